@@ -263,7 +263,7 @@ __global__ void __launch_bounds__((WIDE ? 8 : 4) * 32 + 32, WIDE ? 1 : 2) attent
     __syncthreads();                          // the only block-wide barrier before the warps part ways
     if (warp == CW) {
         const int ps = p.page_size;
-        if (TMA && lane != 0) return;         // one elected lane issues the TMA loads; the copies of the other path take all 32
+        if (TMA && !elect_one()) return;      // one elected lane issues the TMA loads; the copies of the other path take all 32
         bool waited = !EARLY;
         // a launch that makes the new keys itself finds only keys of earlier steps in the pages: nothing there is the
         // work of the kernel before this one (the rows of this step's positions are replaced in shared memory)

@@ -9,7 +9,7 @@
 //
 // A CTA takes up to 256 query rows of one request and one KV head as two halves of 128 (row =
 // token_in_half * G + head_in_group) and walks key tiles of 128 keys, which both halves share.
-//   warp 0      producers: one lane brings the K tiles, another the V tiles, as TMA boxes
+//   warps 0, 10 producers of the K tiles and of the V tiles, as TMA boxes
 //               [page rows x 64] into rings of three and two tiles ([2 column halves][128 keys]
 //               [128 bytes], 128-byte swizzle; keys without a page are zero-filled through an
 //               out-of-range coordinate)
@@ -174,7 +174,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
         : "memory");
 }
 
-constexpr int TC_THREADS = 320;
+constexpr int TC_THREADS = 352;
 
 __global__ void __launch_bounds__(TC_THREADS) attention_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                   const __grid_constant__ CUtensorMap tm_k_run,
@@ -242,10 +242,10 @@ __global__ void __launch_bounds__(TC_THREADS) attention_tc_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
 
-    if (warp == 0) {
-        // ---- producers: lane 0 brings the K tiles, lane 1 the V tiles (each at its ring's pace)
-        if (lane < 2) {
-            const bool is_k = lane == 0;
+    if (warp == 0 || warp == TC_THREADS / 32 - 1) {
+        // ---- producers: warp 0 brings the K tiles, the last warp the V tiles (each at its ring's pace)
+        if (elect_one()) {
+            const bool is_k = warp == 0;
             const int ps = p.page_size, ring = is_k ? KS : VS;
             const uint32_t full0 = is_k ? k_full0 : v_full0, empty0 = is_k ? k_empty0 : v_empty0, base = is_k ? k_s : v_s;
             const CUtensorMap* map = is_k ? &tm_k : &tm_v;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(TC_THREADS) attention_tc_kernel(const __grid_c
         // tensor memory, then at once S_h = Q_h K_(r+1)^T into the columns P_h has just been read
         // from (the tensor pipe runs its instructions in the order of issue), half 0 and half 1 in
         // turn: while one half's softmax runs, the other half's products do.
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = idesc_128x128(false), idesc_o = idesc_128x128(true);
             int pv_cnt[2] = {0, 0};
             bool q_ready[2] = {false, false}, ok = true;

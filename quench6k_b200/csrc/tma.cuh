@@ -39,6 +39,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
     }
 }
 
+// True in one lane of a converged warp, the same one every time.  Copies and matrix instructions take their operands from the
+// warp's uniform registers: behind `if (elect_one())` the compiler knows that a single thread is there and moves them over
+// directly, behind `if (lane == 0)` it emits a loop over the active threads' values around every such instruction (about 100
+// clocks each, measured on a producer's copies and on an issuer's MMAs alike).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
