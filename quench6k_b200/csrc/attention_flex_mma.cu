@@ -437,15 +437,41 @@ __global__ void __launch_bounds__(128) attention_flex_merge_kernel(const float* 
     }
 }
 
-// out[t, h] = sum_g talk[h, g] * part[t, g, KV head of h], FP32 sums in the order of g.
+// out[t, h] = sum_g talk[h, g] * part[t, g, KV head of h], FP32 sums in the order of g.  A block per token: a thread takes four
+// columns of a value head and reads every head's part of them once for four query heads at a time, all loads independent.  (A block
+// per token and query head read each part once per head of the group, 4 bytes a load: 66 us for 2,048 tokens of 16 heads on 4 value
+// heads of 128; the parts are 67 MB, most of which still lie in L2.)
 __global__ void __launch_bounds__(128) attention_talk_mix_kernel(const float* part, const float* talk, int H, int Hkv, int dv,
                                                                  __nv_bfloat16* out) {
     pdl_enter();
-    const int t = blockIdx.x, h = blockIdx.y, kv = h / (H / Hkv);
-    for (int d = threadIdx.x; d < dv; d += blockDim.x) {
-        float acc = 0.0f;
-        for (int g = 0; g < H; ++g) acc = fmaf(talk[h * H + g], part[(((size_t)t * H + g) * Hkv + kv) * dv + d], acc);
-        out[((size_t)t * H + h) * dv + d] = __float2bfloat16_rn(acc);
+    extern __shared__ float mix[];                                               // talk, transposed: [g][h]
+    for (int i = threadIdx.x; i < H * H; i += blockDim.x) mix[(i % H) * H + i / H] = talk[i];
+    __syncthreads();
+    const int t = blockIdx.x, G = H / Hkv, width = Hkv * dv;
+    const float* src = part + (size_t)t * H * width;
+    for (int col = threadIdx.x * 4; col < width; col += blockDim.x * 4) {
+        const int kv = col / dv, d = col - kv * dv;
+        for (int h0 = 0; h0 < G; h0 += 4) {
+            float4 acc[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+            for (int g = 0; g < H; ++g) {
+                const float4 x = *reinterpret_cast<const float4*>(src + (size_t)g * width + col);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float w = h0 + j < G ? mix[g * H + kv * G + h0 + j] : 0.0f;
+                    acc[j].x = fmaf(w, x.x, acc[j].x), acc[j].y = fmaf(w, x.y, acc[j].y), acc[j].z = fmaf(w, x.z, acc[j].z), acc[j].w = fmaf(w, x.w, acc[j].w);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (h0 + j < G) {
+                    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + ((size_t)t * H + kv * G + h0 + j) * dv + d);
+                    o[0] = __floats2bfloat162_rn(acc[j].x, acc[j].y);
+                    o[1] = __floats2bfloat162_rn(acc[j].z, acc[j].w);
+                }
+        }
     }
 }
 
@@ -512,12 +538,49 @@ Q6K_API int q6k_attention_flex_mma(const float* qa, int da, const void* qb, int 
 #undef FLEX_LAUNCH
     if (int rc = q6k_check_launch("attention_flex_mma")) return rc;
     if (talk) {
-        q6k_launch(attention_talk_mix_kernel, dim3(T_, H), 128, 0, st, (const float*)workspace, talk, H, Hkv, dv, (__nv_bfloat16*)out);
+        q6k_launch(attention_talk_mix_kernel, T_, 128, (size_t)H * H * 4, st, (const float*)workspace, talk, H, Hkv, dv, (__nv_bfloat16*)out);
         return q6k_check_launch("attention_talk_mix");
     }
     if (nsplit > 1) {
         q6k_launch(attention_flex_merge_kernel, dim3(T_, H), 128, 0, st, (const float*)a.part_o, (const float*)a.part_ml, nsplit, T_, H, dv,
                    (__nv_bfloat16*)out, out_head_major, sinks, out_f32);
+        return q6k_check_launch("attention_flex_merge");
+    }
+    return 0;
+}
+
+int q6k_attention_flex_tc_launch(const void* qa, int da, const void* qb, int db, int q_head_major, const void* k_pages, int k_ld, const void* v_pages,
+                                 int v_ld, int dv, int num_pages, const int* block_table, int max_blocks, int page_size, const int* req_of_token,
+                                 const int* positions, const int* tile_tok0, const int* tile_ntok, int n_tiles, int window, int chunk, float scale, void* out,
+                                 int out_head_major, int T_, int H, int Hkv, int nsplit, int split_keys, float* part_o, float* part_ml, int talk,
+                                 const float* sinks, float softcap, int maps, float* out_f32, cudaStream_t st);
+
+// The same on tcgen05 for prompt portions (attention_flex_tc.cu), with the row tiles and the shapes of
+// q6k_attention_flex_tc_tile_tokens / q6k_attention_flex_tc_parts; both parts of the
+// query are bfloat16; num_pages: pages of a head, heads one after the other.
+Q6K_API int q6k_attention_flex_tc(const void* qa, int da, const void* qb, int db, int q_head_major, const void* k_pages, int k_ld, const void* v_pages,
+                                  int v_ld, int dv, int num_pages, const int* block_table, int max_blocks, int page_size, const int* req_of_token,
+                                  const int* positions, const int* tile_tok0, const int* tile_ntok, int n_tiles, int window, int chunk, float scale, void* out,
+                                  int out_head_major, int T_, int H, int Hkv, int nsplit, int split_keys, float* workspace, const float* talk, const float* sinks,
+                                  float softcap, int maps, float* out_f32, cudaStream_t st) {
+    if (T_ == 0 || n_tiles == 0) return 0;
+    Q6K_REQUIRE(maps >= 1 && Hkv > 0 && Hkv % maps == 0 && softcap >= 0.0f, "attention_flex_tc: %d maps over %d key heads, softcap %f", maps, Hkv, softcap);
+    Q6K_REQUIRE((da == 0 || qa) && (db == 0 || qb) && nsplit >= 1 && (nsplit == 1 || (workspace && split_keys > 0 && split_keys % KEYS == 0)),
+                "attention_flex_tc: bad query parts or key split");
+    Q6K_REQUIRE(!talk || (maps == 1 && softcap == 0.0f && !out_f32 && nsplit == 1 && workspace && !out_head_major && !sinks),
+                "attention_flex_tc: mixed heads take one map, no cap, bfloat16 token-major results, one key range, scratch and no sinks");
+    float* ml = workspace ? workspace + (size_t)nsplit * T_ * H * dv : nullptr;
+    if (int rc = q6k_attention_flex_tc_launch(qa, da, qb, db, q_head_major, k_pages, k_ld, v_pages, v_ld, dv, num_pages, block_table, max_blocks, page_size,
+                                              req_of_token, positions, tile_tok0, tile_ntok, n_tiles, window, chunk, scale, out, out_head_major, T_, H, Hkv,
+                                              nsplit, split_keys, workspace, ml, talk != nullptr, sinks, softcap, maps, out_f32, st))
+        return rc;
+    if (talk) {
+        q6k_launch(attention_talk_mix_kernel, T_, 128, (size_t)H * H * 4, st, (const float*)workspace, talk, H, Hkv, dv, (__nv_bfloat16*)out);
+        return q6k_check_launch("attention_talk_mix");
+    }
+    if (nsplit > 1) {
+        q6k_launch(attention_flex_merge_kernel, dim3(T_, H), 128, 0, st, (const float*)workspace, (const float*)ml, nsplit, T_, H, dv, (__nv_bfloat16*)out,
+                   out_head_major, sinks, out_f32);
         return q6k_check_launch("attention_flex_merge");
     }
     return 0;

@@ -39,7 +39,7 @@ constexpr int BK = 64;                 // bf16 per k-block: one 128-byte swizzle
 constexpr int WM = 128;                // weight rows per tile (UMMA M)
 constexpr int MAX_STAGES = 12;
 
-enum { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_PARTIAL = 3, EPI_ACT = 4 };   // EPI_ACT: one matrix, out = bfloat16(act(A.W))
+enum { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_PARTIAL = 3, EPI_ACT = 4, EPI_BF16 = 5 };   // EPI_ACT: one matrix, out = bfloat16(act(A.W)); EPI_BF16: bfloat16(A.W)
 
 __device__ int g_tc_status = 0;
 
@@ -371,6 +371,8 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                             ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(p.act == 0 ? gte / (1.0f + expf(-gte)) * u[DUAL ? j : 0] : q6k_gated(gte, u[DUAL ? j : 0], p.act, p.act_limit));
                         } else if (p.epilogue == EPI_ACT) {
                             ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(q6k_activation(v[j], p.act));
+                        } else if (p.epilogue == EPI_BF16) {
+                            ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(v[j]);
                         } else {
                             p.partial[((size_t)tl.z * p.rows_total + row) * p.N + n] = v[j];
                         }
@@ -786,9 +788,9 @@ Q6K_API int q6k_gemm_tc(const void* A, long long lda, int rows_total, const void
                 "gemm_tc: operands must be 16-byte aligned");
     const int act = epilogue >> 8;
     epilogue &= 255;
-    Q6K_REQUIRE(((epilogue >= 0 && epilogue <= 2) || epilogue == EPI_ACT) && act >= 0 && act <= (epilogue == EPI_SWIGLU ? 3 : 2),
+    Q6K_REQUIRE(((epilogue >= 0 && epilogue <= 2) || epilogue == EPI_ACT || epilogue == EPI_BF16) && act >= 0 && act <= (epilogue == EPI_SWIGLU ? 3 : 2),
                 "gemm_tc: unknown epilogue %d (activation %d)", epilogue, act);
-    Q6K_REQUIRE(epilogue != EPI_ACT || tile_group != nullptr, "gemm_tc: the activation of a single product is for grouped rows");
+    Q6K_REQUIRE((epilogue != EPI_ACT && epilogue != EPI_BF16) || tile_group != nullptr, "gemm_tc: bfloat16 results of a single product are for grouped rows");
     const bool dual = epilogue == EPI_SWIGLU;
     Q6K_REQUIRE(!dual || W2, "gemm_tc: the SwiGLU epilogue needs two weight matrices");
     const bool grouped = tile_group != nullptr;

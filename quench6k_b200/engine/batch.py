@@ -57,19 +57,27 @@ class StepContext:
     position: int = 0                             # the executed position (index into the model's order) whose block is running
     side_rows: Optional[torch.Tensor] = None      # FP32 [T, columns]: the tokens' rows of the model's side table, if it has one
 
-    def query_tiles(self, tokens_per_tile: int, at_most: Optional[int] = None):
+    def query_tiles(self, tokens_per_tile: int, at_most: Optional[int] = None, most_keys_first=None):
         """Tiles of at most `tokens_per_tile` consecutive tokens of one request, as device arrays
         (first row, token count) and their number; made once per step and size.  at_most: only
-        the requests that bring at most that many tokens to the step."""
-        key = ("query_tiles", tokens_per_tile, at_most)
+        the requests that bring at most that many tokens to the step.  most_keys_first = (window, chunk): sorted by the
+        number of keys a tile sees under that mask (0 or None: no limit), so that a launch's long blocks start in its first wave."""
+        key = ("query_tiles", tokens_per_tile, at_most, most_keys_first)
         if key not in self.plans:
-            first, count, at = [], [], 0
-            for n in self.q_lens:
+            first, count, keys, at = [], [], [], 0
+            for r, n in enumerate(self.q_lens):
                 if at_most is None or n <= at_most:
                     for i in range(0, n, tokens_per_tile):
                         first.append(at + i)
                         count.append(min(tokens_per_tile, n - i))
+                        if most_keys_first is not None:
+                            window, chunk = most_keys_first
+                            p0 = (self.pos_starts[r] if r < len(self.pos_starts) else 0) + i
+                            keys.append(p0 + count[-1] - max(p0 - window + 1 if window else 0, p0 // chunk * chunk if chunk else 0, 0))
                 at += n
+            if most_keys_first is not None:
+                order = sorted(range(len(first)), key=lambda j: -keys[j])
+                first, count = [first[j] for j in order], [count[j] for j in order]
             both = torch.tensor([first, count], dtype=torch.int32).reshape(2, -1).to(self.token_ids.device, non_blocking=True)
             self.plans[key] = (both[0], both[1], len(first))
         return self.plans[key]

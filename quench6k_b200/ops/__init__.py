@@ -57,7 +57,7 @@ def _need(t: torch.Tensor, name: str, dtype=None, shape=None):
 
 
 # kernels launched per exported function (for launch accounting in benchmarks)
-_LAUNCHES = {"q6k_gated_delta": 1, "q6k_delta_channel": 1, "q6k_attention_flex_mma": 2, "q6k_selective_scan": 1, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
+_LAUNCHES = {"q6k_gated_delta": 1, "q6k_delta_channel": 1, "q6k_retention_chunked": 2, "q6k_attention_flex_mma": 2, "q6k_attention_flex_tc": 2, "q6k_selective_scan": 1, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
 launch_count = 0
 
 
@@ -240,7 +240,7 @@ def swiglu(gu: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
 
 
 # --------------------------------------------------------------------------- matrix products (CUDA cores)
-EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_ACT = 0, 1, 2, 4
+EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_ACT, EPI_BF16 = 0, 1, 2, 4, 5
 ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "relu2": 2}
 # A gate that takes a constant is named with it, ("clamped", limit): with g the gate's product and u the other one,
 # g' = min(g, limit), u' = clamp(u, -limit, limit), and the result is g' sigmoid(1.702 g') (u' + 1).  Gated epilogues only.
@@ -375,7 +375,9 @@ def tc_status() -> int:
     lib.q6k_attention_status.restype = ctypes.c_int
     lib.q6k_attention_tc_status.restype = ctypes.c_int
     lib.q6k_router_status.restype = ctypes.c_int
-    return lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_router_status()
+    lib.q6k_attention_flex_tc_status.restype = ctypes.c_int
+    return (lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_attention_flex_tc_status()
+            or lib.q6k_router_status())
 
 
 def selftest_wait_runs_out(limit_cycles: int = 2_000_000):
@@ -404,13 +406,13 @@ def _workspace(nbytes: int, device, which: str = "") -> torch.Tensor:
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
             w2: Optional[torch.Tensor] = None, groups=None, bt: int = 0, rows: Optional[int] = None,
-            keep_partials: bool = False, act: Optional[str] = None) -> torch.Tensor:
+            keep_partials: bool = False, act: Optional[str] = None, rounded: bool = False) -> torch.Tensor:
     """The same contract as gemm_simt without the row gather, on tcgen05 tensor cores: bfloat16
     operands, FP32 accumulation in tensor memory.  Grouped calls pass the tile list made for
     token tile `bt` (tile_list(offsets, pairs, bt)).  keep_partials (dense, plain store): when the
     kernel slices K over CTAs the result is the FP32 partial products [slices, M, N], a view of the
     device's scratch buffer that stays valid until the next kernel that uses scratch; the consumer
-    sums the slices in order."""
+    sums the slices in order.  rounded (plain grouped products): the result leaves in bfloat16."""
     if not tc_supported(a, w):
         raise KernelError("gemm_tc: operands must be bfloat16 with K a multiple of 8 and 16-byte aligned rows")
     K = a.shape[1]
@@ -422,8 +424,10 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None
     if grouped and groups is None:
         raise KernelError("gemm_tc: a grouped weight needs group offsets and a tile list")
     M = rows if rows is not None else a.shape[0]
-    epi = _epilogue(w2, accumulate, act)             # act: the gate's activation with w2; alone (grouped rows only): out = act(a w^T) in bfloat16
-    out_dtype = torch.bfloat16 if w2 is not None or act is not None else torch.float32
+    epi = EPI_BF16 if rounded else _epilogue(w2, accumulate, act)             # act: the gate's activation with w2; alone (grouped rows only): out = act(a w^T) in bfloat16
+    if rounded and (not grouped or w2 is not None or accumulate or act is not None):
+        raise KernelError("gemm_tc: results rounded to bfloat16 are for plain grouped products")
+    out_dtype = torch.bfloat16 if w2 is not None or act is not None or rounded else torch.float32
     lib = library()
     splits = 1
     if keep_partials:
@@ -1263,7 +1267,7 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
                    block_table: torch.Tensor, req_of_token: torch.Tensor, positions: torch.Tensor, H: int, scale: float,
                    window: Optional[int] = None, chunk: Optional[int] = None, talk: Optional[torch.Tensor] = None,
                    out_head_major: bool = False, tiles=None, max_context: int = 0, sinks: Optional[torch.Tensor] = None,
-                   softcap: float = 0.0, maps: int = 1, out_f32: bool = False) -> torch.Tensor:
+                   softcap: float = 0.0, maps: int = 1, out_f32: bool = False, wide_tiles=None) -> torch.Tensor:
     """Causal attention of every row over its request's pages, for any key and value widths.  A query row is the FP32
     part q_f32 [H*T or T*H rows, da] followed by q [rows, db] in the pages' dtype (either may be None); rows are head-major
     (h T + t) or token-major.  k_pages [Hkv, P, page, dk]; v_pages [Hkv, P, page, dv], possibly a view into k_pages (the
@@ -1277,13 +1281,15 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
     Returns [H, T, dv] (out_head_major) or [T, H dv].
     tiles = (first row, token count, number) of row tiles of attention_flex_tile_tokens(H, Hkv) tokens of one request
     each, with max_context the largest position + 1 of the step: bfloat16 pages then go to the tensor-core kernel where
-    it takes the shapes; with few tiles it splits the keys into fixed ranges and merges them."""
+    it takes the shapes; with few tiles it splits the keys into fixed ranges and merges them.  wide_tiles: the same for tiles of
+    attention_flex_wide_tokens(...) tokens, where that says the tcgen05 kernel should run instead; the first part of the query
+    is then bfloat16 too."""
     da = q_f32.shape[-1] if q_f32 is not None else 0
     db = q.shape[-1] if q is not None else 0
     rows = (q_f32 if q_f32 is not None else q).numel() // (da if q_f32 is not None else db)
     T = rows // H
     if q_f32 is not None:
-        _need(q_f32, "q_f32", torch.float32)
+        _need(q_f32, "q_f32", torch.float32 if wide_tiles is None else k_pages.dtype)
     if q is not None:
         _need(q, "q", k_pages.dtype)
     Hkv, num_pages, page_size, dk = k_pages.shape
@@ -1303,6 +1309,30 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
     out = torch.empty((H, T, dv) if out_head_major else (T, H * dv), dtype=torch.float32 if out_f32 else k_pages.dtype, device=k_pages.device)
     as_f32 = out if out_f32 and k_pages.dtype != torch.float32 else None      # FP32 pages: the kernel's own result type
     shared_v = v_pages.data_ptr() == k_pages.data_ptr() and v_pages.stride() == k_pages.stride()
+    if wide_tiles is not None:
+        parts = _flex_tc_parts(H, Hkv, da, db, dv, talk is not None, shared_v, page_size)
+        for p in (k_pages, v_pages):
+            if p.shape[0] > 1 and p.stride(0) != num_pages * page_size * p.stride(2):
+                raise KernelError("attention_flex: the heads' pages do not follow one another")
+        if not parts or k_pages.dtype != torch.bfloat16:
+            raise KernelError("attention_flex: the tcgen05 kernel does not take these shapes")
+        tok0, ntok, n_tiles = wide_tiles
+        nsplit, split_keys, ws = 1, 0, None
+        lib = library()
+        if talk is not None:                     # every head's weights against every KV head's values, then the mixture
+            lib.q6k_attention_flex_mma_talk_workspace.restype = ctypes.c_longlong
+            ws = _workspace(lib.q6k_attention_flex_mma_talk_workspace(_i(T), _i(H), _i(Hkv), _i(dv)), k_pages.device, "flex")
+        elif not chunk:
+            nsplit, split_keys = _key_ranges(n_tiles * Hkv * parts, 148, max_context, window, attention_flex_tc_tile_tokens(H, Hkv))
+            if nsplit > 1:
+                lib.q6k_attention_flex_mma_workspace.restype = ctypes.c_longlong
+                ws = _workspace(lib.q6k_attention_flex_mma_workspace(_i(T), _i(H), _i(dv), _i(nsplit)), k_pages.device, "flex")
+        _call("q6k_attention_flex_tc", _ptr(q_f32), _i(da), _ptr(q), _i(db), _i(1 if head_major else 0), _ptr(k_pages), _i(k_pages.stride(2)),
+              _ptr(v_pages), _i(v_pages.stride(2)), _i(dv), _i(num_pages), _ptr(block_table), _i(block_table.shape[1]), _i(page_size),
+              _ptr(req_of_token), _ptr(positions), _ptr(tok0), _ptr(ntok), _i(n_tiles), _i(window or 0), _i(chunk or 0), _f(scale), _ptr(out),
+              _i(1 if out_head_major else 0), _i(T), _i(H), _i(Hkv), _i(nsplit), _i(split_keys), _ptr(ws), _ptr(talk), _ptr(sinks), _f(softcap),
+              _i(maps), _ptr(out if out_f32 else None), _stream())
+        return out
     if (tiles is not None and k_pages.dtype == torch.bfloat16 and not (talk is not None and out_head_major)
             and attention_flex_mma_supported(H, Hkv, dk, dv, k_pages.stride(2), v_pages.stride(2), db, shared_v)):
         tok0, ntok, n_tiles = tiles
@@ -1312,13 +1342,8 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
             lib = library()
             lib.q6k_attention_flex_mma_talk_workspace.restype = ctypes.c_longlong
             ws = _workspace(lib.q6k_attention_flex_mma_talk_workspace(_i(T), _i(H), _i(Hkv), _i(dv)), k_pages.device, "flex")
-        elif ctas < 120 and not chunk and max_context > 256:     # few row tiles: fixed key ranges over more CTAs
-            want = max(1, 296 // ctas)
-            # under a window a tile sees its window and its own tokens: ranges sized for that span (the ranges that lie
-            # outside it cost a block that finds no key), and no more than 128 of them
-            span = min(max_context, window + attention_flex_tile_tokens(H, Hkv)) if window else max_context
-            split_keys = max(256, (-(-span // want) + 63) // 64 * 64, (-(-max_context // 128) + 63) // 64 * 64)
-            nsplit = -(-max_context // split_keys)
+        elif ctas < 120 and not chunk:           # few row tiles: fixed key ranges over more CTAs
+            nsplit, split_keys = _key_ranges(ctas, 296, max_context, window, attention_flex_tile_tokens(H, Hkv))
             if nsplit > 1:
                 lib = library()
                 lib.q6k_attention_flex_mma_workspace.restype = ctypes.c_longlong
@@ -1347,6 +1372,46 @@ def map_difference(a: torch.Tensor, H: int, dv: int, weight: float, eps: float, 
     out = torch.empty((T, H * dv), dtype=out_dtype, device=a.device)
     _call("q6k_map_difference", _ptr(a), _ptr(out), _i(T), _i(H), _i(dv), _f(weight), _f(eps), _f(mult), _i(dtype_code(out_dtype)), _stream())
     return out
+
+
+def _key_ranges(ctas: int, slots: int, max_context: int, window: Optional[int], tile_tokens: int):
+    """(ranges, keys of a range) that spread a launch of few row tiles over `slots` CTAs; (1, 0): whole."""
+    if max_context <= 256 or ctas > slots // 2:
+        return 1, 0
+    want = max(1, slots // max(1, ctas))
+    # under a window a tile sees its window and its own tokens: ranges sized for that span (the ranges that lie
+    # outside it cost a block that finds no key), and no more than 128 of them
+    span = min(max_context, window + tile_tokens) if window else max_context
+    split_keys = max(256, (-(-span // want) + 63) // 64 * 64, (-(-max_context // 128) + 63) // 64 * 64)
+    return -(-max_context // split_keys), split_keys
+
+
+@functools.lru_cache(maxsize=None)          # a question about sizes: asked of the library once
+def _flex_tc_parts(H: int, Hkv: int, da: int, db: int, dv: int, mixed: bool, shared_v: bool, page_size: int) -> int:
+    lib = library()
+    lib.q6k_attention_flex_tc_parts.restype = ctypes.c_int
+    return lib.q6k_attention_flex_tc_parts(_i(H), _i(Hkv), _i(da), _i(db), _i(dv), _i(Hkv if mixed else 0), _i(1 if shared_v else 0), _i(page_size))
+
+
+@functools.lru_cache(maxsize=None)
+def attention_flex_tc_tile_tokens(H: int, Hkv: int) -> int:
+    """Tokens of one request in a row tile of the tcgen05 flexible attention kernel."""
+    lib = library()
+    lib.q6k_attention_flex_tc_tile_tokens.restype = ctypes.c_int
+    return lib.q6k_attention_flex_tc_tile_tokens(_i(H), _i(Hkv))
+
+
+def attention_flex_wide_tokens(max_q_len: int, H: int, Hkv: int, da: int, db: int, dv: int, mixed: bool, shared_v: bool, page_size: int,
+                               scale: float) -> int:
+    """Tokens of the row tiles the tcgen05 kernel should be given in a step whose longest portion has max_q_len tokens, or 0
+    where the mma.sync kernel (tiles of a quarter of the rows) serves the step: shapes this one does not take, and steps in
+    which no portion fills half of one of its tiles.  Both measured: a latent of 512 under 16 heads at 4,096 keys, 4 tokens 54 us
+    (mma.sync) and 40 us, 64 tokens 139 and 49 us; mixed heads in chunks of 1,024, 64 tokens 25 and 26 us, 256 tokens 48 and
+    32 us; two tokens of two maps of 64, 20 and 21 us."""
+    if scale <= 0 or not _flex_tc_parts(H, Hkv, da, db, dv, mixed, shared_v, page_size):
+        return 0
+    tokens = attention_flex_tc_tile_tokens(H, Hkv)
+    return tokens if 2 * max_q_len >= tokens else 0
 
 
 @functools.lru_cache(maxsize=None)

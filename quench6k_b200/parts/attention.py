@@ -210,10 +210,17 @@ class Attention(Mixer):
                           ctx.positions, ctx.req_of_token, table if write else None, cache.page_size, cache.k if write else None,
                           cache.v if write else None, rt.dtype, v_heads=self.Hkv, bias=self.prep_bias, values_are_keys=self.values_are_keys, value_norm=self.value_norm)
         ops.current_tag = "attention.keys"
-        tiles = None if rt.is_fp32 or not rt.tensor_cores else ctx.query_tiles(ops.attention_flex_tile_tokens(self.Hq, self.Hkv))
+        tiles = wide = None
+        if not rt.is_fp32 and rt.tensor_cores:
+            tokens = ops.attention_flex_wide_tokens(ctx.max_q_len, self.Hq * M, self.Hkv * M, 0, self.hd, self.vd, self.talk, False, cache.page_size,
+                                                    self.scale)
+            if tokens:
+                wide = ctx.query_tiles(tokens, most_keys_first=(self.window, self.chunk))
+            else:
+                tiles = ctx.query_tiles(ops.attention_flex_tile_tokens(self.Hq, self.Hkv))
         a = ops.attention_flex(None, q.view(-1, self.hd), False, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, self.Hq * M,
                                self.scale, window=self.window, chunk=self.chunk, talk=self.w_talk, tiles=tiles, max_context=ctx.max_context,
-                               sinks=self.sinks, softcap=self.softcap, maps=M, out_f32=M > 1)
+                               sinks=self.sinks, softcap=self.softcap, maps=M, out_f32=M > 1, wide_tiles=wide)
         if M > 1:                                   # a head's two maps, FP32, into the head's one result
             ops.current_tag = "attention.maps"
             a = ops.map_difference(a, self.Hq, self.vd, self.map_weight, self.eps, 1.0 - self.diff, rt.dtype)

@@ -109,13 +109,19 @@ class LatentAttention(Mixer):
         inv_freq, turn, neighbours = (None, 0, False) if self.pos.is_identity else self.pos.rotary_table()
         qn, qr = ops.latent_prep(x, H, self.dim, self.rd, self.rank, self.c_norm, self.eps, inv_freq, turn, ctx.positions,
                                  ctx.req_of_token, table, cache.page_size, cache.k, neighbours=neighbours, write=not self.borrows, latent=latent)
+        tiles = wide = None
+        if not rt.is_fp32 and rt.tensor_cores:
+            tokens = ops.attention_flex_wide_tokens(ctx.max_q_len, H, 1, self.rank, self.rd, self.rank, False, True, cache.page_size, self.scale)
+            if tokens:
+                wide = ctx.query_tiles(tokens, most_keys_first=(self.window, None))
+            else:
+                tiles = ctx.query_tiles(ops.attention_flex_tile_tokens(H, 1))
         ops.current_tag = "latent.absorb"
-        ql = linear.batched_matmul(qn.view(H * T, self.dim), self.w_ukT, rt, T)          # FP32 [H T, rank]
+        ql = linear.batched_matmul(qn.view(H * T, self.dim), self.w_ukT, rt, T, rounded=wide is not None)      # [H T, rank], FP32 or as the tcgen05 kernel reads it
         ops.current_tag = "latent.keys"
-        tiles = None if rt.is_fp32 or not rt.tensor_cores else ctx.query_tiles(ops.attention_flex_tile_tokens(H, 1))
         o = ops.attention_flex(ql, qr.view(H * T, self.rd) if self.rd else None, True, cache.k, cache.v, table, ctx.req_of_token,
                                ctx.positions, H, self.scale, window=self.window, out_head_major=True, tiles=tiles,
-                               max_context=ctx.max_context, sinks=self.sinks)                                       # [H, T, rank]
+                               max_context=ctx.max_context, sinks=self.sinks, wide_tiles=wide)                                       # [H, T, rank]
         ops.current_tag = "latent.values"
         ov = linear.batched_matmul(o.view(H * T, self.rank), self.w_uv, rt, T)           # FP32 [H T, vd]
         a = ops.heads_to_rows(ov, H, rt.dtype)

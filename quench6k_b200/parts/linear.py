@@ -115,12 +115,13 @@ def _uniform_groups(groups: int, rows_per_group: int, bm: int, device):
     return _uniform[key]
 
 
-def batched_matmul(a: torch.Tensor, w: torch.Tensor, rt, rows_per_group: int) -> torch.Tensor:
+def batched_matmul(a: torch.Tensor, w: torch.Tensor, rt, rows_per_group: int, rounded: bool = False) -> torch.Tensor:
     """FP32 y[g M + r] = a[g M + r] @ w[g]^T for G groups of M = rows_per_group rows each: one product per head, the rows
-    laid out head by head.  a: [G M, K], w: [G, N, K]."""
+    laid out head by head.  a: [G M, K], w: [G, N, K].  rounded: y in bfloat16 (for a consumer that would round it first)."""
     G = w.shape[0]
     total = G * rows_per_group
     if _tc(a, w, rt) and a.is_contiguous():
         bt = ops.tc_token_tile(rows_per_group, False)
-        return ops.gemm_tc(a, w, groups=_uniform_groups(G, rows_per_group, bt, a.device), bt=bt, rows=total)
-    return ops.gemm_simt(a, w, groups=_uniform_groups(G, rows_per_group, ops.simt_tile_rows(), a.device), rows=total)
+        return ops.gemm_tc(a, w, groups=_uniform_groups(G, rows_per_group, bt, a.device), bt=bt, rows=total, rounded=rounded)
+    y = ops.gemm_simt(a, w, groups=_uniform_groups(G, rows_per_group, ops.simt_tile_rows(), a.device), rows=total)
+    return ops.cast_columns(y, 0, y.shape[1], torch.bfloat16) if rounded else y
