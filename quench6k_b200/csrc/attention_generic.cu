@@ -92,13 +92,173 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(const T* q, cons
     }
 }
 
+// The same for steps that bring several tokens per request: the same sums in the same order (a row's scores are summed over ascending
+// dimensions, its keys come in tiles of 32 whose weights a warp adds with the same butterfly, values are added in ascending order
+// of the keys), so a row's result is the same bit for bit whichever of the two kernels runs it.
+//
+// The kernel above reads a key row per lane and a value row per (head, key) from global memory: 500 us for 509 tokens of 8 heads
+// over 509 keys, waiting for loads.  Here a block takes up to 32 rows (the query heads of a KV head for consecutive tokens of the step)
+// and brings each key tile into shared memory once; 8 threads share a row: each makes the scores of four keys and owns every
+// eighth group of four dimensions of the result, so that a 16-byte read of keys or values serves four rows and a warp's reads fall into
+// different banks: 92 us.  Tokens of several requests in one block are taken request by request.
+constexpr int GT_ROWS = 32, GT_KEYS = 32, GT_THREADS = 256;
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+
+template <typename T, int NI>          // NI: groups of 32 dimensions (hd <= 32 NI)
+__global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q, const T* k_pages, const T* v_pages, const int* block_table, int max_blocks,
+                                                                     int page_size, int num_pages, const int* req_of_token, const int* positions,
+                                                                     int window, const float* sinks, float scale, T* out, int T_, int Hq, int Hkv, int hd,
+                                                                     int tokens, int heads) {
+    pdl_enter();
+    extern __shared__ __align__(16) float gt_smem[];
+    const int ld = hd + 4;
+    float* qs = gt_smem;                              // [GT_ROWS][ld]
+    float* ks = qs + GT_ROWS * ld;                    // [GT_KEYS][ld]
+    float* vs = ks + GT_KEYS * ld;                    // [GT_KEYS][ld]
+    float* ss = vs + GT_KEYS * ld;                    // [GT_ROWS][GT_KEYS + 4]: scores, then weights
+    float* corr_s = ss + GT_ROWS * (GT_KEYS + 4);     // [GT_ROWS]: what a row's result is multiplied by before the tile, at the end by
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = Hq / Hkv;
+    const int t0 = blockIdx.x * tokens, t1 = min(T_, t0 + tokens), kh = blockIdx.y, g0 = blockIdx.z * heads, here = min(heads, G - g0);
+    const int row = tid >> 3, c = tid & 7;            // this thread's row and place in it; row = token * heads + head
+    const size_t head_base = (size_t)kh * num_pages;
+    for (int ta = t0; ta < t1;) {
+        const int req = req_of_token[ta];
+        int tb = ta + 1;
+        while (tb < t1 && req_of_token[tb] == req) ++tb;
+        const int* bt = block_table + (size_t)req * max_blocks;
+        const int rows = (tb - ta) * heads, k_end = positions[tb - 1] + 1;
+        const int lo_first = window > 0 ? max(0, positions[ta] - window + 1) : 0;
+        __syncthreads();                              // the rows before are done with
+        for (int i = tid; i < rows * (hd / 4); i += GT_THREADS) {
+            const int r = i / (hd / 4), d = (i % (hd / 4)) * 4, g = g0 + r % heads;
+            *reinterpret_cast<float4*>(qs + r * ld + d) = load4(q + ((size_t)(ta + r / heads) * Hq + kh * G + (g < G ? g : 0)) * hd + d);
+        }
+        // the softmax state of rows 4 warp .. 4 warp + 3, the same in every lane
+        float m[4], l[4];
+        int pos4[4], lo4[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int r = warp * 4 + x;
+            m[x] = -INFINITY, l[x] = 0.0f;
+            pos4[x] = r < rows ? positions[ta + r / heads] : -1;
+            lo4[x] = window > 0 ? max(0, pos4[x] - window + 1) : 0;
+        }
+        float4 o[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) o[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int j0 = lo_first & ~(GT_KEYS - 1); j0 < k_end; j0 += GT_KEYS) {
+            __syncthreads();                          // the tile before is done with
+            for (int i = tid; i < GT_KEYS * (hd / 4); i += GT_THREADS) {
+                const int kk = i / (hd / 4), d = (i % (hd / 4)) * 4, j = j0 + kk;
+                float4 kv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv = kv;
+                if (j >= lo_first && j < k_end) {
+                    const size_t at = ((head_base + bt[j / page_size]) * page_size + j % page_size) * hd + d;
+                    kv = load4(k_pages + at);
+                    vv = load4(v_pages + at);
+                }
+                *reinterpret_cast<float4*>(ks + kk * ld + d) = kv;
+                *reinterpret_cast<float4*>(vs + kk * ld + d) = vv;
+            }
+            __syncthreads();
+            if (row < rows) {
+                float s[4] = {};
+                const float* qr = qs + row * ld;
+                const float* kr = ks + c * ld;
+#pragma unroll 4
+                for (int d = 0; d < hd; d += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(qr + d);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const float4 b = *reinterpret_cast<const float4*>(kr + x * 8 * ld + d);
+                        s[x] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s[x]))));
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) ss[row * (GT_KEYS + 4) + c + 8 * x] = s[x];
+            }
+            __syncwarp();                             // a row's eight threads, its state and its weights belong to one warp
+            // softmax: a lane per key, the warp's four rows in turn
+            const int j = j0 + lane;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int r = warp * 4 + x;
+                if (j0 > pos4[x] || j0 + GT_KEYS <= lo4[x]) {              // no key of this tile for the row: it does not see the tile at all
+                    if (lane == 0) corr_s[r] = -1.0f;
+                    continue;
+                }
+                const bool ok = j >= lo4[x] && j <= pos4[x];
+                const float s = ok ? ss[r * (GT_KEYS + 4) + lane] * scale : -INFINITY;
+                const float mn = fmaxf(m[x], warp_max(s));
+                const float corr = m[x] == -INFINITY ? 0.0f : expf(m[x] - mn);
+                const float p = ok ? round_to<T>(expf(s - mn)) : 0.0f;
+                l[x] = l[x] * corr + warp_sum(p);
+                m[x] = mn;
+                ss[r * (GT_KEYS + 4) + lane] = p;
+                if (lane == 0) corr_s[r] = corr;
+            }
+            __syncwarp();
+            const float corr = row < rows ? corr_s[row] : -1.0f;
+            if (corr != -1.0f) {
+#pragma unroll
+                for (int i = 0; i < NI; ++i) o[i].x *= corr, o[i].y *= corr, o[i].z *= corr, o[i].w *= corr;
+                const float* pr = ss + row * (GT_KEYS + 4);
+#pragma unroll 4
+                for (int kk = 0; kk < GT_KEYS; ++kk) {
+                    const float p = pr[kk];
+                    if (p != 0.0f) {
+                        const float* vr = vs + kk * ld + c * 4;
+#pragma unroll
+                        for (int i = 0; i < NI; ++i)
+                            if (NI * 32 == hd || c * 4 + 32 * i < hd) {
+                                const float4 b = *reinterpret_cast<const float4*>(vr + 32 * i);
+                                o[i].x = fmaf(p, b.x, o[i].x), o[i].y = fmaf(p, b.y, o[i].y), o[i].z = fmaf(p, b.z, o[i].z), o[i].w = fmaf(p, b.w, o[i].w);
+                            }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int r = warp * 4 + x;
+            if (lane == 0 && r < rows) {
+                float den = l[x], osc = 1.0f;
+                if (sinks && g0 + r % heads < G) {
+                    const float sk = sinks[kh * G + g0 + r % heads], M = fmaxf(m[x], sk);
+                    osc = expf(m[x] - M);
+                    den = l[x] * osc + expf(sk - M);
+                }
+                corr_s[r] = osc / den;
+            }
+        }
+        __syncwarp();
+        if (row < rows && row % heads < here) {
+            const float inv = corr_s[row];
+            T* dst = out + ((size_t)(ta + row / heads) * Hq + kh * G + g0 + row % heads) * hd + c * 4;
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+                if (NI * 32 == hd || c * 4 + 32 * i < hd) {
+                    dst[32 * i] = from_f32<T>(o[i].x * inv), dst[32 * i + 1] = from_f32<T>(o[i].y * inv);
+                    dst[32 * i + 2] = from_f32<T>(o[i].z * inv), dst[32 * i + 3] = from_f32<T>(o[i].w * inv);
+                }
+        }
+        ta = tb;
+    }
+}
+
 }  // namespace
 
 // q: [T, Hq, hd]; pages: [Hkv, num_pages, page_size, hd]; block_table: [R, max_blocks];
-// window 0: every earlier key is visible; sinks: FP32 [Hq] or null; out: [T, Hq*hd].
+// window 0: every earlier key is visible; sinks: FP32 [Hq] or null; out: [T, Hq*hd].  requests: how many the step's rows belong to
+// (0: not said).
 Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void* v_pages, int num_pages, const int* block_table,
                                   int max_blocks, int page_size, const int* req_of_token, const int* positions, int window,
-                                  const float* sinks, float scale, void* out, int T_, int Hq, int Hkv, int hd, int dtype,
+                                  const float* sinks, float scale, void* out, int T_, int Hq, int Hkv, int hd, int dtype, int requests,
                                   cudaStream_t st) {
     if (T_ == 0) return 0;
     Q6K_REQUIRE(T_ > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0, "attention: bad head counts Hq=%d Hkv=%d", Hq, Hkv);
@@ -107,6 +267,28 @@ Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void
                 page_size, max_blocks, window);
     Q6K_REQUIRE(Hkv <= 65535, "attention: %d KV heads exceed the grid limit", Hkv);
     const int G = Hq / Hkv;
+    // Several tokens per request: row tiles (92 us against 500 where a step brings 509 tokens of one request).  A decode step (a token
+    // each) would leave most of a tile's rows empty and keeps a block per token.
+    if (requests > 0 && T_ >= 4 * requests && (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+        const int heads = G < GT_ROWS ? G : GT_ROWS, tokens = GT_ROWS / heads;
+        const size_t smem = (size_t)((GT_ROWS + 2 * GT_KEYS) * (hd + 4) + GT_ROWS * (GT_KEYS + 4) + GT_ROWS) * sizeof(float);
+        const dim3 tiles((T_ + tokens - 1) / tokens, Hkv, (G + heads - 1) / heads);
+#define TILED(NI)                                                                                                                                       \
+    do {                                                                                                                                                \
+        if (cudaFuncSetAttribute(attention_tiled_kernel<T, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)                 \
+            return q6k_check_launch("attention_tiled: shared memory attribute");                                                                        \
+        q6k_launch(attention_tiled_kernel<T, NI>, tiles, GT_THREADS, smem, st, (const T*)q, (const T*)k_pages, (const T*)v_pages, block_table,          \
+                   max_blocks, page_size, num_pages, req_of_token, positions, window, sinks, scale, (T*)out, T_, Hq, Hkv, hd, tokens, heads);           \
+    } while (0)
+        Q6K_DISPATCH(dtype, {
+            if (hd <= 32) TILED(1);
+            else if (hd <= 64) TILED(2);
+            else if (hd <= 128) TILED(4);
+            else TILED(8);
+        });
+#undef TILED
+        return q6k_check_launch("attention_tiled");
+    }
     const int warps = G < 4 ? G : 4;
     dim3 grid(T_, Hkv);
     Q6K_DISPATCH(dtype, q6k_launch(attention_generic_kernel<T>, grid, warps * 32, warps * hd * sizeof(float), st, 

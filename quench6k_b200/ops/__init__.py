@@ -639,7 +639,7 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
     _call("q6k_attention_generic", _ptr(q), _ptr(k_pages), _ptr(v_pages), _i(num_pages), _ptr(block_table), _i(block_table.shape[1]),
           _i(page_size), _ptr(req_of_token), _ptr(positions), _i(window or 0), _ptr(sinks),
           _f(scale if scale is not None else 1.0 / math.sqrt(hd)), _ptr(out), _i(T), _i(Hq), _i(Hkv), _i(hd),
-          _i(dtype_code(q.dtype)), _stream())
+          _i(dtype_code(q.dtype)), _i(block_table.shape[0]), _stream())
     return out
 
 
