@@ -25,6 +25,7 @@
 //    weight shared by the heads and by silu (or the sigmoid) of a gate projection, and leaves in the operand dtype for the
 //    output product.  Called with ONE head of all heads' values it norms them together.
 #include "common.cuh"
+#include "short_conv.cuh"
 
 namespace {
 
@@ -438,13 +439,17 @@ __global__ void __launch_bounds__(256) delta_out_row_kernel(const float* o, cons
 // copied (their slices summed).  act: 0 none, 1 silu.  Then call q6k_short_conv_tail with the same x.
 Q6K_API int q6k_short_conv(const float* x, int slices, long long slice_stride, int ldx, const float* bias, const float* w, const float* tail,
                            const int* req_of_token, const int* q_start, const int* slot_ids, float* out, int ldo, int T_, int C, int copy_to,
-                           int taps, int act, cudaStream_t st) {
+                           int taps, int act, int requests, cudaStream_t st) {
     if (T_ == 0) return 0;
     Q6K_REQUIRE(T_ > 0 && C > 0 && copy_to >= C && taps >= 1 && taps <= CONV_MAX_TAPS && slices >= 1,
                 "short_conv: bad sizes T=%d C=%d taps=%d (at most %d taps) slices=%d", T_, C, taps, CONV_MAX_TAPS, slices);
     Q6K_REQUIRE(ldx >= copy_to && ldo >= copy_to && (act == 0 || act == 1), "short_conv: rows of %d and %d for %d columns, act %d", ldx, ldo, copy_to, act);
     dim3 grid(T_, (copy_to + 255) / 256);
     Q6K_REQUIRE(grid.y <= 65535, "short_conv: %d channels exceed the grid limit", copy_to);
+    if (slices == 1 && copy_to == C && conv_rows_taken(T_, requests, x, ldx, bias, tail, out, ldo, C, taps)) {
+        conv_rows<float, false>(x, ldx, w, bias, tail, req_of_token, q_start, slot_ids, out, ldo, T_, C, taps, act, st);
+        return q6k_check_launch("short_conv");
+    }
     q6k_launch(short_conv_kernel, grid, 256, 0, st, x, slices, (size_t)slice_stride, ldx, bias, w, tail, req_of_token, q_start, slot_ids, out,
                ldo, C, copy_to, taps, act);
     return q6k_check_launch("short_conv");

@@ -18,7 +18,7 @@
 // is the decay it applies to what came before).  A first launch (MODE 1) leaves that pair per segment; the second (MODE 2)
 // folds the pairs of the segments before its own into the state it starts from, in order, and then runs as the single
 // launch (MODE 0) does.  This only regroups the sums of the recurrence: the result differs by rounding.
-#include "common.cuh"
+#include "short_conv.cuh"
 
 namespace {
 
@@ -210,11 +210,15 @@ __global__ void cast_columns_kernel(const float* src, int ld, int col0, int n, T
 // w: FP32 [C, taps] (last column: the current token's), bias FP32 [C], tail FP32 [slots, taps-1, C] (read only here; the scan
 // kernel moves it on).
 Q6K_API int q6k_conv_silu(const float* x, int ldx, const float* w, const float* bias, const float* tail, const int* req_of_token,
-                          const int* q_start, const int* slot_ids, void* out, int T_, int C, int taps, int dtype, cudaStream_t st) {
+                          const int* q_start, const int* slot_ids, void* out, int T_, int C, int taps, int dtype, int requests, cudaStream_t st) {
     if (T_ == 0) return 0;
     Q6K_REQUIRE(T_ > 0 && C > 0 && taps >= 1 && taps <= MAX_TAPS, "conv_silu: bad sizes T=%d C=%d taps=%d (at most %d taps)", T_, C, taps, MAX_TAPS);
     dim3 grid(T_, (C + 255) / 256);
     Q6K_REQUIRE(grid.y <= 65535, "conv_silu: %d channels exceed the grid limit", C);
+    if (conv_rows_taken(T_, requests, x, ldx, bias, tail, out, C, C, taps)) {
+        Q6K_DISPATCH(dtype, (conv_rows<T, true>(x, ldx, w, bias, tail, req_of_token, q_start, slot_ids, (T*)out, C, T_, C, taps, 1, st)););
+        return q6k_check_launch("conv_silu");
+    }
     Q6K_DISPATCH(dtype, q6k_launch(conv_silu_kernel<T>, grid, 256, 0, st, x, ldx, w, bias, tail, req_of_token, q_start, slot_ids,
                                    (T*)out, C, taps););
     return q6k_check_launch("conv_silu");

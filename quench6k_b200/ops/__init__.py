@@ -1125,7 +1125,7 @@ def conv_silu(x: torch.Tensor, channels: int, w: torch.Tensor, bias: torch.Tenso
         raise KernelError("conv_silu: shapes disagree")
     out = torch.empty((T, channels), dtype=out_dtype, device=x.device)
     _call("q6k_conv_silu", _ptr(x), _i(x.stride(0)), _ptr(w), _ptr(bias), _ptr(tail), _ptr(req_of_token), _ptr(q_start), _ptr(slot_ids),
-          _ptr(out), _i(T), _i(channels), _i(taps), _i(dtype_code(out_dtype)), _stream())
+          _ptr(out), _i(T), _i(channels), _i(taps), _i(dtype_code(out_dtype)), _i(q_start.numel() - 1), _stream())
     return out
 
 
@@ -1458,7 +1458,8 @@ def short_conv(x: torch.Tensor, channels: int, w: torch.Tensor, bias: Optional[t
         raise KernelError(f"short_conv: unknown activation {act!r}")
     out = torch.empty((T, copy_to), dtype=torch.float32, device=x.device)
     _call("q6k_short_conv", _ptr(x), _i(slices), _ll(stride), _i(N), _ptr(bias), _ptr(w), _ptr(tail), _ptr(req_of_token), _ptr(q_start),
-          _ptr(slot_ids), _ptr(out), _i(copy_to), _i(T), _i(channels), _i(copy_to), _i(taps), _i(1 if act == "silu" else 0), _stream())
+          _ptr(slot_ids), _ptr(out), _i(copy_to), _i(T), _i(channels), _i(copy_to), _i(taps), _i(1 if act == "silu" else 0),
+          _i(q_start.numel() - 1), _stream())
     if taps > 1:
         _call("q6k_short_conv_tail", _ptr(x), _i(slices), _ll(stride), _i(N), _ptr(bias), _ptr(tail), _ptr(q_start), _ptr(slot_ids), _i(R),
               _i(channels), _i(taps), _stream())
