@@ -9,15 +9,18 @@
 //
 // The state S, dt, the decay and every sum of the recurrence are FP32; u leaves the convolution in
 // the operand dtype (it is the next product's input) and enters the recurrence as stored.  A group of
-// L lanes owns a channel (state index n = lane + L * k); the sum over n is a butterfly over those
-// lanes, so its order depends on nothing but N.  Tokens of a request are walked in order, so a prompt
+// L lanes owns a channel, each lane eight states side by side (B and C come to them 16 bytes at a time); the sum over n is
+// a lane's own and then a butterfly over those lanes, so its order depends on nothing but N.  Tokens of a request are walked in order, so a prompt
 // cut anywhere leaves the same state as the whole prompt.
 //
 // A long portion is walked in segments of `seg_len` tokens by different blocks (the recurrence is linear in S, so a
-// segment's effect on the state is a pair: the state it builds from zero and the sum of dt A over it, whose exponential
-// is the decay it applies to what came before).  A first launch (MODE 1) leaves that pair per segment; the second (MODE 2)
-// folds the pairs of the segments before its own into the state it starts from, in order, and then runs as the single
-// launch (MODE 0) does.  This only regroups the sums of the recurrence: the result differs by rounding.
+// segment's effect on the state is a pair: the state it builds from zero and the sum of dt over it, from which follows
+// the decay it applies to what came before).  A first launch (MODE 1) leaves that pair per segment; a small kernel walks a
+// request's pairs in order and puts the state that each segment starts from in its state's place; the last launch (MODE 2)
+// runs as the single launch (MODE 0) does.  This only regroups the sums of the recurrence: the result differs by rounding.
+// 2,048 tokens, 4,096 channels of 16 states: the launches were 545 us when each segment folded all of its predecessors
+// itself (254 MB of pairs) and a lane read its states' B and C one by one.  Now 135 + 20 + 216 us.  What bounds it: issue slots,
+// about 16 a token and state in either launch, and the special-function unit (an exponential each).
 #include "short_conv.cuh"
 
 namespace {
@@ -60,9 +63,32 @@ __global__ void __launch_bounds__(256) conv_silu_kernel(const float* x, int ldx,
     out[(size_t)t * C + c] = from_f32<T>(silu_f(acc));
 }
 
-// grid (R, ceil(C / (128 / L)), segments), 128 threads; dynamic shared memory SCAN_TILE * (2 N + 4 * 128 / L) floats.
-// ws (MODE 1, 2): per segment slot q = seg_base[r] + segment, [q][2][C][N] (the state built from zero, the sum of dt A),
-// then per request [r][C][N], the state the step found in the request's slot.
+// The state every segment of request r starts from, in place of the state it builds from zero.  grid (R * blocks), blocks = ceil(C N / 256).
+__global__ void __launch_bounds__(256) scan_fold_kernel(float* ws, const float* A, const float* state, const int* q_start, const int* slot_ids,
+                                                        const int* seg_base, int seg_len, int seg_slots, int C, int N) {
+    pdl_enter();
+    const size_t CN = (size_t)C * N;
+    const unsigned blocks = (unsigned)((CN + 255) / 256);
+    const int r = blockIdx.x / blocks, n_req = q_start[r + 1] - q_start[r];
+    const size_t i = (size_t)(blockIdx.x % blocks) * 256 + threadIdx.x;
+    if (i >= CN) return;
+    const float a = A[i];
+    float S = state[(size_t)slot_ids[r] * CN + i];
+    float* at = ws + (size_t)seg_base[r] * CN + i;
+    const float* sums = ws + (size_t)seg_slots * CN + (size_t)seg_base[r] * C + i / N;
+    const int segments = (n_req + seg_len - 1) / seg_len;
+#pragma unroll 4
+    for (int q = 0; q < segments; ++q, at += CN, sums += C) {
+        const bool more = q + 1 < segments;                                     // the last segment leaves no pair
+        const float built = more ? *at : 0.0f, dts = more ? *sums : 0.0f;
+        *at = S;
+        S = fmaf(expm1f(dts * a), S, S) + built;
+    }
+}
+
+// grid (R, ceil(C / (128 / L)), segments), 128 threads; dynamic shared memory SCAN_TILE * (16 L + 4 * 128 / L) floats.
+// ws (MODE 1, 2): per segment slot q = seg_base[r] + segment, [q][C][N] the state built from zero (MODE 2: the state to start
+// from), then [q][C] the sum of dt.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp,
                                                              int b_col, int c_col, const float* A, const float* Dskip, const float* xz,
@@ -70,7 +96,7 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
                                                              const int* slot_ids, T* out, int C, int N, int L, int taps, float* ws,
                                                              const int* seg_base, int seg_len, int seg_slots) {
     pdl_enter();
-    extern __shared__ float bc[];              // [SCAN_TILE][N] of B, the same of C, then four [SCAN_TILE][channels of the block]
+    extern __shared__ __align__(16) float bc[];    // [SCAN_TILE][8 L] of B, the same of C, then four [SCAN_TILE][channels of the block]
     const int r = blockIdx.x, seg = MODE == 0 ? 0 : blockIdx.z;
     const int per_block = blockDim.x / L;
     const int c = blockIdx.y * per_block + threadIdx.x / L, sub = threadIdx.x % L;
@@ -81,33 +107,21 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
     const int n_tok = MODE == 0 ? n_req : min(n_req - t_begin, seg_len);       // this block's tokens
     const int first = first_req + t_begin;
     const bool last_segment = t_begin + n_tok == n_req;
+    if (MODE == 1 && last_segment) return;     // no later segment follows this one
     const size_t CN = (size_t)C * N, own = ((size_t)(live ? c : 0)) * N;
-    float S[MAX_PER_LANE], a[MAX_PER_LANE], dsum[MAX_PER_LANE];
+    const int n0 = sub * MAX_PER_LANE, NP = L * MAX_PER_LANE;                  // this lane's first state; states with padding
+    float S[MAX_PER_LANE], a[MAX_PER_LANE], dt_sum = 0.0f;
     float* Sg = state + (size_t)slot * CN + own;
-    float* seg_pair = MODE == 0 ? nullptr : ws + (size_t)(seg_base[r] + seg) * 2 * CN + own;
-    float* found = MODE == 0 ? nullptr : ws + (size_t)seg_slots * 2 * CN + (size_t)r * CN + own;
+    float* seg_state = MODE == 0 ? Sg : ws + (size_t)(seg_base[r] + seg) * CN + own;
 #pragma unroll
     for (int k = 0; k < MAX_PER_LANE; ++k) {
-        const int n = sub + L * k;
-        const bool has = live && n < N;
-        a[k] = has ? A[(size_t)c * N + n] : 0.0f;
-        dsum[k] = 0.0f;
-        if (MODE == 0) {
-            S[k] = has ? Sg[n] : 0.0f;
-        } else if (MODE == 1) {
-            S[k] = 0.0f;
-            if (has && seg == 0) found[n] = Sg[n];
-        } else {
-            S[k] = has ? found[n] : 0.0f;
-            const float* pair = ws + (size_t)seg_base[r] * 2 * CN + own;
-            for (int q = 0; q < seg; ++q, pair += 2 * CN)
-                if (has) S[k] = fmaf(expm1f(pair[CN + n]), S[k], S[k]) + pair[n];
-        }
+        const bool has = live && n0 + k < N;   // a state beyond N has A = B = C = 0 and stays zero
+        a[k] = has ? A[(size_t)c * N + n0 + k] : 0.0f;
+        S[k] = has && MODE != 1 ? seg_state[n0 + k] : 0.0f;
     }
-    if (MODE == 1 && last_segment) return;     // no later segment folds this one (segment 0 has left the state it found)
     // Per tile of SCAN_TILE tokens the block first makes, once per (token, channel) and with coalesced loads, what the
     // recurrence needs of them: dt = softplus(dt_raw + bias), dt u, the gate silu(z) and the skip D u; then B and C.
-    float* s_dt = bc + 2 * SCAN_TILE * N;          // [SCAN_TILE][per_block]
+    float* s_dt = bc + 2 * SCAN_TILE * NP;         // [SCAN_TILE][per_block]
     float* s_du = s_dt + SCAN_TILE * per_block;
     float* s_gate = s_du + SCAN_TILE * per_block;
     float* s_skip = s_gate + SCAN_TILE * per_block;
@@ -115,11 +129,11 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
     for (int t0 = 0; t0 < n_tok; t0 += SCAN_TILE) {
         const int nt = min(SCAN_TILE, n_tok - t0);
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * N; i += blockDim.x) {
-            const int tt = i / N, n = i % N;
+        for (int i = threadIdx.x; i < nt * NP; i += blockDim.x) {
+            const int tt = i / NP, n = i % NP;
             const float* pr = proj + (size_t)(first + t0 + tt) * ldp;
-            bc[i] = pr[b_col + n];
-            bc[SCAN_TILE * N + i] = pr[c_col + n];
+            bc[i] = n < N ? pr[b_col + n] : 0.0f;
+            bc[SCAN_TILE * NP + i] = n < N ? pr[c_col + n] : 0.0f;
         }
         for (int i = threadIdx.x; i < nt * per_block; i += blockDim.x) {
             const int tt = i / per_block, ch = c0 + i % per_block;
@@ -139,19 +153,20 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
 #pragma unroll 2
         for (int tt = 0; tt < nt; ++tt) {
             const float dt = s_dt[tt * per_block + cc], du = s_du[tt * per_block + cc];
-            const float* Bt = bc + tt * N;
-            const float* Ct = bc + SCAN_TILE * N + tt * N;
+            const float4* Bt = reinterpret_cast<const float4*>(bc + tt * NP + n0);
+            const float4* Ct = reinterpret_cast<const float4*>(bc + (SCAN_TILE + tt) * NP + n0);
             float y = 0.0f;
+            if (MODE == 1) dt_sum += dt;
 #pragma unroll
-            for (int k = 0; k < MAX_PER_LANE; ++k) {
-                const int n = sub + L * k;
-                if (n < N) {
+            for (int k = 0; k < MAX_PER_LANE; k += 4) {
+                const float4 b4 = Bt[k / 4], c4 = MODE == 1 ? b4 : Ct[k / 4];
+                const float bb[4] = {b4.x, b4.y, b4.z, b4.w}, cc4[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
                     // exp(dt A) S as S + expm1(dt A) S: a decay close to 1 keeps its distance from 1 to full precision, so
                     // that no rounding of the factor itself (always the same way for a given dt A) adds up over a long context
-                    const float da = dt * a[k];
-                    S[k] = fmaf(decay_minus_one<sizeof(T) == 2>(da), S[k], S[k]) + du * Bt[n];
-                    if (MODE == 1) dsum[k] += da;
-                    else y = fmaf(S[k], Ct[n], y);
+                    S[k + e] = fmaf(du, bb[e], fmaf(decay_minus_one<sizeof(T) == 2>(dt * a[k + e]), S[k + e], S[k + e]));
+                    if (MODE != 1) y = fmaf(S[k + e], cc4[e], y);
                 }
             }
             if (MODE != 1) {
@@ -164,21 +179,15 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
     if (!live) return;
     if (MODE == 1) {
 #pragma unroll
-        for (int k = 0; k < MAX_PER_LANE; ++k) {
-            const int n = sub + L * k;
-            if (n < N) {
-                seg_pair[n] = S[k];
-                seg_pair[CN + n] = dsum[k];
-            }
-        }
+        for (int k = 0; k < MAX_PER_LANE; ++k)
+            if (n0 + k < N) seg_state[n0 + k] = S[k];
+        if (sub == 0) ws[(size_t)seg_slots * CN + (size_t)(seg_base[r] + seg) * C + c] = dt_sum;
         return;
     }
     if (!last_segment) return;
 #pragma unroll
-    for (int k = 0; k < MAX_PER_LANE; ++k) {
-        const int n = sub + L * k;
-        if (n < N) Sg[n] = S[k];
-    }
+    for (int k = 0; k < MAX_PER_LANE; ++k)
+        if (n0 + k < N) Sg[n0 + k] = S[k];
     if (sub == 0 && taps > 1) {
         // the last taps-1 inputs of the convolution: the end of this portion, preceded by what is left of the old tail
         float* tl = tail + (size_t)slot * (taps - 1) * C + c;
@@ -239,7 +248,7 @@ Q6K_API int q6k_selective_scan_lanes(int N) {
 Q6K_API int q6k_selective_scan_segment() { return 64; }
 
 // Floats of scratch for `seg_slots` segments in all and R requests.
-Q6K_API long long q6k_selective_scan_workspace(int seg_slots, int R, int C, int N) { return ((long long)seg_slots * 2 + R) * C * N; }
+Q6K_API long long q6k_selective_scan_workspace(int seg_slots, int R, int C, int N) { return R > 0 ? (long long)seg_slots * C * (N + 1) : 0; }
 
 // segments > 1: portions are walked in segments of q6k_selective_scan_segment() tokens (`segments`: the most of any request;
 // seg_base: int32 [R], the first segment slot of each request; seg_slots: their total; ws: the scratch above).
@@ -255,7 +264,7 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
     const int per_block = 128 / L;
     dim3 grid(R, (C + per_block - 1) / per_block);
     Q6K_REQUIRE(grid.y <= 65535, "selective_scan: %d channels exceed the grid limit", C);
-    const size_t smem = (size_t)SCAN_TILE * (2 * N + 4 * per_block) * sizeof(float);
+    const size_t smem = (size_t)SCAN_TILE * (2 * L * MAX_PER_LANE + 4 * per_block) * sizeof(float);
     const int seg_len = q6k_selective_scan_segment();
 #define SCAN_LAUNCH(MODE, GRID)                                                                                                      \
     Q6K_DISPATCH(dtype, if (smem > 48 * 1024) cudaFuncSetAttribute(selective_scan_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -269,6 +278,8 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
     dim3 grid3(R, grid.y, segments);
     SCAN_LAUNCH(1, grid3);
     if (int rc = q6k_check_launch("selective_scan (segments)")) return rc;
+    q6k_launch(scan_fold_kernel, dim3((unsigned)(R * (((size_t)C * N + 255) / 256))), 256, 0, st, ws, A, state, q_start, slot_ids, seg_base, seg_len, seg_slots, C, N);
+    if (int rc = q6k_check_launch("selective_scan (fold)")) return rc;
     SCAN_LAUNCH(2, grid3);
 #undef SCAN_LAUNCH
     return q6k_check_launch("selective_scan");
