@@ -24,7 +24,7 @@
 //    delta_out_kernel closes the mixer: every head's o is divided by its root mean square over dv, multiplied by a
 //    weight shared by the heads and by silu (or the sigmoid) of a gate projection, and leaves in the operand dtype for the
 //    output product.  Called with ONE head of all heads' values it norms them together.
-#include "common.cuh"
+#include "chunks.cuh"
 #include "short_conv.cuh"
 
 namespace {
@@ -111,9 +111,9 @@ __device__ __forceinline__ void delta_unit_vectors(float* ur, int q_at, int k_at
     }
 }
 
-// grid (T), 128 threads.
+// grid (T), 128 threads.  logs: the decays' logarithms in the decays' place (for the chunked kernels below).
 __global__ void __launch_bounds__(128) delta_prepare_kernel(float* u, int ldu, const float* p, int ldp, int b_col, int a_col, const float* A_log,
-                                                            const float* dt_bias, float* bg, int H, int G, int dk) {
+                                                            const float* dt_bias, float* bg, int H, int G, int dk, int logs) {
     pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* ur = u + (size_t)t * ldu;
@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(float* u, int ldu, c
     for (int h = threadIdx.x; h < H; h += blockDim.x) {
         const float* pr = p + (size_t)t * ldp;
         out[h] = 1.0f / (1.0f + expf(-pr[b_col + h]));
-        out[H + h] = expf(-expf(A_log[h]) * softplus_f(pr[a_col + h] + dt_bias[h]));
+        const float log_decay = -expf(A_log[h]) * softplus_f(pr[a_col + h] + dt_bias[h]);
+        out[H + h] = logs ? (log_decay < -200.0f ? -200.0f : log_decay) : expf(log_decay);      // e^-200 is 0; sums of such stay exact enough
     }
 }
 
@@ -364,6 +365,266 @@ __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float*
     }
 }
 
+// ---------------------------------------------------------------------------------------- long portions, chunk by chunk
+//
+// The walk above takes a step of a few scalars per column and four tokens, each behind a butterfly and a barrier: 235 ns a token
+// (2,048 tokens of 16 heads of 128 x 128: 482 us), latency that no other work hides.  Over a chunk of C = 32 tokens the recurrence is
+// a triangular system: with P_i the product of the chunk's decays up to token i and S the state before the chunk,
+//
+//   (I + A) U = B (V - diag(P) K S),    A[i][m] = beta_i (P_i / P_m) (k_i . k_m) for m < i,    B = diag(beta)
+//   O = diag(P) Q S + M U,              M[i][m] = (P_i / P_m) (q_i . k_m) for m <= i
+//   S <- P_C S + sum_m (P_C / P_m) k_m u_m^T
+//
+// delta_chunk_kernel makes (I + A)^-1 and M of every (chunk, head), which do not depend on the state, for all chunks at once (the
+// inverse's entries are products of the rule's contractions and stay below 1; the decays' ratios come from their logarithms,
+// summed and subtracted in double precision).  delta_walk_kernel takes the chunks in order: five small FP32 products a chunk, a
+// block per (request, head, 16 columns), the next chunk's K, Q, inverse and M on their way meanwhile, S in registers with a copy in
+// shared memory for the products that read it.  C = 32: a chunk of 64 would double the triangular work and the bytes of the two
+// matrices per token.  15 + 237 us.  What bounds it: the FP32 pipe
+// (3 x dk x 16 multiply-adds a token and block), its reads of shared memory and four barriers a chunk.
+constexpr int CHUNK_FLOATS = 2 * WC * WC + 3 * WC;              // per (chunk, head): inverse, M, beta, P, P_C / P_m
+
+// grid (chunks, G), 128 threads; dynamic shared memory: K and Q [WC][dk + 4] each, then six [WC][WLD] squares (four of them a warp's).
+__global__ void __launch_bounds__(128) delta_chunk_kernel(const float* u, int ldu, const float* bg, const int* q_start, int R, float* chunks, int H, int G, int dk) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    const int ld = dk + 4, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *ks = sm, *qs = ks + WC * ld, *kk = qs + WC * ld, *kq = kk + WC * WLD, *aw = kq + WC * WLD + warp * WC * WLD;
+    int first = 0, n = 0;
+    chunk_of(q_start, R, blockIdx.x, first, n);
+    if (n == 0) return;
+    for (int i = tid; i < WC * (dk / 4); i += 128) {
+        const int t = i / (dk / 4), d = (i % (dk / 4)) * 4;
+        float4 k4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q4 = k4;
+        if (t < n) {
+            const float* ur = u + (size_t)(first + t) * ldu + kvh * dk + d;
+            q4 = *reinterpret_cast<const float4*>(ur);
+            k4 = *reinterpret_cast<const float4*>(ur + G * dk);
+        }
+        *reinterpret_cast<float4*>(ks + t * ld + d) = k4;
+        *reinterpret_cast<float4*>(qs + t * ld + d) = q4;
+    }
+    __syncthreads();
+    {   // kk[i][m] = k_i . k_m, kq[i][m] = q_i . k_m: a thread one row i, eight m
+        const int i = tid >> 2, m0 = tid & 3;
+        float a[8] = {}, b[8] = {};
+        for (int d = 0; d < dk; d += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(ks + i * ld + d), q4 = *reinterpret_cast<const float4*>(qs + i * ld + d);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                const float4 m4 = *reinterpret_cast<const float4*>(ks + (m0 + 4 * x) * ld + d);
+                a[x] = dot4(k4, m4, a[x]);
+                b[x] = dot4(q4, m4, b[x]);
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 8; ++x) kk[i * WLD + m0 + 4 * x] = a[x], kq[i * WLD + m0 + 4 * x] = b[x];
+    }
+    __syncthreads();
+    const int per = H / G;
+    for (int hh = warp; hh < per; hh += 4) {
+        const int head = kvh * per + hh;
+        float* out = chunks + ((size_t)blockIdx.x * H + head) * CHUNK_FLOATS;
+        // lane = token: its beta and the sum of the decays' logarithms up to it (tokens beyond the portion change nothing)
+        const float* pr = bg + (size_t)(first + (lane < n ? lane : 0)) * 2 * H;
+        const float beta = lane < n ? pr[head] : 0.0f;
+        double L = lane < n ? (double)pr[H + head] : 0.0;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double other = __shfl_up_sync(0xffffffffu, L, off);
+            if (lane >= off) L += other;
+        }
+        const double all = __shfl_sync(0xffffffffu, L, 31);
+        out[2 * WC * WC + lane] = beta;
+        out[2 * WC * WC + WC + lane] = expf((float)L);
+        out[2 * WC * WC + 2 * WC + lane] = expf((float)(all - L));
+        // lane = column m from here on
+#pragma unroll 4
+        for (int i = 0; i < WC; ++i) {
+            const double Li = __shfl_sync(0xffffffffu, L, i);
+            const float ratio = lane <= i ? expf((float)(Li - L)) : 0.0f;
+            const float bi = __shfl_sync(0xffffffffu, beta, i);
+            aw[i * WLD + lane] = lane < i ? bi * ratio * kk[i * WLD + lane] : 0.0f;
+            out[WC * WC + i * WC + lane] = lane <= i ? ratio * kq[i * WLD + lane] : 0.0f;
+        }
+        __syncwarp();
+        float t[WC];                                            // column `lane` of the inverse, by forward substitution
+#pragma unroll
+        for (int i = 0; i < WC; ++i) {
+            float acc = i == lane ? 1.0f : 0.0f;
+#pragma unroll
+            for (int m = 0; m < i; ++m) acc = fmaf(-aw[i * WLD + m], t[m], acc);
+            t[i] = acc;
+            out[i * WC + lane] = acc;
+        }
+        __syncwarp();
+    }
+}
+
+__host__ __device__ constexpr int walk_stage_floats(int dkp) { return 2 * WC * (dkp + 4) + 2 * WC * WLD + 3 * WC + WC * WALK_COLS; }
+__host__ __device__ constexpr int walk_floats(int dkp) { return 2 * walk_stage_floats(dkp) + WALK_COLS * (dkp + 4) + 2 * WC * (WALK_COLS + 4) + 3 * WALK_COLS * WLD; }
+
+// grid (H * ceil(dv / 16), R), 256 threads.  dkp: dk rounded up to a multiple of 8.  GROUPS: ceil(dkp / 128), groups of four rows of the
+// state a thread holds.
+template <int GROUPS>
+__global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(const float* u, int ldu, const float* chunks, float* state, const int* q_start,
+                                                                  const int* slot_ids, float* o, int H, int G, int dk, int dv, int dkp) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    const int ld = dkp + 4, stage = walk_stage_floats(dkp);
+    // a stage: K [WC][ld] | Q [WC][ld] | inverse [WC][WLD] | M [WC][WLD] | beta, P, P_C / P_m [3][WC] | V [WC][16]
+    float* S = sm + 2 * stage;                          // [16][ld]: a column's rows side by side
+    float* xy = S + WALK_COLS * ld;                     // [2][WC][20]: half sums of K S and Q S on their way between the halves, then P (Q S)
+    float* rt = xy + 2 * WC * (WALK_COLS + 4);          // [16][WLD]: right-hand sides, a column's tokens side by side
+    float* ut = rt + WALK_COLS * WLD;                   // [16][WLD]: U
+    float* uw = ut + WALK_COLS * WLD;                   // [16][WLD]: U times P_C / P_m
+    const int col_blocks = (dv + WALK_COLS - 1) / WALK_COLS, head = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * WALK_COLS, r = blockIdx.y;
+    const int kvh = head / (H / G), tid = threadIdx.x, tx = tid & 7, row8 = tid >> 3;
+    const int first = q_start[r], n = q_start[r + 1] - first;
+    if (n <= 0) return;
+    const int chunk0 = first_chunk_of(q_start, r), count = (n + WC - 1) / WC;
+    float* mine = state + ((size_t)slot_ids[r] * H + head) * dv * dk;
+    // rows 4 (row8 + 32 g) .. + 3 of columns tx and tx + 8
+    float4 s[GROUPS][2];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int row = 4 * (row8 + 32 * g), col = col0 + tx + 8 * c;
+            s[g][c] = row < dk && col < dv ? *reinterpret_cast<const float4*>(mine + (size_t)col * dk + row) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row < dkp) *reinterpret_cast<float4*>(S + (tx + 8 * c) * ld + row) = s[g][c];
+        }
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+    auto copy = [&](uint32_t to, const float* from, bool in) { copy16(to, in ? from : u, in); };
+    auto fetch = [&](int c) {
+        if (c < count) {
+            const uint32_t at = base + 4 * (c & 1) * stage;
+            const int left = n - c * WC;
+            const float* row = u + (size_t)(first + c * WC + row8) * ldu + kvh * dk;        // eight threads a row
+            for (int d = tx * 4; d < dkp; d += 32) {
+                copy(at + 4 * (row8 * ld + d), row + G * dk + d, row8 < left && d < dk);
+                copy(at + 4 * ((WC + row8) * ld + d), row + d, row8 < left && d < dk);
+            }
+            const float* from = chunks + ((size_t)(chunk0 + c) * H + head) * CHUNK_FLOATS;
+            const uint32_t sq = at + 4 * 2 * WC * ld;
+            for (int i = tid; i < 2 * WC * WC / 4; i += WALK_THREADS) copy(sq + 4 * ((i / (WC / 4)) * WLD + (i % (WC / 4)) * 4), from + 4 * i, true);
+            if (tid < 3 * WC / 4) copy(sq + 4 * (2 * WC * WLD + 4 * tid), from + 2 * WC * WC + 4 * tid, true);
+            else if (tid >= 128) {
+                const int t = (tid - 128) >> 2, d = (tid & 3) * 4;
+                copy(sq + 4 * (2 * WC * WLD + 3 * WC + t * WALK_COLS + d), u + (size_t)(first + c * WC + t) * ldu + 2 * G * dk + head * dv + col0 + d,
+                     t < left && col0 + d < dv);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    for (int c = 0; c < count; ++c) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                // the chunk has landed, S is whole, and nobody is in the chunk before any more
+        fetch(c + 1);
+        const float* K = sm + (c & 1) * stage;
+        const float *inv = K + 2 * WC * ld, *M = inv + WC * WLD, *beta = M + WC * WLD, *P = beta + WC, *E = P + WC, *V = E + WC;
+        {   // K S and Q S: rows row + 8 i of K (y 0) or Q (y 1), columns tx and tx + 8, half of the sum each
+            const int half = tid >> 7, y = (tid >> 6) & 1, row = (tid >> 3) & 7;
+            const float *a = K + (size_t)(y * WC + row) * ld + half * (dkp / 2), *b = S + tx * ld + half * (dkp / 2);
+            float acc[4][2] = {};
+#pragma unroll 4
+            for (int d = 0; d < dkp / 2; d += 4) {
+                const float4 b0 = *reinterpret_cast<const float4*>(b + d), b1 = *reinterpret_cast<const float4*>(b + 8 * ld + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 x = *reinterpret_cast<const float4*>(a + i * 8 * ld + d);
+                    acc[i][0] = dot4(x, b0, acc[i][0]);
+                    acc[i][1] = dot4(x, b1, acc[i][1]);
+                }
+            }
+            // the first half of the threads finishes K S, the second Q S
+            if (half != y) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) xy[(y * WC + row + 8 * i) * (WALK_COLS + 4) + tx + 8 * j] = acc[i][j];
+            }
+            __syncthreads();
+            if (half == y) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int t = row + 8 * i;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int col = tx + 8 * j;
+                        float* at = xy + (y * WC + t) * (WALK_COLS + 4) + col;
+                        const float sum = (*at + acc[i][j]) * P[t];
+                        if (y == 0) rt[col * WLD + t] = beta[t] * (V[t * WALK_COLS + col] - sum);
+                        else *at = sum;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const int t = row8;                             // U and O: token t, columns tx and tx + 8
+        auto triangle = [&](const float* m, const float* x, float* acc) {
+#pragma unroll
+            for (int d = 0; d < WC; d += 4) {
+                if (d > t) break;
+                const float4 a = *reinterpret_cast<const float4*>(m + t * WLD + d);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) acc[j] = dot4(a, up_to(*reinterpret_cast<const float4*>(x + (tx + 8 * j) * WLD + d), t - d), acc[j]);
+            }
+        };
+        {
+            float acc[2] = {};
+            triangle(inv, rt, acc);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) ut[(tx + 8 * j) * WLD + t] = acc[j], uw[(tx + 8 * j) * WLD + t] = acc[j] * E[t];
+        }
+        __syncthreads();
+        {
+            float acc[2] = {xy[(WC + t) * (WALK_COLS + 4) + tx], xy[(WC + t) * (WALK_COLS + 4) + tx + 8]};
+            triangle(M, ut, acc);
+            if (c * WC + t < n) {
+                float* dst = o + (size_t)(first + c * WC + t) * H * dv + head * dv + col0;
+                if (col0 + tx < dv) dst[tx] = acc[0];
+                if (col0 + tx + 8 < dv) dst[tx + 8] = acc[1];
+            }
+        }
+        const float decay = P[WC - 1];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            const int row = 4 * (row8 + 32 * g);
+            if (row < dkp) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) s[g][j].x *= decay, s[g][j].y *= decay, s[g][j].z *= decay, s[g][j].w *= decay;
+#pragma unroll 2
+                for (int m = 0; m < WC; m += 4) {
+                    float4 w[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) w[j] = *reinterpret_cast<const float4*>(uw + (tx + 8 * j) * WLD + m);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const float4 k4 = *reinterpret_cast<const float4*>(K + (m + x) * ld + row);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const float ww = x == 0 ? w[j].x : x == 1 ? w[j].y : x == 2 ? w[j].z : w[j].w;
+                            s[g][j].x = fmaf(k4.x, ww, s[g][j].x), s[g][j].y = fmaf(k4.y, ww, s[g][j].y);
+                            s[g][j].z = fmaf(k4.z, ww, s[g][j].z), s[g][j].w = fmaf(k4.w, ww, s[g][j].w);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) *reinterpret_cast<float4*>(S + (tx + 8 * j) * ld + row) = s[g][j];
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int row = 4 * (row8 + 32 * g), col = col0 + tx + 8 * j;
+            if (row < dk && col < dv) *reinterpret_cast<float4*>(mine + (size_t)col * dk + row) = s[g][j];
+        }
+}
+
 // grid (T, ceil(H / 4)), a warp per (token, head): out = T(o / rms(o) * w * silu(gate)).  Heads up to 256 wide keep their
 // values and gates in registers, all loads asked for before the sum; wider ones read the row twice.  w_stride: floats from a
 // head's weights to the next head's (0: shared by the heads).
@@ -466,18 +727,35 @@ Q6K_API int q6k_short_conv_tail(const float* x, int slices, long long slice_stri
 
 Q6K_API int q6k_gated_delta_max_dim() { return 32 * DELTA_LANES; }
 
-// state: FP32 [slots, H, dv, dk]; o: FP32 [T, H * dv].  bg: null, or FP32 scratch [T, 2 H]: the per-token values are then made
+// Floats of scratch for walking the portions of a step of T_ rows and R requests chunk by chunk.
+Q6K_API long long q6k_gated_delta_chunk_floats(int T_, int R, int H) { return (long long)(T_ / WC + R) * H * CHUNK_FLOATS; }
+
+// state: FP32 [slots, H, dv, dk]; o: FP32 [T, H * dv].  chunks: null, or (with bg) the scratch above.  bg: null, or FP32 scratch [T, 2 H]: the per-token values are then made
 // by a kernel of their own first, which also turns q and k in u into unit vectors (for steps with long portions).
 Q6K_API int q6k_gated_delta(float* u, int ldu, const float* p, int ldp, int b_col, int a_col, const float* A_log, const float* dt_bias,
-                            float* bg, float* state, const int* q_start, const int* slot_ids, float* o, int T_, int R, int H, int G, int dk,
+                            float* bg, float* chunks, float* state, const int* q_start, const int* slot_ids, float* o, int T_, int R, int H, int G, int dk,
                             int dv, cudaStream_t st) {
     if (R == 0 || T_ == 0) return 0;
     Q6K_REQUIRE(R > 0 && T_ > 0 && H > 0 && G > 0 && H % G == 0 && dk > 0 && dv > 0, "gated_delta: bad sizes R=%d H=%d G=%d dk=%d dv=%d", R, H, G, dk, dv);
     Q6K_REQUIRE(dk <= 32 * DELTA_LANES, "gated_delta: keys of %d entries exceed the supported %d", dk, 32 * DELTA_LANES);
     Q6K_REQUIRE(R <= 65535, "gated_delta: %d requests exceed the grid limit", R);
     if (bg) {
-        q6k_launch(delta_prepare_kernel, T_, 128, 0, st, u, ldu, p, ldp, b_col, a_col, A_log, dt_bias, bg, H, G, dk);
+        q6k_launch(delta_prepare_kernel, T_, 128, 0, st, u, ldu, p, ldp, b_col, a_col, A_log, dt_bias, bg, H, G, dk, chunks != nullptr);
         if (int rc = q6k_check_launch("delta_prepare")) return rc;
+    }
+    if (chunks) {
+        Q6K_REQUIRE(bg && dk % 4 == 0 && dv % 4 == 0 && ldu % 4 == 0 && (((uintptr_t)u | (uintptr_t)state | (uintptr_t)chunks) & 15) == 0,
+                    "gated_delta: chunks take prepared inputs, keys, values and rows of multiples of 4 entries, on 16 bytes");
+        const size_t smem1 = (size_t)(2 * WC * (dk + 4) + 6 * WC * WLD) * sizeof(float);
+        if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return q6k_check_launch("delta_chunk: shared memory attribute");
+        q6k_launch(delta_chunk_kernel, dim3(T_ / WC + R, G), 128, smem1, st, u, ldu, bg, q_start, R, chunks, H, G, dk);
+        if (int rc = q6k_check_launch("delta_chunk")) return rc;
+        const int dkp = (dk + 7) / 8 * 8;
+        const size_t smem2 = (size_t)walk_floats(dkp) * sizeof(float);
+        auto* walk = dkp <= 128 ? delta_walk_kernel<1> : delta_walk_kernel<2>;
+        if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess) return q6k_check_launch("delta_walk: shared memory attribute");
+        q6k_launch(walk, dim3(H * ((dv + WALK_COLS - 1) / WALK_COLS), R), WALK_THREADS, smem2, st, u, ldu, chunks, state, q_start, slot_ids, o, H, G, dk, dv, dkp);
+        return q6k_check_launch("delta_walk");
     }
     const dim3 grid(H * ((dv + DELTA_COLS - 1) / DELTA_COLS), R);
     const int rpl = ((dk + DELTA_LANES - 1) / DELTA_LANES + 3) / 4 * 4;

@@ -1473,14 +1473,23 @@ def gated_delta_max_dim() -> int:
     return lib.q6k_gated_delta_max_dim()
 
 
+def gated_delta_chunks(longest: int, G: int, H: int, dk: int, dv: int) -> bool:
+    """Whether a step whose longest portion has `longest` tokens should be walked chunk by chunk: rows of u and of the state that
+    start on 16 bytes, and more tokens than the walk token by token (235 ns each) gets through while the chunks' own kernel
+    runs (about 12 us)."""
+    return longest > 64 and dk % 4 == 0 and dv % 4 == 0 and (2 * G * dk + H * dv) % 4 == 0
+
+
 def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
-                q_start: torch.Tensor, slot_ids: torch.Tensor, R: int, H: int, G: int, dk: int, dv: int, prepare: bool = False) -> torch.Tensor:
+                q_start: torch.Tensor, slot_ids: torch.Tensor, R: int, H: int, G: int, dk: int, dv: int, prepare: bool = False,
+                chunked: bool = False) -> torch.Tensor:
     """The gated delta rule over the step's rows, request by request, from and into state [slots, H, dv, dk] (FP32):
     S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, with unit q (times dk^-1/2) and k.  u: FP32 [T, >= 2 G dk + H dv]
     = [q | k | v]; p: FP32 rows holding the H beta logits at b_col and the H decay inputs at a_col.  Returns FP32 o [T, H dv].
     prepare: a kernel of its own first makes every token's unit vectors (in place over q and k in u), beta, decay and k . q,
     and the recurrence fetches a tile of tokens while it walks the one before (for steps with long portions); else the
-    recurrence makes them itself.  The results are the same bit for bit."""
+    recurrence makes them itself.  The results are the same bit for bit.  chunked (with prepare, where gated_delta_chunks(...)
+    says so): 32 tokens at a time as a triangular system, equal to the others up to rounding."""
     _need(u, "u", torch.float32)
     _need(p, "p", torch.float32)
     _need(A_log, "A_log", torch.float32, (H,))
@@ -1491,8 +1500,15 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
         raise KernelError("gated_delta: shapes disagree")
     o = torch.empty((T, H * dv), dtype=torch.float32, device=u.device)
     bg = torch.empty((T, 2 * H + G), dtype=torch.float32, device=u.device) if prepare else None
+    chunks = None
+    if chunked:
+        if not prepare:
+            raise KernelError("gated_delta: chunks go with prepared inputs")
+        lib = library()
+        lib.q6k_gated_delta_chunk_floats.restype = ctypes.c_longlong
+        chunks = torch.empty(lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H)), dtype=torch.float32, device=u.device)
     _call("q6k_gated_delta", _ptr(u), _i(u.stride(0)), _ptr(p), _i(p.stride(0)), _i(b_col), _i(a_col), _ptr(A_log), _ptr(dt_bias), _ptr(bg),
-          _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
+          _ptr(chunks), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
     return o
 
 

@@ -126,7 +126,8 @@ class GatedDelta(Mixer):
                                   ctx.R, self.H, self.G, self.dk, self.dv, prepare=prepare, single=ctx.max_q_len == 1)
         else:
             o = ops.gated_delta(u, p, self.b_col, self.a_col, self.A_log, self.dt_bias, state["S"], ctx.q_start, ctx.slot_ids, ctx.R,
-                                self.H, self.G, self.dk, self.dv, prepare=prepare)
+                                self.H, self.G, self.dk, self.dv, prepare=prepare,
+                                chunked=prepare and ops.gated_delta_chunks(ctx.max_q_len, self.G, self.H, self.dk, self.dv))
         ops.current_tag = "delta.out"
         y = ops.delta_out(o, low, g_col, self.norm_w, self.eps, self.H, self.dv, rt.dtype, gate=self.gate)
         ops.current_tag = "delta.o"
