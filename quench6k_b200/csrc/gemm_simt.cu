@@ -8,7 +8,7 @@
 // runs them through one grouped kernel, crates/cuda/kernels/moe.cu:142-255) and may be gathered
 // through an index.  With two weight matrices the epilogue is SwiGLU: out = silu(A.Wg) * (A.Wu).
 //
-// Each output element is one accumulator summed over k in ascending order, so its value does not
+// Each output element is summed over k in an order that follows from K alone, so its value does not
 // depend on which tile or batch the row was in.
 #include "common.cuh"
 
@@ -102,25 +102,36 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* A, int lda, con
     }
 }
 
-// FP32 operands.  The same tiles and the same sums (one accumulator per element, ascending k) as the kernel above, whose loads, one
-// value at a time into a transposed tile that everyone then waits for, left the multipliers idle two thirds of the time (509 x
-// 1,024 x 1,024: 15 TFLOP/s).  Here rows go to shared memory as they lie, 16 bytes a copy, two k-blocks ahead of the one in use;
-// a thread reads four k of its 4 + 4 rows at a time (rows 144 bytes apart: 8 threads' reads fall into different banks), 8 loads for
-// 64 multiply-adds.  The 20 products of a step of 509 tokens through four layers (1,024 wide, experts of 512): 2,930 -> 1,835 us.
-// What bounds it now: the FP32 pipe (12 shared-memory wavefronts against 16 issue slots of multiply-adds a warp)
-// and, below 148 tiles, the SMs without one.  WIDE: rows start on 16 bytes and K is a multiple of 4; else copies of 4 bytes.
-constexpr int FK = 32, FLD = FK + 4, FSTAGES = 3;
+// FP32 operands.  The kernel above loads one value at a time into a transposed tile that everyone then waits for, and leaves the
+// multipliers idle two thirds of the time.  Here rows go to shared memory as they lie, 16 bytes a copy, two blocks of 32 k ahead of the one in
+// use, and the products go through the packed multiply-add, which takes two FP32 products an instruction: with operands read four k at a time,
+// the even and the odd k of an output are its two halves, so nothing has to be rearranged.  An output is then four sums over ascending k (even and
+// odd, of either half of each block of 32), added in the end: no larger an error than one sum, and the same for a row whatever its tile.
+// A block makes 32 x 64 outputs, half of its threads the first 16 k of every block and half the others: small enough that 512
+// rows fill the chip and that experts of some 60 rows waste little, with 4 x 4 outputs a thread all the same (8 loads of 16 bytes
+// for 64 products; rows 144 bytes apart, so that eight threads' reads fall into different banks).
+// The 20 products of a step of 509 tokens through four layers (1,024 wide, experts of 512): 1,835 -> 1,670 us against tiles of 64 x 64 with
+// an instruction per product (2,930 us with the kernel above).  What bounds it now: the FP32 pipe, half of its cycles, and reads of
+// shared memory, two thirds (3.3 wavefronts a read).  Warps of 8 x 128 outputs, whose reads of one address were to cost less, took 2,100 us.
+// WIDE: rows start on 16 bytes and K is a multiple of 4; else copies of 4 bytes.
+constexpr int FM = 32, FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 3;
+static_assert(BM == 2 * FM, "a tile of the tile lists is two of these");
 
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum_pair(unsigned long long v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+
+// grid (ceil(N / 64), tiles of 64 rows, 2), 256 threads.
 template <int EPI, bool WIDE>
-__global__ void __launch_bounds__(256, EPI == EPI_SWIGLU ? 2 : 3) gemm_f32_kernel(const float* A, int lda, const int* a_rows, const float* W, const float* W2,
+__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(const float* A, int lda, const int* a_rows, const float* W, const float* W2,
                                                                                   size_t w_group_stride, float* out, int ldo, int M, int N, int K,
                                                                                   const int* tile_group, const int* tile_row0, const int* group_offsets,
                                                                                   const int* num_tiles, int act, float act_limit) {
     pdl_enter();
     constexpr bool DUAL = EPI == EPI_SWIGLU;
-    constexpr int MATS = DUAL ? 3 : 2, TILE = BM * FLD, STAGE = MATS * TILE;
-    static_assert(BM == BN, "the loader takes tiles of equal height");
-    extern __shared__ __align__(16) float f_smem[];          // [FSTAGES][A | W | W2][64 rows][FLD]
+    constexpr int MATS = DUAL ? 2 : 1, STAGE = (FM + MATS * FN) * FLD;
+    extern __shared__ __align__(16) float f_smem[];          // [FSTAGES][A 32 rows | W 64 | W2 64][FLD]
     int g = 0, row0 = blockIdx.y * BM, row_end = M;
     if (tile_group) {
         if ((int)blockIdx.y >= *num_tiles) return;
@@ -128,83 +139,102 @@ __global__ void __launch_bounds__(256, EPI == EPI_SWIGLU ? 2 : 3) gemm_f32_kerne
         row0 = tile_row0[blockIdx.y];
         row_end = group_offsets[g + 1];
     }
+    row0 += blockIdx.z * FM;
     if (row0 >= row_end) return;
-    const int n0 = blockIdx.x * BN, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    // loader: WIDE pieces of 4 k of rows tid / 8 and tid / 8 + 32, else single k of rows tid / 32 + 8 e
-    constexpr int ROWS = WIDE ? 2 : 8, STEP = WIDE ? 32 : 8;
+    const int n0 = blockIdx.x * FN, tid = threadIdx.x;
+    // loader: WIDE pieces of 4 k of rows tid / 8 (+ 32), else single k of rows tid / 32 + 8 e
+    constexpr int STEP = WIDE ? 32 : 8, A_ROWS = FM / STEP, W_ROWS = FN / STEP;
     const int lr = WIDE ? tid >> 3 : tid >> 5, lk = WIDE ? (tid & 7) * 4 : tid & 31;
-    const float* src[MATS][ROWS];
+    const float *a_src[A_ROWS], *w_src[MATS][W_ROWS];
 #pragma unroll
-    for (int e = 0; e < ROWS; ++e) {
-        const int r = lr + e * STEP;
-        src[0][e] = row0 + r < row_end ? A + (size_t)(a_rows ? a_rows[row0 + r] : row0 + r) * lda : nullptr;
-        src[1][e] = n0 + r < N ? W + (size_t)g * w_group_stride + (size_t)(n0 + r) * K : nullptr;
-        if (DUAL) src[MATS - 1][e] = n0 + r < N ? W2 + (size_t)g * w_group_stride + (size_t)(n0 + r) * K : nullptr;
+    for (int e = 0; e < A_ROWS; ++e) {
+        const int r = row0 + lr + e * STEP;
+        a_src[e] = r < row_end ? A + (size_t)(a_rows ? a_rows[r] : r) * lda : nullptr;
+    }
+#pragma unroll
+    for (int e = 0; e < W_ROWS; ++e) {
+        const int n = n0 + lr + e * STEP;
+        w_src[0][e] = n < N ? W + (size_t)g * w_group_stride + (size_t)n * K : nullptr;
+        if (DUAL) w_src[MATS - 1][e] = n < N ? W2 + (size_t)g * w_group_stride + (size_t)n * K : nullptr;
     }
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(f_smem);
     const int blocks = (K + FK - 1) / FK;
     auto fetch = [&](int b) {
         if (b < blocks) {
             const int k = b * FK + lk;
+            const uint32_t at = base + 4 * ((b % FSTAGES) * STAGE + lr * FLD + lk);
+            auto copy = [&](const float* row, int to_row) {
+                const bool in = row != nullptr && k < K;
+                const float* from = in ? row + k : A;
+                if (WIDE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + 4 * to_row * FLD), "l"(from), "r"(in ? 16 : 0) : "memory");
+                else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + 4 * to_row * FLD), "l"(from), "r"(in ? 4 : 0) : "memory");
+            };
+#pragma unroll
+            for (int e = 0; e < A_ROWS; ++e) copy(a_src[e], e * STEP);
 #pragma unroll
             for (int m = 0; m < MATS; ++m)
 #pragma unroll
-                for (int e = 0; e < ROWS; ++e) {
-                    const bool in = src[m][e] != nullptr && k < K;
-                    const float* from = in ? src[m][e] + k : A;
-                    const uint32_t to = base + 4 * ((b % FSTAGES) * STAGE + m * TILE + (lr + e * STEP) * FLD + lk);
-                    if (WIDE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
-                    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(in ? 4 : 0) : "memory");
-                }
+                for (int e = 0; e < W_ROWS; ++e) copy(w_src[m][e], FM + m * FN + e * STEP);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[4][4] = {}, acc2[DUAL ? 4 : 1][4] = {};
+    // this thread's outputs: rows ty + 4 i, columns tx + 8 j; its k: 16 of each block's 32
+    const int half = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31, tx = (warp & 1) * 32 + (lane & 7), ty = (warp >> 1) * 16 + (lane >> 3);
+    unsigned long long acc[MATS][4][4] = {};
     fetch(0);
     fetch(1);
     for (int b = 0; b < blocks; ++b) {
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();                                     // this block has landed for everyone; the one before it is done with
         fetch(b + 2);
-        const float* As = f_smem + (b % FSTAGES) * STAGE + ty * FLD;
-        const float* Ws = f_smem + (b % FSTAGES) * STAGE + TILE + tx * FLD;
-        const float* Ws2 = Ws + TILE;
+        const float* As = f_smem + (b % FSTAGES) * STAGE + ty * FLD + half * (FK / 2);
+        const float* Ws = f_smem + (b % FSTAGES) * STAGE + (FM + tx) * FLD + half * (FK / 2);
 #pragma unroll
-        for (int k = 0; k < FK; k += 4) {
-            float4 a[4], w[4];
+        for (int k = 0; k < FK / 2; k += 4) {
+            ulonglong2 a[4], w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(As + i * 16 * FLD + k);
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(As + i * 4 * FLD + k);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(Ws + j * 16 * FLD + k);
+            for (int m = 0; m < MATS; ++m) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc[i][j]))));
-            if (DUAL) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(Ws2 + j * 16 * FLD + k);
+                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + (m * FN + j * 8) * FLD + k);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        acc2[DUAL ? i : 0][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc2[DUAL ? i : 0][j]))));
+                    for (int j = 0; j < 4; ++j) fma_pair(acc[m][i][j], a[i].x, w[j].x);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma_pair(acc[m][i][j], a[i].y, w[j].y);
             }
         }
     }
+    // the second half of the threads hands its sums over
+    __syncthreads();
+    float* sums = f_smem + (tid & 127);                      // [matrix, i, j][128 threads]
+    if (half == 1) {
+#pragma unroll
+        for (int e = 0; e < MATS * 16; ++e) sums[e * 128] = sum_pair(acc[e / 16][e / 4 % 4][e % 4]);
+    }
+    __syncthreads();
+    if (half == 1) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = row0 + ty + 16 * i;
+        const int r = row0 + ty + 4 * i;
         if (r >= row_end) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 16 * j;
+            const int n = n0 + tx + 8 * j;
             if (n >= N) continue;
             float* o = out + (size_t)r * ldo + n;
-            const float v = acc[i][j];
+            const float v = sum_pair(acc[0][i][j]) + sums[(i * 4 + j) * 128];
             if (EPI == EPI_STORE) *o = v;
             else if (EPI == EPI_ADD) *o += v;
             else if (EPI == EPI_ACT) *o = q6k_activation(v, act);
-            else *o = act == 0 ? v / (1.0f + expf(-v)) * acc2[DUAL ? i : 0][j] : q6k_gated(v, acc2[DUAL ? i : 0][j], act, act_limit);
+            else {
+                const float up = sum_pair(acc[MATS - 1][i][j]) + sums[(MATS * 16 - 16 + i * 4 + j) * 128];
+                *o = act == 0 ? v / (1.0f + expf(-v)) * up : q6k_gated(v, up, act, act_limit);
+            }
         }
     }
 }
@@ -213,7 +243,8 @@ template <int EPI>
 int launch_f32(dim3 grid, bool wide, cudaStream_t st, const float* A, int lda, const int* a_rows, const float* W, const float* W2, size_t w_group_stride,
                float* out, int ldo, int M, int N, int K, const int* tile_group, const int* tile_row0, const int* group_offsets, const int* num_tiles, int act,
                float act_limit) {
-    const size_t smem = (size_t)FSTAGES * (EPI == EPI_SWIGLU ? 3 : 2) * BM * FLD * sizeof(float);
+    const size_t smem = (size_t)FSTAGES * (FM + (EPI == EPI_SWIGLU ? 2 : 1) * FN) * FLD * sizeof(float);
+    grid.z = BM / FM;
     auto* kernel = wide ? gemm_f32_kernel<EPI, true> : gemm_f32_kernel<EPI, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return q6k_check_launch("gemm_f32: shared memory attribute");
     q6k_launch(kernel, grid, 256, smem, st, A, lda, a_rows, W, W2, w_group_stride, out, ldo, M, N, K, tile_group, tile_row0, group_offsets, num_tiles, act, act_limit);
