@@ -7,28 +7,41 @@ namespace {
 constexpr int WC = 32, WLD = WC + 4;                            // tokens of a chunk; pitch of a row of 32 in shared memory
 constexpr int WALK_THREADS = 256, WALK_COLS = 16;               // threads of a walking block and columns of the state it owns
 
-// Chunk c of all requests' chunks side by side: its first row and its tokens (0: there is no such chunk).
+// Chunk c (of CT tokens) of all requests' chunks side by side: its first row and its tokens (0: there is no such chunk).
+template <int CT = WC>
 __device__ __forceinline__ void chunk_of(const int* q_start, int R, int c, int& first, int& tokens) {
     tokens = 0;
     for (int r = 0; r < R; ++r) {
-        const int n = q_start[r + 1] - q_start[r], chunks = (n + WC - 1) / WC;
+        const int n = q_start[r + 1] - q_start[r], chunks = (n + CT - 1) / CT;
         if (c < chunks) {
-            first = q_start[r] + c * WC;
-            tokens = min(WC, n - c * WC);
+            first = q_start[r] + c * CT;
+            tokens = min(CT, n - c * CT);
             return;
         }
         c -= chunks;
     }
 }
 // The first chunk of request r among all requests' chunks.
+template <int CT = WC>
 __device__ __forceinline__ int first_chunk_of(const int* q_start, int r) {
     int c = 0;
-    for (int x = 0; x < r; ++x) c += (q_start[x + 1] - q_start[x] + WC - 1) / WC;
+    for (int x = 0; x < r; ++x) c += (q_start[x + 1] - q_start[x] + CT - 1) / CT;
     return c;
 }
 __device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc)))); }
 // v with zeros behind its entry n: no value of a later token, were it infinite, reaches an earlier one.
 __device__ __forceinline__ float4 up_to(float4 v, int n) { return make_float4(v.x, n >= 1 ? v.y : 0.0f, n >= 2 ? v.z : 0.0f, n >= 3 ? v.w : 0.0f); }
+// Two FP32 multiply-adds in one instruction; a value in both halves; the halves added.
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long both(float v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "r"(__float_as_uint(v)));
+    return r;
+}
+__device__ __forceinline__ float low(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 // 16 bytes global -> shared without passing registers; !in: zeros (nothing is read from `from`, which has to be an address all the same).
 __device__ __forceinline__ void copy16(uint32_t to, const float* from, bool in) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");

@@ -25,7 +25,7 @@
 //  * time_mix_prep_kernel makes the decays w = exp(-exp(z + w0)) in place and the token's bonus number per head.
 //
 // Everything is FP32: angles, the rotation, decays and their powers, the state and every sum.
-#include "common.cuh"
+#include "chunks.cuh"
 
 namespace {
 
@@ -355,6 +355,233 @@ __global__ void __launch_bounds__(128) time_mix_prep_kernel(const float* r, cons
     if (lane == 0) bonus[row] = sum;
 }
 
+// ---------------------------------------------------------------------------------------- long portions, chunk by chunk
+//
+// The walk above takes 200 ns a token whatever runs beside it.  Over a chunk of C = 64 tokens, with S the state before it and d the head's
+// decay,
+//
+//   O_i = d^(i+1) S^T q_i + sum_(m <= i) M[i][m] v_m,   M[i][m] = d^(i-m) (q_i . k_m);      S <- d^C S + sum_m d^(C-1-m) k_m v_m^T
+//
+// so only a sum of matrices goes from chunk to chunk.  ret_outer_kernel makes every chunk's sum of k v^T, all at once; ret_fold_kernel
+// walks a request's chunks entry by entry and leaves in each one's place the state it starts from; ret_out_kernel makes every
+// chunk's results, [d^(i+1) Q | M] times [S | V] as one product of 64 x 128 outputs whose second factor comes by in slices of 32 rows.
+// FP32 throughout; powers of d are made in double precision.  C = 64: 32 would double the bytes of the states (one per chunk and head).
+// 2,552 tokens in three portions, 16 heads of 128 x 128: 202 us token by token, 41 + 14 + 95 us so.  What bounds the two products: reads of
+// shared memory beside the FP32 pipe, each about half of the time.
+constexpr int RC = 64;
+
+__device__ __forceinline__ float ret_power(float d, int n) {
+    double p = 1.0, x = (double)d;
+    for (; n > 0; n >>= 1, x *= x)
+        if (n & 1) p *= x;
+    return (float)p;
+}
+
+// grid (chunks, H, ceil(dk / 128) ceil(dv / 128)), 256 threads, 64 KB of dynamic shared memory; KV: FP32 [chunks, H, dk, dv].
+__global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const float* vp, int ld, const float* decay, const int* q_start, int R, float* KV, int H, int dk,
+                                                        int dv) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    float *ks = sm, *vs = sm + RC * 128;                    // [64][128] each, k times its token's power of d
+    const int head = blockIdx.y, tid = threadIdx.x, cols = (dv + 127) / 128, row0 = blockIdx.z / cols * 128, col0 = blockIdx.z % cols * 128;
+    int first = 0, n = 0;
+    chunk_of<RC>(q_start, R, blockIdx.x, first, n);
+    if (n == 0) return;
+    const float d = decay[head];
+    const int at = (tid & 31) * 4;
+    float4 k4[8], v4[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int t = (tid >> 5) + 8 * e;
+        const size_t row = (size_t)(first + t) * ld;
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        k4[e] = t < n && row0 + at < dk ? *reinterpret_cast<const float4*>(kp + row + (size_t)head * dk + row0 + at) : zero;
+        v4[e] = t < n && col0 + at < dv ? *reinterpret_cast<const float4*>(vp + row + (size_t)head * dv + col0 + at) : zero;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int t = (tid >> 5) + 8 * e;
+        const float p = ret_power(d, t < n ? n - 1 - t : 0);
+        *reinterpret_cast<float4*>(ks + t * 128 + at) = make_float4(k4[e].x * p, k4[e].y * p, k4[e].z * p, k4[e].w * p);
+        *reinterpret_cast<float4*>(vs + t * 128 + at) = v4[e];
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, row = (warp >> 1) * 32 + (lane >> 3) * 4, col = (warp & 1) * 64 + (lane & 7) * 4;
+    unsigned long long acc[8][4] = {};                      // rows row .. row + 3 and row + 16 .. row + 19; columns col .. and col + 32 ..
+#pragma unroll 2
+    for (int m = 0; m < n; ++m) {
+        const float4 a0 = *reinterpret_cast<const float4*>(ks + m * 128 + row), a1 = *reinterpret_cast<const float4*>(ks + m * 128 + row + 16);
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(vs + m * 128 + col), b1 = *reinterpret_cast<const ulonglong2*>(vs + m * 128 + col + 32);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned long long aa = both(a[i]);
+            fma_pair(acc[i][0], aa, b0.x), fma_pair(acc[i][1], aa, b0.y), fma_pair(acc[i][2], aa, b1.x), fma_pair(acc[i][3], aa, b1.y);
+        }
+    }
+    float* out = KV + ((size_t)blockIdx.x * H + head) * dk * dv;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int rr = row0 + row + (i & 3) + (i >> 2) * 16;
+        if (rr >= dk) continue;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (col0 + col + 32 * j < dv) *reinterpret_cast<ulonglong2*>(out + (size_t)rr * dv + col0 + col + 32 * j) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
+    }
+}
+
+// The state every chunk starts from, in its sum's place, and the state a portion leaves.  grid (R * blocks), blocks = ceil(H dk dv / 1024).
+__global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, const int* slot_ids, int H, int cells) {
+    pdl_enter();
+    const size_t all = (size_t)H * cells;                   // cells = dk dv, a multiple of 4
+    const unsigned blocks = (unsigned)((all + 1023) / 1024);
+    const int r = blockIdx.x / blocks, n = q_start[r + 1] - q_start[r], count = (n + RC - 1) / RC;
+    const size_t i = ((size_t)(blockIdx.x % blocks) * 256 + threadIdx.x) * 4;
+    if (i >= all || n <= 0) return;
+    const float d = decay[i / cells], full = ret_power(d, RC), rest = ret_power(d, n - (count - 1) * RC);
+    float4* mine = reinterpret_cast<float4*>(state + (size_t)slot_ids[r] * all + i);
+    float4 S = *mine;
+    float* at = KV + (size_t)first_chunk_of<RC>(q_start, r) * all + i;
+    for (int c0 = 0; c0 < count; c0 += 4) {
+        float4 built[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c0 + e < count) built[e] = *reinterpret_cast<const float4*>(at + (size_t)(c0 + e) * all);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c0 + e < count) {
+                *reinterpret_cast<float4*>(at + (size_t)(c0 + e) * all) = S;
+                const float p = c0 + e + 1 == count ? rest : full;
+                S = make_float4(fmaf(p, S.x, built[e].x), fmaf(p, S.y, built[e].y), fmaf(p, S.z, built[e].z), fmaf(p, S.w, built[e].w));
+            }
+    }
+    *mine = S;
+}
+
+constexpr int RO_SLICE = 32, RO_STAGES = 3, RO_MLD = RC + 4;
+__host__ __device__ constexpr int ret_out_slices(int dkp) { return RC * (dkp + 4) > RO_STAGES * RO_SLICE * 128 ? RC * (dkp + 4) : RO_STAGES * RO_SLICE * 128; }
+__host__ __device__ constexpr int ret_out_floats(int dkp) { return RC * (dkp + 4) + RC * RO_MLD + ret_out_slices(dkp) + RC + 4; }
+
+// grid (chunks, H, ceil(dv / 128)), 256 threads.  dkp: dk rounded up to a multiple of 32.
+__global__ void __launch_bounds__(256, 2) ret_out_kernel(const float* qp, const float* kp, const float* vp, int ld, const float* decay, const float* KV, const int* q_start,
+                                                         int R, float* o, int H, int dk, int dv, int dkp) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    const int ldq = dkp + 4;
+    float* Q = sm;                                          // [64][ldq]
+    float* M = Q + RC * ldq;                                // [64][68]
+    float* B = M + RC * RO_MLD;                             // K [64][ldq], then the slices [3][32][128] of S and V
+    float* pw = B + ret_out_slices(dkp);                    // [65]
+    const int head = blockIdx.y, col0 = blockIdx.z * 128, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int first = 0, n = 0;
+    chunk_of<RC>(q_start, R, blockIdx.x, first, n);
+    if (n == 0) return;
+    if (tid <= RC) pw[tid] = ret_power(decay[head], tid);
+    for (int t = warp; t < RC; t += 8)
+        for (int d = lane * 4; d < dkp; d += 128) {
+            const bool in = t < n && d < dk;
+            const size_t at = (size_t)(first + (in ? t : 0)) * ld + (size_t)head * dk + (in ? d : 0);
+            copy16((uint32_t)__cvta_generic_to_shared(Q + t * ldq + d), qp + at, in);
+            copy16((uint32_t)__cvta_generic_to_shared(B + t * ldq + d), kp + at, in);
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int row = (warp >> 2) * 32 + (lane >> 3);         // rows row + 4 i
+    {   // M: columns mc and mc + 8
+        const int mc = (warp & 3) * 16 + (lane & 7);
+        unsigned long long acc[8][2] = {};
+#pragma unroll 2
+        for (int d = 0; d < dkp; d += 4) {
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(B + mc * ldq + d), b1 = *reinterpret_cast<const ulonglong2*>(B + (mc + 8) * ldq + d);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(Q + (row + 4 * i) * ldq + d);
+                fma_pair(acc[i][0], a.x, b0.x), fma_pair(acc[i][0], a.y, b0.y);
+                fma_pair(acc[i][1], a.x, b1.x), fma_pair(acc[i][1], a.y, b1.y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int t = row + 4 * i, m = mc + 8 * j;
+                M[t * RO_MLD + m] = m <= t ? pw[t - m] * (low(acc[i][j]) + high(acc[i][j])) : 0.0f;
+            }
+    }
+    __syncthreads();                                        // K is done with, M whole
+    const int state_slices = dkp / RO_SLICE, slices = state_slices + (n + RO_SLICE - 1) / RO_SLICE;
+    const float* S = KV + ((size_t)blockIdx.x * H + head) * dk * dv;
+    auto fetch = [&](int s) {
+        if (s < slices) {
+            const int c = col0 + lane * 4;
+#pragma unroll
+            for (int e = 0; e < RO_SLICE / 8; ++e) {
+                const int rr = warp + 8 * e, x = (s < state_slices ? s : s - state_slices) * RO_SLICE + rr;
+                const bool in = c < dv && x < (s < state_slices ? dk : n);
+                const float* from = s < state_slices ? S + (size_t)x * dv + c : vp + (size_t)(first + x) * ld + (size_t)head * dv + c;
+                copy16((uint32_t)__cvta_generic_to_shared(B + ((s % RO_STAGES) * RO_SLICE + rr) * 128 + lane * 4), in ? from : vp, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    fetch(1);
+    for (int t = warp; t < RC; t += 8)                      // d^(i+1) Q, seen by all at the first slice's barrier
+        for (int d = lane; d < dkp; d += 32) Q[t * ldq + d] *= pw[t + 1];
+    const int col = (warp & 3) * 32 + (lane & 7) * 4;
+    unsigned long long acc[8][2] = {};
+    for (int s = 0; s < slices; ++s) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                    // the slice has landed for everyone; the one before it is done with
+        fetch(s + 2);
+        const float* b = B + (s % RO_STAGES) * RO_SLICE * 128 + col;
+        if (s < state_slices) {
+            const float* a = Q + row * ldq + s * RO_SLICE;
+#pragma unroll 2
+            for (int d = 0; d < RO_SLICE; d += 4) {
+                float4 x[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(a + 4 * i * ldq + d);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(b + (d + e) * 128);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const unsigned long long aa = both(e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w);
+                        fma_pair(acc[i][0], aa, w.x), fma_pair(acc[i][1], aa, w.y);
+                    }
+                }
+            }
+        } else {
+            const int m0 = (s - state_slices) * RO_SLICE;
+            const float* a = M + row * RO_MLD + m0;
+#pragma unroll 1
+            for (int d = 0; d < RO_SLICE; d += 4) {
+                float4 x[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(a + 4 * i * RO_MLD + d);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(b + (d + e) * 128);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (m0 + d + e <= row + 4 * i) {    // no value of a later token, were it infinite, reaches an earlier one
+                            const unsigned long long aa = both(e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w);
+                            fma_pair(acc[i][0], aa, w.x), fma_pair(acc[i][1], aa, w.y);
+                        }
+                }
+            }
+        }
+    }
+    if (col0 + col < dv) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = row + 4 * i;
+            if (t < n) *reinterpret_cast<ulonglong2*>(o + ((size_t)(first + t) * H + head) * dv + col0 + col) = make_ulonglong2(acc[i][0], acc[i][1]);
+        }
+    }
+}
+
 }  // namespace
 
 Q6K_API int q6k_retention_max_dim() { return RET_MAX_DK; }
@@ -392,6 +619,29 @@ Q6K_API int q6k_retention(const float* p, int ld, int q_col, int k_col, int v_co
     else RET_LAUNCH(16);
 #undef RET_LAUNCH
     return q6k_check_launch("retention");
+}
+
+// Floats of scratch for the same walk chunk by chunk.
+Q6K_API long long q6k_retention_chunk_floats(int T_, int R, int H, int dk, int dv) { return (long long)(T_ / RC + R) * H * dk * dv; }
+
+// Chunks of 64 tokens (T_: rows of the step): rows and heads of q, k and v that start on 16 bytes, dk and dv multiples of 4.
+Q6K_API int q6k_retention_chunked(const float* p, int ld, int q_col, int k_col, int v_col, const float* decay, float* chunks, float* state, const int* q_start,
+                                  const int* slot_ids, int T_, int R, float* o, int H, int dk, int dv, cudaStream_t st) {
+    if (R == 0 || T_ == 0) return 0;
+    Q6K_REQUIRE(R > 0 && R <= 65535 && H > 0 && H <= 65535 && dk > 0 && dv > 0 && dk <= RET_MAX_DK, "retention: bad sizes R=%d H=%d dk=%d (at most %d) dv=%d", R, H, dk, RET_MAX_DK, dv);
+    Q6K_REQUIRE(dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0 && (((uintptr_t)p | (uintptr_t)chunks | (uintptr_t)state) & 15) == 0,
+                "retention: chunks take rows and heads that start on 16 bytes");
+    const int n_chunks = T_ / RC + R, cols = (dv + 127) / 128, dkp = (dk + 31) / 32 * 32;
+    const size_t smem1 = (size_t)2 * RC * 128 * sizeof(float), smem2 = (size_t)ret_out_floats(dkp) * sizeof(float);
+    if (cudaFuncSetAttribute(ret_outer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
+        cudaFuncSetAttribute(ret_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess)
+        return q6k_check_launch("retention: shared memory attribute");
+    q6k_launch(ret_outer_kernel, dim3(n_chunks, H, (dk + 127) / 128 * cols), 256, smem1, st, p + k_col, p + v_col, ld, decay, q_start, R, chunks, H, dk, dv);
+    if (int rc = q6k_check_launch("ret_outer")) return rc;
+    q6k_launch(ret_fold_kernel, dim3((unsigned)(R * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, slot_ids, H, dk * dv);
+    if (int rc = q6k_check_launch("ret_fold")) return rc;
+    q6k_launch(ret_out_kernel, dim3(n_chunks, H, cols), 256, smem2, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, o, H, dk, dv, dkp);
+    return q6k_check_launch("ret_out");
 }
 
 // x: [T, D] in the storage type; mu: FP32 [n, D]; prev: FP32 [slots, D]; out: [n, T, D] in the storage type.

@@ -57,7 +57,7 @@ def _need(t: torch.Tensor, name: str, dtype=None, shape=None):
 
 
 # kernels launched per exported function (for launch accounting in benchmarks)
-_LAUNCHES = {"q6k_gated_delta": 1, "q6k_delta_channel": 1, "q6k_retention_chunked": 2, "q6k_attention_flex_mma": 2, "q6k_attention_flex_tc": 2, "q6k_selective_scan": 1, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
+_LAUNCHES = {"q6k_gated_delta": 1, "q6k_delta_channel": 1, "q6k_retention_chunked": 3, "q6k_attention_flex_mma": 2, "q6k_attention_flex_tc": 2, "q6k_selective_scan": 1, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
 launch_count = 0
 
 
@@ -1695,15 +1695,27 @@ def retention_prep(p: torch.Tensor, H: int, dk: int, q_col: int, k_col: int, rot
 
 
 def retention(p: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
-              slot_ids: torch.Tensor, R: int, H: int, dk: int, dv: int) -> torch.Tensor:
+              slot_ids: torch.Tensor, R: int, H: int, dk: int, dv: int, longest: int = 0) -> torch.Tensor:
     """Per request and head, in token order: S <- decay[h] S + k v^T, o = S^T q.  p FP32 [T, N] with q, k (prepared) and v
-    at their columns; state FP32 [slots, H, dk, dv], updated in place; returns o FP32 [T, H dv]."""
+    at their columns; state FP32 [slots, H, dk, dv], updated in place; returns o FP32 [T, H dv].  longest: tokens of the step's
+    longest portion; beyond 64 (the walk token by token takes 200 ns each), rows that start on 16 bytes go 64 tokens at a time, equal up to
+    rounding, if the states of all the chunks take no more than 256 MB."""
     _need(p, "p", torch.float32)
     _need(decay, "decay", torch.float32, (H,))
     _need(state, "state", torch.float32)
     if tuple(state.shape[1:]) != (H, dk, dv) or p.dim() != 2 or max(q_col, k_col) + H * dk > p.shape[1] or v_col + H * dv > p.shape[1]:
         raise KernelError("retention: shapes disagree")
     o = torch.empty((p.shape[0], H * dv), dtype=torch.float32, device=p.device)
+    aligned = dk % 4 == 0 and dv % 4 == 0 and p.stride(0) % 4 == 0 and q_col % 4 == 0 and k_col % 4 == 0 and v_col % 4 == 0
+    if longest > 64 and aligned and p.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
+        lib = library()
+        lib.q6k_retention_chunk_floats.restype = ctypes.c_longlong
+        floats = lib.q6k_retention_chunk_floats(_i(p.shape[0]), _i(R), _i(H), _i(dk), _i(dv))
+        if floats <= 64 << 20:
+            ws = torch.empty(floats, dtype=torch.float32, device=p.device)
+            _call("q6k_retention_chunked", _ptr(p), _i(p.stride(0)), _i(q_col), _i(k_col), _i(v_col), _ptr(decay), _ptr(ws), _ptr(state), _ptr(q_start),
+                  _ptr(slot_ids), _i(p.shape[0]), _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _stream())
+            return o
     _call("q6k_retention", _ptr(p), _i(p.stride(0)), _i(q_col), _i(k_col), _i(v_col), _ptr(decay), _ptr(state), _ptr(q_start), _ptr(slot_ids),
           _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _stream())
     return o
