@@ -394,6 +394,75 @@ __global__ void __launch_bounds__(256) qkv_pages_warp_kernel(const float* qkv, i
     }
 }
 
+__device__ __forceinline__ void store4(float* out, float4 v) { *reinterpret_cast<float4*>(out) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* out, float4 v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+
+// The same again for heads of 16 to 128 entries (powers of two) that fill rows of 128 columns evenly: a warp takes stretches of 128
+// columns, 16 bytes a lane, asks for two of them first, and a head's lanes add its squares among themselves.  The kernel
+// above, which reads 4 bytes a lane and starts a warp per head, took 45 us for 2,113 tokens of 44 heads (18 MB), waiting
+// for its chain of loads; this one takes 20 (16 for 23 where 2,048 tokens have 24 heads of 128).
+constexpr int QR_WARPS = 8, QR_EACH = 2;
+
+// grid (T, ceil(stretches / 16)), 256 threads.
+template <typename T>
+__global__ void __launch_bounds__(QR_WARPS * 32) qkv_rows_kernel(const float* qkv, int ld, int splits, size_t split_stride, int Hq, int Hkv, int Hv, int hd, int vd,
+                                                                 const float* q_norm, const float* k_norm, float eps, const float* inv_freq, int rd,
+                                                                 int neighbours, const int* positions, const int* req_of_token, const int* block_table,
+                                                                 int max_blocks, int page_size, int num_pages, T* q_out, T* k_pages, T* v_pages,
+                                                                 int write_kv, const float* bias, int v_is_k, int v_norm) {
+    pdl_enter();
+    __shared__ float stage[QR_WARPS][128];
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pos = positions[t];
+    const int q_end = Hq * hd / 128, k_end = q_end + (write_kv ? Hkv * hd / 128 : 0), end = k_end + (write_kv ? Hv * vd / 128 : 0);
+    const int page = write_kv ? block_table[(size_t)req_of_token[t] * max_blocks + pos / page_size] : -1;
+    float4 x[QR_EACH];
+#pragma unroll
+    for (int e = 0; e < QR_EACH; ++e) {
+        const int s = blockIdx.y * QR_WARPS * QR_EACH + e * QR_WARPS + warp;
+        const int from = (s < k_end || !v_is_k ? s : s - k_end + q_end) * 128 + lane * 4;       // v_is_k: a value head reads the key head of its number
+        x[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (s >= end) continue;
+        const float* src = qkv + (size_t)t * ld + from;
+        x[e] = *reinterpret_cast<const float4*>(src);
+        for (int i = 1; i < splits; ++i) {
+            const float4 y = *reinterpret_cast<const float4*>(src + i * split_stride);
+            x[e].x += y.x, x[e].y += y.y, x[e].z += y.z, x[e].w += y.w;
+        }
+        if (bias) {
+            const float4 y = *reinterpret_cast<const float4*>(bias + from);
+            x[e].x += y.x, x[e].y += y.y, x[e].z += y.z, x[e].w += y.w;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < QR_EACH; ++e) {
+        const int s = blockIdx.y * QR_WARPS * QR_EACH + e * QR_WARPS + warp;
+        if (s >= end) break;
+        const int kind = s < q_end ? 0 : s < k_end ? 1 : 2, n = kind == 2 ? vd : hd;
+        const int col = (s - (kind == 0 ? 0 : kind == 1 ? q_end : k_end)) * 128 + lane * 4, h = col / n, d = col % n;     // head of its kind, entry in it
+        const float* nw = kind == 0 ? q_norm : kind == 1 ? k_norm : nullptr;
+        if (nw || (kind == 2 && v_norm)) {
+            float ss = fmaf(x[e].w, x[e].w, fmaf(x[e].z, x[e].z, fmaf(x[e].y, x[e].y, x[e].x * x[e].x)));
+            for (int o = n / 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float inv = rsqrtf(ss / (float)n + eps);
+            const float4 w = nw ? make_float4(nw[d], nw[d + 1], nw[d + 2], nw[d + 3]) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+            x[e] = make_float4(x[e].x * inv * w.x, x[e].y * inv * w.y, x[e].z * inv * w.z, x[e].w * inv * w.w);
+        }
+        if (inv_freq && kind != 2 && rd > 0) {
+            *reinterpret_cast<float4*>(&stage[warp][lane * 4]) = x[e];
+            __syncwarp();
+            const float* xs = &stage[warp][lane * 4 - d];
+            x[e] = make_float4(rotated(xs, d, rd, neighbours, pos, inv_freq), rotated(xs, d + 1, rd, neighbours, pos, inv_freq),
+                               rotated(xs, d + 2, rd, neighbours, pos, inv_freq), rotated(xs, d + 3, rd, neighbours, pos, inv_freq));
+            __syncwarp();
+        }
+        if (kind == 0) store4(q_out + ((size_t)t * Hq + h) * hd + d, x[e]);
+        else if (page >= 0) store4((kind == 1 ? k_pages : v_pages) + (((size_t)h * num_pages + page) * page_size + pos % page_size) * n + d, x[e]);
+    }
+}
+
 // The inputs of attention over a cached latent.  x: FP32 [T, ld] = [H query heads of (dim + rd) | latent of `rank` | rd].
 // Block (t, h < H): the head's first `dim` values -> qn[(h T + t) dim] (they go through the key up-projection next), its
 // last rd values, the first `turn` of them rotated -> qr[(h T + t) rd].  Block (t, H): the latent, RMS-normed with weight
@@ -431,7 +500,71 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const float* x, int ld
     for (int d = threadIdx.x; d < rd; d += blockDim.x) dst[rank + d] = from_f32<T>(rotated(xs, d, turn, neighbours, pos, inv_freq));
 }
 
-// src: FP32 [H, T, n] -> out: [T, H n] in the storage type.
+// The same with a block for all of a token's heads, 16 bytes a read (dim, rd and ld multiples of 4), and the sines and cosines of a
+// token's angles made once: a block of 128 threads per (token, head) took 39 us for 2,048 tokens of 16 heads of 128 + 64;
+// this one takes 17.  The second block of a token is the latent's, as above.
+// grid (T, pages ? 2 : 1), 256 threads; dynamic shared memory: cos [turn / 2] | sin [turn / 2] | the rotated parts [H][rd].
+template <typename T>
+__global__ void __launch_bounds__(256) latent_rows_kernel(const float* x, int ld, const float* xc, int ldc, int H, int dim, int rd, int rank, const float* cw, float eps,
+                                                          const float* inv_freq, int turn, int neighbours, const int* positions,
+                                                          const int* req_of_token, const int* block_table, int max_blocks, int page_size,
+                                                          T* qn, T* qr, T* pages, int T_) {
+    pdl_enter();
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float red[32];
+    const int t = blockIdx.x, pos = positions[t], half = turn / 2;
+    float *xs = sm, *cs = sm + (blockIdx.y == 0 ? H : 1) * rd, *sn = cs + half;
+    auto turned = [&](const float* v, int d) {              // rotated() with the angles' table
+        if (d >= turn) return v[d];
+        const int i = neighbours ? d >> 1 : (d < half ? d : d - half);
+        const bool first = neighbours ? !(d & 1) : d < half;
+        const int partner = neighbours ? d ^ 1 : (first ? d + half : d - half);
+        return first ? v[d] * cs[i] - v[partner] * sn[i] : v[d] * cs[i] + v[partner] * sn[i];
+    };
+    for (int i = threadIdx.x; i < half; i += 256) sincosf((float)pos * inv_freq[i], &sn[i], &cs[i]);
+    if (blockIdx.y == 0) {
+        const float* src = x + (size_t)t * ld;
+        const int head4 = (dim + rd) / 4;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < H * head4; i += 256) {
+            const float4 v = *reinterpret_cast<const float4*>(src + 4 * i);
+            const int h = i / head4, d = (i - h * head4) * 4;
+            if (d < dim) store4(qn + ((size_t)h * T_ + t) * dim + d, v);
+            else *reinterpret_cast<float4*>(xs + h * rd + d - dim) = v;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x * 4; i < H * rd; i += 1024) {
+            const int h = i / rd, d = i - h * rd;
+            const float* v = xs + h * rd;
+            store4(qr + ((size_t)h * T_ + t) * rd + d, make_float4(turned(v, d), turned(v, d + 1), turned(v, d + 2), turned(v, d + 3)));
+        }
+        return;
+    }
+    const float* src = xc + (size_t)t * ldc;
+    float ss = 0.0f;
+    for (int d = threadIdx.x; d < rank; d += 256) ss = fmaf(src[d], src[d], ss);
+    for (int d = threadIdx.x; d < rd; d += 256) xs[d] = src[rank + d];
+    const float inv = rsqrtf(block_sum(ss, red) / (float)rank + eps);
+    __syncthreads();
+    const int page = block_table[(size_t)req_of_token[t] * max_blocks + pos / page_size];
+    if (page < 0) return;
+    T* dst = pages + ((size_t)page * page_size + pos % page_size) * (rank + rd);
+    for (int d = threadIdx.x; d < rank; d += 256) dst[d] = from_f32<T>(src[d] * inv * cw[d]);
+    for (int d = threadIdx.x; d < rd; d += 256) dst[rank + d] = from_f32<T>(turned(xs, d));
+}
+
+// src: FP32 [H, T, n] -> out: [T, H n] in the storage type, four values a thread (n4 = n / 4; a value a thread took 19 us for 2,048 rows
+// of 16 x 128, 25 MB; so 6).
+template <typename T>
+__global__ void __launch_bounds__(256) heads_to_rows4_kernel(const float4* src, T* out, int H, int T_, int n4, int total) {
+    pdl_enter();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= total) return;
+    const int th = i / n4, t = th / H, h = th - t * H;
+    store4(out + 4 * (size_t)i, src[((size_t)h * T_ + t) * n4 + (i - th * n4)]);
+}
+
+// The same for any n.
 template <typename T>
 __global__ void heads_to_rows_kernel(const float* src, T* out, int H, int T_, int n) {
     pdl_enter();
@@ -460,6 +593,29 @@ __global__ void __launch_bounds__(128) map_difference_kernel(const float* a, T* 
     }
     const float inv = rsqrtf(warp_sum(ss) / (float)dv + eps) * mult;
     for (int d = lane; d < dv; d += 32) out[(size_t)row * dv + d] = from_f32<T>((a1[d] - lambda * a2[d]) * inv);
+}
+
+// The same, 16 bytes a read (dv a multiple of 4).
+template <typename T>
+__global__ void __launch_bounds__(128) map_difference4_kernel(const float* a, T* out, int rows, int dv, float lambda, float eps, float mult) {
+    pdl_enter();
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const float* a1 = a + (size_t)row * 2 * dv;
+    auto at = [&](int d) {
+        const float4 x = *reinterpret_cast<const float4*>(a1 + d), y = *reinterpret_cast<const float4*>(a1 + dv + d);
+        return make_float4(x.x - lambda * y.x, x.y - lambda * y.y, x.z - lambda * y.z, x.w - lambda * y.w);
+    };
+    float ss = 0.0f;
+    for (int d = lane * 4; d < dv; d += 128) {
+        const float4 o = at(d);
+        ss = fmaf(o.w, o.w, fmaf(o.z, o.z, fmaf(o.y, o.y, fmaf(o.x, o.x, ss))));
+    }
+    const float inv = rsqrtf(warp_sum(ss) / (float)dv + eps) * mult;
+    for (int d = lane * 4; d < dv; d += 128) {
+        const float4 o = at(d);
+        store4(out + (size_t)row * dv + d, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
+    }
 }
 
 // Every head's result times the sigmoid of its number: a [T, H, n] in the storage type, in place; the numbers are columns
@@ -570,6 +726,10 @@ Q6K_API int q6k_map_difference(const float* a, void* out, int T_, int H, int dv,
     Q6K_REQUIRE(T_ > 0 && H > 0 && dv > 0, "map_difference: bad sizes T=%d H=%d dv=%d", T_, H, dv);
     const long long rows = (long long)T_ * H;
     Q6K_REQUIRE(rows <= 0x7fffffffLL, "map_difference: too many rows");
+    if (dv % 4 == 0 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)out & (dtype == Q6K_F32 ? 15 : 7)) == 0) {
+        Q6K_DISPATCH(dtype, q6k_launch(map_difference4_kernel<T>, dim3((unsigned)((rows + 3) / 4)), 128, 0, st, a, (T*)out, (int)rows, dv, lambda, eps, mult););
+        return q6k_check_launch("map_difference");
+    }
     Q6K_DISPATCH(dtype, q6k_launch(map_difference_kernel<T>, dim3((unsigned)((rows + 3) / 4)), 128, 0, st, a, (T*)out, (int)rows, dv, lambda, eps, mult););
     return q6k_check_launch("map_difference");
 }
@@ -626,6 +786,18 @@ Q6K_API int q6k_qkv_pages(const float* qkv, int ld, int splits, long long split_
     Q6K_REQUIRE(heads <= 65535, "qkv_pages: %d heads exceed the grid limit", heads);
     const size_t smem = (size_t)(hd > vd ? hd : vd) * sizeof(float);
     Q6K_REQUIRE(smem <= 48 * 1024, "qkv_pages: heads of %d do not fit shared memory", hd > vd ? hd : vd);
+    const auto fills = [](int n, int count) { return n >= 16 && n <= 128 && (n & (n - 1)) == 0 && (long long)n * count % 128 == 0; };
+    const size_t align = dtype == Q6K_F32 ? 15 : 7;
+    if (fills(hd, Hq) && (!write_kv || (fills(hd, Hkv) && fills(vd, Hv))) && ld % 4 == 0 && split_stride % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)bias) & 15) == 0 &&
+        (((uintptr_t)q_out | (uintptr_t)(write_kv ? k_pages : nullptr) | (uintptr_t)(write_kv ? v_pages : nullptr)) & align) == 0) {
+        const long long stretches = ((long long)Hq * hd + (write_kv ? (long long)Hkv * hd + (long long)Hv * vd : 0)) / 128;
+        if ((stretches + 15) / 16 <= 65535) {
+            Q6K_DISPATCH(dtype, q6k_launch(qkv_rows_kernel<T>, dim3(T_, (unsigned)((stretches + 15) / 16)), QR_WARPS * 32, 0, st, qkv, ld, splits, (size_t)split_stride, Hq, Hkv, Hv,
+                                           hd, vd, q_norm, k_norm, eps, inv_freq, inv_freq ? rotary_dim : 0, neighbours, positions, req_of_token,
+                                           block_table, max_blocks, page_size, num_pages, (T*)q_out, (T*)k_pages, (T*)v_pages, write_kv, bias, v_is_k, v_norm););
+            return q6k_check_launch("qkv_pages");
+        }
+    }
     if (hd <= 256 && vd <= 256 && (heads + 7) / 8 <= 65535) {                 // narrow heads: a warp per head
         Q6K_DISPATCH(dtype, q6k_launch(qkv_pages_warp_kernel<T>, dim3(T_, (heads + 7) / 8), 256, 0, st, qkv, ld, splits, (size_t)split_stride, Hq, Hkv,
                                        hd, vd, q_norm, k_norm, eps, inv_freq, inv_freq ? rotary_dim : 0, neighbours, positions, req_of_token,
@@ -645,7 +817,13 @@ Q6K_API int q6k_latent_prep(const float* x, int ld, const float* xc, int ldc, in
     Q6K_REQUIRE(T_ > 0 && H > 0 && dim > 0 && rd >= 0 && ((rank > 0 && xc) || !pages), "latent_prep: bad sizes T=%d H=%d dim=%d rd=%d rank=%d", T_, H, dim, rd, rank);
     Q6K_REQUIRE(turn >= 0 && turn % 2 == 0 && turn <= rd && (turn == 0 || inv_freq), "latent_prep: %d turning dimensions of %d", turn, rd);
     Q6K_REQUIRE(H + 1 <= 65535 && (!pages || (page_size > 0 && max_blocks > 0 && cw)), "latent_prep: bad grid or pages");
-    const size_t smem = (size_t)(rd > 0 ? rd : 1) * sizeof(float);
+    const size_t smem = (size_t)(rd > 0 ? rd : 1) * sizeof(float), smem_rows = ((size_t)H * rd + turn) * sizeof(float), align = dtype == Q6K_F32 ? 15 : 7;
+    if (dim % 4 == 0 && rd % 4 == 0 && ld % 4 == 0 && ((uintptr_t)x & 15) == 0 && (((uintptr_t)qn | (uintptr_t)qr) & align) == 0 && smem_rows <= 40 * 1024 &&
+        (long long)H * (dim + rd) <= 0x7fffffffLL) {
+        Q6K_DISPATCH(dtype, q6k_launch(latent_rows_kernel<T>, dim3(T_, pages ? 2 : 1), 256, smem_rows, st, x, ld, xc, ldc, H, dim, rd, rank, cw, eps, inv_freq, turn,
+                                       neighbours, positions, req_of_token, block_table, max_blocks, page_size, (T*)qn, (T*)qr, (T*)pages, T_););
+        return q6k_check_launch("latent_prep");
+    }
     Q6K_DISPATCH(dtype, q6k_launch(latent_prep_kernel<T>, dim3(T_, pages ? H + 1 : H), 128, smem, st, x, ld, xc, ldc, H, dim, rd, rank, cw, eps, inv_freq, turn,
                                    neighbours, positions, req_of_token, block_table, max_blocks, page_size, (T*)qn, (T*)qr, (T*)pages, T_););
     return q6k_check_launch("latent_prep");
@@ -654,6 +832,10 @@ Q6K_API int q6k_latent_prep(const float* x, int ld, const float* xc, int ldc, in
 Q6K_API int q6k_heads_to_rows(const float* src, void* out, int H, int T_, int n, int dtype, cudaStream_t st) {
     if (T_ == 0) return 0;
     const size_t total = (size_t)H * T_ * n;
+    if (n % 4 == 0 && total / 4 < 0x7fffff00 && ((uintptr_t)src & 15) == 0 && ((uintptr_t)out & (dtype == Q6K_F32 ? 15 : 7)) == 0) {
+        Q6K_DISPATCH(dtype, q6k_launch(heads_to_rows4_kernel<T>, dim3((unsigned)((total / 4 + 255) / 256)), 256, 0, st, (const float4*)src, (T*)out, H, T_, n / 4, (int)(total / 4)););
+        return q6k_check_launch("heads_to_rows");
+    }
     Q6K_DISPATCH(dtype, q6k_launch(heads_to_rows_kernel<T>, dim3((unsigned)((total + 255) / 256)), 256, 0, st, src, (T*)out, H, T_, n););
     return q6k_check_launch("heads_to_rows");
 }

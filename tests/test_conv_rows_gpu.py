@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("taps, C, dtype", [(4, 516, torch.bfloat16), (3, 8, torch.float32), (2, 1028, torch.float32), (4, 514, torch.float32)])
+@pytest.mark.parametrize("taps, C, dtype", [(4, 516, torch.bfloat16), (3, 8, torch.float32), (2, 1028, torch.float32), (4, 514, torch.float32), (1, 64, torch.float32)])
 def test_the_same_bits_as_token_by_token(taps, C, dtype):
     from quench6k_b200 import ops
     g = torch.Generator().manual_seed(taps * C)
