@@ -23,6 +23,8 @@
 // about 16 a token and state in either launch, and the special-function unit (an exponential each).
 #include "short_conv.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int MAX_TAPS = 16;
@@ -41,7 +43,8 @@ __device__ __forceinline__ float decay_minus_one(float x) {
     p = fmaf(x, p, 1.0f / 6.0f);
     p = fmaf(x, p, 0.5f);
     p = fmaf(x, p, 1.0f);
-    return x > -0.25f ? x * p : (FAST ? __expf(x) : expf(x)) - 1.0f;
+    const float near = x * p, far = (FAST ? __expf(x) : expf(x)) - 1.0f;      // both, so that no warp splits over it
+    return x > -0.25f ? near : far;
 }
 
 // grid (T, ceil(C / 256)); x: FP32 [T, ldx] (first C columns); tail: FP32 [slots, taps-1, C].
@@ -84,6 +87,20 @@ __global__ void __launch_bounds__(256) scan_fold_kernel(float* ws, const float* 
         *at = S;
         S = fmaf(expm1f(dts * a), S, S) + built;
     }
+}
+
+// The last taps - 1 inputs of a channel's convolution: the end of a portion of n tokens, preceded by what is left of the old tail.
+__device__ __forceinline__ void scan_move_tail(float* tl, const float* x, int ldx, int C, int n, int taps) {
+    float keep[MAX_TAPS];
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS; ++j)
+        if (j < taps - 1) {
+            const int src = n - (taps - 1) + j;              // index within the portion
+            keep[j] = src >= 0 ? x[(size_t)src * ldx] : tl[(size_t)(j + n) * C];
+        }
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS; ++j)
+        if (j < taps - 1) tl[(size_t)j * C] = keep[j];
 }
 
 // grid (R, ceil(C / (128 / L)), segments), 128 threads; dynamic shared memory SCAN_TILE * (16 L + 4 * 128 / L) floats.
@@ -188,21 +205,164 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
 #pragma unroll
     for (int k = 0; k < MAX_PER_LANE; ++k)
         if (n0 + k < N) Sg[n0 + k] = S[k];
-    if (sub == 0 && taps > 1) {
-        // the last taps-1 inputs of the convolution: the end of this portion, preceded by what is left of the old tail
-        float* tl = tail + (size_t)slot * (taps - 1) * C + c;
-        float keep[MAX_TAPS];
+    if (sub == 0 && taps > 1) scan_move_tail(tail + (size_t)slot * (taps - 1) * C + c, xz + (size_t)first_req * ldx + c, ldx, C, n_req, taps);
+}
+
+// ---------------------------------------------------------------------------------------- a lane per state, one pass
+//
+// With up to 16 states a channel and enough channels, a portion needs no segments: a lane per state gives 16 C chains (2,048 warps for
+// 4,096 channels), which walk all the tokens once where the segments' two launches compute every decay twice.  A block takes 16
+// channels.  Per tile of 64 tokens its threads make dt, dt u, the gate and the skip of each (token, channel) once, from loads asked for
+// before the tile before was walked; then a lane steps through the tile, reading four tokens' dt, dt u, B and C at a time and leaving
+// S C in shared memory, and every 16 tokens the lanes sum the 16 values of each (token, channel).  The decays of two
+// tokens go through packed instructions.  2,048 tokens, 4,096 channels of 16 states: 171 us against 371 in segments (186 with tiles of 32
+// tokens).  What bounds it: issue slots, two thirds of them taken where four warps share a scheduler, and the chain through a tile's
+// preparation and its two barriers.
+// decay_minus_one of two tokens' dt (FP32, the first in the low half) times a, with packed arithmetic where FAST.
+template <bool FAST>
+__device__ __forceinline__ void decay_minus_one_pair(unsigned long long dt, float a, float* out) {
+    const float d0 = __uint_as_float((uint32_t)dt), d1 = __uint_as_float((uint32_t)(dt >> 32));
+    if (!FAST) {
+        out[0] = decay_minus_one<false>(d0 * a), out[1] = decay_minus_one<false>(d1 * a);
+        return;
+    }
+    auto both = [](float v) {
+        unsigned long long r;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+        return r;
+    };
+    auto mul = [](unsigned long long x, unsigned long long y) {
+        unsigned long long r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+        return r;
+    };
+    auto fma = [](unsigned long long x, unsigned long long y, unsigned long long z) {
+        unsigned long long r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+        return r;
+    };
+    const unsigned long long x = mul(dt, both(a)), y = mul(dt, both(a * 1.44269504088896341f));
+    unsigned long long p = fma(x, both(1.0f / 120.0f), both(1.0f / 24.0f));
+    p = fma(x, p, both(1.0f / 6.0f));
+    p = fma(x, p, both(0.5f));
+    p = mul(x, fma(x, p, both(1.0f)));
+    float e0, e1;                            // beyond e^-87 a decay is zero beside the 1 that is taken from it
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(__uint_as_float((uint32_t)y)));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(__uint_as_float((uint32_t)(y >> 32))));
+    out[0] = __uint_as_float((uint32_t)x) > -0.25f ? __uint_as_float((uint32_t)p) : e0 - 1.0f;
+    out[1] = __uint_as_float((uint32_t)(x >> 32)) > -0.25f ? __uint_as_float((uint32_t)(p >> 32)) : e1 - 1.0f;
+}
+
+constexpr int LS_N = 16, LS_CH = 16, LS_THREADS = LS_N * LS_CH, LS_TILE = 64, LS_LD = LS_TILE + 4;
+
+template <typename T>
+__global__ void __launch_bounds__(LS_THREADS) scan_lanes_kernel(const T* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col,
+                                                                int c_col, const float* A, const float* Dskip, const float* xz, int ldx, int z_col,
+                                                                float* state, float* tail, const int* q_start, const int* slot_ids, T* out, int C, int N,
+                                                                int taps) {
+    pdl_enter();
+    __shared__ __align__(16) float s_dt[LS_CH][LS_LD], s_du[LS_CH][LS_LD], s_gate[LS_CH][LS_LD], s_skip[LS_CH][LS_LD];       // [channel][token]
+    __shared__ __align__(16) float s_bc[2 * LS_N][LS_LD];                    // [state of B, then of C][token]
+    __shared__ __align__(16) float s_y[LS_THREADS / 32][8][68];              // a warp's S C: [pair of tokens][lane][token of it]
+    __shared__ T s_out[LS_TILE][LS_CH];
+    const int r = blockIdx.x, c0 = blockIdx.y * LS_CH, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int first = q_start[r], n_tok = q_start[r + 1] - first;
+    if (n_tok <= 0) return;
+    const int slot = slot_ids[r], cc = tid >> 4, n = tid & 15, c = c0 + cc;
+    const bool has = c < C && n < N;                                         // a state beyond N has A = B = C = 0 and stays zero
+    const float a = has ? A[(size_t)c * N + n] : 0.0f;
+    float S = has ? state[((size_t)slot * C + c) * N + n] : 0.0f;
+    // a thread's share of a tile: four (token, channel) and eight entries of B and C
+    const int pc = tid & 15, pt = tid >> 4, bn = tid & 31, bt = tid >> 5;
+    const bool p_in = c0 + pc < C, b_in = (bn & 15) < N;
+    const float bias = p_in ? dt_bias[c0 + pc] : 0.0f, skip = p_in ? Dskip[c0 + pc] : 0.0f;
+    const int col = bn < LS_N ? b_col + bn : c_col + bn - LS_N;
+    float f_dt[LS_TILE / 16], f_u[LS_TILE / 16], f_z[LS_TILE / 16], f_bc[LS_TILE / 8];
+    auto fetch = [&](int t0) {
 #pragma unroll
-        for (int j = 0; j < MAX_TAPS; ++j) {
-            if (j < taps - 1) {
-                const int src = n_req - (taps - 1) + j;          // index within the portion
-                keep[j] = src >= 0 ? xz[(size_t)(first_req + src) * ldx + c] : tl[(size_t)(j + n_req) * C];
-            }
+        for (int j = 0; j < LS_TILE / 16; ++j) {
+            const int t = t0 + pt + 16 * j;
+            const size_t row = (size_t)(first + t);
+            const bool in = p_in && t < n_tok;
+            f_dt[j] = in ? dt_raw[row * C + c0 + pc] : 0.0f;
+            f_u[j] = in ? to_f32(u[row * C + c0 + pc]) : 0.0f;
+            f_z[j] = in ? xz[row * ldx + z_col + c0 + pc] : 0.0f;
         }
 #pragma unroll
-        for (int j = 0; j < MAX_TAPS; ++j)
-            if (j < taps - 1) tl[(size_t)j * C] = keep[j];
+        for (int j = 0; j < LS_TILE / 8; ++j) {
+            const int t = t0 + bt + 8 * j;
+            f_bc[j] = b_in && t < n_tok ? proj[(size_t)(first + t) * ldp + col] : 0.0f;
+        }
+    };
+    fetch(0);
+    for (int t0 = 0; t0 < n_tok; t0 += LS_TILE) {
+        const int nt = min(LS_TILE, n_tok - t0);
+#pragma unroll
+        for (int j = 0; j < LS_TILE / 16; ++j) {
+            const int t = pt + 16 * j;
+            const float dt = softplus_f(f_dt[j] + bias);
+            s_dt[pc][t] = dt;
+            s_du[pc][t] = dt * f_u[j];
+            s_gate[pc][t] = silu_f(f_z[j]);
+            s_skip[pc][t] = skip * f_u[j];
+        }
+#pragma unroll
+        for (int j = 0; j < LS_TILE / 8; ++j) s_bc[bn][bt + 8 * j] = f_bc[j];
+        __syncthreads();
+        if (t0 + LS_TILE < n_tok) fetch(t0 + LS_TILE);
+#pragma unroll 1
+        for (int g = 0; g < LS_TILE; g += 16) {
+            if (g >= nt) break;
+            auto walk = [&](auto whole) {                    // whole: 16 tokens; else the nt - g that there are
+#pragma unroll
+                for (int q = 0; q < 16; q += 4) {
+                    const ulonglong2 dt4 = *reinterpret_cast<const ulonglong2*>(&s_dt[cc][g + q]);
+                    const float4 du4 = *reinterpret_cast<const float4*>(&s_du[cc][g + q]), b4 = *reinterpret_cast<const float4*>(&s_bc[n][g + q]);
+                    const float4 c4 = *reinterpret_cast<const float4*>(&s_bc[LS_N + n][g + q]);
+                    const float du_[4] = {du4.x, du4.y, du4.z, du4.w}, b_[4] = {b4.x, b4.y, b4.z, b4.w};
+                    float SS[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e += 2) {
+                        float near_one[2];
+                        decay_minus_one_pair<sizeof(T) == 2>(e ? dt4.y : dt4.x, a, near_one);
+#pragma unroll
+                        for (int f = 0; f < 2; ++f) {
+                            // exp(dt A) S as S + expm1(dt A) S, as above
+                            const float next = fmaf(du_[e + f], b_[e + f], fmaf(near_one[f], S, S));
+                            if (decltype(whole)::value || g + q + e + f < nt) S = next;
+                            SS[e + f] = S;
+                        }
+                    }
+                    *reinterpret_cast<float2*>(&s_y[warp][q / 2][lane * 2]) = make_float2(SS[0] * c4.x, SS[1] * c4.y);
+                    *reinterpret_cast<float2*>(&s_y[warp][q / 2 + 1][lane * 2]) = make_float2(SS[2] * c4.z, SS[3] * c4.w);
+                }
+            };
+            if (g + 16 <= nt) walk(std::true_type{});
+            else walk(std::false_type{});
+            __syncwarp();
+            // a lane adds eight states' values of two tokens, then takes the other eight's sum of one of them from the lane 16 away
+            const int pair = lane & 7, ch = (lane >> 3) & 1, part = lane >> 4;
+            const float4* p = reinterpret_cast<const float4*>(&s_y[warp][pair][ch * 32 + part * 16]);
+            float y0 = 0.0f, y1 = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 v = p[k];
+                y0 += v.x, y1 += v.y, y0 += v.z, y1 += v.w;
+            }
+            const float other = __shfl_xor_sync(0xffffffffu, part ? y0 : y1, 16), y = (part ? y1 : y0) + other;
+            const int tok = g + 2 * pair + part, c_at = 2 * warp + ch;
+            s_out[tok][c_at] = from_f32<T>((y + s_skip[c_at][tok]) * s_gate[c_at][tok]);
+            __syncwarp();
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < LS_TILE / 16; ++j) {
+            const int t = pt + 16 * j;
+            if (p_in && t < nt) out[(size_t)(first + t0 + t) * C + c0 + pc] = s_out[t][pc];
+        }
     }
+    if (has) state[((size_t)slot * C + c) * N + n] = S;
+    if (c < C && n == 0 && taps > 1) scan_move_tail(tail + (size_t)slot * (taps - 1) * C + c, xz + (size_t)first * ldx + c, ldx, C, n_tok, taps);
 }
 
 template <typename T>
@@ -247,6 +407,16 @@ Q6K_API int q6k_selective_scan_lanes(int N) {
 // Tokens per segment when a portion is walked by several blocks.
 Q6K_API int q6k_selective_scan_segment() { return 64; }
 
+// Whether a step of T_ rows whose longest portion has up to `segments` segments goes a lane per state in one pass.  More than 16 states
+// take more lanes; fewer than 9 leave half of them idle.  A chain takes about 35 clocks a token however few there are; the segments'
+// launches take their 30 instructions per token and state, spread over the chip: with 592 schedulers the lines meet where the tokens of all
+// requests bring 24,000 chains for each token of the longest (65,536 chains: 171 against 371 us).  Without segments (up to 64 tokens) a walk of eight states a lane
+// is slower from a few tokens on; a step of single tokens keeps it (nothing to fetch ahead).
+Q6K_API int q6k_selective_scan_lanes_taken(int T_, int R, int C, int N, int segments) {
+    if (N <= 8 || N > LS_N || T_ < 8 * R) return 0;
+    return segments <= 1 || (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 24000;
+}
+
 // Floats of scratch for `seg_slots` segments in all and R requests.
 Q6K_API long long q6k_selective_scan_workspace(int seg_slots, int R, int C, int N) { return R > 0 ? (long long)seg_slots * C * (N + 1) : 0; }
 
@@ -255,7 +425,7 @@ Q6K_API long long q6k_selective_scan_workspace(int seg_slots, int R, int C, int 
 Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col, int c_col,
                                const float* A, const float* Dskip, const float* xz, int ldx, int z_col, float* state, float* tail,
                                const int* q_start, const int* slot_ids, void* out, int R, int C, int N, int taps, int dtype,
-                               int segments, const int* seg_base, int seg_slots, float* ws, cudaStream_t st) {
+                               int segments, const int* seg_base, int seg_slots, float* ws, int T_, cudaStream_t st) {
     if (R == 0) return 0;
     const int L = q6k_selective_scan_lanes(N);
     Q6K_REQUIRE(R > 0 && C > 0 && N > 0 && N <= L * MAX_PER_LANE, "selective_scan: bad sizes R=%d C=%d N=%d (at most %d states)", R, C, N,
@@ -264,6 +434,11 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
     const int per_block = 128 / L;
     dim3 grid(R, (C + per_block - 1) / per_block);
     Q6K_REQUIRE(grid.y <= 65535, "selective_scan: %d channels exceed the grid limit", C);
+    if (q6k_selective_scan_lanes_taken(T_, R, C, N, segments)) {
+        Q6K_DISPATCH(dtype, q6k_launch(scan_lanes_kernel<T>, dim3(R, (C + LS_CH - 1) / LS_CH), LS_THREADS, 0, st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
+                                       A, Dskip, xz, ldx, z_col, state, tail, q_start, slot_ids, (T*)out, C, N, taps););
+        return q6k_check_launch("selective_scan (lanes)");
+    }
     const size_t smem = (size_t)SCAN_TILE * (2 * L * MAX_PER_LANE + 4 * per_block) * sizeof(float);
     const int seg_len = q6k_selective_scan_segment();
 #define SCAN_LAUNCH(MODE, GRID)                                                                                                      \

@@ -1167,10 +1167,11 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
         most, seg_base, slots = segments
         lib = library()
         lib.q6k_selective_scan_workspace.restype = ctypes.c_longlong
-        ws = _workspace(4 * lib.q6k_selective_scan_workspace(_i(slots), _i(R), _i(C), _i(N)), u.device, "scan")
+        if not lib.q6k_selective_scan_lanes_taken(_i(T), _i(R), _i(C), _i(N), _i(most)):
+            ws = _workspace(4 * lib.q6k_selective_scan_workspace(_i(slots), _i(R), _i(C), _i(N)), u.device, "scan")
     _call("q6k_selective_scan", _ptr(u), _ptr(dt_raw), _ptr(dt_bias), _ptr(proj), _i(proj.stride(0)), _i(b_col), _i(c_col), _ptr(A), _ptr(D),
           _ptr(xz), _i(xz.stride(0)), _i(z_col), _ptr(state), _ptr(tail), _ptr(q_start), _ptr(slot_ids), _ptr(out), _i(R), _i(C), _i(N),
-          _i(taps), _i(dtype_code(u.dtype)), _i(most), _ptr(seg_base), _i(slots), _ptr(ws), _stream())
+          _i(taps), _i(dtype_code(u.dtype)), _i(most), _ptr(seg_base), _i(slots), _ptr(ws), _i(T), _stream())
     return out
 
 

@@ -1,0 +1,39 @@
+"""The selective scan with a lane per state, in one pass, against float64 and against the walk of eight states a lane (which a step of
+fewer than eight tokens per request keeps), at the edges of its tiles (32 tokens, 16 channels) and for state sizes below 16."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("C, N, taps, dtype, lens", [(40, 16, 4, torch.bfloat16, [33, 1, 32, 97]), (19, 9, 2, torch.float32, [64, 31, 2]),
+                                                     (1600, 16, 4, torch.bfloat16, [129]), (16, 12, 1, torch.float32, [16, 48])])
+def test_lanes_against_float64(C, N, taps, dtype, lens):
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(C + N)
+    T, R = sum(lens), len(lens)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    starts, slots = [sum(lens[:i]) for i in range(R + 1)], list(range(R, 0, -1))
+    u, dt_raw, dt_b, proj = rnd(T, C).to(dtype), rnd(T, C) * 0.5 - 2, rnd(C) * 0.5, rnd(T, 2 * N + 5)
+    A, D, xz = -torch.exp(rnd(C, N)), rnd(C), rnd(T, 2 * C)
+    state, tail = rnd(R + 1, C, N), rnd(R + 1, taps - 1, C)
+    assert ops.library().q6k_selective_scan_lanes_taken(T, R, C, N, 1) == 1 and ops.library().q6k_selective_scan_lanes_taken(1, 1, C, N, 1) == 0
+    s1, t1 = state.clone(), tail.clone()
+    got = ops.selective_scan(u, dt_raw, dt_b, proj, 5, 5 + N, A, D, xz, C, s1, t1, i32(starts), i32(slots), R)
+    s2, t2, walked = state.clone(), tail.clone(), []
+    for r, n in enumerate(lens):
+        for t in range(starts[r], starts[r] + n):
+            walked.append(ops.selective_scan(u[t:t + 1], dt_raw[t:t + 1], dt_b, proj[t:t + 1], 5, 5 + N, A, D, xz[t:t + 1], C, s2, t2, i32([0, 1]), i32([slots[r]]), 1))
+    walked = torch.cat(walked)
+    d = lambda x: x.double()
+    dt = torch.nn.functional.softplus(d(dt_raw) + d(dt_b))
+    want, S = torch.zeros(T, C, dtype=torch.float64, device="cuda"), d(state)
+    for r, n in enumerate(lens):
+        for t in range(starts[r], starts[r] + n):
+            S[slots[r]] = torch.exp(dt[t][:, None] * d(A)) * S[slots[r]] + (dt[t] * d(u[t]))[:, None] * d(proj[t, 5:5 + N])
+            want[t] = (S[slots[r]] @ d(proj[t, 5 + N:5 + 2 * N]) + d(D) * d(u[t])) * torch.nn.functional.silu(d(xz[t, C:]))
+    far = lambda x, y: float((d(x) - y).norm() / y.norm())
+    # the same products in the same order over time; a token's 16 are added in another order
+    assert far(s1, S) <= 1.01 * far(s2, S) + 1e-8 and torch.equal(t1, t2)
+    assert far(got, want) <= 1.05 * far(walked, want) + 1e-7
