@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float*
 // summed and subtracted in double precision).  delta_walk_kernel takes the chunks in order: five small FP32 products a chunk, a
 // block per (request, head, 16 columns), the next chunk's K, Q, inverse and M on their way meanwhile, S in registers with a copy in
 // shared memory for the products that read it.  C = 32: a chunk of 64 would double the triangular work and the bytes of the two
-// matrices per token.  15 + 237 us.  What bounds it: the FP32 pipe
+// matrices per token.  15 + 227 us.  What bounds it: the FP32 pipe
 // (3 x dk x 16 multiply-adds a token and block), its reads of shared memory and four barriers a chunk.
 constexpr int CHUNK_FLOATS = 2 * WC * WC + 3 * WC;              // per (chunk, head): inverse, M, beta, P, P_C / P_m
 
@@ -461,21 +461,23 @@ __global__ void __launch_bounds__(128) delta_chunk_kernel(const float* u, int ld
     }
 }
 
+constexpr int XY_LD = WALK_COLS + 4;
 __host__ __device__ constexpr int walk_stage_floats(int dkp) { return 2 * WC * (dkp + 4) + 2 * WC * WLD + 3 * WC + WC * WALK_COLS; }
-__host__ __device__ constexpr int walk_floats(int dkp) { return 2 * walk_stage_floats(dkp) + WALK_COLS * (dkp + 4) + 2 * WC * (WALK_COLS + 4) + 3 * WALK_COLS * WLD; }
+__host__ __device__ constexpr int walk_floats(int dkp) { return 2 * walk_stage_floats(dkp) + WALK_COLS * (dkp + 4) + 9 * WC * XY_LD + 3 * WALK_COLS * WLD; }
 
-// grid (H * ceil(dv / 16), R), 256 threads.  dkp: dk rounded up to a multiple of 8.  GROUPS: ceil(dkp / 128), groups of four rows of the
+// grid (H * ceil(dv / 16), R), 256 threads.  dkp: dk rounded up to a multiple of 16.  GROUPS: ceil(dkp / 128), groups of four rows of the
 // state a thread holds.
 template <int GROUPS>
-__global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(const float* u, int ldu, const float* chunks, float* state, const int* q_start,
+__global__ void __launch_bounds__(WALK_THREADS, 1) delta_walk_kernel(const float* u, int ldu, const float* chunks, float* state, const int* q_start,
                                                                   const int* slot_ids, float* o, int H, int G, int dk, int dv, int dkp) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int ld = dkp + 4, stage = walk_stage_floats(dkp);
     // a stage: K [WC][ld] | Q [WC][ld] | inverse [WC][WLD] | M [WC][WLD] | beta, P, P_C / P_m [3][WC] | V [WC][16]
     float* S = sm + 2 * stage;                          // [16][ld]: a column's rows side by side
-    float* xy = S + WALK_COLS * ld;                     // [2][WC][20]: half sums of K S and Q S on their way between the halves, then P (Q S)
-    float* rt = xy + 2 * WC * (WALK_COLS + 4);          // [16][WLD]: right-hand sides, a column's tokens side by side
+    float* xy = S + WALK_COLS * ld;                     // [4][K, Q][WC][20]: quarters of K S and Q S
+    float* qs = xy + 8 * WC * XY_LD;                    // [WC][20]: P (Q S)
+    float* rt = qs + WC * XY_LD;                        // [16][WLD]: right-hand sides, a column's tokens side by side
     float* ut = rt + WALK_COLS * WLD;                   // [16][WLD]: U
     float* uw = ut + WALK_COLS * WLD;                   // [16][WLD]: U times P_C / P_m
     const int col_blocks = (dv + WALK_COLS - 1) / WALK_COLS, head = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * WALK_COLS, r = blockIdx.y;
@@ -524,41 +526,40 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(const float* u
         fetch(c + 1);
         const float* K = sm + (c & 1) * stage;
         const float *inv = K + 2 * WC * ld, *M = inv + WC * WLD, *beta = M + WC * WLD, *P = beta + WC, *E = P + WC, *V = E + WC;
-        {   // K S and Q S: rows row + 8 i of K (y 0) or Q (y 1), columns tx and tx + 8, half of the sum each
-            const int half = tid >> 7, y = (tid >> 6) & 1, row = (tid >> 3) & 7;
-            const float *a = K + (size_t)(y * WC + row) * ld + half * (dkp / 2), *b = S + tx * ld + half * (dkp / 2);
-            float acc[4][2] = {};
-#pragma unroll 4
-            for (int d = 0; d < dkp / 2; d += 4) {
-                const float4 b0 = *reinterpret_cast<const float4*>(b + d), b1 = *reinterpret_cast<const float4*>(b + 8 * ld + d);
+        {   // K S and Q S: rows row + 16 i of K and Q (one below the other), columns tc + 4 j, a quarter of the sum each: 8 reads for 64 products
+            const int quarter = tid >> 6, row = (tid >> 2) & 15, tc = tid & 3;
+            const float *a = K + (size_t)row * ld + quarter * (dkp / 4), *b = S + tc * ld + quarter * (dkp / 4);
+            float acc[4][4] = {};
+#pragma unroll 2
+            for (int d = 0; d < dkp / 4; d += 4) {
+                float4 y[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) y[j] = *reinterpret_cast<const float4*>(b + j * 4 * ld + d);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float4 x = *reinterpret_cast<const float4*>(a + i * 8 * ld + d);
-                    acc[i][0] = dot4(x, b0, acc[i][0]);
-                    acc[i][1] = dot4(x, b1, acc[i][1]);
+                    const float4 x = *reinterpret_cast<const float4*>(a + i * 16 * ld + d);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = dot4(x, y[j], acc[i][j]);
                 }
             }
-            // the first half of the threads finishes K S, the second Q S
-            if (half != y) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(xy + (quarter * 2 * WC + row + 16 * i) * XY_LD + tc * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+        __syncthreads();
+        {   // the quarters added: row tid / 4, columns tc + 4 j
+            const int row = tid >> 2, tc = tid & 3, t = row & (WC - 1);
+            float sum[4] = {};
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) xy[(y * WC + row + 8 * i) * (WALK_COLS + 4) + tx + 8 * j] = acc[i][j];
+            for (int e = 0; e < 4; ++e) {
+                const float4 v = *reinterpret_cast<const float4*>(xy + (e * 2 * WC + row) * XY_LD + tc * 4);
+                sum[0] += v.x, sum[1] += v.y, sum[2] += v.z, sum[3] += v.w;
             }
-            __syncthreads();
-            if (half == y) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int t = row + 8 * i;
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const int col = tx + 8 * j;
-                        float* at = xy + (y * WC + t) * (WALK_COLS + 4) + col;
-                        const float sum = (*at + acc[i][j]) * P[t];
-                        if (y == 0) rt[col * WLD + t] = beta[t] * (V[t * WALK_COLS + col] - sum);
-                        else *at = sum;
-                    }
-                }
+            for (int j = 0; j < 4; ++j) {
+                const int col = tc + 4 * j;
+                if (row < WC) rt[col * WLD + t] = beta[t] * (V[t * WALK_COLS + col] - sum[j] * P[t]);
+                else qs[t * XY_LD + col] = sum[j] * P[t];
             }
         }
         __syncthreads();
@@ -580,7 +581,7 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(const float* u
         }
         __syncthreads();
         {
-            float acc[2] = {xy[(WC + t) * (WALK_COLS + 4) + tx], xy[(WC + t) * (WALK_COLS + 4) + tx + 8]};
+            float acc[2] = {qs[t * XY_LD + tx], qs[t * XY_LD + tx + 8]};
             triangle(M, ut, acc);
             if (c * WC + t < n) {
                 float* dst = o + (size_t)(first + c * WC + t) * H * dv + head * dv + col0;
@@ -750,7 +751,7 @@ Q6K_API int q6k_gated_delta(float* u, int ldu, const float* p, int ldp, int b_co
         if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return q6k_check_launch("delta_chunk: shared memory attribute");
         q6k_launch(delta_chunk_kernel, dim3(T_ / WC + R, G), 128, smem1, st, u, ldu, bg, q_start, R, chunks, H, G, dk);
         if (int rc = q6k_check_launch("delta_chunk")) return rc;
-        const int dkp = (dk + 7) / 8 * 8;
+        const int dkp = (dk + 15) / 16 * 16;
         const size_t smem2 = (size_t)walk_floats(dkp) * sizeof(float);
         auto* walk = dkp <= 128 ? delta_walk_kernel<1> : delta_walk_kernel<2>;
         if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess) return q6k_check_launch("delta_walk: shared memory attribute");
