@@ -665,6 +665,37 @@ __global__ void __launch_bounds__(128) delta_out_kernel(const float* o, const fl
     for (int i = lane; i < dv; i += 32) dst[i] = from_f32<T>(orow[i] * inv * w[i] * gate_f(grow[i], gate));
 }
 
+// The same 16 bytes at a time, for heads of up to 256 that are multiples of 4 and start on 16 bytes: 13 us for 2,048 tokens of 16 heads
+// of 128 four bytes at a time, 11 so.
+template <typename T>
+__global__ void __launch_bounds__(128) delta_out4_kernel(const float* o, const float* p, int ldp, int g_col, const float* w, int w_stride, float eps, T* out,
+                                                         int H, int dv, int gate) {
+    pdl_enter();
+    const int t = blockIdx.x, head = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (head >= H) return;
+    const size_t at = ((size_t)t * H + head) * dv;
+    const float* grow = p + (size_t)t * ldp + g_col + head * dv;
+    w += (size_t)head * w_stride;
+    float4 v[2], g[2], ww[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = lane * 4 + 128 * j;
+        v[j] = g[j] = ww[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < dv) v[j] = *reinterpret_cast<const float4*>(o + at + i), g[j] = *reinterpret_cast<const float4*>(grow + i), ww[j] = *reinterpret_cast<const float4*>(w + i);
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) ss = dot4(v[j], v[j], ss);
+    const float inv = rsqrtf(warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = lane * 4 + 128 * j;
+        if (i < dv)
+            conv_store(out + at + i, make_float4(v[j].x * inv * ww[j].x * gate_f(g[j].x, gate), v[j].y * inv * ww[j].y * gate_f(g[j].y, gate),
+                                                 v[j].z * inv * ww[j].z * gate_f(g[j].z, gate), v[j].w * inv * ww[j].w * gate_f(g[j].w, gate)));
+    }
+}
+
 // The same for ONE wide head (all heads' values normed together): a block per token, the row's values kept in registers
 // between the sum of squares and the products (up to 16 a thread), read again beyond that.
 template <typename T>
@@ -785,6 +816,11 @@ Q6K_API int q6k_delta_out(const float* o, const float* p, int ldp, int g_col, co
     Q6K_REQUIRE((H + 3) / 4 <= 65535, "delta_out: %d heads exceed the grid limit", H);
     if (H == 1 && dv > 256) {                 // one wide head: a block per token
         Q6K_DISPATCH(dtype, q6k_launch(delta_out_row_kernel<T>, dim3(T_), 256, 0, st, o, p, ldp, g_col, w, eps, (T*)out, dv, gate););
+        return q6k_check_launch("delta_out");
+    }
+    if (dv <= 256 && dv % 4 == 0 && ldp % 4 == 0 && g_col % 4 == 0 && w_stride % 4 == 0 && (((uintptr_t)o | (uintptr_t)p | (uintptr_t)w) & 15) == 0 &&
+        ((uintptr_t)out & (dtype == Q6K_F32 ? 15 : 7)) == 0) {
+        Q6K_DISPATCH(dtype, q6k_launch(delta_out4_kernel<T>, dim3(T_, (H + 3) / 4), 128, 0, st, o, p, ldp, g_col, w, w_stride, eps, (T*)out, H, dv, gate););
         return q6k_check_launch("delta_out");
     }
     Q6K_DISPATCH(dtype, q6k_launch(delta_out_kernel<T>, dim3(T_, (H + 3) / 4), 128, 0, st, o, p, ldp, g_col, w, w_stride, eps, (T*)out, H, dv, gate););

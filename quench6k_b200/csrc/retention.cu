@@ -65,6 +65,50 @@ __global__ void __launch_bounds__(256) retention_prep_kernel(float* p, int ld, i
     }
 }
 
+// The same for halves that pair up 16 bytes at a time (rd / 2 a multiple of 4, rows and heads on 16 bytes, no activation before it): a
+// thread asks for two pairs before the angles are made.  26 us for 2,552 tokens of 16 heads of 128, 84 MB, four bytes at a time;
+// this one takes 14.
+__global__ void __launch_bounds__(256) retention_turn4_kernel(float* p, int ld, int H, int dk, int q_col, int k_col, const float* inv_freq, int rd, float k_scale,
+                                                              const int* positions) {
+    pdl_enter();
+    extern __shared__ __align__(16) float xs[];            // cos [rd / 2] | sin [rd / 2]
+    const int t = blockIdx.x, half = rd / 2, half4 = half / 4, all = 2 * H * half4;
+    float* row = p + (size_t)t * ld;
+    auto at = [&](int w) { return row + (w >= all / 2 ? k_col : q_col) + (size_t)(w / half4 % H) * dk + w % half4 * 4; };      // (q or k, head, four pairs)
+    bool made = false;
+    for (int w0 = threadIdx.x; w0 < all || !made; w0 += 512) {
+        float4 u[2], v[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (w0 + 256 * e < all) {
+                const float* x = at(w0 + 256 * e);
+                u[e] = *reinterpret_cast<const float4*>(x), v[e] = *reinterpret_cast<const float4*>(x + half);
+            }
+        if (!made) {
+            const float pos = (float)positions[t];
+            for (int i = threadIdx.x; i < half; i += 256) sincosf(pos * inv_freq[i], &xs[half + i], &xs[i]);
+            __syncthreads();
+            made = true;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (w0 + 256 * e < all) {
+                float* x = at(w0 + 256 * e);
+                const int i = (w0 + 256 * e) % half4 * 4;
+                const float mul = w0 + 256 * e >= all / 2 ? k_scale : 1.0f;
+                const float4 c = *reinterpret_cast<const float4*>(xs + i), s = *reinterpret_cast<const float4*>(xs + half + i);
+                *reinterpret_cast<float4*>(x) = make_float4((u[e].x * c.x - v[e].x * s.x) * mul, (u[e].y * c.y - v[e].y * s.y) * mul,
+                                                            (u[e].z * c.z - v[e].z * s.z) * mul, (u[e].w * c.w - v[e].w * s.w) * mul);
+                *reinterpret_cast<float4*>(x + half) = make_float4((v[e].x * c.x + u[e].x * s.x) * mul, (v[e].y * c.y + u[e].y * s.y) * mul,
+                                                                   (v[e].z * c.z + u[e].z * s.z) * mul, (v[e].w * c.w + u[e].w * s.w) * mul);
+            }
+    }
+    if (k_scale != 1.0f) {
+        const int rest = dk - rd;
+        for (int w = threadIdx.x; w < H * rest; w += 256) row[k_col + (size_t)(w / rest) * dk + rd + w % rest] *= k_scale;
+    }
+}
+
 // Four bytes from global to shared memory without passing registers; `in` false writes a zero and reads nothing.
 __device__ __forceinline__ void ret_copy(float* dst, const float* src, bool in) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -595,6 +639,10 @@ Q6K_API int q6k_retention_prep(float* p, int ld, int T_, int H, int dk, int q_co
     Q6K_REQUIRE(rd >= 0 && rd % 2 == 0 && rd <= dk && (rd == 0 || inv_freq), "retention_prep: %d turning dimensions of %d", rd, dk);
     Q6K_REQUIRE(act_cols >= 0 && act_cols <= ld, "retention_prep: %d activated columns of %d", act_cols, ld);
     if (rd == 0 && k_scale == 1.0f && act_cols == 0) return 0;
+    if (rd > 0 && rd % 8 == 0 && !neighbours && act_cols == 0 && dk % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && ((uintptr_t)p & 15) == 0) {
+        q6k_launch(retention_turn4_kernel, dim3(T_), 256, (size_t)rd * sizeof(float), st, p, ld, H, dk, q_col, k_col, inv_freq, rd, k_scale, positions);
+        return q6k_check_launch("retention_prep");
+    }
     q6k_launch(retention_prep_kernel, dim3(T_), 256, (size_t)rd * sizeof(float), st, p, ld, H, dk, q_col, k_col,
                inv_freq, rd, neighbours, k_scale, positions, act_cols);
     return q6k_check_launch("retention_prep");

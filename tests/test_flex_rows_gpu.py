@@ -62,3 +62,22 @@ def test_latent_rows_against_a_block_per_head(H, dim, rd, rank, turn, near, writ
     assert torch.allclose(one.float(), other.float(), rtol=2.0 ** -7, atol=1e-6)
     src = torch.randn(H * T, dim, generator=g).cuda()
     assert torch.equal(ops.heads_to_rows(_at(src, True), H, torch.bfloat16), ops.heads_to_rows(_at(src, False), H, torch.bfloat16))
+
+
+@pytest.mark.parametrize("H, dk, rd, scale, dv", [(16, 128, 128, 0.3, 128), (3, 24, 8, 1.0, 20), (40, 64, 32, 0.5, 256), (1, 8, 8, 2.0, 4)])
+def test_recurrent_rows_against_four_bytes_at_a_time(H, dk, rd, scale, dv):
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(H * dk + dv)
+    T, width = 7, 4 + 2 * H * dk + H * dv
+    p, o, w = (torch.randn(*s, generator=g).cuda() for s in ((T, width), (T, H * dv), (dv,)))
+    rot = (torch.rand(rd // 2, generator=g).cuda(), rd, False)
+    pos = torch.arange(11, 11 + T, dtype=torch.int32, device="cuda")
+    turned = []
+    for aligned in (True, False):
+        x = _at(p, aligned)
+        ops.retention_prep(x, H, dk, 4, 4 + H * dk, rot, scale, pos)
+        turned.append(x)
+    assert torch.allclose(*turned, rtol=1e-6, atol=1e-6 * float(p.abs().max()))          # the same products; their sums may be contracted otherwise
+    for dtype in (torch.bfloat16, torch.float32):
+        one, other = (ops.delta_out(_at(o, a), _at(p, a), 4 + 2 * H * dk, _at(w, a), 1e-6, H, dv, dtype) for a in (True, False))
+        assert torch.allclose(one.float(), other.float(), rtol=2.0 ** -7 if dtype == torch.bfloat16 else 1e-6, atol=1e-6)       # squares in another order
