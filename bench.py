@@ -233,7 +233,8 @@ def kernel_gated_delta(args):
     A_log, dt_bias = torch.randn(H, device=dev) - 3.0, torch.randn(H, device=dev)
     state = torch.zeros(R, H, dv, dk, device=dev)
     q_start, slots = i32([i * n for i in range(R + 1)]), i32(list(range(R)))
-    run = lambda: ops.gated_delta(u.clone() if not decode else u, p, 0, H, A_log, dt_bias, state, q_start, slots, R, H, G, dk, dv, prepare=n > 16)
+    run = lambda: ops.gated_delta(u.clone() if not decode else u, p, 0, H, A_log, dt_bias, state, q_start, slots, R, H, G, dk, dv, prepare=n > 16,
+                                  chunked=n > 16 and ops.gated_delta_chunks(n, G, H, dk, dv))
     for _ in range(max(3, args.warmup)):
         run()
     torch.cuda.synchronize()
@@ -267,7 +268,7 @@ def kernel_retention(args):
     decay = 1.0 - 2.0 ** (-5.0 - 5.0 * torch.arange(H, device=dev, dtype=torch.float32) / H)
     state = torch.zeros(R, H, dk, dv, device=dev)
     q_start, slots = i32([i * n for i in range(R + 1)]), i32(list(range(R)))
-    run = lambda: ops.retention(p, 0, H * dk, 2 * H * dk, decay, state, q_start, slots, R, H, dk, dv)
+    run = lambda: ops.retention(p, 0, H * dk, 2 * H * dk, decay, state, q_start, slots, R, H, dk, dv, longest=n)
     for _ in range(max(3, args.warmup)):
         run()
     torch.cuda.synchronize()

@@ -402,7 +402,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* out, float4 v) {
 
 // The same again for heads of 16 to 128 entries (powers of two) that fill rows of 128 columns evenly: a warp takes stretches of 128
 // columns, 16 bytes a lane, asks for two of them first, and a head's lanes add its squares among themselves.  The kernel
-// above, which reads 4 bytes a lane and starts a warp per head, took 45 us for 2,113 tokens of 44 heads (18 MB), waiting
+// above, which reads 4 bytes a lane and starts a warp per head, took 45 us for 2,465 tokens of 44 heads (30 MB), waiting
 // for its chain of loads; this one takes 20 (16 for 23 where 2,048 tokens have 24 heads of 128).
 constexpr int QR_WARPS = 8, QR_EACH = 2;
 

@@ -21,7 +21,7 @@
 // What bounds it: chains, not a unit (tensor pipe 30 % active): a tile is its loads, its scores, its softmax and its value product, each
 // 700 to 1,900 clocks, overlapped two tiles deep for the widest rows and four for others; then the boxes of shuffled pages (a TMA
 // box of 16 rows takes about 60 clocks).  B200, 2,048 tokens, pages in shuffled order: latent of 512 + 64 under 16 heads 941 us on
-// mma.sync, 194 us here; 16 heads on 4 value heads of 128 in chunks of 1,024, mixed, 564 -> 107 us; two maps of 64, 2,113 tokens
+// mma.sync, 194 us here; 16 heads on 4 value heads of 128 in chunks of 1,024, mixed, 564 -> 107 us; two maps of 64, 2,465 tokens
 // in chunks of 1,024, 326 -> 77 us.
 // Every wait is bounded; one that runs out records a code that q6k_attention_flex_tc_status() returns.
 #include "umma.cuh"

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) retention_prep_kernel(float* p, int ld, i
 }
 
 // The same for halves that pair up 16 bytes at a time (rd / 2 a multiple of 4, rows and heads on 16 bytes, no activation before it): a
-// thread asks for two pairs before the angles are made.  26 us for 2,552 tokens of 16 heads of 128, 84 MB, four bytes at a time;
+// thread asks for two pairs before the angles are made.  26 us for 2,550 tokens of 16 heads of 128, 84 MB, four bytes at a time;
 // this one takes 14.
 __global__ void __launch_bounds__(256) retention_turn4_kernel(float* p, int ld, int H, int dk, int q_col, int k_col, const float* inv_freq, int rd, float k_scale,
                                                               const int* positions) {
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(128) time_mix_prep_kernel(const float* r, cons
 // walks a request's chunks entry by entry and leaves in each one's place the state it starts from; ret_out_kernel makes every
 // chunk's results, [d^(i+1) Q | M] times [S | V] as one product of 64 x 128 outputs whose second factor comes by in slices of 32 rows.
 // FP32 throughout; powers of d are made in double precision.  C = 64: 32 would double the bytes of the states (one per chunk and head).
-// 2,552 tokens in three portions, 16 heads of 128 x 128: 202 us token by token, 41 + 14 + 95 us so.  What bounds the two products: reads of
+// 2,550 tokens in three portions, 16 heads of 128 x 128: 202 us token by token, 41 + 14 + 95 us so.  What bounds the two products: reads of
 // shared memory beside the FP32 pipe, each about half of the time.
 constexpr int RC = 64;
 
