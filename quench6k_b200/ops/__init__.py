@@ -1490,7 +1490,8 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
     prepare: a kernel of its own first makes every token's unit vectors (in place over q and k in u), beta, decay and k . q,
     and the recurrence fetches a tile of tokens while it walks the one before (for steps with long portions); else the
     recurrence makes them itself.  The results are the same bit for bit.  chunked (with prepare, where gated_delta_chunks(...)
-    says so): 32 tokens at a time as a triangular system, equal to the others up to rounding."""
+    says so): 32 tokens at a time as a triangular system, equal to the others up to rounding, if the chunks' matrices take no more than
+    256 MB."""
     _need(u, "u", torch.float32)
     _need(p, "p", torch.float32)
     _need(A_log, "A_log", torch.float32, (H,))
@@ -1507,7 +1508,9 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
             raise KernelError("gated_delta: chunks go with prepared inputs")
         lib = library()
         lib.q6k_gated_delta_chunk_floats.restype = ctypes.c_longlong
-        chunks = torch.empty(lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H)), dtype=torch.float32, device=u.device)
+        floats = lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H))
+        if floats <= 64 << 20:
+            chunks = torch.empty(floats, dtype=torch.float32, device=u.device)
     _call("q6k_gated_delta", _ptr(u), _i(u.stride(0)), _ptr(p), _i(p.stride(0)), _i(b_col), _i(a_col), _ptr(A_log), _ptr(dt_bias), _ptr(bg),
           _ptr(chunks), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
     return o
