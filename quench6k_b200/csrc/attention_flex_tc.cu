@@ -92,10 +92,10 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
     const int n_q = p.dkb - p.qt;                               // Q chunks in shared memory: chunks qt .. dkb-1
     const int n_chunks = p.shared_v ? p.dkb : p.dkb + p.nvc;     // chunks of a stage
     const uint32_t q_s = smem_u32(smem), k_s = q_s + n_q * FT_QCHUNK, stage_bytes = n_chunks * FT_CHUNK;
-    __shared__ __align__(8) uint64_t bars[4 * FT_STAGES + 6];
+    __shared__ __align__(8) uint64_t bars[4 * FT_STAGES + 7];
     __shared__ uint32_t tmem_slot;
     const uint32_t fullA = smem_u32(&bars[0]), emptyA = fullA + 8 * FT_STAGES, fullB = fullA + 16 * FT_STAGES, emptyB = fullA + 24 * FT_STAGES;
-    const uint32_t s_full = fullA + 32 * FT_STAGES, p_full = s_full + 16, pv_done = s_full + 32, q_full = s_full + 40;
+    const uint32_t s_full = fullA + 32 * FT_STAGES, p_full = s_full + 16, pv_done = s_full + 32, q_full = s_full + 48;
 
     // every (key head, part of the values) of a row tile side by side, the tiles in the order of the list (those with the most keys first)
     const int kh = blockIdx.x / p.parts, part = blockIdx.x % p.parts, tile = blockIdx.y, split = blockIdx.z;
@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
         for (int s = 0; s < 2; ++s) {
             mbar_init(s_full + 8 * s, 1);
             mbar_init(p_full + 8 * s, 128);
+            mbar_init(pv_done + 8 * s, 1);
         }
-        mbar_init(pv_done, 1);
         mbar_init(q_full, 128 * WARPS4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_k) : "memory");
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
                     for (int k = 0; k < 4; ++k)
                         umma_ts(tmem, pa + t * 32 + k * 8, umma_desc_mn(v + k * 2048, FT_CHUNK), idesc_o, (i | t | k) != 0);
                 umma_commit(emptyB + 8 * s);
-                umma_commit(pv_done);
+                umma_commit(pv_done + 8 * (i & 1));
             };
             const int groups = p.shared_v ? 2 : 1;
             for (int grp = 0; grp < groups && ok; ++grp) {
@@ -289,6 +289,11 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
             }
         }
     } else {
+        // A barrier's parity tells a phase from the one before and the one after it only, and these warps do not wait for every value
+        // product.  So the products take turns on two barriers: when a row has seen the scores of tile i, the product of tile i - 2
+        // is done (the scores were issued behind it), and no product beyond i - 1 can end before the row's weights of tile i are
+        // out.  Product i - 1 is thus the last phase of its barrier that ended or the one at hand, whenever the row comes to ask.
+        // With one barrier product i - 1 could be taken for i - 3, and a row that came late to ask for i - 2 would wait for i.
         // ---- Q (zeros in rows without a token)
         const int quarter = warp & 3, row = quarter * 32 + lane;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
                     corr = m == -INFINITY ? 1.0f : ex2_approx(m - ref);
                 }
                 if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
-                    if (!mbar_wait(pv_done, (i - 1) & 1)) {
+                    if (!mbar_wait(pv_done + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1)) {
                         if (lane == 0) atomicExch(&g_flex_tc_status, 7);
                         ok = false;
                         break;
@@ -448,9 +453,7 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
                 mbar_arrive(p_full + 8 * (i & 1));
             }
             if (ok && n > 0) {
-                // the product before the last may still run (the last scores were asked for before it): its phase first, or the
-                // wait for the last one would see the phase of the same parity two products ago
-                if ((n > 1 && !mbar_wait(pv_done, n & 1)) || !mbar_wait(pv_done, (n - 1) & 1)) {
+                if (!mbar_wait(pv_done + 8 * ((n - 1) & 1), ((n - 1) >> 1) & 1)) {      // the products before it are done when it is
                     if (lane == 0) atomicExch(&g_flex_tc_status, 9);
                     ok = false;
                 }

@@ -75,3 +75,27 @@ def test_against_the_cuda_core_kernel(H, Hkv, da, db, dv, shared, page, extra):
         rel = ((got.float() - want.float()).norm() / want.float().norm()).item()
         assert diff < 1e-2 * size and rel < 4e-3, f"max_context {max_context}: {diff / size:.3e}, {rel:.3e}"
     assert ops.tc_status() == 0
+
+
+def test_every_row_sees_its_last_value_product():
+    """From one key tile to seven, two CTAs to an SM, launched again and again: a row that comes late to ask for the last product
+    has to see that it is done (a wait by a parity two products old would run out, leave a status and store nothing)."""
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(5)
+    H, Hkv, hd, page = 8, 2, 64, 16
+    q_lens, starts = [32] * 48, [(64 * i) % 448 for i in range(48)]
+    n_pages = sum((s + n + page - 1) // page for s, n in zip(starts, q_lens))
+    order, tables, at = torch.randperm(n_pages, generator=g).tolist(), [], 0
+    for s, n in zip(starts, q_lens):
+        tables.append(order[at:at + (s + n + page - 1) // page])
+        at += len(tables[-1])
+    ctx = helpers.make_context(q_lens, starts, [tables])
+    k, v = (_pages(q_lens, starts, page, Hkv, hd, g, order, n_pages) for _ in range(2))
+    q = torch.randn(H * ctx.T, hd, generator=g).to(torch.bfloat16).cuda()
+    tiles = ctx.query_tiles(ops.attention_flex_wide_tokens(32, H, Hkv, 0, hd, hd, False, False, page, 0.125))
+    run = lambda: ops.attention_flex(None, q, False, k, v, ctx.block_tables[0], ctx.req_of_token, ctx.positions, H, 0.125, wide_tiles=tiles, max_context=512)
+    first = run()
+    assert bool(torch.isfinite(first).all())
+    for _ in range(200):
+        assert torch.equal(run(), first)
+    assert ops.tc_status() == 0
