@@ -2,7 +2,9 @@
 // of their own or the leading entries of the key rows, a query given in two parts, causal mask narrowed by a
 // window and/or chunks, sinks, a cap on the scores, several maps per head, and every head against every value head for the mixing
 // kernel.  The scores, maxima, exponentials, sums and accumulators are FP32 and the weights enter the value product as two
-// bfloat16 terms (16 bits of them), as in attention_flex_mma.cu, which keeps the decode steps and the shapes this one does not take.
+// bfloat16 terms (16 bits of them), as in attention_flex_mma.cu, which keeps the steps of short portions and the shapes this one does not
+// take.  Groups of more than 32 query heads, values beyond 512 and whatever else that kernel does not take stay on CUDA cores with
+// FP32 weights.
 //
 // A CTA takes 128 query rows (the G query heads of one key head for 128 / G consecutive tokens of one request) and up to 256
 // value columns (FP32 accumulators in tensor memory: a latent of 512 is two CTAs per row tile, which both make the scores: the
@@ -28,7 +30,7 @@
 
 namespace {
 
-constexpr int FT_ROWS = 128, FT_KEYS = 64;
+constexpr int FT_ROWS = 128, FT_KEYS = 64, FT_GROUP = 32;   // FT_GROUP: query heads of a key head, at most (as in attention_flex_mma.cu)
 constexpr uint32_t FT_CHUNK = FT_KEYS * 128;           // bytes of a [64 keys x 64 columns] chunk
 constexpr uint32_t FT_QCHUNK = FT_ROWS * 128;          // bytes of a [128 rows x 64 columns] chunk of Q
 constexpr int FT_STAGES = 4;
@@ -43,6 +45,7 @@ struct FlexTc {
     int dkb, qt;                        // chunks of a key row; how many of Q's lie in tensor memory
     int nvc, shared_v;                  // value chunks of a CTA; values are the leading columns of the key rows
     int stages, parts;                  // stages of the ring; CTAs that share a row tile's value columns
+    int per_tile;                       // CTAs of a row tile: key heads x parts
     int k_head_rows, v_head_rows;       // page rows of a head
     const int* block_table; int max_blocks, page_size, box;
     int oob_k, oob_v;                   // a row beyond the pages: reads zeros
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(64 + 128 * WARPS4, WARPS4 == 1 ? 2 : 1) attent
     const uint32_t s_full = fullA + 32 * FT_STAGES, p_full = s_full + 16, pv_done = s_full + 32, q_full = s_full + 48;
 
     // every (key head, part of the values) of a row tile side by side, the tiles in the order of the list (those with the most keys first)
-    const int kh = blockIdx.x / p.parts, part = blockIdx.x % p.parts, tile = blockIdx.y, split = blockIdx.z;
+    const int tile = blockIdx.x / p.per_tile, of_tile = blockIdx.x % p.per_tile, kh = of_tile / p.parts, part = of_tile % p.parts, split = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = p.G;
     const int tok0 = p.tile_tok0[tile], ntok = min(p.tile_ntok[tile], FT_ROWS / G);
     const int pos0 = p.positions[tok0], pos_last = pos0 + ntok - 1;
@@ -536,7 +539,7 @@ struct FlexTcPlan {
 };
 
 bool flex_tc_plan(int H, int Hkv, int dk, int dv, int da, int db, int v_heads, bool shared_v, int page_size, FlexTcPlan* o) {
-    if (Hkv <= 0 || H <= 0 || H % Hkv || H / Hkv > FT_ROWS) return false;
+    if (Hkv <= 0 || H <= 0 || H % Hkv || H / Hkv > FT_GROUP || dv > 512) return false;
     if (page_size < 8 || (page_size < FT_KEYS ? FT_KEYS % page_size : page_size % FT_KEYS)) return false;
     const int total = v_heads > 0 ? v_heads * dv : dv;
     if (dk % 8 || da % 8 || db % 8 || dv <= 0 || dv % 64 || total > 2048) return false;
@@ -581,7 +584,7 @@ Q6K_API int q6k_attention_flex_tc_parts(int H, int Hkv, int da, int db, int dv, 
 }
 
 // Tokens of one request a row tile holds.
-Q6K_API int q6k_attention_flex_tc_tile_tokens(int H, int Hkv) { return Hkv > 0 && H % Hkv == 0 && H / Hkv <= FT_ROWS ? FT_ROWS / (H / Hkv) : 0; }
+Q6K_API int q6k_attention_flex_tc_tile_tokens(int H, int Hkv) { return Hkv > 0 && H % Hkv == 0 && H / Hkv <= FT_GROUP ? FT_ROWS / (H / Hkv) : 0; }
 
 // Arguments as q6k_attention_flex_tc's (attention_flex_mma.cu).  talk != 0: mixed heads; the result is part_o FP32
 // [T, H, Hkv, dv], for the mixing kernel.  nsplit > 1: part_o [nsplit, T, H, dv] unnormalised and part_ml [nsplit, T, H, 2], for
@@ -597,7 +600,7 @@ int q6k_attention_flex_tc_launch(const void* qa, int da, const void* qb, int db,
                 Hkv, da + db, dv);
     const int Hv = maps > 1 ? Hkv / maps : Hkv;
     const long long k_rows = (long long)Hkv * num_pages * page_size, v_rows = (long long)Hv * num_pages * page_size;
-    Q6K_REQUIRE(k_rows < (1LL << 31) && n_tiles <= 65535 && nsplit <= 65535 && ((uintptr_t)k_pages & 15) == 0 && ((uintptr_t)v_pages & 15) == 0 && k_ld % 8 == 0 &&
+    Q6K_REQUIRE(k_rows < (1LL << 31) && (long long)n_tiles * Hkv * pl.parts < (1LL << 31) && nsplit <= 65535 && ((uintptr_t)k_pages & 15) == 0 && ((uintptr_t)v_pages & 15) == 0 && k_ld % 8 == 0 &&
                     v_ld % 8 == 0 && ((uintptr_t)qa & 15) == 0 && ((uintptr_t)qb & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)part_o & 15) == 0 && scale > 0.0f,
                 "attention_flex_tc: too many rows or operands not 16-byte aligned");
     const int box = page_size < FT_KEYS ? page_size : FT_KEYS;
@@ -611,7 +614,7 @@ int q6k_attention_flex_tc_launch(const void* qa, int da, const void* qb, int db,
     }
     FlexTc p{};
     p.qa = (const __nv_bfloat16*)qa, p.da = da, p.qb = (const __nv_bfloat16*)qb, p.db = db, p.q_head_major = q_head_major;
-    p.dkb = pl.dkb, p.qt = pl.qt, p.nvc = pl.nvc, p.shared_v = shared_v, p.stages = pl.stages, p.parts = pl.parts;
+    p.dkb = pl.dkb, p.qt = pl.qt, p.nvc = pl.nvc, p.shared_v = shared_v, p.stages = pl.stages, p.parts = pl.parts, p.per_tile = Hkv * pl.parts;
     p.k_head_rows = p.v_head_rows = num_pages * page_size, p.oob_k = (int)k_rows, p.oob_v = (int)v_rows;
     p.block_table = block_table, p.max_blocks = max_blocks, p.page_size = page_size, p.box = box;
     p.req_of_token = req_of_token, p.positions = positions, p.tile_tok0 = tile_tok0, p.tile_ntok = tile_ntok;
@@ -622,6 +625,6 @@ int q6k_attention_flex_tc_launch(const void* qa, int da, const void* qb, int db,
     auto* kernel = pl.two ? (softcap > 0.0f ? attention_flex_tc_kernel<true, 1> : attention_flex_tc_kernel<false, 1>)
                           : (softcap > 0.0f ? attention_flex_tc_kernel<true, 2> : attention_flex_tc_kernel<false, 2>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) != cudaSuccess) return q6k_check_launch("attention_flex_tc: shared memory attribute");
-    q6k_launch(kernel, dim3(Hkv * pl.parts, n_tiles, nsplit), pl.two ? 192 : 320, pl.smem, st, tk, tv, tkr, tvr, p);
+    q6k_launch(kernel, dim3(n_tiles * Hkv * pl.parts, nsplit), pl.two ? 192 : 320, pl.smem, st, tk, tv, tkr, tvr, p);
     return q6k_check_launch("attention_flex_tc");
 }

@@ -1283,7 +1283,7 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
     tiles = (first row, token count, number) of row tiles of attention_flex_tile_tokens(H, Hkv) tokens of one request
     each, with max_context the largest position + 1 of the step: bfloat16 pages then go to the tensor-core kernel where
     it takes the shapes; with few tiles it splits the keys into fixed ranges and merges them.  wide_tiles: the same for tiles of
-    attention_flex_wide_tokens(...) tokens, where that says the tcgen05 kernel should run instead; the first part of the query
+    attention_flex_wide(...) tokens, where that says the tcgen05 kernel should run instead; the first part of the query
     is then bfloat16 too."""
     da = q_f32.shape[-1] if q_f32 is not None else 0
     db = q.shape[-1] if q is not None else 0
@@ -1402,11 +1402,28 @@ def attention_flex_tc_tile_tokens(H: int, Hkv: int) -> int:
     return lib.q6k_attention_flex_tc_tile_tokens(_i(H), _i(Hkv))
 
 
+def attention_flex_wide(max_q_len: int, H: int, da: int, db: int, mixed: bool, k_pages: torch.Tensor, v_pages: torch.Tensor, scale: float) -> int:
+    """attention_flex_wide_tokens(...) for these pages, or 0 where the tcgen05 kernel may not stand in for the one that ran the step
+    before it: shapes the mma.sync kernel does not take (on CUDA cores the query and the weights stay FP32; its first query
+    part and its weights are rounded as the tcgen05 kernel's are), and pages the copies of whole boxes cannot address."""
+    Hkv, num_pages, page_size, dk = k_pages.shape
+    dv, shared_v = v_pages.shape[-1], v_pages.data_ptr() == k_pages.data_ptr() and v_pages.stride() == k_pages.stride()
+    if k_pages.dtype != torch.bfloat16 or Hkv * num_pages * page_size >= 1 << 31:
+        return 0
+    for p in (k_pages, v_pages):
+        if p.data_ptr() % 16 or (p.shape[0] > 1 and p.stride(0) != num_pages * page_size * p.stride(2)):
+            return 0
+    if not attention_flex_mma_supported(H, Hkv, dk, dv, k_pages.stride(2), v_pages.stride(2), db, shared_v):
+        return 0
+    return attention_flex_wide_tokens(max_q_len, H, Hkv, da, db, dv, mixed, shared_v, page_size, scale)
+
+
 def attention_flex_wide_tokens(max_q_len: int, H: int, Hkv: int, da: int, db: int, dv: int, mixed: bool, shared_v: bool, page_size: int,
                                scale: float) -> int:
     """Tokens of the row tiles the tcgen05 kernel should be given in a step whose longest portion has max_q_len tokens, or 0
     where the mma.sync kernel (tiles of a quarter of the rows) serves the step: shapes this one does not take, and steps in
-    which no portion fills half of one of its tiles.  Both measured: a latent of 512 under 16 heads at 4,096 keys, 4 tokens 54 us
+    which no portion fills half of one of its tiles (a tile has at least four tokens, so steps of single tokens are among them).
+    attention_flex_wide says whether a layer may use it.  Both measured: a latent of 512 under 16 heads at 4,096 keys, 4 tokens 54 us
     (mma.sync) and 40 us, 64 tokens 139 and 49 us; mixed heads in chunks of 1,024, 64 tokens 25 and 26 us, 256 tokens 48 and
     32 us; two tokens of two maps of 64, 20 and 21 us."""
     if scale <= 0 or not _flex_tc_parts(H, Hkv, da, db, dv, mixed, shared_v, page_size):

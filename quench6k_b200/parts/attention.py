@@ -212,8 +212,7 @@ class Attention(Mixer):
         ops.current_tag = "attention.keys"
         tiles = wide = None
         if not rt.is_fp32 and rt.tensor_cores:
-            tokens = ops.attention_flex_wide_tokens(ctx.max_q_len, self.Hq * M, self.Hkv * M, 0, self.hd, self.vd, self.talk, False, cache.page_size,
-                                                    self.scale)
+            tokens = ops.attention_flex_wide(ctx.max_q_len, self.Hq * M, 0, self.hd, self.talk, cache.k, cache.v, self.scale)
             if tokens:
                 wide = ctx.query_tiles(tokens, most_keys_first=(self.window, self.chunk))
             else:
