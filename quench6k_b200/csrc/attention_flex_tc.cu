@@ -553,7 +553,10 @@ bool flex_tc_plan(int H, int Hkv, int dk, int dv, int da, int db, int v_heads, b
     o->qt = 0;
     // narrow values: half of an SM's tensor memory and shared memory, so that two CTAs hide each other's softmax
     o->two = o->nvc <= 2 && o->dkb * FT_QCHUNK + 2 * stage <= half;
-    if (!o->two && o->dkb * FT_QCHUNK + 2 * stage > most) o->qt = o->dkb < 4 ? o->dkb : 4;
+    if (!o->two && o->dkb * FT_QCHUNK + 2 * stage > most) {
+        if (o->dkb <= 4) return false;   // some of Q stays in shared memory: what goes to tensor memory passes through its place
+        o->qt = 4;
+    }
     const size_t q_bytes = (size_t)(o->dkb - o->qt) * FT_QCHUNK, room = o->two ? half : most;
     if (q_bytes + 2 * stage > room) return false;
     o->stages = (int)((room - q_bytes) / stage);
