@@ -440,13 +440,16 @@ __global__ void __launch_bounds__(128) attention_flex_merge_kernel(const float* 
 // out[t, h] = sum_g talk[h, g] * part[t, g, KV head of h], FP32 sums in the order of g.  A block per token: a thread takes four
 // columns of a value head and reads every head's part of them once for four query heads at a time, all loads independent.  (A block
 // per token and query head read each part once per head of the group, 4 bytes a load: 66 us for 2,048 tokens of 16 heads on 4 value
-// heads of 128; the parts are 67 MB, most of which still lie in L2.)
+// heads of 128; the parts are 67 MB, most of which still lie in L2.)  STAGED: the matrix fits shared memory.
+template <bool STAGED>
 __global__ void __launch_bounds__(128) attention_talk_mix_kernel(const float* part, const float* talk, int H, int Hkv, int dv,
                                                                  __nv_bfloat16* out) {
     pdl_enter();
     extern __shared__ float mix[];                                               // talk, transposed: [g][h]
-    for (int i = threadIdx.x; i < H * H; i += blockDim.x) mix[(i % H) * H + i / H] = talk[i];
-    __syncthreads();
+    if (STAGED) {
+        for (int i = threadIdx.x; i < H * H; i += blockDim.x) mix[(i % H) * H + i / H] = talk[i];
+        __syncthreads();
+    }
     const int t = blockIdx.x, G = H / Hkv, width = Hkv * dv;
     const float* src = part + (size_t)t * H * width;
     for (int col = threadIdx.x * 4; col < width; col += blockDim.x * 4) {
@@ -460,7 +463,8 @@ __global__ void __launch_bounds__(128) attention_talk_mix_kernel(const float* pa
                 const float4 x = *reinterpret_cast<const float4*>(src + (size_t)g * width + col);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float w = h0 + j < G ? mix[g * H + kv * G + h0 + j] : 0.0f;
+                    const int h = kv * G + h0 + j;
+                    const float w = h0 + j >= G ? 0.0f : STAGED ? mix[g * H + h] : talk[(size_t)h * H + g];
                     acc[j].x = fmaf(w, x.x, acc[j].x), acc[j].y = fmaf(w, x.y, acc[j].y), acc[j].z = fmaf(w, x.z, acc[j].z), acc[j].w = fmaf(w, x.w, acc[j].w);
                 }
             }
@@ -473,6 +477,14 @@ __global__ void __launch_bounds__(128) attention_talk_mix_kernel(const float* pa
                 }
         }
     }
+}
+
+// More than 110 heads: the matrix is read where it lies.
+int launch_talk_mix(const float* part, const float* talk, int T_, int H, int Hkv, int dv, void* out, cudaStream_t st) {
+    const size_t bytes = (size_t)H * H * sizeof(float);
+    if (bytes <= 48 * 1024) q6k_launch(attention_talk_mix_kernel<true>, T_, 128, bytes, st, part, talk, H, Hkv, dv, (__nv_bfloat16*)out);
+    else q6k_launch(attention_talk_mix_kernel<false>, T_, 128, 0, st, part, talk, H, Hkv, dv, (__nv_bfloat16*)out);
+    return q6k_check_launch("attention_talk_mix");
 }
 
 size_t flex_mma_smem(int dk, int dv, bool shared_v, int nbuf) {
@@ -537,10 +549,7 @@ Q6K_API int q6k_attention_flex_mma(const float* qa, int da, const void* qb, int 
     else FLEX_LAUNCH(8);
 #undef FLEX_LAUNCH
     if (int rc = q6k_check_launch("attention_flex_mma")) return rc;
-    if (talk) {
-        q6k_launch(attention_talk_mix_kernel, T_, 128, (size_t)H * H * 4, st, (const float*)workspace, talk, H, Hkv, dv, (__nv_bfloat16*)out);
-        return q6k_check_launch("attention_talk_mix");
-    }
+    if (talk) return launch_talk_mix(workspace, talk, T_, H, Hkv, dv, out, st);
     if (nsplit > 1) {
         q6k_launch(attention_flex_merge_kernel, dim3(T_, H), 128, 0, st, (const float*)a.part_o, (const float*)a.part_ml, nsplit, T_, H, dv,
                    (__nv_bfloat16*)out, out_head_major, sinks, out_f32);
@@ -574,10 +583,7 @@ Q6K_API int q6k_attention_flex_tc(const void* qa, int da, const void* qb, int db
                                               req_of_token, positions, tile_tok0, tile_ntok, n_tiles, window, chunk, scale, out, out_head_major, T_, H, Hkv,
                                               nsplit, split_keys, workspace, ml, talk != nullptr, sinks, softcap, maps, out_f32, st))
         return rc;
-    if (talk) {
-        q6k_launch(attention_talk_mix_kernel, T_, 128, (size_t)H * H * 4, st, (const float*)workspace, talk, H, Hkv, dv, (__nv_bfloat16*)out);
-        return q6k_check_launch("attention_talk_mix");
-    }
+    if (talk) return launch_talk_mix(workspace, talk, T_, H, Hkv, dv, out, st);
     if (nsplit > 1) {
         q6k_launch(attention_flex_merge_kernel, dim3(T_, H), 128, 0, st, (const float*)workspace, (const float*)ml, nsplit, T_, H, dv, (__nv_bfloat16*)out,
                    out_head_major, sinks, out_f32);

@@ -99,3 +99,22 @@ def test_every_row_sees_its_last_value_product():
     for _ in range(200):
         assert torch.equal(run(), first)
     assert ops.tc_status() == 0
+
+
+@pytest.mark.parametrize("H, Hkv", [(96, 8), (112, 8)])                   # a mixing matrix that fits 48 KB, or does not
+def test_mixed_heads_of_any_number(H, Hkv):
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(H)
+    T, hd, dv, page, chunk = 21, 64, 64, 16, 8
+    ctx = helpers.make_context([T], [0], [[[1, 0]]])
+    k, v = (torch.randn(Hkv, 2, page, n, generator=g).to(torch.bfloat16).cuda() for n in (hd, dv))
+    q = torch.randn(T * H, hd, generator=g).to(torch.bfloat16).cuda()
+    talk = (torch.randn(H, H, generator=g) * H ** -0.5).cuda()
+    run = lambda **tiles: ops.attention_flex(None, q, False, k, v, ctx.block_tables[0], ctx.req_of_token, ctx.positions, H, 0.125, chunk=chunk, talk=talk, max_context=T, **tiles)
+    pos = torch.arange(T, device="cuda")
+    seen = (pos[:, None] >= pos) & (pos[:, None] // chunk == pos // chunk)
+    rows = [x[:, [1, 0]].reshape(Hkv, -1, x.shape[-1])[:, :T].double().repeat_interleave(H // Hkv, 0) for x in (k, v)]
+    w = torch.softmax((torch.einsum("thd,hjd->htj", q.view(T, H, hd).double(), rows[0]) * 0.125).masked_fill(~seen, float("-inf")), -1)
+    want = torch.einsum("hgtj,hjd->thd", talk.double()[:, :, None, None] * w[None], rows[1]).reshape(T, H * dv)
+    for got in (run(tiles=ctx.query_tiles(ops.attention_flex_tile_tokens(H, Hkv))), run(wide_tiles=ctx.query_tiles(ops.attention_flex_tc_tile_tokens(H, Hkv)))):
+        assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8          # a rounding to bfloat16 (2^-9), weights of 16 bits
