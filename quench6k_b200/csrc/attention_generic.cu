@@ -128,11 +128,11 @@ __global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q,
     const size_t head_base = (size_t)kh * num_pages;
     for (int ta = t0; ta < t1;) {
         const int req = req_of_token[ta];
-        int tb = ta + 1;
-        while (tb < t1 && req_of_token[tb] == req) ++tb;
+        int tb = ta + 1, pos_min = positions[ta], pos_max = pos_min;        // the rows' positions may come in any order
+        for (; tb < t1 && req_of_token[tb] == req; ++tb) pos_min = min(pos_min, positions[tb]), pos_max = max(pos_max, positions[tb]);
         const int* bt = block_table + (size_t)req * max_blocks;
-        const int rows = (tb - ta) * heads, k_end = positions[tb - 1] + 1;
-        const int lo_first = window > 0 ? max(0, positions[ta] - window + 1) : 0;
+        const int rows = (tb - ta) * heads, k_end = pos_max + 1;
+        const int lo_first = window > 0 ? max(0, pos_min - window + 1) : 0;
         __syncthreads();                              // the rows before are done with
         for (int i = tid; i < rows * (hd / 4); i += GT_THREADS) {
             const int r = i / (hd / 4), d = (i % (hd / 4)) * 4, g = g0 + r % heads;
@@ -156,8 +156,9 @@ __global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q,
             for (int i = tid; i < GT_KEYS * (hd / 4); i += GT_THREADS) {
                 const int kk = i / (hd / 4), d = (i % (hd / 4)) * 4, j = j0 + kk;
                 float4 kv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv = kv;
-                if (j >= lo_first && j < k_end) {
-                    const size_t at = ((head_base + bt[j / page_size]) * page_size + j % page_size) * hd + d;
+                const int page = j >= lo_first && j < k_end ? bt[j / page_size] : -1;
+                if (page >= 0) {                      // a page between the rows' windows may be gone
+                    const size_t at = ((head_base + page) * page_size + j % page_size) * hd + d;
                     kv = load4(k_pages + at);
                     vv = load4(v_pages + at);
                 }

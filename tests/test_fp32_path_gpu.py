@@ -39,6 +39,26 @@ def test_row_tiles_give_the_bits_of_the_decode_kernel(Hq, Hkv, hd, window, page,
     assert bool(torch.isfinite(whole).all())
 
 
+@pytest.mark.parametrize("window", [None, 9])
+def test_rows_in_any_order(window):
+    """Rows of one request whose positions do not ascend: every row sees its own keys."""
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(3)
+    Hq, Hkv, hd, page, T = 4, 2, 32, 4, 50
+    k, v = (torch.randn(Hkv, 13, page, hd, generator=g).cuda() for _ in range(2))
+    q, table = torch.randn(T, Hq, hd, generator=g).cuda(), torch.randperm(13, generator=g).to(torch.int32).cuda()[None]
+    orders = [torch.arange(T).flip(0), torch.randperm(T, generator=g), torch.randint(0, T, (T,), generator=g)]
+    if window:                                              # two stretches, and no pages between their windows
+        table[0, 3:9] = -1
+        orders = [torch.cat([torch.arange(11, -1, -1), torch.arange(49, 43, -1)])]
+    for order in orders:
+        T = len(order)
+        pos, req = order.to(torch.int32).cuda(), torch.zeros(T, dtype=torch.int32, device="cuda")
+        whole = ops.attention_generic(q[:T], k, v, table, req, pos, window, None)
+        for t in range(T):
+            assert torch.equal(ops.attention_generic(q[t:t + 1], k, v, table, req[:1], pos[t:t + 1], window, None)[0], whole[t]), (t, int(pos[t]))
+
+
 @pytest.mark.parametrize("M, N, K, offset", [(1, 1, 1, 0), (64, 64, 32, 0), (65, 63, 33, 0), (3, 130, 36, 0), (130, 70, 100, 1), (17, 257, 1000, 0), (200, 65, 4, 0)])
 def test_fp32_product_at_the_edges_of_its_tiles(M, N, K, offset):
     """offset: the operands start off a 16-byte boundary (copies of 4 bytes)."""
