@@ -142,15 +142,15 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(float* u, int ldu, c
 //
 // u: FP32 [T, ldu] with q at column 0 (G heads of dk), k after it, v after that (H heads of dv); p: FP32 [T, ldp] with
 // the H beta logits at b_col and the H decay inputs at a_col.  PREPARED: q and k in u are unit vectors already and bg
-// holds [beta | decay] per token (delta_prepare_kernel); the next tile's inputs are then fetched into registers while
-// this tile is walked.
+// holds [beta | decay] per token (delta_prepare_kernel; logs: the decays' logarithms); the next tile's inputs are then fetched into
+// registers while this tile is walked.  Requests of more than `most` tokens are not this launch's.
 constexpr int DELTA_CHUNK = 4;
 
 template <int RPL, bool PREPARED>
 __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float* u, int ldu, const float* p, int ldp, int b_col, int a_col,
                                                                               const float* A_log, const float* dt_bias, const float* bg,
                                                                               float* state, const int* q_start, const int* slot_ids, float* o,
-                                                                              int H, int G, int dk, int dv) {
+                                                                              int H, int G, int dk, int dv, int logs, int most) {
     pdl_enter();
     constexpr int SEG = RPL + 4, KS = DELTA_LANES * SEG, NT = DELTA_THREADS, CH = DELTA_CHUNK, PER = DELTA_PER, CT = DELTA_COLS / DELTA_PER;
     constexpr int PRE = PREPARED ? DELTA_TILE * DELTA_LANES * RPL / NT : 1;      // k (and q) entries of a tile per thread
@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int sub = threadIdx.x % DELTA_LANES, cl = threadIdx.x / DELTA_LANES;       // the thread's columns: col0 + cl + CT j
     const int first = q_start[r], n = q_start[r + 1] - first;
+    if (n > most) return;
     const int q_at = kvh * dk, k_at = G * dk + kvh * dk, v_at = 2 * G * dk + head * dv;
     const float decay_rate = PREPARED ? 0.0f : -expf(A_log[head]), bias = PREPARED ? 0.0f : dt_bias[head], q_mult = rsqrtf((float)dk);
     float* mine = state + ((size_t)slot_ids[r] * H + head) * dv * dk;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float*
         if (threadIdx.x < 2 * DELTA_TILE) {
             const int what = threadIdx.x / DELTA_TILE, t = threadIdx.x % DELTA_TILE;
             pre_s = t < nt ? bg[(size_t)(first + t0 + t) * 2 * H + what * H + head] : 0.0f;
+            if (logs && what) pre_s = expf(pre_s);
         }
     };
     if (PREPARED && n > 0) fetch(0);
@@ -385,13 +387,13 @@ __global__ void __launch_bounds__(DELTA_THREADS) gated_delta_kernel(const float*
 constexpr int CHUNK_FLOATS = 2 * WC * WC + 3 * WC;              // per (chunk, head): inverse, M, beta, P, P_C / P_m
 
 // grid (chunks, G), 128 threads; dynamic shared memory: K and Q [WC][dk + 4] each, then six [WC][WLD] squares (four of them a warp's).
-__global__ void __launch_bounds__(128) delta_chunk_kernel(const float* u, int ldu, const float* bg, const int* q_start, int R, float* chunks, int H, int G, int dk) {
+__global__ void __launch_bounds__(128) delta_chunk_kernel(const float* u, int ldu, const float* bg, const int* q_start, int R, int beyond, float* chunks, int H, int G, int dk) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int ld = dk + 4, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *ks = sm, *qs = ks + WC * ld, *kk = qs + WC * ld, *kq = kk + WC * WLD, *aw = kq + WC * WLD + warp * WC * WLD;
     int first = 0, n = 0;
-    chunk_of(q_start, R, blockIdx.x, first, n);
+    chunk_of(q_start, R, beyond, blockIdx.x, first, n);
     if (n == 0) return;
     for (int i = tid; i < WC * (dk / 4); i += 128) {
         const int t = i / (dk / 4), d = (i % (dk / 4)) * 4;
@@ -465,10 +467,10 @@ constexpr int XY_LD = WALK_COLS + 4;
 __host__ __device__ constexpr int walk_stage_floats(int dkp) { return 2 * WC * (dkp + 4) + 2 * WC * WLD + 3 * WC + WC * WALK_COLS; }
 __host__ __device__ constexpr int walk_floats(int dkp) { return 2 * walk_stage_floats(dkp) + WALK_COLS * (dkp + 4) + 9 * WC * XY_LD + 3 * WALK_COLS * WLD; }
 
-// grid (H * ceil(dv / 16), R), 256 threads.  dkp: dk rounded up to a multiple of 16.  GROUPS: ceil(dkp / 128), groups of four rows of the
+// grid (H * ceil(dv / 16), long requests), 256 threads.  dkp: dk rounded up to a multiple of 16.  GROUPS: ceil(dkp / 128), groups of four rows of the
 // state a thread holds.
 template <int GROUPS>
-__global__ void __launch_bounds__(WALK_THREADS, 1) delta_walk_kernel(const float* u, int ldu, const float* chunks, float* state, const int* q_start,
+__global__ void __launch_bounds__(WALK_THREADS, 1) delta_walk_kernel(const float* u, int ldu, const float* chunks, float* state, const int* q_start, int R, int beyond,
                                                                   const int* slot_ids, float* o, int H, int G, int dk, int dv, int dkp) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
@@ -480,11 +482,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) delta_walk_kernel(const float
     float* rt = qs + WC * XY_LD;                        // [16][WLD]: right-hand sides, a column's tokens side by side
     float* ut = rt + WALK_COLS * WLD;                   // [16][WLD]: U
     float* uw = ut + WALK_COLS * WLD;                   // [16][WLD]: U times P_C / P_m
-    const int col_blocks = (dv + WALK_COLS - 1) / WALK_COLS, head = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * WALK_COLS, r = blockIdx.y;
+    const int col_blocks = (dv + WALK_COLS - 1) / WALK_COLS, head = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * WALK_COLS;
     const int kvh = head / (H / G), tid = threadIdx.x, tx = tid & 7, row8 = tid >> 3;
-    const int first = q_start[r], n = q_start[r + 1] - first;
-    if (n <= 0) return;
-    const int chunk0 = first_chunk_of(q_start, r), count = (n + WC - 1) / WC;
+    int chunk0;
+    const int r = long_request(q_start, R, beyond, blockIdx.y, chunk0);
+    if (r < 0) return;
+    const int first = q_start[r], n = q_start[r + 1] - first, count = (n + WC - 1) / WC;
     float* mine = state + ((size_t)slot_ids[r] * H + head) * dv * dk;
     // rows 4 (row8 + 32 g) .. + 3 of columns tx and tx + 8
     float4 s[GROUPS][2];
@@ -760,12 +763,13 @@ Q6K_API int q6k_short_conv_tail(const float* x, int slices, long long slice_stri
 Q6K_API int q6k_gated_delta_max_dim() { return 32 * DELTA_LANES; }
 
 // Floats of scratch for walking the portions of a step of T_ rows and R requests chunk by chunk.
-Q6K_API long long q6k_gated_delta_chunk_floats(int T_, int R, int H) { return (long long)(T_ / WC + R) * H * CHUNK_FLOATS; }
+Q6K_API long long q6k_gated_delta_chunk_floats(int T_, int R, int H, int beyond) { return (long long)most_chunks(T_, R, beyond) * H * CHUNK_FLOATS; }
 
 // state: FP32 [slots, H, dv, dk]; o: FP32 [T, H * dv].  chunks: null, or (with bg) the scratch above.  bg: null, or FP32 scratch [T, 2 H]: the per-token values are then made
-// by a kernel of their own first, which also turns q and k in u into unit vectors (for steps with long portions).
+// by a kernel of their own first, which also turns q and k in u into unit vectors (for steps with long portions).  beyond: with
+// chunks, requests of up to so many tokens are walked token by token (0: none is).
 Q6K_API int q6k_gated_delta(float* u, int ldu, const float* p, int ldp, int b_col, int a_col, const float* A_log, const float* dt_bias,
-                            float* bg, float* chunks, float* state, const int* q_start, const int* slot_ids, float* o, int T_, int R, int H, int G, int dk,
+                            float* bg, float* chunks, int beyond, float* state, const int* q_start, const int* slot_ids, float* o, int T_, int R, int H, int G, int dk,
                             int dv, cudaStream_t st) {
     if (R == 0 || T_ == 0) return 0;
     Q6K_REQUIRE(R > 0 && T_ > 0 && H > 0 && G > 0 && H % G == 0 && dk > 0 && dv > 0, "gated_delta: bad sizes R=%d H=%d G=%d dk=%d dv=%d", R, H, G, dk, dv);
@@ -776,24 +780,28 @@ Q6K_API int q6k_gated_delta(float* u, int ldu, const float* p, int ldp, int b_co
         if (int rc = q6k_check_launch("delta_prepare")) return rc;
     }
     if (chunks) {
-        Q6K_REQUIRE(bg && dk % 4 == 0 && dv % 4 == 0 && ldu % 4 == 0 && (((uintptr_t)u | (uintptr_t)state | (uintptr_t)chunks) & 15) == 0,
+        Q6K_REQUIRE(bg && beyond >= 0 && dk % 4 == 0 && dv % 4 == 0 && ldu % 4 == 0 && (((uintptr_t)u | (uintptr_t)state | (uintptr_t)chunks) & 15) == 0,
                     "gated_delta: chunks take prepared inputs, keys, values and rows of multiples of 4 entries, on 16 bytes");
-        const size_t smem1 = (size_t)(2 * WC * (dk + 4) + 6 * WC * WLD) * sizeof(float);
-        if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return q6k_check_launch("delta_chunk: shared memory attribute");
-        q6k_launch(delta_chunk_kernel, dim3(T_ / WC + R, G), 128, smem1, st, u, ldu, bg, q_start, R, chunks, H, G, dk);
-        if (int rc = q6k_check_launch("delta_chunk")) return rc;
-        const int dkp = (dk + 15) / 16 * 16;
-        const size_t smem2 = (size_t)walk_floats(dkp) * sizeof(float);
-        auto* walk = dkp <= 128 ? delta_walk_kernel<1> : delta_walk_kernel<2>;
-        if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess) return q6k_check_launch("delta_walk: shared memory attribute");
-        q6k_launch(walk, dim3(H * ((dv + WALK_COLS - 1) / WALK_COLS), R), WALK_THREADS, smem2, st, u, ldu, chunks, state, q_start, slot_ids, o, H, G, dk, dv, dkp);
-        return q6k_check_launch("delta_walk");
+        if (most_long(T_, R, beyond) > 0) {
+            const size_t smem1 = (size_t)(2 * WC * (dk + 4) + 6 * WC * WLD) * sizeof(float);
+            if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return q6k_check_launch("delta_chunk: shared memory attribute");
+            q6k_launch(delta_chunk_kernel, dim3(most_chunks(T_, R, beyond), G), 128, smem1, st, u, ldu, bg, q_start, R, beyond, chunks, H, G, dk);
+            if (int rc = q6k_check_launch("delta_chunk")) return rc;
+            const int dkp = (dk + 15) / 16 * 16;
+            const size_t smem2 = (size_t)walk_floats(dkp) * sizeof(float);
+            auto* walk = dkp <= 128 ? delta_walk_kernel<1> : delta_walk_kernel<2>;
+            if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess) return q6k_check_launch("delta_walk: shared memory attribute");
+            q6k_launch(walk, dim3(H * ((dv + WALK_COLS - 1) / WALK_COLS), most_long(T_, R, beyond)), WALK_THREADS, smem2, st, u, ldu, chunks, state, q_start, R, beyond, slot_ids, o, H, G, dk, dv, dkp);
+            if (int rc = q6k_check_launch("delta_walk")) return rc;
+        }
+        if (beyond == 0) return 0;
     }
     const dim3 grid(H * ((dv + DELTA_COLS - 1) / DELTA_COLS), R);
     const int rpl = ((dk + DELTA_LANES - 1) / DELTA_LANES + 3) / 4 * 4;
     const int RPL_ = rpl <= 4 ? 4 : rpl <= 8 ? 8 : rpl <= 16 ? 16 : 32;
     const size_t smem = (size_t)(2 * DELTA_TILE * DELTA_LANES * (RPL_ + 4) + DELTA_TILE * DELTA_COLS + 2 * DELTA_TILE + 2 * DELTA_TILE * DELTA_CHUNK) * sizeof(float);
-#define Q6K_DELTA_GO(R_, P_) q6k_launch(gated_delta_kernel<R_, P_>, grid, DELTA_THREADS, smem, st, u, ldu, p, ldp, b_col, a_col, A_log, dt_bias, bg, state, q_start, slot_ids, o, H, G, dk, dv)
+#define Q6K_DELTA_GO(R_, P_) q6k_launch(gated_delta_kernel<R_, P_>, grid, DELTA_THREADS, smem, st, u, ldu, p, ldp, b_col, a_col, A_log, dt_bias, bg, state, q_start, slot_ids, o, H, G, dk, dv, \
+                                              chunks != nullptr, chunks ? beyond : 0x7fffffff)
     if (bg) {
         if (RPL_ == 4) Q6K_DELTA_GO(4, true);
         else if (RPL_ == 8) Q6K_DELTA_GO(8, true);

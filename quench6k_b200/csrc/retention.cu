@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const f
     float *ks = sm, *vs = sm + RC * 128;                    // [64][128] each, k times its token's power of d
     const int head = blockIdx.y, tid = threadIdx.x, cols = (dv + 127) / 128, row0 = blockIdx.z / cols * 128, col0 = blockIdx.z % cols * 128;
     int first = 0, n = 0;
-    chunk_of<RC>(q_start, R, blockIdx.x, first, n);
+    chunk_of<RC>(q_start, R, 0, blockIdx.x, first, n);
     if (n == 0) return;
     const float d = decay[head];
     const int at = (tid & 31) * 4;
@@ -475,17 +475,20 @@ __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const f
 }
 
 // The state every chunk starts from, in its sum's place, and the state a portion leaves.  grid (R * blocks), blocks = ceil(H dk dv / 1024).
-__global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, const int* slot_ids, int H, int cells) {
+__global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, int R, const int* slot_ids, int H, int cells) {
     pdl_enter();
     const size_t all = (size_t)H * cells;                   // cells = dk dv, a multiple of 4
     const unsigned blocks = (unsigned)((all + 1023) / 1024);
-    const int r = blockIdx.x / blocks, n = q_start[r + 1] - q_start[r], count = (n + RC - 1) / RC;
+    int chunk0;
+    const int r = long_request<RC>(q_start, R, 0, blockIdx.x / blocks, chunk0);
+    if (r < 0) return;
+    const int n = q_start[r + 1] - q_start[r], count = (n + RC - 1) / RC;
     const size_t i = ((size_t)(blockIdx.x % blocks) * 256 + threadIdx.x) * 4;
-    if (i >= all || n <= 0) return;
+    if (i >= all) return;
     const float d = decay[i / cells], full = ret_power(d, RC), rest = ret_power(d, n - (count - 1) * RC);
     float4* mine = reinterpret_cast<float4*>(state + (size_t)slot_ids[r] * all + i);
     float4 S = *mine;
-    float* at = KV + (size_t)first_chunk_of<RC>(q_start, r) * all + i;
+    float* at = KV + (size_t)chunk0 * all + i;
     for (int c0 = 0; c0 < count; c0 += 4) {
         float4 built[4];
 #pragma unroll
@@ -518,7 +521,7 @@ __global__ void __launch_bounds__(256, 2) ret_out_kernel(const float* qp, const 
     float* pw = B + ret_out_slices(dkp);                    // [65]
     const int head = blockIdx.y, col0 = blockIdx.z * 128, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int first = 0, n = 0;
-    chunk_of<RC>(q_start, R, blockIdx.x, first, n);
+    chunk_of<RC>(q_start, R, 0, blockIdx.x, first, n);
     if (n == 0) return;
     if (tid <= RC) pw[tid] = ret_power(decay[head], tid);
     for (int t = warp; t < RC; t += 8)
@@ -686,7 +689,7 @@ Q6K_API int q6k_retention_chunked(const float* p, int ld, int q_col, int k_col, 
         return q6k_check_launch("retention: shared memory attribute");
     q6k_launch(ret_outer_kernel, dim3(n_chunks, H, (dk + 127) / 128 * cols), 256, smem1, st, p + k_col, p + v_col, ld, decay, q_start, R, chunks, H, dk, dv);
     if (int rc = q6k_check_launch("ret_outer")) return rc;
-    q6k_launch(ret_fold_kernel, dim3((unsigned)(R * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, slot_ids, H, dk * dv);
+    q6k_launch(ret_fold_kernel, dim3((unsigned)(R * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, R, slot_ids, H, dk * dv);
     if (int rc = q6k_check_launch("ret_fold")) return rc;
     q6k_launch(ret_out_kernel, dim3(n_chunks, H, cols), 256, smem2, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, o, H, dk, dv, dkp);
     return q6k_check_launch("ret_out");

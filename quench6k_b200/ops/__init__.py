@@ -1491,16 +1491,25 @@ def gated_delta_max_dim() -> int:
     return lib.q6k_gated_delta_max_dim()
 
 
-def gated_delta_chunks(longest: int, G: int, H: int, dk: int, dv: int) -> bool:
-    """Whether a step whose longest portion has `longest` tokens should be walked chunk by chunk: rows of u and of the state that
-    start on 16 bytes, and more tokens than the walk token by token (235 ns each) gets through while the chunks' own kernel
-    runs (about 12 us)."""
-    return longest > 64 and dk % 4 == 0 and dv % 4 == 0 and (2 * G * dk + H * dv) % 4 == 0
+CHUNKS_BEYOND = 64      # where a step goes chunk by chunk, its portions of up to so many tokens are walked token by token
+
+
+def gated_delta_chunks(longest: int, G: int, H: int, dk: int, dv: int, q_lens=()) -> bool:
+    """Whether a step whose longest portion has `longest` tokens may be walked chunk by chunk: rows of u and of the state that start on 16
+    bytes, and a portion that does not go token by token all the same.  q_lens, the tokens of the step's portions: whether it
+    should be.  Token by token a portion takes 235 ns a token, by chunks 110 after the chunks' own kernel (12 us); portions of up to
+    CHUNKS_BEYOND tokens then wait for a launch of their own.  A whole layer of 16 heads of 128 x 128, token by token and by chunks, in
+    us: 97 tokens 64 and 65, 130 tokens 76 and 72 (8 heads: 112 tokens 60 and 61, 130 tokens 70 and 68); 130 beside one of 8
+    tokens 78 and 80, beside 32 of one 105 and 125; 200 beside one of 32 107 and 105; 256 beside 32 of one 154 and 140."""
+    if longest <= CHUNKS_BEYOND or dk % 4 or dv % 4 or (2 * G * dk + H * dv) % 4:
+        return False
+    short = [n for n in q_lens if n <= CHUNKS_BEYOND]
+    return not q_lens or longest > 116 + (30 + 2 * max(short) + 3 * len(short) if short else 0)
 
 
 def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                 q_start: torch.Tensor, slot_ids: torch.Tensor, R: int, H: int, G: int, dk: int, dv: int, prepare: bool = False,
-                chunked: bool = False) -> torch.Tensor:
+                chunked: bool = False, shortest: int = 0) -> torch.Tensor:
     """The gated delta rule over the step's rows, request by request, from and into state [slots, H, dv, dk] (FP32):
     S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, with unit q (times dk^-1/2) and k.  u: FP32 [T, >= 2 G dk + H dv]
     = [q | k | v]; p: FP32 rows holding the H beta logits at b_col and the H decay inputs at a_col.  Returns FP32 o [T, H dv].
@@ -1508,7 +1517,8 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
     and the recurrence fetches a tile of tokens while it walks the one before (for steps with long portions); else the
     recurrence makes them itself.  The results are the same bit for bit.  chunked (with prepare, where gated_delta_chunks(...)
     says so): 32 tokens at a time as a triangular system, equal to the others up to rounding, if the chunks' matrices take no more than
-    256 MB."""
+    256 MB.  shortest: tokens of the step's shortest portion; where it says that there are portions of up to CHUNKS_BEYOND tokens beside
+    the long ones, those are walked token by token all the same (the same bits as in a step of their own)."""
     _need(u, "u", torch.float32)
     _need(p, "p", torch.float32)
     _need(A_log, "A_log", torch.float32, (H,))
@@ -1519,17 +1529,17 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
         raise KernelError("gated_delta: shapes disagree")
     o = torch.empty((T, H * dv), dtype=torch.float32, device=u.device)
     bg = torch.empty((T, 2 * H + G), dtype=torch.float32, device=u.device) if prepare else None
-    chunks = None
+    chunks, beyond = None, CHUNKS_BEYOND if 0 < shortest <= CHUNKS_BEYOND else 0
     if chunked:
         if not prepare:
             raise KernelError("gated_delta: chunks go with prepared inputs")
         lib = library()
         lib.q6k_gated_delta_chunk_floats.restype = ctypes.c_longlong
-        floats = lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H))
+        floats = lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H), _i(beyond))
         if floats <= 64 << 20:
             chunks = torch.empty(floats, dtype=torch.float32, device=u.device)
     _call("q6k_gated_delta", _ptr(u), _i(u.stride(0)), _ptr(p), _i(p.stride(0)), _i(b_col), _i(a_col), _ptr(A_log), _ptr(dt_bias), _ptr(bg),
-          _ptr(chunks), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
+          _ptr(chunks), _i(beyond), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
     return o
 
 

@@ -127,7 +127,8 @@ class GatedDelta(Mixer):
         else:
             o = ops.gated_delta(u, p, self.b_col, self.a_col, self.A_log, self.dt_bias, state["S"], ctx.q_start, ctx.slot_ids, ctx.R,
                                 self.H, self.G, self.dk, self.dv, prepare=prepare,
-                                chunked=prepare and ops.gated_delta_chunks(ctx.max_q_len, self.G, self.H, self.dk, self.dv))
+                                chunked=prepare and ops.gated_delta_chunks(ctx.max_q_len, self.G, self.H, self.dk, self.dv, ctx.q_lens),
+                                shortest=min(ctx.q_lens, default=0))
         ops.current_tag = "delta.out"
         y = ops.delta_out(o, low, g_col, self.norm_w, self.eps, self.H, self.dv, rt.dtype, gate=self.gate)
         ops.current_tag = "delta.o"

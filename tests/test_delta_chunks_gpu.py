@@ -40,3 +40,30 @@ def test_chunks_against_the_walk(H, G, dk, dv, rate):
         # both sum the same FP32 products, in another order; a chunk's are shorter sums.  1e-6: eight roundings of the result
         assert far(got, want) <= max(1.2 * far(walk, want), 1e-6), (far(got, want), far(walk, want))
     assert torch.equal(s_chunk[4], state[4])                   # a slot of no request of this step
+
+
+@pytest.mark.parametrize("lens", [[1, 100, 64, 65, 1, 7, 130], [65], [64, 1, 66], [1] * 30 + [97]])
+def test_short_portions_beside_long_ones_are_walked(lens):
+    """Said that there are short portions, a step walks them as a step of their own would, bit for bit; the long ones go chunk by chunk."""
+    from quench6k_b200 import ops
+    H, G, dk, dv = 4, 2, 64, 36
+    g = torch.Generator().manual_seed(len(lens))
+    T, R = sum(lens), len(lens)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    u, p = rnd(T, 2 * G * dk + H * dv), rnd(T, 2 * H)
+    A_log, dt_bias, state = rnd(H) * 0.5 - 2.0, rnd(H) * 0.5, rnd(R, H, dv, dk) * 0.3
+    A_log[0] = 6.0                                                       # decays whose logarithms are below -200
+    starts = [sum(lens[:i]) for i in range(R + 1)]
+
+    def run(rows, q_start, slots, **kw):
+        s = state.clone()
+        o = ops.gated_delta(u[rows].clone(), p[rows].contiguous(), 0, H, A_log, dt_bias, s, i32(q_start), i32(slots), len(slots), H, G, dk, dv, prepare=True, **kw)
+        return o, s
+
+    mixed, s_mixed = run(slice(0, T), starts, list(range(R)), chunked=True, shortest=min(lens))
+    chunked, s_chunked = run(slice(0, T), starts, list(range(R)), chunked=True)
+    for r, n in enumerate(lens):
+        rows = slice(starts[r], starts[r + 1])
+        o, s = run(rows, [0, n], [r]) if n <= ops.CHUNKS_BEYOND else (chunked[rows], s_chunked)
+        assert torch.equal(mixed[rows], o) and torch.equal(s_mixed[r], s[r]), (r, n)
