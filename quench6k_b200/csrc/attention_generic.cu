@@ -17,79 +17,92 @@ namespace {
 
 constexpr int MAX_HD = 256, DPL = MAX_HD / 32;   // head dims per lane
 
+// One query head h of row t, by a warp; qw: hd floats of shared memory of its own.
+template <typename T>
+__device__ __forceinline__ void attention_row(const T* q, const T* k_pages, const T* v_pages, const int* bt, int page_size, size_t head_base, int pos, int lo,
+                                              const float* sinks, float scale, T* out, int t, int h, int Hq, int hd, float* qw) {
+    const int lane = threadIdx.x & 31;
+    for (int d = lane; d < hd; d += 32) qw[d] = to_f32(q[((size_t)t * Hq + h) * hd + d]);
+    __syncwarp();
+    float m = -INFINITY, l = 0.0f, o[DPL];
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) o[i] = 0.0f;
+    for (int j0 = lo & ~31; j0 <= pos; j0 += 32) {
+        const int j = j0 + lane;
+        const bool ok = j >= lo && j <= pos;
+        float s = -INFINITY;
+        size_t row = 0;
+        if (ok) {
+            const int page = bt[j / page_size];
+            row = ((head_base + page) * page_size + j % page_size) * hd;
+            const T* kr = k_pages + row;
+            float acc = 0.0f;
+            for (int d = 0; d < hd; ++d) acc = fmaf(qw[d], to_f32(kr[d]), acc);
+            s = acc * scale;
+        }
+        const float mt = warp_max(s);
+        const float mn = fmaxf(m, mt);          // finite: the tile holds at least one visible key
+        const float corr = m == -INFINITY ? 0.0f : expf(m - mn);
+        float p = ok ? round_to<T>(expf(s - mn)) : 0.0f;
+        l = l * corr + warp_sum(p);
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) o[i] *= corr;
+        const int nk = min(32, pos - j0 + 1);
+        for (int jj = 0; jj < nk; ++jj) {
+            const float pj = __shfl_sync(0xffffffffu, p, jj);
+            const unsigned long long rj = __shfl_sync(0xffffffffu, (unsigned long long)row, jj);
+            if (pj == 0.0f) continue;           // uniform across the warp
+            const T* vr = v_pages + rj;
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                const int d = lane + 32 * i;
+                if (d < hd) o[i] = fmaf(pj, to_f32(vr[d]), o[i]);
+            }
+        }
+        m = mn;
+    }
+    float den = l;
+    float osc = 1.0f;
+    if (sinks) {
+        const float sk = sinks[h];
+        const float M = fmaxf(m, sk);
+        osc = expf(m - M);
+        den = l * osc + expf(sk - M);
+    }
+    const float inv = osc / den;
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) {
+        const int d = lane + 32 * i;
+        if (d < hd) out[((size_t)t * Hq + h) * hd + d] = from_f32<T>(o[i] * inv);
+    }
+    __syncwarp();
+}
+
+// Whether fewer than `least` rows of the step, one after the other, belong to row t's request (rows [ta, tb) around t are known to).
+__device__ __forceinline__ bool few_rows(const int* req_of_token, int ta, int tb, int T_, int least) {
+    const int req = req_of_token[ta];
+    while (tb - ta < least && ta > 0 && req_of_token[ta - 1] == req) --ta;
+    while (tb - ta < least && tb < T_ && req_of_token[tb] == req) ++tb;
+    return tb - ta < least;
+}
+
+// least > 0: requests of at least so many rows belong to the launch of row tiles.
 template <typename T>
 __global__ void __launch_bounds__(128) attention_generic_kernel(const T* q, const T* k_pages, const T* v_pages,
                                                                 const int* block_table, int max_blocks, int page_size,
                                                                 int num_pages, const int* req_of_token, const int* positions, int window,
-                                                                const float* sinks, float scale, T* out, int Hq, int Hkv,
-                                                                int hd) {
+                                                                const float* sinks, float scale, T* out, int T_, int Hq, int Hkv,
+                                                                int hd, int least) {
     pdl_enter();
     extern __shared__ float qs[];             // [warps][hd]
     const int t = blockIdx.x, kh = blockIdx.y, G = Hq / Hkv;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (least > 0 && !few_rows(req_of_token, t, t + 1, T_, least)) return;
+    const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int pos = positions[t];
     const int* bt = block_table + (size_t)req_of_token[t] * max_blocks;
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
-    float* qw = qs + warp * hd;
-    const size_t head_base = (size_t)kh * num_pages;          // pools are [Hkv, num_pages, page_size, hd]
-
-    for (int g = warp; g < G; g += nwarps) {
-        const int h = kh * G + g;
-        for (int d = lane; d < hd; d += 32) qw[d] = to_f32(q[((size_t)t * Hq + h) * hd + d]);
-        __syncwarp();
-        float m = -INFINITY, l = 0.0f, o[DPL];
-#pragma unroll
-        for (int i = 0; i < DPL; ++i) o[i] = 0.0f;
-        for (int j0 = lo & ~31; j0 <= pos; j0 += 32) {
-            const int j = j0 + lane;
-            const bool ok = j >= lo && j <= pos;
-            float s = -INFINITY;
-            size_t row = 0;
-            if (ok) {
-                const int page = bt[j / page_size];
-                row = ((head_base + page) * page_size + j % page_size) * hd;
-                const T* kr = k_pages + row;
-                float acc = 0.0f;
-                for (int d = 0; d < hd; ++d) acc = fmaf(qw[d], to_f32(kr[d]), acc);
-                s = acc * scale;
-            }
-            const float mt = warp_max(s);
-            const float mn = fmaxf(m, mt);          // finite: the tile holds at least one visible key
-            const float corr = m == -INFINITY ? 0.0f : expf(m - mn);
-            float p = ok ? round_to<T>(expf(s - mn)) : 0.0f;
-            l = l * corr + warp_sum(p);
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) o[i] *= corr;
-            const int nk = min(32, pos - j0 + 1);
-            for (int jj = 0; jj < nk; ++jj) {
-                const float pj = __shfl_sync(0xffffffffu, p, jj);
-                const unsigned long long rj = __shfl_sync(0xffffffffu, (unsigned long long)row, jj);
-                if (pj == 0.0f) continue;           // uniform across the warp
-                const T* vr = v_pages + rj;
-#pragma unroll
-                for (int i = 0; i < DPL; ++i) {
-                    const int d = lane + 32 * i;
-                    if (d < hd) o[i] = fmaf(pj, to_f32(vr[d]), o[i]);
-                }
-            }
-            m = mn;
-        }
-        float den = l;
-        float osc = 1.0f;
-        if (sinks) {
-            const float sk = sinks[h];
-            const float M = fmaxf(m, sk);
-            osc = expf(m - M);
-            den = l * osc + expf(sk - M);
-        }
-        const float inv = osc / den;
-#pragma unroll
-        for (int i = 0; i < DPL; ++i) {
-            const int d = lane + 32 * i;
-            if (d < hd) out[((size_t)t * Hq + h) * hd + d] = from_f32<T>(o[i] * inv);
-        }
-        __syncwarp();
-    }
+    for (int g = warp; g < G; g += nwarps)       // pools are [Hkv, num_pages, page_size, hd]
+        attention_row(q, k_pages, v_pages, bt, page_size, (size_t)kh * num_pages, pos, lo, sinks, scale, out, t, kh * G + g, Hq, hd, qs + warp * hd);
 }
 
 // The same for steps that bring several tokens per request: the same sums in the same order (a row's scores are summed over ascending
@@ -100,7 +113,9 @@ __global__ void __launch_bounds__(128) attention_generic_kernel(const T* q, cons
 // over 509 keys, waiting for loads.  Here a block takes up to 32 rows (the query heads of a KV head for consecutive tokens of the step)
 // and brings each key tile into shared memory once; 8 threads share a row: each makes the scores of four keys and owns every
 // eighth group of four dimensions of the result, so that a 16-byte read of keys or values serves four rows and a warp's reads fall into
-// different banks: 92 us.  Tokens of several requests in one block are taken request by request.
+// different banks: 92 us.  Tokens of several requests in one block are taken request by request, so where a block could meet many,
+// requests of fewer than `least` tokens are left to the kernel above.  8 heads on 8 KV heads, 509 tokens beside 32 requests of 4,000 keys: a
+// block walked the contexts of 32 tokens one after the other, 15,700 us; all rows in the kernel above 4,470; so 2,830.
 constexpr int GT_ROWS = 32, GT_KEYS = 32, GT_THREADS = 256;
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -113,7 +128,7 @@ template <typename T, int NI>          // NI: groups of 32 dimensions (hd <= 32 
 __global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q, const T* k_pages, const T* v_pages, const int* block_table, int max_blocks,
                                                                      int page_size, int num_pages, const int* req_of_token, const int* positions,
                                                                      int window, const float* sinks, float scale, T* out, int T_, int Hq, int Hkv, int hd,
-                                                                     int tokens, int heads) {
+                                                                     int tokens, int heads, int least) {
     pdl_enter();
     extern __shared__ __align__(16) float gt_smem[];
     const int ld = hd + 4;
@@ -123,13 +138,18 @@ __global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q,
     float* ss = vs + GT_KEYS * ld;                    // [GT_ROWS][GT_KEYS + 4]: scores, then weights
     float* corr_s = ss + GT_ROWS * (GT_KEYS + 4);     // [GT_ROWS]: what a row's result is multiplied by before the tile, at the end by
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = Hq / Hkv;
-    const int t0 = blockIdx.x * tokens, t1 = min(T_, t0 + tokens), kh = blockIdx.y, g0 = blockIdx.z * heads, here = min(heads, G - g0);
-    const int row = tid >> 3, c = tid & 7;            // this thread's row and place in it; row = token * heads + head
+    const int kh = blockIdx.y, g0 = blockIdx.z * heads, here = min(heads, G - g0);
     const size_t head_base = (size_t)kh * num_pages;
+    const int t0 = blockIdx.x * tokens, t1 = min(T_, t0 + tokens);
+    const int row = tid >> 3, c = tid & 7;            // this thread's row and place in it; row = token * heads + head
     for (int ta = t0; ta < t1;) {
         const int req = req_of_token[ta];
         int tb = ta + 1, pos_min = positions[ta], pos_max = pos_min;        // the rows' positions may come in any order
         for (; tb < t1 && req_of_token[tb] == req; ++tb) pos_min = min(pos_min, positions[tb]), pos_max = max(pos_max, positions[tb]);
+        if (least > 0 && few_rows(req_of_token, ta, tb, T_, least)) {
+            ta = tb;
+            continue;
+        }
         const int* bt = block_table + (size_t)req * max_blocks;
         const int rows = (tb - ta) * heads, k_end = pos_max + 1;
         const int lo_first = window > 0 ? max(0, pos_min - window + 1) : 0;
@@ -256,10 +276,10 @@ __global__ void __launch_bounds__(GT_THREADS) attention_tiled_kernel(const T* q,
 
 // q: [T, Hq, hd]; pages: [Hkv, num_pages, page_size, hd]; block_table: [R, max_blocks];
 // window 0: every earlier key is visible; sinks: FP32 [Hq] or null; out: [T, Hq*hd].  requests: how many the step's rows belong to
-// (0: not said).
+// (0: not said); shortest: the rows of the one with the fewest (0: not said).
 Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void* v_pages, int num_pages, const int* block_table,
                                   int max_blocks, int page_size, const int* req_of_token, const int* positions, int window,
-                                  const float* sinks, float scale, void* out, int T_, int Hq, int Hkv, int hd, int dtype, int requests,
+                                  const float* sinks, float scale, void* out, int T_, int Hq, int Hkv, int hd, int dtype, int requests, int shortest,
                                   cudaStream_t st) {
     if (T_ == 0) return 0;
     Q6K_REQUIRE(T_ > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0, "attention: bad head counts Hq=%d Hkv=%d", Hq, Hkv);
@@ -269,9 +289,13 @@ Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void
     Q6K_REQUIRE(Hkv <= 65535, "attention: %d KV heads exceed the grid limit", Hkv);
     const int G = Hq / Hkv;
     // Several tokens per request: row tiles (92 us against 500 where a step brings 509 tokens of one request).  A decode step (a token
-    // each) would leave most of a tile's rows empty and keeps a block per token.
-    if (requests > 0 && T_ >= 4 * requests && (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
-        const int heads = G < GT_ROWS ? G : GT_ROWS, tokens = GT_ROWS / heads;
+    // each) would leave most of a tile's rows empty and keeps a block per token.  A tile takes 0.30 us a key for each request it
+    // meets in turn, a warp of the other kernel 0.70 for a fourth of the heads: tiles of up to 4 tokens take every request; larger ones those that
+    // fill half of one, so that none meets more than three.  The others then wait for a launch of their own, which pays where they are
+    // few beside the rows of long portions (8 heads on 2, window of 128: 509 tokens beside 32 of one 315 -> 150 us, 60 beside 8 95 -> 114).
+    const int heads = G < GT_ROWS ? G : GT_ROWS, tokens = GT_ROWS / heads;
+    int least = tokens > 4 && requests > 1 && shortest < tokens / 2 ? tokens / 2 : 0;
+    if (requests > 0 && T_ >= (least > 0 ? 16 : 4) * requests && (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
         const size_t smem = (size_t)((GT_ROWS + 2 * GT_KEYS) * (hd + 4) + GT_ROWS * (GT_KEYS + 4) + GT_ROWS) * sizeof(float);
         const dim3 tiles((T_ + tokens - 1) / tokens, Hkv, (G + heads - 1) / heads);
 #define TILED(NI)                                                                                                                                       \
@@ -279,7 +303,7 @@ Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void
         if (cudaFuncSetAttribute(attention_tiled_kernel<T, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)                 \
             return q6k_check_launch("attention_tiled: shared memory attribute");                                                                        \
         q6k_launch(attention_tiled_kernel<T, NI>, tiles, GT_THREADS, smem, st, (const T*)q, (const T*)k_pages, (const T*)v_pages, block_table,          \
-                   max_blocks, page_size, num_pages, req_of_token, positions, window, sinks, scale, (T*)out, T_, Hq, Hkv, hd, tokens, heads);           \
+                   max_blocks, page_size, num_pages, req_of_token, positions, window, sinks, scale, (T*)out, T_, Hq, Hkv, hd, tokens, heads, least);    \
     } while (0)
         Q6K_DISPATCH(dtype, {
             if (hd <= 32) TILED(1);
@@ -288,12 +312,15 @@ Q6K_API int q6k_attention_generic(const void* q, const void* k_pages, const void
             else TILED(8);
         });
 #undef TILED
-        return q6k_check_launch("attention_tiled");
+        const int rc = q6k_check_launch("attention_tiled");
+        if (rc || least == 0) return rc;
+    } else {
+        least = 0;
     }
     const int warps = G < 4 ? G : 4;
     dim3 grid(T_, Hkv);
     Q6K_DISPATCH(dtype, q6k_launch(attention_generic_kernel<T>, grid, warps * 32, warps * hd * sizeof(float), st, 
                             (const T*)q, (const T*)k_pages, (const T*)v_pages, block_table, max_blocks, page_size,
-                            num_pages, req_of_token, positions, window, sinks, scale, (T*)out, Hq, Hkv, hd););
+                            num_pages, req_of_token, positions, window, sinks, scale, (T*)out, T_, Hq, Hkv, hd, least););
     return q6k_check_launch("attention_generic");
 }

@@ -621,8 +621,9 @@ def qk_prep(qkv: torch.Tensor, Hq: int, Hkv: int, hd: int, q_norm, k_norm, eps: 
 
 def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
                       req_of_token: torch.Tensor, positions: torch.Tensor, window: Optional[int],
-                      sinks: Optional[torch.Tensor], scale: Optional[float] = None) -> torch.Tensor:
-    """Causal (optionally windowed, optionally with sinks) attention of every row over its request's pages."""
+                      sinks: Optional[torch.Tensor], scale: Optional[float] = None, shortest: int = 0) -> torch.Tensor:
+    """Causal (optionally windowed, optionally with sinks) attention of every row over its request's pages.  shortest: rows of the
+    request with the fewest, if known (it chooses the kernels, not the result)."""
     _need(q, "q")
     T, Hq, hd = q.shape
     _need(k_pages, "k_pages", q.dtype)
@@ -639,7 +640,7 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
     _call("q6k_attention_generic", _ptr(q), _ptr(k_pages), _ptr(v_pages), _i(num_pages), _ptr(block_table), _i(block_table.shape[1]),
           _i(page_size), _ptr(req_of_token), _ptr(positions), _i(window or 0), _ptr(sinks),
           _f(scale if scale is not None else 1.0 / math.sqrt(hd)), _ptr(out), _i(T), _i(Hq), _i(Hkv), _i(hd),
-          _i(dtype_code(q.dtype)), _i(block_table.shape[0]), _stream())
+          _i(dtype_code(q.dtype)), _i(block_table.shape[0]), _i(shortest), _stream())
     return out
 
 

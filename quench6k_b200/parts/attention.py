@@ -331,7 +331,8 @@ class Attention(Mixer):
 
     def _attend(self, q, cache, table, ctx, how):
         if how[0] == "generic":
-            return ops.attention_generic(q, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, self.window, self.sinks, self.scale)
+            return ops.attention_generic(q, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, self.window, self.sinks, self.scale,
+                                         shortest=min(ctx.q_lens, default=0))
         if how[0] == "tc":
             (tok0, ntok), short = how[1], how[2]
             out = ops.attention_tc(q, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, tok0, ntok, self.window,

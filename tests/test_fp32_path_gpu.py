@@ -59,6 +59,32 @@ def test_rows_in_any_order(window):
             assert torch.equal(ops.attention_generic(q[t:t + 1], k, v, table, req[:1], pos[t:t + 1], window, None)[0], whole[t]), (t, int(pos[t]))
 
 
+@pytest.mark.parametrize("Hq, Hkv, hd", [(8, 8, 64), (8, 2, 128), (12, 2, 32)])          # tiles of 32, 8 and 5 tokens
+def test_decoding_requests_beside_a_portion_do_not_wait_for_one_another(Hq, Hkv, hd):
+    """A portion beside 32 requests deep in their contexts takes less than three times what it takes beside one of them: each is
+    walked by warps of its own, not one after the other in the block of a row tile (32 times)."""
+    from quench6k_b200 import ops
+    depth, page, portion, most = 2000, 16, 640, 32
+    pages = -(-depth // page)
+    k, v = (torch.randn(Hkv, pages * (most + 1), page, hd, device="cuda") for _ in range(2))
+    table = torch.arange(pages * (most + 1), dtype=torch.int32, device="cuda").view(most + 1, pages)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    def took(n):
+        q = torch.randn(portion + n, Hq, hd, device="cuda")
+        req, pos = i32([0] * portion + list(range(1, n + 1))), i32(list(range(portion)) + [depth - 1] * n)
+        run = lambda: ops.attention_generic(q, k, v, table[:n + 1].contiguous(), req, pos, None, None)
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(); run(); b.record(); torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[1:])
+
+    one, many = took(1), took(most)
+    assert many < 3 * one, (one, many)
+
+
 @pytest.mark.parametrize("M, N, K, offset", [(1, 1, 1, 0), (64, 64, 32, 0), (65, 63, 33, 0), (3, 130, 36, 0), (130, 70, 100, 1), (17, 257, 1000, 0), (200, 65, 4, 0)])
 def test_fp32_product_at_the_edges_of_its_tiles(M, N, K, offset):
     """offset: the operands start off a 16-byte boundary (copies of 4 bytes)."""
