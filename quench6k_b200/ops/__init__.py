@@ -56,8 +56,8 @@ def _need(t: torch.Tensor, name: str, dtype=None, shape=None):
         raise KernelError(f"{name} has shape {tuple(t.shape)}, expected {tuple(shape)}")
 
 
-# kernels launched per exported function (for launch accounting in benchmarks)
-_LAUNCHES = {"q6k_gated_delta": 1, "q6k_delta_channel": 1, "q6k_retention_chunked": 3, "q6k_attention_flex_mma": 2, "q6k_attention_flex_tc": 2, "q6k_selective_scan": 1, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
+# kernels launched per exported function (for launch accounting in benchmarks), unless the call says how many
+_LAUNCHES = {"q6k_delta_channel": 1, "q6k_retention_chunked": 3, "q6k_attention_flex_mma": 2, "q6k_moe_permute": 3, "q6k_moe_plan": 3, "q6k_gemm_tc": 1, "q6k_attention_mma": 2, "q6k_argmax": 2, "q6k_gemm_tc_pairs_scratch": 0}
 launch_count = 0
 
 
@@ -91,9 +91,9 @@ def profile_end():
     return out
 
 
-def _call(fn_name: str, *args):
+def _call(fn_name: str, *args, launches: Optional[int] = None):
     global launch_count
-    launch_count += _LAUNCHES.get(fn_name, 1)
+    launch_count += _LAUNCHES.get(fn_name, 1) if launches is None else launches
     fn = _functions.get(fn_name)
     if fn is None:
         fn = _functions[fn_name] = getattr(library(), fn_name)
@@ -1333,7 +1333,7 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
               _ptr(v_pages), _i(v_pages.stride(2)), _i(dv), _i(num_pages), _ptr(block_table), _i(block_table.shape[1]), _i(page_size),
               _ptr(req_of_token), _ptr(positions), _ptr(tok0), _ptr(ntok), _i(n_tiles), _i(window or 0), _i(chunk or 0), _f(scale), _ptr(out),
               _i(1 if out_head_major else 0), _i(T), _i(H), _i(Hkv), _i(nsplit), _i(split_keys), _ptr(ws), _ptr(talk), _ptr(sinks), _f(softcap),
-              _i(maps), _ptr(out if out_f32 else None), _stream())
+              _i(maps), _ptr(out if out_f32 else None), _stream(), launches=2 if talk is not None or nsplit > 1 else 1)
         return out
     if (tiles is not None and k_pages.dtype == torch.bfloat16 and not (talk is not None and out_head_major)
             and attention_flex_mma_supported(H, Hkv, dk, dv, k_pages.stride(2), v_pages.stride(2), db, shared_v)):
@@ -1540,7 +1540,8 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
         if floats <= 64 << 20:
             chunks = torch.empty(floats, dtype=torch.float32, device=u.device)
     _call("q6k_gated_delta", _ptr(u), _i(u.stride(0)), _ptr(p), _i(p.stride(0)), _i(b_col), _i(a_col), _ptr(A_log), _ptr(dt_bias), _ptr(bg),
-          _ptr(chunks), _i(beyond), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream())
+          _ptr(chunks), _i(beyond), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream(),
+          launches=int(prepare) + (2 if chunks is not None and T > beyond else 0) + (1 if chunks is None or beyond else 0))
     return o
 
 
