@@ -1493,6 +1493,7 @@ def gated_delta_max_dim() -> int:
 
 
 CHUNKS_BEYOND = 64      # where a step goes chunk by chunk, its portions of up to so many tokens are walked token by token
+CHUNK_SCRATCH_FLOATS = 64 << 20      # 256 MB: a step whose chunks need more is walked token by token
 
 
 def gated_delta_chunks(longest: int, G: int, H: int, dk: int, dv: int, q_lens=()) -> bool:
@@ -1537,7 +1538,7 @@ def gated_delta(u: torch.Tensor, p: torch.Tensor, b_col: int, a_col: int, A_log:
         lib = library()
         lib.q6k_gated_delta_chunk_floats.restype = ctypes.c_longlong
         floats = lib.q6k_gated_delta_chunk_floats(_i(T), _i(R), _i(H), _i(beyond))
-        if floats <= 64 << 20:
+        if floats <= CHUNK_SCRATCH_FLOATS:
             chunks = torch.empty(floats, dtype=torch.float32, device=u.device)
     _call("q6k_gated_delta", _ptr(u), _i(u.stride(0)), _ptr(p), _i(p.stride(0)), _i(b_col), _i(a_col), _ptr(A_log), _ptr(dt_bias), _ptr(bg),
           _ptr(chunks), _i(beyond), _ptr(state), _ptr(q_start), _ptr(slot_ids), _ptr(o), _i(T), _i(R), _i(H), _i(G), _i(dk), _i(dv), _stream(),

@@ -67,3 +67,22 @@ def test_short_portions_beside_long_ones_are_walked(lens):
         rows = slice(starts[r], starts[r + 1])
         o, s = run(rows, [0, n], [r]) if n <= ops.CHUNKS_BEYOND else (chunked[rows], s_chunked)
         assert torch.equal(mixed[rows], o) and torch.equal(s_mixed[r], s[r]), (r, n)
+
+
+def test_more_scratch_than_the_limit_is_walked(monkeypatch):
+    """A step whose chunks' matrices would pass the limit goes token by token: decays, not their logarithms, and the walk's bits."""
+    from quench6k_b200 import ops
+    H, G, dk, dv, T = 2, 1, 32, 16, 100
+    g = torch.Generator().manual_seed(1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    u, p, A_log, dt_bias, state = rnd(T, 2 * G * dk + H * dv), rnd(T, 2 * H), rnd(H), rnd(H), rnd(1, H, dv, dk)
+
+    def run(**kw):
+        s = state.clone()
+        return ops.gated_delta(u.clone(), p, 0, H, A_log, dt_bias, s, i32([0, T]), i32([0]), 1, H, G, dk, dv, prepare=True, **kw), s
+
+    walk, chunks = run(), run(chunked=True)
+    assert not torch.equal(walk[0], chunks[0])
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_FLOATS", 1000)
+    assert all(torch.equal(a, b) for a, b in zip(run(chunked=True), walk))
