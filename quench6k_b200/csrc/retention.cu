@@ -126,10 +126,11 @@ __device__ __forceinline__ void ret_copy16(float* dst, const float* src, bool in
 // [slots, H, dk, dv]; o: FP32 [T, H dv].  RPT: rows per thread (dk <= 16 RPT).  STAGES tiles are in flight or in use.
 // WIDE: every head's q and k (and decays) start on 16 bytes in every row and dk is a multiple of 4 (copies of 16 bytes).
 // TM: the second recurrence; q is r, wt: FP32 [T, ld_w] with the decays of head h from column h dk on, bonus: FP32 [T, H].
+// Requests of more than `most` tokens are not this launch's.
 template <int RPT, int STAGES, bool WIDE, bool TM>
 __global__ void __launch_bounds__(RET_THREADS) retention_kernel(const float* qp, const float* kp, const float* vp, int ld, const float* decay,
                                                                 const float* wt, int ld_w, const float* bonus, float* state, const int* q_start,
-                                                                const int* slot_ids, float* o, int H, int dk, int dv) {
+                                                                const int* slot_ids, float* o, int H, int dk, int dv, int most) {
     pdl_enter();
     constexpr int DKP = RET_CHUNKS * RPT;                                // rows, padded
     constexpr int PER_THREAD = RET_TILE * DKP / RET_THREADS;             // elements of q (and of k) a thread stages per tile
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(RET_THREADS) retention_kernel(const float* qp,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = lane % RET_COLS, col = c0 + cl;
     const int row0 = (warp * 2 + lane / RET_COLS) * RPT;                 // this thread's first row
     const int t0 = q_start[r], t1 = q_start[r + 1];
-    if (t0 >= t1) return;
+    if (t0 >= t1 || t1 - t0 > most) return;
     const float d = TM ? 0.0f : decay[head];
     float* mine = state + ((size_t)slot_ids[r] * H + head) * dk * dv + (col < dv ? col : 0);
     float s[RPT];
@@ -294,11 +295,11 @@ __global__ void __launch_bounds__(RET_THREADS) retention_kernel(const float* qp,
 
 template <int RPT, int STAGES, bool WIDE, bool TM>
 int launch_retention(dim3 grid, cudaStream_t st, const float* q, const float* k, const float* v, int ld, const float* decay, const float* wt, int ld_w,
-                     const float* bonus, float* state, const int* q_start, const int* slot_ids, float* o, int H, int dk, int dv) {
+                     const float* bonus, float* state, const int* q_start, const int* slot_ids, float* o, int H, int dk, int dv, int most) {
     const size_t smem = (size_t)(STAGES * RET_TILE * ((TM ? 3 : 2) * RET_CHUNKS * RPT + RET_COLS + (TM ? 1 : 0)) + 2 * RET_TILE * RET_WARPS * RET_COLS) * sizeof(float);
     auto kernel = retention_kernel<RPT, STAGES, WIDE, TM>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    q6k_launch(kernel, grid, RET_THREADS, smem, st, q, k, v, ld, decay, wt, ld_w, bonus, state, q_start, slot_ids, o, H, dk, dv);
+    q6k_launch(kernel, grid, RET_THREADS, smem, st, q, k, v, ld, decay, wt, ld_w, bonus, state, q_start, slot_ids, o, H, dk, dv, most);
     return 0;
 }
 
@@ -421,15 +422,15 @@ __device__ __forceinline__ float ret_power(float d, int n) {
     return (float)p;
 }
 
-// grid (chunks, H, ceil(dk / 128) ceil(dv / 128)), 256 threads, 64 KB of dynamic shared memory; KV: FP32 [chunks, H, dk, dv].
-__global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const float* vp, int ld, const float* decay, const int* q_start, int R, float* KV, int H, int dk,
+// grid (H, chunks, ceil(dk / 128) ceil(dv / 128)) (blocks of chunks that there are not come last), 256 threads, 64 KB of dynamic shared memory; KV: FP32 [chunks, H, dk, dv].
+__global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const float* vp, int ld, const float* decay, const int* q_start, int R, int beyond, float* KV, int H, int dk,
                                                         int dv) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     float *ks = sm, *vs = sm + RC * 128;                    // [64][128] each, k times its token's power of d
-    const int head = blockIdx.y, tid = threadIdx.x, cols = (dv + 127) / 128, row0 = blockIdx.z / cols * 128, col0 = blockIdx.z % cols * 128;
+    const int head = blockIdx.x, tid = threadIdx.x, cols = (dv + 127) / 128, row0 = blockIdx.z / cols * 128, col0 = blockIdx.z % cols * 128;
     int first = 0, n = 0;
-    chunk_of<RC>(q_start, R, 0, blockIdx.x, first, n);
+    chunk_of<RC>(q_start, R, beyond, blockIdx.y, first, n);
     if (n == 0) return;
     const float d = decay[head];
     const int at = (tid & 31) * 4;
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const f
             fma_pair(acc[i][0], aa, b0.x), fma_pair(acc[i][1], aa, b0.y), fma_pair(acc[i][2], aa, b1.x), fma_pair(acc[i][3], aa, b1.y);
         }
     }
-    float* out = KV + ((size_t)blockIdx.x * H + head) * dk * dv;
+    float* out = KV + ((size_t)blockIdx.y * H + head) * dk * dv;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int rr = row0 + row + (i & 3) + (i >> 2) * 16;
@@ -474,13 +475,13 @@ __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const f
     }
 }
 
-// The state every chunk starts from, in its sum's place, and the state a portion leaves.  grid (R * blocks), blocks = ceil(H dk dv / 1024).
-__global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, int R, const int* slot_ids, int H, int cells) {
+// The state every chunk starts from, in its sum's place, and the state a portion leaves.  grid (long requests * blocks), blocks = ceil(H dk dv / 1024).
+__global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, int R, int beyond, const int* slot_ids, int H, int cells) {
     pdl_enter();
     const size_t all = (size_t)H * cells;                   // cells = dk dv, a multiple of 4
     const unsigned blocks = (unsigned)((all + 1023) / 1024);
     int chunk0;
-    const int r = long_request<RC>(q_start, R, 0, blockIdx.x / blocks, chunk0);
+    const int r = long_request<RC>(q_start, R, beyond, blockIdx.x / blocks, chunk0);
     if (r < 0) return;
     const int n = q_start[r + 1] - q_start[r], count = (n + RC - 1) / RC;
     const size_t i = ((size_t)(blockIdx.x % blocks) * 256 + threadIdx.x) * 4;
@@ -509,9 +510,9 @@ constexpr int RO_SLICE = 32, RO_STAGES = 3, RO_MLD = RC + 4;
 __host__ __device__ constexpr int ret_out_slices(int dkp) { return RC * (dkp + 4) > RO_STAGES * RO_SLICE * 128 ? RC * (dkp + 4) : RO_STAGES * RO_SLICE * 128; }
 __host__ __device__ constexpr int ret_out_floats(int dkp) { return RC * (dkp + 4) + RC * RO_MLD + ret_out_slices(dkp) + RC + 4; }
 
-// grid (chunks, H, ceil(dv / 128)), 256 threads.  dkp: dk rounded up to a multiple of 32.
+// grid (H, chunks, ceil(dv / 128)), 256 threads.  dkp: dk rounded up to a multiple of 32.
 __global__ void __launch_bounds__(256, 2) ret_out_kernel(const float* qp, const float* kp, const float* vp, int ld, const float* decay, const float* KV, const int* q_start,
-                                                         int R, float* o, int H, int dk, int dv, int dkp) {
+                                                         int R, int beyond, float* o, int H, int dk, int dv, int dkp) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int ldq = dkp + 4;
@@ -519,9 +520,9 @@ __global__ void __launch_bounds__(256, 2) ret_out_kernel(const float* qp, const 
     float* M = Q + RC * ldq;                                // [64][68]
     float* B = M + RC * RO_MLD;                             // K [64][ldq], then the slices [3][32][128] of S and V
     float* pw = B + ret_out_slices(dkp);                    // [65]
-    const int head = blockIdx.y, col0 = blockIdx.z * 128, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int head = blockIdx.x, col0 = blockIdx.z * 128, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int first = 0, n = 0;
-    chunk_of<RC>(q_start, R, 0, blockIdx.x, first, n);
+    chunk_of<RC>(q_start, R, beyond, blockIdx.y, first, n);
     if (n == 0) return;
     if (tid <= RC) pw[tid] = ret_power(decay[head], tid);
     for (int t = warp; t < RC; t += 8)
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(256, 2) ret_out_kernel(const float* qp, const 
     }
     __syncthreads();                                        // K is done with, M whole
     const int state_slices = dkp / RO_SLICE, slices = state_slices + (n + RO_SLICE - 1) / RO_SLICE;
-    const float* S = KV + ((size_t)blockIdx.x * H + head) * dk * dv;
+    const float* S = KV + ((size_t)blockIdx.y * H + head) * dk * dv;
     auto fetch = [&](int s) {
         if (s < slices) {
             const int c = col0 + lane * 4;
@@ -651,8 +652,9 @@ Q6K_API int q6k_retention_prep(float* p, int ld, int T_, int H, int dk, int q_co
     return q6k_check_launch("retention_prep");
 }
 
+// most: requests of up to so many tokens (the others are left alone).
 Q6K_API int q6k_retention(const float* p, int ld, int q_col, int k_col, int v_col, const float* decay, float* state, const int* q_start,
-                          const int* slot_ids, int R, float* o, int H, int dk, int dv, cudaStream_t st) {
+                          const int* slot_ids, int R, float* o, int H, int dk, int dv, int most, cudaStream_t st) {
     if (R == 0) return 0;
     Q6K_REQUIRE(R > 0 && H > 0 && dk > 0 && dv > 0 && dk <= RET_MAX_DK, "retention: bad sizes R=%d H=%d dk=%d (at most %d) dv=%d", R, H, dk, RET_MAX_DK, dv);
     const int zb = (dv + RET_COLS - 1) / RET_COLS;
@@ -662,8 +664,8 @@ Q6K_API int q6k_retention(const float* p, int ld, int q_col, int k_col, int v_co
     const bool wide = dk % 4 == 0 && ld % 4 == 0 && on16(p + q_col) && on16(p + k_col);
 #define RET_LAUNCH(RPT)                                                                                                               \
     do {                                                                                                                              \
-        if (wide) launch_retention<RPT, RET_STAGES, true, false>(grid, st, p + q_col, p + k_col, p + v_col, ld, decay, nullptr, 0, nullptr, state, q_start, slot_ids, o, H, dk, dv); \
-        else launch_retention<RPT, RET_STAGES, false, false>(grid, st, p + q_col, p + k_col, p + v_col, ld, decay, nullptr, 0, nullptr, state, q_start, slot_ids, o, H, dk, dv);     \
+        if (wide) launch_retention<RPT, RET_STAGES, true, false>(grid, st, p + q_col, p + k_col, p + v_col, ld, decay, nullptr, 0, nullptr, state, q_start, slot_ids, o, H, dk, dv, most); \
+        else launch_retention<RPT, RET_STAGES, false, false>(grid, st, p + q_col, p + k_col, p + v_col, ld, decay, nullptr, 0, nullptr, state, q_start, slot_ids, o, H, dk, dv, most);     \
     } while (0)
     if (dk <= 64) RET_LAUNCH(4);
     else if (dk <= 128) RET_LAUNCH(8);
@@ -673,25 +675,27 @@ Q6K_API int q6k_retention(const float* p, int ld, int q_col, int k_col, int v_co
 }
 
 // Floats of scratch for the same walk chunk by chunk.
-Q6K_API long long q6k_retention_chunk_floats(int T_, int R, int H, int dk, int dv) { return (long long)(T_ / RC + R) * H * dk * dv; }
+Q6K_API long long q6k_retention_chunk_floats(int T_, int R, int H, int dk, int dv, int beyond) { return (long long)most_chunks<RC>(T_, R, beyond) * H * dk * dv; }
 
-// Chunks of 64 tokens (T_: rows of the step): rows and heads of q, k and v that start on 16 bytes, dk and dv multiples of 4.
+// Requests of more than `beyond` tokens in chunks of 64 (T_: rows of the step): rows and heads of q, k and v that start on 16 bytes,
+// dk and dv multiples of 4.
 Q6K_API int q6k_retention_chunked(const float* p, int ld, int q_col, int k_col, int v_col, const float* decay, float* chunks, float* state, const int* q_start,
-                                  const int* slot_ids, int T_, int R, float* o, int H, int dk, int dv, cudaStream_t st) {
+                                  const int* slot_ids, int T_, int R, float* o, int H, int dk, int dv, int beyond, cudaStream_t st) {
     if (R == 0 || T_ == 0) return 0;
-    Q6K_REQUIRE(R > 0 && R <= 65535 && H > 0 && H <= 65535 && dk > 0 && dv > 0 && dk <= RET_MAX_DK, "retention: bad sizes R=%d H=%d dk=%d (at most %d) dv=%d", R, H, dk, RET_MAX_DK, dv);
+    Q6K_REQUIRE(R > 0 && beyond >= 0 && H > 0 && dk > 0 && dv > 0 && dk <= RET_MAX_DK, "retention: bad sizes R=%d H=%d dk=%d (at most %d) dv=%d", R, H, dk, RET_MAX_DK, dv);
     Q6K_REQUIRE(dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0 && (((uintptr_t)p | (uintptr_t)chunks | (uintptr_t)state) & 15) == 0,
                 "retention: chunks take rows and heads that start on 16 bytes");
-    const int n_chunks = T_ / RC + R, cols = (dv + 127) / 128, dkp = (dk + 31) / 32 * 32;
+    const int n_long = most_long(T_, R, beyond), n_chunks = most_chunks<RC>(T_, R, beyond), cols = (dv + 127) / 128, dkp = (dk + 31) / 32 * 32;
+    if (n_long == 0) return 0;
     const size_t smem1 = (size_t)2 * RC * 128 * sizeof(float), smem2 = (size_t)ret_out_floats(dkp) * sizeof(float);
     if (cudaFuncSetAttribute(ret_outer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
         cudaFuncSetAttribute(ret_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess)
         return q6k_check_launch("retention: shared memory attribute");
-    q6k_launch(ret_outer_kernel, dim3(n_chunks, H, (dk + 127) / 128 * cols), 256, smem1, st, p + k_col, p + v_col, ld, decay, q_start, R, chunks, H, dk, dv);
+    q6k_launch(ret_outer_kernel, dim3(H, n_chunks, (dk + 127) / 128 * cols), 256, smem1, st, p + k_col, p + v_col, ld, decay, q_start, R, beyond, chunks, H, dk, dv);
     if (int rc = q6k_check_launch("ret_outer")) return rc;
-    q6k_launch(ret_fold_kernel, dim3((unsigned)(R * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, R, slot_ids, H, dk * dv);
+    q6k_launch(ret_fold_kernel, dim3((unsigned)(n_long * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, R, beyond, slot_ids, H, dk * dv);
     if (int rc = q6k_check_launch("ret_fold")) return rc;
-    q6k_launch(ret_out_kernel, dim3(n_chunks, H, cols), 256, smem2, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, o, H, dk, dv, dkp);
+    q6k_launch(ret_out_kernel, dim3(H, n_chunks, cols), 256, smem2, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, beyond, o, H, dk, dv, dkp);
     return q6k_check_launch("ret_out");
 }
 
@@ -731,8 +735,8 @@ Q6K_API int q6k_time_mix(const float* r, const float* k, const float* v, int ld,
     const bool wide = dk % 4 == 0 && ld % 4 == 0 && on16(r) && on16(k) && on16(w);
 #define RET_LAUNCH(RPT)                                                                                                               \
     do {                                                                                                                              \
-        if (wide) launch_retention<RPT, RET_STAGES, true, true>(grid, st, r, k, v, ld, nullptr, w, H * dk, bonus, state, q_start, slot_ids, o, H, dk, dv); \
-        else launch_retention<RPT, RET_STAGES, false, true>(grid, st, r, k, v, ld, nullptr, w, H * dk, bonus, state, q_start, slot_ids, o, H, dk, dv);     \
+        if (wide) launch_retention<RPT, RET_STAGES, true, true>(grid, st, r, k, v, ld, nullptr, w, H * dk, bonus, state, q_start, slot_ids, o, H, dk, dv, 0x7fffffff); \
+        else launch_retention<RPT, RET_STAGES, false, true>(grid, st, r, k, v, ld, nullptr, w, H * dk, bonus, state, q_start, slot_ids, o, H, dk, dv, 0x7fffffff);     \
     } while (0)
     if (dk <= 64) RET_LAUNCH(4);
     else if (dk <= 128) RET_LAUNCH(8);

@@ -1728,12 +1728,37 @@ def retention_prep(p: torch.Tensor, H: int, dk: int, q_col: int, k_col: int, rot
           _i(1 if neighbours else 0), _f(k_scale), _ptr(positions), _i(act_cols), _stream())
 
 
+def retention_chunks(q_lens, H: int, dk: int, dv: int) -> bool:
+    """Whether a step of these portions should go chunk by chunk: the recurrence's time (us) by either form, from measurements of 65 to
+    1,024 tokens in 1 to 8 portions, alone and beside 1 to 32 requests of a token, with 8 and 16 heads of 64, 128 and 256 keys.  Token by token
+    the longest portion decides (its blocks slow one another down once several share an SM); by chunks the rounds of 64-token chunks
+    over the SMs do, and short portions wait for a launch of their own.  16 heads of 128 x 128, walk and chunks: 65 tokens 10 and
+    35, 320 tokens 36 and 37, 512 tokens 56 and 38, eight portions of 200 91 and 118, two of 1,024 146 and 120, 65 beside 32 of one 30 and 54,
+    512 beside 8 of one 105 and 45."""
+    longest = max(q_lens, default=0)
+    if longest <= CHUNKS_BEYOND:
+        return False
+    short = [n for n in q_lens if n <= CHUNKS_BEYOND]
+    long_ones, sms = len(q_lens) - len(short), 148
+    per_token = 0.070 if dk <= 64 else 0.104 if dk <= 128 else 0.134
+    load = long_ones * H * -(-dv // 16) / sms                        # the long portions' walking blocks on an SM
+    shared = 0.72 * load if load < 4 else 2.9 + 0.45 * (load - 4)
+    walk = 3 + per_token * longest * max(shared, 1.3 if len(q_lens) * H * -(-dv // 16) > sms else 1.0)
+    rounds = -(-sum(-(-n // 64) for n in q_lens if n > CHUNKS_BEYOND) * H * -(-dv // 128) // sms)
+    chunks = 5 + rounds * (10 + 0.17 * dk)
+    if short:
+        chunks += 5 + per_token * max(short) + 0.55 * len(short) * (H * dk * dv / 262144)
+    return 1.04 * chunks < walk
+
+
 def retention(p: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
-              slot_ids: torch.Tensor, R: int, H: int, dk: int, dv: int, longest: int = 0) -> torch.Tensor:
+              slot_ids: torch.Tensor, R: int, H: int, dk: int, dv: int, longest: int = 0, shortest: int = 0) -> torch.Tensor:
     """Per request and head, in token order: S <- decay[h] S + k v^T, o = S^T q.  p FP32 [T, N] with q, k (prepared) and v
     at their columns; state FP32 [slots, H, dk, dv], updated in place; returns o FP32 [T, H dv].  longest: tokens of the step's
     longest portion; beyond 64 (the walk token by token takes 200 ns each), rows that start on 16 bytes go 64 tokens at a time, equal up to
-    rounding, if the states of all the chunks take no more than 256 MB."""
+    rounding, if the states of all the chunks take no more than 256 MB.  shortest: tokens of its shortest portion; where it says that
+    there are portions of up to CHUNKS_BEYOND tokens beside the long ones, those are walked token by token all the same (the same bits as
+    in a step of their own)."""
     _need(p, "p", torch.float32)
     _need(decay, "decay", torch.float32, (H,))
     _need(state, "state", torch.float32)
@@ -1741,17 +1766,21 @@ def retention(p: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.
         raise KernelError("retention: shapes disagree")
     o = torch.empty((p.shape[0], H * dv), dtype=torch.float32, device=p.device)
     aligned = dk % 4 == 0 and dv % 4 == 0 and p.stride(0) % 4 == 0 and q_col % 4 == 0 and k_col % 4 == 0 and v_col % 4 == 0
-    if longest > 64 and aligned and p.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
+    most = 0x7fffffff
+    if longest > CHUNKS_BEYOND and aligned and p.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
         lib = library()
         lib.q6k_retention_chunk_floats.restype = ctypes.c_longlong
-        floats = lib.q6k_retention_chunk_floats(_i(p.shape[0]), _i(R), _i(H), _i(dk), _i(dv))
-        if floats <= 64 << 20:
+        beyond = CHUNKS_BEYOND if 0 < shortest <= CHUNKS_BEYOND else 0
+        floats = lib.q6k_retention_chunk_floats(_i(p.shape[0]), _i(R), _i(H), _i(dk), _i(dv), _i(beyond))
+        if floats <= CHUNK_SCRATCH_FLOATS:
             ws = torch.empty(floats, dtype=torch.float32, device=p.device)
             _call("q6k_retention_chunked", _ptr(p), _i(p.stride(0)), _i(q_col), _i(k_col), _i(v_col), _ptr(decay), _ptr(ws), _ptr(state), _ptr(q_start),
-                  _ptr(slot_ids), _i(p.shape[0]), _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _stream())
-            return o
+                  _ptr(slot_ids), _i(p.shape[0]), _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _i(beyond), _stream())
+            if beyond == 0:
+                return o
+            most = beyond
     _call("q6k_retention", _ptr(p), _i(p.stride(0)), _i(q_col), _i(k_col), _i(v_col), _ptr(decay), _ptr(state), _ptr(q_start), _ptr(slot_ids),
-          _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _stream())
+          _i(R), _ptr(o), _i(H), _i(dk), _i(dv), _i(most), _stream())
     return o
 
 

@@ -87,8 +87,12 @@ class Retention(Mixer):
         ops.retention_prep(p, self.H, self.dk, 0, self.k_col, None if self.pos.is_identity else self.pos.rotary_table(), self.k_scale,
                            ctx.positions, act_cols=self.g_col if self.act else 0)
         ops.current_tag = "retention.recurrence"
+        key = ("retention_chunks", self.H, self.dk, self.dv)
+        if key not in ctx.plans:                                      # once per step for all layers of these sizes
+            ctx.plans[key] = ops.retention_chunks(ctx.q_lens, self.H, self.dk, self.dv)
+        chunked = ctx.plans[key]
         o = ops.retention(p, 0, self.k_col, self.v_col, self.decay_t, state["S"], ctx.q_start, ctx.slot_ids, ctx.R, self.H, self.dk, self.dv,
-                          longest=ctx.max_q_len)
+                          longest=ctx.max_q_len if chunked else 0, shortest=min(ctx.q_lens, default=0))
         ops.current_tag = "retention.out"
         if self.out_norm == "all_heads":
             y = ops.delta_out(o, p, self.g_col, self.out_w, self.eps, 1, self.H * self.dv, rt.dtype, gate=self.gate)
