@@ -411,21 +411,27 @@ Q6K_API int q6k_selective_scan_segment() { return 64; }
 // take more lanes; fewer than 9 leave half of them idle.  A chain takes about 35 clocks a token however few there are; the segments'
 // launches take their 30 instructions per token and state, spread over the chip: with 592 schedulers the lines meet where the tokens of all
 // requests bring 24,000 chains for each token of the longest (65,536 chains: 171 against 371 us).  Without segments (up to 64 tokens) a walk of eight states a lane
-// is slower from a few tokens on; a step of single tokens keeps it (nothing to fetch ahead).
-Q6K_API int q6k_selective_scan_lanes_taken(int T_, int R, int C, int N, int segments) {
-    if (N <= 8 || N > LS_N || T_ < 8 * R) return 0;
-    return segments <= 1 || (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 24000;
+// takes 0.58 us a token of the longest portion, a lane per state 6.6 us for every round of blocks (four are resident on an SM), whatever their
+// tokens (4,096 channels: 64 tokens 40 and 9 us, 64 beside 8 of one 40 and 31, 32 portions of 8 28 and 88); from 25 tokens a request on the
+// latter has the fewer instructions too.  A step of single tokens keeps the former (nothing to fetch ahead).
+static bool lanes_taken(int T_, int R, int C, int N, int segments, int longest) {
+    const long long blocks = (C + LS_CH - 1) / LS_CH;
+    if (N <= 8 || N > LS_N || T_ < 8 * R || blocks > 65535) return false;
+    if (segments > 1) return (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 24000;
+    return T_ >= 25 * R || 5.0f + 6.6f * (float)(R * blocks) / (4 * 148) < 3.0f + 0.58f * (float)longest;
 }
+Q6K_API int q6k_selective_scan_lanes_taken(int T_, int R, int C, int N, int segments) { return lanes_taken(T_, R, C, N, segments, R > 0 ? T_ / R : 0); }
 
 // Floats of scratch for `seg_slots` segments in all and R requests.
 Q6K_API long long q6k_selective_scan_workspace(int seg_slots, int R, int C, int N) { return R > 0 ? (long long)seg_slots * C * (N + 1) : 0; }
 
 // segments > 1: portions are walked in segments of q6k_selective_scan_segment() tokens (`segments`: the most of any request;
-// seg_base: int32 [R], the first segment slot of each request; seg_slots: their total; ws: the scratch above).
+// seg_base: int32 [R], the first segment slot of each request; seg_slots: their total; ws: the scratch above).  longest: tokens of the
+// longest portion (0: not said).
 Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col, int c_col,
                                const float* A, const float* Dskip, const float* xz, int ldx, int z_col, float* state, float* tail,
                                const int* q_start, const int* slot_ids, void* out, int R, int C, int N, int taps, int dtype,
-                               int segments, const int* seg_base, int seg_slots, float* ws, int T_, cudaStream_t st) {
+                               int segments, const int* seg_base, int seg_slots, float* ws, int T_, int longest, cudaStream_t st) {
     if (R == 0) return 0;
     const int L = q6k_selective_scan_lanes(N);
     Q6K_REQUIRE(R > 0 && C > 0 && N > 0 && N <= L * MAX_PER_LANE, "selective_scan: bad sizes R=%d C=%d N=%d (at most %d states)", R, C, N,
@@ -434,7 +440,7 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
     const int per_block = 128 / L;
     dim3 grid(R, (C + per_block - 1) / per_block);
     Q6K_REQUIRE(grid.y <= 65535, "selective_scan: %d channels exceed the grid limit", C);
-    if (q6k_selective_scan_lanes_taken(T_, R, C, N, segments)) {
+    if (lanes_taken(T_, R, C, N, segments, longest > 0 ? longest : T_ / R)) {
         Q6K_DISPATCH(dtype, q6k_launch(scan_lanes_kernel<T>, dim3(R, (C + LS_CH - 1) / LS_CH), LS_THREADS, 0, st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
                                        A, Dskip, xz, ldx, z_col, state, tail, q_start, slot_ids, (T*)out, C, N, taps););
         return q6k_check_launch("selective_scan (lanes)");

@@ -1140,14 +1140,15 @@ def cast_columns(src: torch.Tensor, col0: int, n: int, out_dtype: torch.dtype) -
 
 def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, proj: torch.Tensor, b_col: int, c_col: int,
                    A: torch.Tensor, D: torch.Tensor, xz: torch.Tensor, z_col: int, state: torch.Tensor, tail: torch.Tensor,
-                   q_start: torch.Tensor, slot_ids: torch.Tensor, R: int, segments=None) -> torch.Tensor:
+                   q_start: torch.Tensor, slot_ids: torch.Tensor, R: int, segments=None, longest: int = 0) -> torch.Tensor:
     """The selective-scan recurrence over each request's tokens in order, from and into the request's state slot:
     dt = softplus(dt_raw + dt_bias); S <- exp(dt A) S + dt u B; y = (S . C + D u) * silu(z).  u [T, C] (operand dtype),
     dt_raw FP32 [T, C], proj FP32 [T, *] holding B and C (N columns each from b_col, c_col), A FP32 [C, N], xz FP32 [T, *]
     holding the convolution's inputs (columns 0..) and z (columns z_col..), state FP32 [slots, C, N], tail FP32
     [slots, taps-1, C] (moved on to the portion's end).  Returns [T, C] in u's dtype.
     segments = (most segments of any request, seg_base int32 [R] on the device, segments in all) from
-    selective_scan_segments(q_lens): long portions are then walked by several blocks each (two launches)."""
+    selective_scan_segments(q_lens): long portions are then walked by several blocks each (three launches), unless a lane per state
+    takes the step in one pass.  longest: tokens of the longest portion, if known."""
     _need(u, "u")
     T, C = u.shape
     N = A.shape[1]
@@ -1172,7 +1173,7 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
             ws = _workspace(4 * lib.q6k_selective_scan_workspace(_i(slots), _i(R), _i(C), _i(N)), u.device, "scan")
     _call("q6k_selective_scan", _ptr(u), _ptr(dt_raw), _ptr(dt_bias), _ptr(proj), _i(proj.stride(0)), _i(b_col), _i(c_col), _ptr(A), _ptr(D),
           _ptr(xz), _i(xz.stride(0)), _i(z_col), _ptr(state), _ptr(tail), _ptr(q_start), _ptr(slot_ids), _ptr(out), _i(R), _i(C), _i(N),
-          _i(taps), _i(dtype_code(u.dtype)), _i(most), _ptr(seg_base), _i(slots), _ptr(ws), _i(T), _stream())
+          _i(taps), _i(dtype_code(u.dtype)), _i(most), _ptr(seg_base), _i(slots), _ptr(ws), _i(T), _i(longest), _stream(), launches=1 if ws is None else 3)
     return out
 
 

@@ -65,6 +65,6 @@ class SelectiveScan(Mixer):
         if key not in ctx.plans:                # long portions are walked in segments by several blocks: the same plan for every layer
             ctx.plans[key] = ops.selective_scan_segments(ctx.q_lens, rt.device)
         y = ops.selective_scan(u, dt_raw, self.dt_b, proj, R, R + N, self.A, self.skip, xz, C, state["ssm"], state["conv"],
-                               ctx.q_start, ctx.slot_ids, ctx.R, segments=ctx.plans[key])
+                               ctx.q_start, ctx.slot_ids, ctx.R, segments=ctx.plans[key], longest=ctx.max_q_len)
         ops.current_tag = "scan.out"
         return linear.matmul(y, self.w_o, rt, partials_ok=True)
