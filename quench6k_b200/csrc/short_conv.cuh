@@ -57,11 +57,13 @@ __global__ void __launch_bounds__(128) conv_rows_kernel(const float* x, int ldx,
     }
 }
 
-// Whether these rows go four channels at a time; else the kernels that take any.  A step of a token or two per request keeps a block
-// per token: eight requests' tokens in a row would be eight trips to memory one after the other.  (Measured in prompts of 2,048 tokens: 60 -> 24 us, 45 -> 19 us; with one tap, which only
-// adds a bias, 23 -> 9 us.)
+// Whether these rows go four channels at a time; else the kernels that take any.  A thread's walk over eight tokens takes some 5 us however
+// few there are, a thread per channel and token 2.5 and more with every token: the lines meet at about 750,000 values (4,096 channels:
+// 130 tokens 5.6 and 5.4 us, 64 tokens 3.8 and 5.3; 3,072 channels with a tail to move on: 130 tokens 7.4 and 9.3, 256 tokens 9.9 and 9.7, 512 tokens 15.0 and
+// 10.5; 2,048 tokens 60 and 24).  Beside many requests of a token each, eight requests' tokens in a row are eight trips to memory one
+// after the other (256 tokens beside 32 requests 11.0 and 13.8 us, 512 beside 32 16.0 and 14.8).
 inline bool conv_rows_taken(int T_, int requests, const float* x, int ldx, const float* bias, const float* tail, const void* out, int ldo, int C, int taps) {
-    return requests > 0 && T_ >= 4 * requests && taps >= 1 && taps <= 4 && C % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 &&
+    return requests > 0 && (long long)T_ * C >= 750000 && T_ >= 16 * requests && taps >= 1 && taps <= 4 && C % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 &&
            (((uintptr_t)x | (uintptr_t)bias | (uintptr_t)tail | (uintptr_t)out) & 15) == 0;
 }
 

@@ -8,9 +8,18 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("taps, C, dtype", [(4, 516, torch.bfloat16), (3, 8, torch.float32), (2, 1028, torch.float32), (4, 514, torch.float32), (1, 64, torch.float32)])
 def test_the_same_bits_as_token_by_token(taps, C, dtype):
+    _check(taps, C, dtype, [19, 1, 8, 2, 30])
+
+
+# steps large enough (750,000 values) for the kernel of four channels a thread
+@pytest.mark.parametrize("taps, C, dtype", [(4, 4100, torch.bfloat16), (3, 4096, torch.float32), (2, 5000, torch.float32), (1, 4096, torch.float32)])
+def test_the_same_bits_in_large_steps(taps, C, dtype):
+    _check(taps, C, dtype, [19, 1, 8, 2, 170])
+
+
+def _check(taps, C, dtype, lens):
     from quench6k_b200 import ops
     g = torch.Generator().manual_seed(taps * C)
-    lens = [19, 1, 8, 2, 30]
     T, R = sum(lens), len(lens)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     starts, slots = [sum(lens[:i]) for i in range(R + 1)], [4, 0, 2, 1, 3]
