@@ -1326,7 +1326,7 @@ def attention_flex(q_f32: Optional[torch.Tensor], q: Optional[torch.Tensor], hea
             lib.q6k_attention_flex_mma_talk_workspace.restype = ctypes.c_longlong
             ws = _workspace(lib.q6k_attention_flex_mma_talk_workspace(_i(T), _i(H), _i(Hkv), _i(dv)), k_pages.device, "flex")
         elif not chunk:
-            nsplit, split_keys = _key_ranges(n_tiles * Hkv * parts, 148, max_context, window, attention_flex_tc_tile_tokens(H, Hkv))
+            nsplit, split_keys = _wide_ranges(n_tiles * Hkv * parts, max_context, window, attention_flex_tc_tile_tokens(H, Hkv))
             if nsplit > 1:
                 lib.q6k_attention_flex_mma_workspace.restype = ctypes.c_longlong
                 ws = _workspace(lib.q6k_attention_flex_mma_workspace(_i(T), _i(H), _i(dv), _i(nsplit)), k_pages.device, "flex")
@@ -1404,10 +1404,31 @@ def attention_flex_tc_tile_tokens(H: int, Hkv: int) -> int:
     return lib.q6k_attention_flex_tc_tile_tokens(_i(H), _i(Hkv))
 
 
-def attention_flex_wide(max_q_len: int, H: int, da: int, db: int, mixed: bool, k_pages: torch.Tensor, v_pages: torch.Tensor, scale: float) -> int:
+def _wide_ranges(ctas: int, max_context: int, window: Optional[int], tile_tokens: int):
+    """_key_ranges for the tcgen05 kernel.  Under a window of up to 2,048 keys a tile is short already, and the ranges that lie outside it,
+    a whole SM each, cost more than they give (32 tokens beside 16 requests at 16,000 keys, window of 512: a layer of 109 us on mma.sync,
+    163 with ranges)."""
+    return (1, 0) if window and window + tile_tokens <= 2048 else _key_ranges(ctas, 148, max_context, window, tile_tokens)
+
+
+def _ranges_beat_tiles(q_lens, wide: int, narrow: int, heads: int, wide_heads: int, max_context: int, window: Optional[int]) -> bool:
+    """Whether short portions beside requests deep in their contexts are left to the mma.sync kernel: its many small tiles can
+    still be split over the keys where the tcgen05 kernel's, on fewer and larger CTAs, fill the chip already, and then every decoded token
+    walks its whole context in one of them.  A key range of the former takes about four times as long a key (a latent of 512 under 16 heads).
+    A whole layer at 4,096 keys, mma.sync and tcgen05: 64 tokens beside 32 of one 184 and 202 us (four ranges and one), 128
+    beside 32 245 and 214 (three and one), 40 beside 4 106 and 74 (12 and 8)."""
+    narrow_ctas, wide_ctas = (sum(-(-n // t) for n in q_lens) * h for t, h in ((narrow, heads), (wide, wide_heads)))
+    if narrow_ctas >= 120 or (window and window + wide <= 2048):
+        return False
+    return _key_ranges(narrow_ctas, 296, max_context, window, narrow)[0] >= 4 * _wide_ranges(wide_ctas, max_context, window, wide)[0]
+
+
+def attention_flex_wide(max_q_len: int, H: int, da: int, db: int, mixed: bool, k_pages: torch.Tensor, v_pages: torch.Tensor, scale: float,
+                        q_lens=(), max_context: int = 0, window: Optional[int] = None, chunk: Optional[int] = None) -> int:
     """attention_flex_wide_tokens(...) for these pages, or 0 where the tcgen05 kernel may not stand in for the one that ran the step
     before it: shapes the mma.sync kernel does not take (on CUDA cores the query and the weights stay FP32; its first query
-    part and its weights are rounded as the tcgen05 kernel's are), and pages the copies of whole boxes cannot address."""
+    part and its weights are rounded as the tcgen05 kernel's are), and pages the copies of whole boxes cannot address.  q_lens, max_context:
+    the step's portions and its largest position + 1; 0 too where requests deep in their contexts make the other kernel the faster one."""
     Hkv, num_pages, page_size, dk = k_pages.shape
     dv, shared_v = v_pages.shape[-1], v_pages.data_ptr() == k_pages.data_ptr() and v_pages.stride() == k_pages.stride()
     if k_pages.dtype != torch.bfloat16 or Hkv * num_pages * page_size >= 1 << 31:
@@ -1417,7 +1438,12 @@ def attention_flex_wide(max_q_len: int, H: int, da: int, db: int, mixed: bool, k
             return 0
     if not attention_flex_mma_supported(H, Hkv, dk, dv, k_pages.stride(2), v_pages.stride(2), db, shared_v):
         return 0
-    return attention_flex_wide_tokens(max_q_len, H, Hkv, da, db, dv, mixed, shared_v, page_size, scale)
+    tokens = attention_flex_wide_tokens(max_q_len, H, Hkv, da, db, dv, mixed, shared_v, page_size, scale)
+    if tokens and len(q_lens) > 1 and not mixed and not chunk:
+        parts = _flex_tc_parts(H, Hkv, da, db, dv, mixed, shared_v, page_size)
+        if _ranges_beat_tiles(q_lens, tokens, attention_flex_tile_tokens(H, Hkv), Hkv, Hkv * parts, max_context, window):
+            return 0
+    return tokens
 
 
 def attention_flex_wide_tokens(max_q_len: int, H: int, Hkv: int, da: int, db: int, dv: int, mixed: bool, shared_v: bool, page_size: int,

@@ -212,7 +212,8 @@ class Attention(Mixer):
         ops.current_tag = "attention.keys"
         tiles = wide = None
         if not rt.is_fp32 and rt.tensor_cores:
-            tokens = ops.attention_flex_wide(ctx.max_q_len, self.Hq * M, 0, self.hd, self.talk, cache.k, cache.v, self.scale)
+            tokens = ops.attention_flex_wide(ctx.max_q_len, self.Hq * M, 0, self.hd, self.talk, cache.k, cache.v, self.scale, ctx.q_lens, ctx.max_context,
+                                             self.window, self.chunk)
             if tokens:
                 wide = ctx.query_tiles(tokens, most_keys_first=(self.window, self.chunk))
             else:

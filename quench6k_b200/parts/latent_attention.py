@@ -111,7 +111,7 @@ class LatentAttention(Mixer):
                                  ctx.req_of_token, table, cache.page_size, cache.k, neighbours=neighbours, write=not self.borrows, latent=latent)
         tiles = wide = None
         if not rt.is_fp32 and rt.tensor_cores:
-            tokens = ops.attention_flex_wide(ctx.max_q_len, H, self.rank, self.rd, False, cache.k, cache.v, self.scale)
+            tokens = ops.attention_flex_wide(ctx.max_q_len, H, self.rank, self.rd, False, cache.k, cache.v, self.scale, ctx.q_lens, ctx.max_context, self.window)
             if tokens:
                 wide = ctx.query_tiles(tokens, most_keys_first=(self.window, None))
             else:

@@ -36,3 +36,16 @@ def test_what_runs_on_cuda_cores_stays_there(H, Hkv, da, db, dv):
     assert not ops.attention_flex_mma_supported(H, Hkv, da + db, dv, k.stride(2), v.stride(2), db, bool(da))
     for n in (1, 2, 64, 2048):
         assert ops.attention_flex_wide(n, H, da, db, False, k, v, 0.1) == 0
+
+
+@pytest.mark.parametrize("lens, context, taken", [
+    ([64] + [1] * 32, 4000, False),                  # four key ranges on mma.sync, none on tcgen05
+    ([128] + [1] * 32, 4000, True), ([40] + [1] * 4, 4000, True), ([2048] + [1] * 32, 4000, True), ([64] + [1] * 32, 200, True), ([64], 30000, True)])
+def test_short_portions_beside_deep_requests(lens, context, taken):
+    k = _pages(1, 16, 576)
+    assert (ops.attention_flex_wide(max(lens), 16, 512, 64, False, k, k[..., :512], 0.1, lens, context) > 0) == taken
+    assert ops.attention_flex_wide(max(lens), 16, 512, 64, False, k, k[..., :512], 0.1, lens, context, chunk=64) > 0        # chunks are never split
+
+
+def test_windows_are_not_cut_into_ranges_of_the_whole_context():
+    assert ops._wide_ranges(20, 16000, 512, 32) == (1, 0) and ops._wide_ranges(20, 16000, None, 32)[0] > 1 and ops._wide_ranges(20, 16000, 8192, 32)[0] > 1
