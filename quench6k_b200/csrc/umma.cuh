@@ -1,4 +1,4 @@
-// tcgen05 and tensor-memory helpers of the attention kernels that keep scores and probabilities in tensor memory.
+// tcgen05 and tensor-memory helpers of the flexible attention (attention_flex_tc.cu; attention_tc.cu has its own, for its tiles).
 #pragma once
 #include "tma.cuh"
 

@@ -61,7 +61,9 @@ class StepContext:
         """Tiles of at most `tokens_per_tile` consecutive tokens of one request, as device arrays
         (first row, token count) and their number; made once per step and size.  at_most: only
         the requests that bring at most that many tokens to the step.  most_keys_first = (window, chunk): sorted by the
-        number of keys a tile sees under that mask (0 or None: no limit), so that a launch's long blocks start in its first wave."""
+        number of keys a tile sees under that mask (0 or None: no limit), so that a launch's long blocks start in its first wave.  A
+        recorded step keeps the order that its first recording's positions gave (the kernels read positions on the device, so the
+        results do not depend on the order)."""
         key = ("query_tiles", tokens_per_tile, at_most, most_keys_first)
         if key not in self.plans:
             first, count, keys, at = [], [], [], 0
