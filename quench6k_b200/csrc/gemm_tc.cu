@@ -22,7 +22,8 @@
 //              accumulators, or a split-K partial; they hand a buffer back ("accumulator empty") as soon
 //              as its values are in registers, so the next tile's MMAs overlap the stores
 // The producer and the MMA issuer are one elected lane each (elect_one() in tma.cuh says what that saves: 2,048 x 8,192 x 2,048 on
-// CTA pairs 74 -> 56 us, 2,048 x 2,048 x 2,048 23 -> 20 us).
+// CTA pairs 74 -> 56 us, 2,048 x 2,048 x 2,048 23 -> 20 us).  A k-block leaves them about 450 clocks, so their loops hold no division: the
+// ring's place and parity are counted along (1,522 x 2,048 x 8,192 41.4 -> 38.8 us, gate and up of 8,192 rows each 105 -> 95 us).
 // Every wait on an mbarrier is bounded; a wait that runs out records a code in a status word that
 // q6k_tc_status() returns, the roles fall through to the common exit, and tensor memory is freed.
 #include <cstdlib>
@@ -60,6 +61,7 @@ struct Params {
     int lists_old;                     // the pair list was written before the kernel launched before this one started: weights may be fetched before the wait
     int groups;                        // pair mode: matrices there are; a pair of a higher expert number is skipped
     int n_y, n_z;                      // row tiles (or pairs; an upper bound when num_tiles is given) and K slices
+    int out_tma;                       // the output's rows and pitch allow tensor stores (the map below)
     int w_once;                        // every weight tile is fetched by one CTA only (or by a few side by side): its lines may leave the L2 cache first
 };
 
@@ -102,6 +104,64 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 }
 
 __host__ __device__ constexpr int tmem_cols(int want) { return want <= 32 ? 32 : want <= 64 ? 64 : want <= 128 ? 128 : want <= 256 ? 256 : 512; }
+
+// How results leave.  A warp of the epilogue holds 32 weight rows (its lanes) of 16 tokens; stored from registers, each token's 32
+// values are a store of their own (128 bytes, or 64 in bfloat16), and adding into the stream is a load, a wait and a store of each.
+// Instead the warp lays the [16 tokens x 32] block into shared memory (a row's lanes side by side: no bank conflicts) and one lane
+// sends it off as a tensor store, or as a tensor reduction that adds in L2, while the warp turns to the next block: two buffers a warp,
+// 16 KB a CTA, which every tile's ring leaves free.  Blocks that reach beyond a tile's rows go the old way, with their loads asked for
+// before the first store.  One FP32 addition per element either way: the same bits.
+// 1,522 rows, N = 2,048, K = 8,192 on CTA pairs: 42.8 -> 41.4 us stored, 138 -> 41.4 us added; 2,048 x 2,048 x 2,048 20.2 -> 18.1 us (an
+// epilogue of 256 tokens behind the last tile took 11,400 clocks).
+constexpr int EPI_TOKENS = 16, EPI_BLOCK_BYTES = EPI_TOKENS * 32 * 4, EPI_BYTES = 4 * 2 * EPI_BLOCK_BYTES;
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+}
+// The warp's [16 tokens x 32 columns] block, v[j] token j's value of this lane's column, to column x and row y of the output.  buffers: the warp's two;
+// turn: how many blocks it sent before.
+template <typename T>
+__device__ __forceinline__ void send_block(const CUtensorMap* map, uint32_t buffers, int turn, const T* v, int x, int y, bool add) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t at = buffers + (turn & 1) * EPI_BLOCK_BYTES;
+    if (elect_one()) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");       // the block before the last has left this buffer
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < EPI_TOKENS; ++j) {
+        if constexpr (sizeof(T) == 4) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (j * 32 + lane) * 4), "f"(v[j]) : "memory");
+        else asm volatile("st.shared.b16 [%0], %1;" ::"r"(at + (j * 32 + lane) * 2), "h"(__bfloat16_as_ushort(v[j])) : "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (elect_one()) {
+        if (add) tma_add_2d(map, at, x, y);
+        else tma_store_2d(map, at, x, y);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+// Up to 16 rows of one column from registers; add: into what is there, all of it asked for first.
+__device__ __forceinline__ void store_rows(float* o, int ld, const float* v, int rows, bool add) {
+    float old[EPI_TOKENS];
+#pragma unroll
+    for (int j = 0; j < EPI_TOKENS; ++j) old[j] = add && j < rows ? o[(size_t)j * ld] : 0.0f;
+#pragma unroll
+    for (int j = 0; j < EPI_TOKENS; ++j)
+        if (j < rows) o[(size_t)j * ld] = add ? old[j] + v[j] : v[j];
+}
+// Before the kernel ends: what this warp sent has been written.
+__device__ __forceinline__ void sent_blocks_done() {
+    if (elect_one()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+// The value that leaves in bfloat16: of EPI_SWIGLU (DUAL: gate and up), EPI_ACT or EPI_BF16.
+template <bool DUAL>
+__device__ __forceinline__ float rounded_result(const Params& p, float v, float up) {
+    if (DUAL) return p.act == 0 ? v / (1.0f + expf(-v)) * up : q6k_gated(v, up, p.act, p.act_limit);
+    return p.epilogue == EPI_ACT ? q6k_activation(v, p.act) : v;
+}
 
 // One tile of the persistent schedule: which weights, which token rows, which slice of K.
 struct Tile {
@@ -146,7 +206,7 @@ __device__ __forceinline__ bool decode_tile(const Params& p, int t, int n_x, int
 // memory, so the epilogue warps drain one tile while the next one is being multiplied.
 template <int BT, bool DUAL>
 __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_w2,
-                                                       const __grid_constant__ CUtensorMap tm_a, const Params p) {
+                                                       const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_out, const Params p) {
     // Dense tiles follow from the launch alone, so their weights can be on the way before the kernel
     // that makes the activations has ended; tile lists and pair lists come from earlier kernels, and
     // only a caller who knows that another kernel lies between their maker and this one says so.
@@ -220,19 +280,20 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                 }
                 pdl_wait();
             }
-            int it = 0;                                    // k-blocks issued so far, over all tiles
+            int s = 0;                                     // the k-block's stage and the parity of its round through the ring
+            uint32_t st = smem_u32(smem), phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
                 Tile tl;
                 if (!decode_tile<BT>(p, t, n_x, n_y, tl)) continue;
                 const int wy = tl.g * p.N + tl.n0;
-                for (int i = 0; i < tl.nkb; ++i, ++it) {
-                    const int s = it % stages;
-                    const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
+                for (int i = 0; i < tl.nkb; ++i) {
                     const uint32_t fb = full0 + 8 * s;
                     const int kx = (tl.kb0 + i) * BK;
-                    if (it >= pre) {
-                        if (!mbar_wait(empty0 + 8 * s, ((it / stages) & 1) ^ 1)) {
+                    if (pre > 0) {                         // a fresh stage, its weights on the way
+                        --pre;
+                    } else {
+                        if (!mbar_wait(empty0 + 8 * s, phase ^ 1)) {
                             atomicExch(&g_tc_status, 1);
                             ok = false;
                             break;
@@ -242,13 +303,16 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                         if (DUAL) load_w(st + W_BYTES, &tm_w2, kx, wy, fb);
                     }
                     tma_load_2d(st + W_BYTES * (DUAL ? 2 : 1), &tm_a, kx, tl.row0, fb);
+                    if (++s == stages) s = 0, st = smem_u32(smem), phase ^= 1;
+                    else st += STAGE_BYTES;
                 }
             }
         }
     } else if (warp == 1) {
         if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc(BT);
-            int it = 0, nt = 0;                            // k-blocks and tiles consumed so far
+            int s = 0, nt = 0;                             // stage; tiles consumed so far
+            uint32_t st = smem_u32(smem), phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
                 Tile tl;
@@ -260,15 +324,13 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                 }
                 tc_fence_after();
                 const uint32_t acc_addr = tmem_base + buf * ACC_COLS;
-                for (int i = 0; i < tl.nkb; ++i, ++it) {
-                    const int s = it % stages;
-                    if (!mbar_wait(full0 + 8 * s, (it / stages) & 1)) {
+                for (int i = 0; i < tl.nkb; ++i) {
+                    if (!mbar_wait(full0 + 8 * s, phase)) {
                         atomicExch(&g_tc_status, 2);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
                     const uint64_t dw = umma_desc_sw128(st), dw2 = umma_desc_sw128(st + W_BYTES);
                     const uint64_t da = umma_desc_sw128(st + W_BYTES * (DUAL ? 2 : 1));
 #pragma unroll
@@ -278,6 +340,8 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                         if (DUAL) umma_bf16(acc_addr + BT, dw2 + 2 * k, da + 2 * k, idesc, acc);
                     }
                     umma_commit(empty0 + 8 * s);
+                    if (++s == stages) s = 0, st = smem_u32(smem), phase ^= 1;
+                    else st += STAGE_BYTES;
                 }
                 if (!ok) break;
                 umma_commit(acc_full0 + 8 * buf);          // arrives when every MMA issued so far has finished
@@ -288,7 +352,8 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
         // epilogue: this warp owns accumulator lanes 32*(warp%4) .. +31
         const int quarter = warp & 3;
         const int n_local = quarter * 32 + lane;
-        int nt = 0;
+        const uint32_t out_smem = smem_u32(smem + (size_t)stages * STAGE_BYTES) + quarter * 2 * EPI_BLOCK_BYTES;
+        int nt = 0, sent = 0;
         if (early) pdl_wait();                             // the output may still be in use by the kernel before
         for (int t = blockIdx.x; t < total; t += gridDim.x) {
             Tile tl;
@@ -356,31 +421,42 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
                     __syncwarp();
                     if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);
                 }
-                if (n < p.N) {
+                const int row = tl.out0 + c0;
+                if constexpr (BT >= 128) {                    // as blocks; see above
+                    const bool whole = p.out_tma && c0 + 16 <= valid;
+                    if (DUAL || p.epilogue == EPI_ACT || p.epilogue == EPI_BF16) {
+                        __nv_bfloat16 y[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) y[j] = __float2bfloat16_rn(rounded_result<DUAL>(p, v[j], u[DUAL ? j : 0]));
+                        if (whole) {
+                            if (n - lane < p.N) send_block(&tm_out, out_smem, sent++, y, n - lane, row, false);
+                        } else if (n < p.N) {
+                            __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (c0 + j < valid) o[(size_t)j * p.ldo] = y[j];
+                        }
+                    } else if (whole) {
+                        if (n - lane < p.N) send_block(&tm_out, out_smem, sent++, v, n - lane, p.epilogue == EPI_PARTIAL ? tl.z * p.rows_total + row : row, p.epilogue == EPI_ADD);
+                    } else if (n < p.N) {
+                        if (p.epilogue == EPI_PARTIAL) store_rows(p.partial + ((size_t)tl.z * p.rows_total + row) * p.N + n, p.N, v, valid - c0, false);
+                        else store_rows((float*)p.out + (size_t)row * p.ldo + n, p.ldo, v, valid - c0, p.epilogue == EPI_ADD);
+                    }
+                } else if (n < p.N) {                         // few tokens, several CTAs an SM: no room for blocks, and few registers
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const int tt = c0 + j;
-                        if (tt >= valid) break;
-                        const size_t row = (size_t)(tl.out0 + tt);
-                        if (p.epilogue == EPI_STORE) {
-                            ((float*)p.out)[row * p.ldo + n] = v[j];
-                        } else if (p.epilogue == EPI_ADD) {
-                            ((float*)p.out)[row * p.ldo + n] += v[j];
-                        } else if (p.epilogue == EPI_SWIGLU) {
-                            const float gte = v[j];
-                            ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(p.act == 0 ? gte / (1.0f + expf(-gte)) * u[DUAL ? j : 0] : q6k_gated(gte, u[DUAL ? j : 0], p.act, p.act_limit));
-                        } else if (p.epilogue == EPI_ACT) {
-                            ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(q6k_activation(v[j], p.act));
-                        } else if (p.epilogue == EPI_BF16) {
-                            ((__nv_bfloat16*)p.out)[row * p.ldo + n] = __float2bfloat16_rn(v[j]);
-                        } else {
-                            p.partial[((size_t)tl.z * p.rows_total + row) * p.N + n] = v[j];
-                        }
+                        if (c0 + j >= valid) break;
+                        if (DUAL) ((__nv_bfloat16*)p.out)[(size_t)(row + j) * p.ldo + n] = __float2bfloat16_rn(rounded_result<DUAL>(p, v[j], u[DUAL ? j : 0]));
+                        else if (p.epilogue == EPI_STORE) ((float*)p.out)[(size_t)(row + j) * p.ldo + n] = v[j];
+                        else if (p.epilogue == EPI_ADD) ((float*)p.out)[(size_t)(row + j) * p.ldo + n] += v[j];
+                        else if (p.epilogue == EPI_PARTIAL) p.partial[((size_t)tl.z * p.rows_total + row + j) * p.N + n] = v[j];
+                        else ((__nv_bfloat16*)p.out)[(size_t)(row + j) * p.ldo + n] = __float2bfloat16_rn(rounded_result<DUAL>(p, v[j], u[DUAL ? j : 0]));
                     }
                 }
             }
             ++nt;
         }
+        if (BT >= 128) sent_blocks_done();
     }
     tc_fence_before();
     __syncthreads();
@@ -439,7 +515,7 @@ __host__ __device__ constexpr uint32_t umma_idesc_pair(int n) {
 
 template <int BT2>
 __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
-                                                           const Params p) {
+                                                           const __grid_constant__ CUtensorMap tm_out, const Params p) {
     // The tiles follow from the launch alone: the pair sets itself up and sends for the weights of its first ring of
     // k-blocks before it waits for the kernel that makes the activations (and whose reader may still use the output).
     const uint32_t rank = cluster_ctarank();
@@ -494,15 +570,17 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                 }
             }
             pdl_wait();
-            int it = 0;
+            int s = 0;                                     // the k-block's stage and the parity of its round through the ring
+            uint32_t st = smem_u32(smem), phase = 0;
             bool ok = true;
             for (int t = pair; t < total && ok; t += n_pairs) {
                 const int n0 = (t % n_x) * 2 * WM + (int)rank * WM, row0 = (t / n_x) * BT2 + (int)rank * (BT2 / 2);
-                for (int i = 0; i < kb_total; ++i, ++it) {
-                    const int s = it % stages;
-                    const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES), fb = full0 + 8 * s;
-                    if (it >= pre) {                       // the first ring's stages are fresh and their weights on the way
-                        if (!mbar_wait(empty0 + 8 * s, ((it / stages) & 1) ^ 1)) {
+                for (int i = 0; i < kb_total; ++i) {
+                    const uint32_t fb = full0 + 8 * s;
+                    if (pre > 0) {                         // the first ring's stages are fresh and their weights on the way
+                        --pre;
+                    } else {
+                        if (!mbar_wait(empty0 + 8 * s, phase ^ 1)) {
                             atomicExch(&g_tc_status, 11);
                             ok = false;
                             break;
@@ -511,13 +589,16 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                         tma_load_2d_pair(st, &tm_w, i * BK, n0, fb);
                     }
                     tma_load_2d_pair(st + W_BYTES, &tm_a, i * BK, row0, fb);
+                    if (++s == stages) s = 0, st = smem_u32(smem), phase ^= 1;
+                    else st += STAGE_BYTES;
                 }
             }
         }
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = umma_idesc_pair(BT2);
-            int it = 0, nt = 0;
+            int s = 0, nt = 0;
+            uint32_t st = smem_u32(smem), phase = 0;
             bool ok = true;
             for (int t = pair; t < total && ok; t += n_pairs, ++nt) {
                 const int buf = nt & 1;
@@ -527,19 +608,19 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                 }
                 tc_fence_after();
                 const uint32_t acc_addr = tmem_base + buf * ACC_COLS;
-                for (int i = 0; i < kb_total; ++i, ++it) {
-                    const int s = it % stages;
-                    if (!mbar_wait(full0 + 8 * s, (it / stages) & 1)) {
+                for (int i = 0; i < kb_total; ++i) {
+                    if (!mbar_wait(full0 + 8 * s, phase)) {
                         atomicExch(&g_tc_status, 12);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
                     const uint64_t dw = umma_desc_sw128(st), da = umma_desc_sw128(st + W_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) umma_bf16_pair(acc_addr, dw + 2 * k, da + 2 * k, idesc, (i | k) != 0);
                     umma_commit_pair(empty0 + 8 * s);
+                    if (++s == stages) s = 0, st = smem_u32(smem), phase ^= 1;
+                    else st += STAGE_BYTES;
                 }
                 if (!ok) break;
                 umma_commit_pair(acc_full0 + 8 * buf);
@@ -547,7 +628,8 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
         }
     } else {
         const int quarter = warp & 3;
-        int nt = 0;
+        const uint32_t out_smem = smem_u32(smem + (size_t)stages * STAGE_BYTES) + quarter * 2 * EPI_BLOCK_BYTES;
+        int nt = 0, sent = 0;
         pdl_wait();                                        // the output may still be in use by the kernel before
         for (int t = pair; t < total; t += n_pairs, ++nt) {
             const int buf = nt & 1;
@@ -568,16 +650,14 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                     __syncwarp();
                     if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
                 }
-                if (n < p.N) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (c0 + j >= valid) break;
-                        float* o = (float*)p.out + (size_t)(tok0 + c0 + j) * p.ldo + n;
-                        *o = p.epilogue == EPI_ADD ? *o + v[j] : v[j];
-                    }
+                if (p.out_tma && c0 + 16 <= valid) {
+                    if (n - lane < p.N) send_block(&tm_out, out_smem, sent++, v, n - lane, tok0 + c0, p.epilogue == EPI_ADD);
+                } else if (n < p.N) {
+                    store_rows((float*)p.out + (size_t)(tok0 + c0) * p.ldo + n, p.ldo, v, valid - c0, p.epilogue == EPI_ADD);
                 }
             }
         }
+        sent_blocks_done();
     }
     tc_fence_before();
     __syncthreads();
@@ -621,6 +701,21 @@ int weight_map(CUtensorMap* out, const void* base, long long rows, int K) {
     return 0;
 }
 
+// The output [rows, N] of pitch ld in boxes of [16 rows x 32 columns], where its start and pitch are on 16 bytes (*fits); what lies beyond N is left alone.
+int out_map(CUtensorMap* map, int* fits, const void* out, long long rows, int N, int ld, bool bf16) {
+    const int size = bf16 ? 2 : 4;
+    *fits = ((uintptr_t)out & 15) == 0 && (long long)ld * size % 16 == 0;
+    if (!*fits) return 0;
+    EncodeTiled fn = encode_fn();
+    if (!fn) return q6k_fail("gemm_tc: the driver does not offer cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * size};
+    const cuuint32_t box[2] = {32u, (cuuint32_t)EPI_TOKENS}, estr[2] = {1, 1};
+    const CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(out), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return q6k_fail("gemm_tc: cuTensorMapEncodeTiled failed with code %d for the output (rows %lld, columns %d, pitch %d)", (int)r, rows, N, ld);
+    return 0;
+}
+
 int sm_count() {
     static int n = 0;
     if (!n) {
@@ -633,6 +728,12 @@ int sm_count() {
 // n_y: row tiles, pairs, or the tile list's capacity; n_z: K slices.
 template <int BT, bool DUAL>
 int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta, Params p, int n_y, int n_z, cudaStream_t st) {
+    CUtensorMap tout = tw;
+    p.out_tma = 0;
+    if (BT >= 128) {
+        const bool partial = p.epilogue == EPI_PARTIAL, rounds = p.epilogue == EPI_SWIGLU || p.epilogue == EPI_ACT || p.epilogue == EPI_BF16;
+        if (int rc = out_map(&tout, &p.out_tma, partial ? (void*)p.partial : p.out, (long long)p.rows_total * (partial ? n_z : 1), p.N, partial ? p.N : p.ldo, rounds)) return rc;
+    }
     constexpr int stage = WM * BK * 2 * (DUAL ? 2 : 1) + BT * BK * 2;
     // narrow token tiles (weight streaming): two CTAs per SM, each with half of the shared memory;
     // wide ones: one CTA per SM whose ring takes all of it
@@ -643,11 +744,12 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta,
     // deep enough to have its whole K slice on the way at once
     const int need = (int)((total + sm_count() - 1) / sm_count());
     if (need < per_sm) per_sm = need < 1 ? 1 : need;
-    int stages = ((220 / per_sm) * 1024) / stage;
+    const int out_bytes = BT >= 128 ? EPI_BYTES : 0;
+    int stages = BT >= 128 ? (225 * 1024 - out_bytes) / stage : ((220 / per_sm) * 1024) / stage;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.stages = stages;
     p.n_y = n_y, p.n_z = n_z;
-    const size_t smem = (size_t)stages * stage + 1024;
+    const size_t smem = (size_t)stages * stage + out_bytes + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(gemm_tc_kernel<BT, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
@@ -656,7 +758,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta,
     }
     const int slots = sm_count() * per_sm;
     const int grid = (int)(total < slots ? total : slots);
-    q6k_launch_as(p.tile_group == nullptr || p.lists_old != 0, gemm_tc_kernel<BT, DUAL>, grid, 192, smem, st, tw, tw2, ta, p);
+    q6k_launch_as(p.tile_group == nullptr || p.lists_old != 0, gemm_tc_kernel<BT, DUAL>, grid, 192, smem, st, tw, tw2, ta, tout, p);
     return q6k_check_launch("gemm_tc");
 }
 
@@ -664,11 +766,13 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta,
 template <int BT2>
 int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, Params p, cudaStream_t st) {
     constexpr int stage = WM * BK * 2 + (BT2 / 2) * BK * 2;
-    int stages = (200 * 1024) / stage;
+    CUtensorMap tout = tw;
+    if (int rc = out_map(&tout, &p.out_tma, p.out, p.rows_total, p.N, p.ldo, false)) return rc;
+    int stages = (225 * 1024 - EPI_BYTES) / stage;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.stages = stages;
     p.n_y = (p.rows_total + BT2 - 1) / BT2;
-    const size_t smem = (size_t)stages * stage + 1024;
+    const size_t smem = (size_t)stages * stage + EPI_BYTES + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BT2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
@@ -685,7 +789,7 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, Params p, cudaStre
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // the weights of the first ring are fetched under the kernel before
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = q6k_pdl_mode() != 0 ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2>, tw, ta, p);
+    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2>, tw, ta, tout, p);
     return q6k_check_launch("gemm_tc pair");
 }
 
