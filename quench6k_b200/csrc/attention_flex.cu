@@ -553,6 +553,24 @@ __global__ void __launch_bounds__(256) latent_rows_kernel(const float* x, int ld
     for (int d = threadIdx.x; d < rd; d += 256) dst[rank + d] = from_f32<T>(turned(xs, d));
 }
 
+// The latents that prompt portions see, for the product that expands them: row i of `places` (request, position, or a negative position for a row that
+// nobody sees) from its page into lat [rows, rank] (zeros where nobody sees it), its rotated part behind each of the H heads' expanded keys, whose rows
+// of dim entries lie `pitch` apart, [H, rows, pitch].  16 bytes at a time: everything a multiple of 8 entries.  grid (rows), 128 threads.
+__global__ void __launch_bounds__(128) latent_context_kernel(const uint4* pages, const int2* places, const int* block_table, int max_blocks, int page_size, uint4* lat, uint4* keys,
+                                                             int rank8, int rd8, int dim8, int pitch8, int H) {
+    pdl_enter();
+    const int row = blockIdx.x;
+    const int2 at = places[row];
+    const int page = at.y >= 0 ? block_table[(size_t)at.x * max_blocks + at.y / page_size] : -1;
+    const uint4* src = pages + ((size_t)max(page, 0) * page_size + max(at.y, 0) % page_size) * (rank8 + rd8);
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < rank8; i += 128) lat[(size_t)row * rank8 + i] = page >= 0 ? src[i] : zero;
+    for (int i = threadIdx.x; i < H * rd8; i += 128) {
+        const int h = i / rd8, c = i - h * rd8;
+        keys[((size_t)h * gridDim.x + row) * pitch8 + dim8 + c] = page >= 0 ? src[rank8 + c] : zero;
+    }
+}
+
 // src: FP32 [H, T, n] -> out: [T, H n] in the storage type, four values a thread (n4 = n / 4; a value a thread took 19 us for 2,048 rows
 // of 16 x 128, 25 MB; so 6).
 template <typename T>
@@ -827,6 +845,19 @@ Q6K_API int q6k_latent_prep(const float* x, int ld, const float* xc, int ldc, in
     Q6K_DISPATCH(dtype, q6k_launch(latent_prep_kernel<T>, dim3(T_, pages ? H + 1 : H), 128, smem, st, x, ld, xc, ldc, H, dim, rd, rank, cw, eps, inv_freq, turn,
                                    neighbours, positions, req_of_token, block_table, max_blocks, page_size, (T*)qn, (T*)qr, (T*)pages, T_););
     return q6k_check_launch("latent_prep");
+}
+
+// pages: bfloat16 [pages, page_size, rank + rd]; places: int32 [rows, 2]; lat: bfloat16 [rows, rank]; keys: bfloat16 [H, rows, pitch] (columns dim .. dim + rd
+// are written).
+Q6K_API int q6k_latent_context(const void* pages, const int* places, int rows, const int* block_table, int max_blocks, int page_size, void* lat, void* keys, int rank, int rd, int dim,
+                               int pitch, int H, cudaStream_t st) {
+    if (rows == 0) return 0;
+    Q6K_REQUIRE(rows > 0 && rank > 0 && rank % 8 == 0 && rd >= 0 && rd % 8 == 0 && dim % 8 == 0 && pitch % 8 == 0 && pitch >= dim + rd && H > 0 && page_size > 0 &&
+                    (((uintptr_t)pages | (uintptr_t)lat | (uintptr_t)keys) & 15) == 0 && ((uintptr_t)places & 7) == 0,
+                "latent_context: bad sizes rows=%d rank=%d rd=%d dim=%d", rows, rank, rd, dim);
+    q6k_launch(latent_context_kernel, dim3(rows), 128, 0, st, (const uint4*)pages, (const int2*)places, block_table, max_blocks, page_size, (uint4*)lat, (uint4*)keys, rank / 8, rd / 8,
+               dim / 8, pitch / 8, H);
+    return q6k_check_launch("latent_context");
 }
 
 Q6K_API int q6k_heads_to_rows(const float* src, void* out, int H, int T_, int n, int dtype, cudaStream_t st) {

@@ -61,6 +61,7 @@ struct Params {
     int lists_old;                     // the pair list was written before the kernel launched before this one started: weights may be fetched before the wait
     int groups;                        // pair mode: matrices there are; a pair of a higher expert number is skipped
     int n_y, n_z;                      // row tiles (or pairs; an upper bound when num_tiles is given) and K slices
+    int head_cols, head_split, head_gap;      // columns of a head, where every head's results are a matrix of their own; those from head_split on lie head_gap further
     int out_tma;                       // the output's rows and pitch allow tensor stores (the map below)
     int w_once;                        // every weight tile is fetched by one CTA only (or by a few side by side): its lines may leave the L2 cache first
 };
@@ -118,13 +119,17 @@ constexpr int EPI_TOKENS = 16, EPI_BLOCK_BYTES = EPI_TOKENS * 32 * 4, EPI_BYTES 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(src) : "memory");
+}
 __device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
 }
 // The warp's [16 tokens x 32 columns] block, v[j] token j's value of this lane's column, to column x and row y of the output.  buffers: the warp's two;
-// turn: how many blocks it sent before.
+// turn: how many blocks it sent before.  head_cols > 0: the output is a matrix for each of the heads that x runs over, so many columns each, `gap` columns
+// left out before column `split`.
 template <typename T>
-__device__ __forceinline__ void send_block(const CUtensorMap* map, uint32_t buffers, int turn, const T* v, int x, int y, bool add) {
+__device__ __forceinline__ void send_block(const CUtensorMap* map, uint32_t buffers, int turn, const T* v, int x, int y, bool add, int head_cols = 0, int split = 0, int gap = 0) {
     const int lane = threadIdx.x & 31;
     const uint32_t at = buffers + (turn & 1) * EPI_BLOCK_BYTES;
     if (elect_one()) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");       // the block before the last has left this buffer
@@ -138,6 +143,7 @@ __device__ __forceinline__ void send_block(const CUtensorMap* map, uint32_t buff
     __syncwarp();
     if (elect_one()) {
         if (add) tma_add_2d(map, at, x, y);
+        else if (head_cols > 0) tma_store_3d(map, at, x % head_cols + (x % head_cols >= split ? gap : 0), y, x / head_cols);
         else tma_store_2d(map, at, x, y);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
@@ -513,7 +519,8 @@ __host__ __device__ constexpr uint32_t umma_idesc_pair(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
-template <int BT2>
+// HEADS: the results leave in bfloat16, a matrix of p.head_cols columns per head (whole blocks of 16 rows).
+template <int BT2, bool HEADS>
 __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
                                                            const __grid_constant__ CUtensorMap tm_out, const Params p) {
     // The tiles follow from the launch alone: the pair sets itself up and sends for the weights of its first ring of
@@ -650,7 +657,12 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                     __syncwarp();
                     if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
                 }
-                if (p.out_tma && c0 + 16 <= valid) {
+                if constexpr (HEADS) {
+                    __nv_bfloat16 y[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) y[j] = __float2bfloat16_rn(v[j]);
+                    if (n - lane < p.N) send_block(&tm_out, out_smem, sent++, y, n - lane, tok0 + c0, false, p.head_cols, p.head_split, p.head_gap);
+                } else if (p.out_tma && c0 + 16 <= valid) {
                     if (n - lane < p.N) send_block(&tm_out, out_smem, sent++, v, n - lane, tok0 + c0, p.epilogue == EPI_ADD);
                 } else if (n < p.N) {
                     store_rows((float*)p.out + (size_t)(tok0 + c0) * p.ldo + n, p.ldo, v, valid - c0, p.epilogue == EPI_ADD);
@@ -763,11 +775,12 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta,
 }
 
 // The CTA-pair kernel: tiles of [256 weights x BT2 tokens], one cluster of two CTAs per SM pair.
-template <int BT2>
-int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, Params p, cudaStream_t st) {
+template <int BT2, bool HEADS>
+int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const CUtensorMap* heads, Params p, cudaStream_t st) {
     constexpr int stage = WM * BK * 2 + (BT2 / 2) * BK * 2;
     CUtensorMap tout = tw;
-    if (int rc = out_map(&tout, &p.out_tma, p.out, p.rows_total, p.N, p.ldo, false)) return rc;
+    if (HEADS) tout = *heads;
+    else if (int rc = out_map(&tout, &p.out_tma, p.out, p.rows_total, p.N, p.ldo, false)) return rc;
     int stages = (225 * 1024 - EPI_BYTES) / stage;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.stages = stages;
@@ -775,7 +788,7 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, Params p, cudaStre
     const size_t smem = (size_t)stages * stage + EPI_BYTES + 1024;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BT2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BT2, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
             return q6k_check_launch("gemm_tc pair: shared memory attribute");
         configured = true;
     }
@@ -789,12 +802,17 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, Params p, cudaStre
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // the weights of the first ring are fetched under the kernel before
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = q6k_pdl_mode() != 0 ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2>, tw, ta, tout, p);
+    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2, HEADS>, tw, ta, tout, p);
     return q6k_check_launch("gemm_tc pair");
 }
 
 // Token tile of the pair kernel for (rows, N), or 0 when the one-CTA kernel serves the product:
 // plain dense products with at least 512 rows and 256 weight rows.  Q6K_TC_PAIR=0 switches it off.
+static int pair_tile(int rows, int N) {                    // the tile that ends the last round earlier
+    const long long n_x = (N + 2 * WM - 1) / (2 * WM), pairs = sm_count() / 2;
+    const long long r256 = (n_x * ((rows + 255) / 256) + pairs - 1) / pairs, r192 = (n_x * ((rows + 191) / 192) + pairs - 1) / pairs;
+    return r192 * 192 < r256 * 256 ? 192 : 256;
+}
 static int pair_plan(int rows, int N, int K) {
     static const bool off = [] {
         const char* v = getenv("Q6K_TC_PAIR");
@@ -803,8 +821,7 @@ static int pair_plan(int rows, int N, int K) {
     if (off || rows < 512 || N < 2 * WM || K % 8 != 0) return 0;
     const long long n_x = (N + 2 * WM - 1) / (2 * WM), pairs = sm_count() / 2;
     if (n_x * ((rows + 255) / 256) * 2 < pairs) return 0;   // too few tiles for the pairs: the one-CTA kernel narrows its tile
-    const long long r256 = (n_x * ((rows + 255) / 256) + pairs - 1) / pairs, r192 = (n_x * ((rows + 191) / 192) + pairs - 1) / pairs;
-    return r192 * 192 < r256 * 256 ? 192 : 256;            // the tile that ends the last round earlier
+    return pair_tile(rows, N);
 }
 
 }  // namespace
@@ -913,7 +930,7 @@ Q6K_API int q6k_gemm_tc(const void* A, long long lda, int rows_total, const void
             if (int rc = make_map(&ta, A, rows_total, K, lda, bt2 / 2, false)) return rc;
             Params pp{};
             pp.out = out, pp.rows_total = rows_total, pp.N = N, pp.K = K, pp.ldo = ldo, pp.epilogue = epilogue;
-            return bt2 == 192 ? launch_pair<192>(tw, ta, pp, st) : launch_pair<256>(tw, ta, pp, st);
+            return bt2 == 192 ? launch_pair<192, false>(tw, ta, nullptr, pp, st) : launch_pair<256, false>(tw, ta, nullptr, pp, st);
         }
     }
     if (int rc = make_map(&ta, A, rows_total, K, lda, bt, false)) return rc;
@@ -957,6 +974,31 @@ Q6K_API int q6k_gemm_tc(const void* A, long long lda, int rows_total, const void
         return q6k_check_launch("gemm_tc split-K reduce");
     }
     return 0;
+}
+
+// The same product with every head's results in a matrix of its own, rounded to bfloat16: out[h][r][d + (d < split ? 0 : gap)] = A[r] . W[h head_cols + d],
+// rows `pitch` and heads `head_stride` entries apart.  Whole blocks only: rows a multiple of 16, head_cols and split of 32, gap of 8, everything on 16 bytes.
+Q6K_API int q6k_gemm_tc_heads(const void* A, long long lda, int rows, const void* W, int N, int K, void* out, int head_cols, int split, int gap, int pitch, long long head_stride,
+                              cudaStream_t st) {
+    if (rows == 0 || N == 0) return 0;
+    Q6K_REQUIRE(rows > 0 && N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && rows % 16 == 0, "gemm_tc_heads: bad sizes rows=%d N=%d K=%d", rows, N, K);
+    Q6K_REQUIRE(head_cols > 0 && head_cols % 32 == 0 && N % head_cols == 0 && split % 32 == 0 && gap >= 0 && gap % 8 == 0 && pitch >= head_cols + gap && pitch % 8 == 0 && head_stride % 8 == 0 && head_stride > 0,
+                "gemm_tc_heads: heads of %d columns, rows %d and heads %lld entries apart", head_cols, pitch, head_stride);
+    Q6K_REQUIRE((((uintptr_t)A | (uintptr_t)W | (uintptr_t)out) & 15) == 0, "gemm_tc_heads: operands must be 16-byte aligned");
+    EncodeTiled fn = encode_fn();
+    if (!fn) return q6k_fail("gemm_tc: the driver does not offer cuTensorMapEncodeTiled");
+    const cuuint64_t dims[3] = {(cuuint64_t)(head_cols + gap), (cuuint64_t)rows, (cuuint64_t)(N / head_cols)}, strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)head_stride * 2};
+    const cuuint32_t box[3] = {32u, (cuuint32_t)EPI_TOKENS, 1u}, estr[3] = {1, 1, 1};
+    CUtensorMap tw, ta, tout;
+    const CUresult r = fn(&tout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                          CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return q6k_fail("gemm_tc: cuTensorMapEncodeTiled failed with code %d for %d heads of [%d, %d]", (int)r, N / head_cols, rows, head_cols);
+    if (int rc = weight_map(&tw, W, N, K)) return rc;
+    const int bt2 = pair_tile(rows, N);
+    if (int rc = make_map(&ta, A, rows, K, lda, bt2 / 2, false)) return rc;
+    Params p{};
+    p.out = out, p.rows_total = rows, p.N = N, p.K = K, p.epilogue = EPI_BF16, p.head_cols = head_cols, p.head_split = split, p.head_gap = gap;
+    return bt2 == 192 ? launch_pair<192, true>(tw, ta, &tout, p, st) : launch_pair<256, true>(tw, ta, &tout, p, st);
 }
 
 // Few tokens (decode): one tile per (token, slot) pair instead of a permutation.  pair_expert:

@@ -44,6 +44,8 @@ class StepContext:
     made: set = field(default_factory=set)        # keys of plans whose device-side part has been launched in this pass over the
                                                   # layers: the runner empties it before it records the step, so that a kernel
                                                   # that fills a plan from the step's positions is part of the recording
+    replayed: bool = False                        # the pass is, or will be, a recording that later steps replay at other positions: what a part
+                                                  # launches must not depend on the host's positions
     fed: Optional[torch.Tensor] = None            # int32 ids the step before sampled: a token id -(i + 1) stands for fed[i]
     hold_results: bool = False                    # a block that keeps a sublayer's result while other kernels run sets it: results
                                                   # must then be tensors of their own, not views of the products' scratch buffer
@@ -82,6 +84,24 @@ class StepContext:
                 first, count = [first[j] for j in order], [count[j] for j in order]
             both = torch.tensor([first, count], dtype=torch.int32).reshape(2, -1).to(self.token_ids.device, non_blocking=True)
             self.plans[key] = (both[0], both[1], len(first))
+        return self.plans[key]
+
+    def context_rows(self):
+        """Every position that the step's requests see, a request after the other, each beginning at a multiple of 64: as device arrays
+        (request and position of every row, a negative position for the rows between; [R, blocks] the blocks of 64 rows of each request) and the
+        number of rows."""
+        key = "context_rows"
+        if key not in self.plans:
+            reach = [s + n for s, n in zip(self.pos_starts, self.q_lens)]
+            blocks = [-(-c // 64) for c in reach]
+            first = [sum(blocks[:r]) for r in range(len(blocks))]
+            req = torch.repeat_interleave(torch.arange(len(reach), dtype=torch.int32), torch.tensor(blocks) * 64)
+            pos = torch.cat([torch.arange(b * 64, dtype=torch.int32) for b in blocks])
+            pos = torch.where(pos < torch.tensor(reach, dtype=torch.int32)[req.long()], pos, -1)
+            wide = max(blocks)
+            table = torch.tensor([[f + min(i, b - 1) for i in range(wide)] for f, b in zip(first, blocks)], dtype=torch.int32)
+            device = self.token_ids.device
+            self.plans[key] = (torch.stack([req, pos], 1).contiguous().to(device, non_blocking=True), table.to(device, non_blocking=True), 64 * sum(blocks))
         return self.plans[key]
 
     def short_requests(self, at_most: int):

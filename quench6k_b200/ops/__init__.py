@@ -1258,6 +1258,24 @@ def latent_prep(x: torch.Tensor, H: int, dim: int, rd: int, rank: int, c_weight:
     return qn, qr
 
 
+def latent_expanded(pages: torch.Tensor, places: torch.Tensor, block_table: torch.Tensor, w: torch.Tensor, H: int, dim: int, rd: int):
+    """Keys and values of every head for the cached latents at `places` (int32 [rows, 2]: request and position, rows a multiple of 64; a negative position:
+    a row of zeros), as pages of 64 rows that attention_flex reads: views [H, rows / 64, 64, dim + rd] and [H, rows / 64, 64, vd] of one bfloat16 tensor.
+    pages: bfloat16 [1, pages, page, rank + rd]; w: [H (dim + vd), rank], a head's rows of the keys' up-projection before those of the values'."""
+    _need(pages, "pages", torch.bfloat16)
+    _need(places, "places", torch.int32)
+    rows, rank, cols = places.shape[0], w.shape[1], w.shape[0] // H
+    _need(w, "w", torch.bfloat16, (H * cols, rank))
+    if rows % 64 or pages.shape[-1] != rank + rd or cols <= dim:
+        raise KernelError(f"latent_expanded: {rows} rows, pages of {pages.shape[-1]} for a latent of {rank} + {rd}")
+    lat = torch.empty((rows, rank), dtype=torch.bfloat16, device=pages.device)
+    kv = torch.empty((H, rows // 64, 64, cols + rd), dtype=torch.bfloat16, device=pages.device)
+    _call("q6k_latent_context", _ptr(pages), _ptr(places), _i(rows), _ptr(block_table), _i(block_table.shape[1]), _i(pages.shape[2]), _ptr(lat), _ptr(kv), _i(rank), _i(rd), _i(dim),
+          _i(cols + rd), _i(H), _stream())
+    _call("q6k_gemm_tc_heads", _ptr(lat), _ll(rank), _i(rows), _ptr(w), _i(H * cols), _i(rank), _ptr(kv), _i(cols), _i(dim), _i(rd), _i(cols + rd), _ll(rows * (cols + rd)), _stream())
+    return kv[..., :dim + rd], kv[..., dim + rd:]
+
+
 def heads_to_rows(src: torch.Tensor, H: int, out_dtype: torch.dtype) -> torch.Tensor:
     """FP32 [H * T, n] (head-major) -> out_dtype [T, H * n]."""
     _need(src, "src", torch.float32)

@@ -7,11 +7,17 @@ latent space, which needs nothing but the cache: with q_h = [a_h | r_h],
 so every head attends with a query of rank + rot_dim over one shared key row per position whose first `rank` entries
 are also its value: multi-query attention over the pages, between two per-head products.
 
+Prompt portions expand the latents they see instead (`expands`): every position's keys and values of every head, by one product,
+then a key row is dim + rot_dim wide and a value v_dim, a quarter of the operations of a pair of positions (2,048 tokens of 16 heads of 128 + 64
+on a latent of 512: 323 -> 155 us a layer).
+
 Options: queries through a normed low-rank vector of their own (`q_rank`: q = W_uq norm(W_dq x)), a sliding window (position i sees j with 0 <= i - j < window), a learned sink per head (exp(sink_h) joins the
 softmax denominator), either pairing of the rotation, and a layer that has no down-projection of its own but reads the
 pages another layer wrote (`borrows`: its own queries, up-projections, mask and output product).  A layer whose pages
 are read by layers with wider windows keeps them for the widest (`retain`: a window, or None for every key)."""
 from __future__ import annotations
+
+import torch
 
 from .. import ops
 from ..spec import PartSpec, TensorSpec
@@ -21,6 +27,9 @@ from .base import POSITION_ENCODINGS, CacheRequest, Mixer, make_part, register_m
 _NAMES = {"q": "q_proj.weight", "dkv": "kv_down_proj.weight", "c_norm": "kv_norm.weight", "uk": "k_up_proj.weight",
           "uv": "v_up_proj.weight", "out": "o_proj.weight", "sinks": "sinks",
           "dq": "q_down_proj.weight", "q_norm": "q_norm.weight", "uq": "q_up_proj.weight"}
+
+
+EXPAND_BYTES = 256 << 20         # of expanded keys and values, at most
 
 
 @register_mixer("latent_attention")
@@ -65,7 +74,6 @@ class LatentAttention(Mixer):
         return out + [TensorSpec(n["out"], (self.D, H * self.vd))]
 
     def bind(self, get, rt):
-        import torch
         self.rt = rt
         n, H = self.names, self.H
         nq = self.q_rank or H * (self.dim + self.rd)
@@ -82,8 +90,36 @@ class LatentAttention(Mixer):
         # per head: a -> W_uk_h^T a is a product with the [rank, dim] matrix W_uk_h^T; o -> W_uv_h o with [vd, rank]
         self.w_ukT = to_operand(get(n["uk"]), rt).view(H, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = to_operand(get(n["uv"]), rt).view(H, self.vd, self.rank).contiguous()
+        # the same up-projections row by row, a head's keys before its values, for the portions that expand what they see
+        self.w_ukv = None
+        if self.can_expand():
+            self.w_ukv = torch.cat([to_operand(get(n["uk"]), rt).view(H, self.dim, self.rank), self.w_uv], 1).view(H * (self.dim + self.vd), self.rank)
         self.w_o = to_operand(get(n["out"]), rt)
         self.pos.bind(lambda name: get("position." + name), rt)
+
+    def can_expand(self) -> bool:
+        """Whether the kernels that expand latents take these sizes."""
+        return (not self.rt.is_fp32 and self.rt.tensor_cores and self.window is None and self.dim % 32 == 0 and self.vd % 64 == 0 and self.rd % 8 == 0
+                and self.rank % 8 == 0 and ops.attention_flex_wide_tokens(1 << 30, self.H, self.H, self.dim, self.rd, self.vd, False, False, 64, self.scale) > 0)
+
+    def expands(self, ctx) -> bool:
+        """Whether this step's requests expand the latents they see: by what either form takes, in us (fitted to layers of 8 heads on a latent of 256 and 16
+        on 512, 64 to 2,048 tokens after 0 to 16,000, of one to three requests).  Absorbed, a million (head, query, key) take 4.1e-3 for each column of
+        a row's two products, and a further 15 go to the products around the attention.  Expanded they take 2.5, in tiles of 128 tokens; the rows to
+        expand take their product at 1.1 PFLOP/s and 1 a thousand for the copies.  Absorbed and expanded, both measured: 16 heads, 2,048 tokens 310 and 145; 130 tokens
+        at 4,096 111 and 105, at 16,000 217 and 246; 8 heads, 300 tokens at 4,096 85 and 74, at 16,000 137 and 163."""
+        if self.w_ukv is None or ctx.replayed or ctx.max_q_len < 64:         # a portion fills half a tile of its heads
+            return False
+        key = ("latent.expands", self.H, self.dim, self.rd, self.vd, self.rank)
+        if key not in ctx.plans:
+            reach = [s + n for s, n in zip(ctx.pos_starts, ctx.q_lens)]
+            pairs = self.H * 1e-6 * sum(n * (c - n / 2) for n, c in zip(ctx.q_lens, reach))
+            tiled = self.H * 1e-6 * sum(-(-n // 128) * 128 * (c - n / 2) for n, c in zip(ctx.q_lens, reach))
+            rows = sum(-(-c // 64) * 64 for c in reach)
+            flops = 2.0 * self.H * (self.dim + self.vd) * self.rank
+            fits = rows * (self.rank + self.H * (self.dim + self.rd + self.vd)) * 2 <= EXPAND_BYTES
+            ctx.plans[key] = fits and 2.5 * tiled + rows * (flops / 1.1e9 + 1e-3) < 4.1e-3 * (3 * self.rank + self.rd) * pairs + 15.0
+        return ctx.plans[key]
 
     def cache_request(self):
         if self.borrows:
@@ -109,6 +145,16 @@ class LatentAttention(Mixer):
         inv_freq, turn, neighbours = (None, 0, False) if self.pos.is_identity else self.pos.rotary_table()
         qn, qr = ops.latent_prep(x, H, self.dim, self.rd, self.rank, self.c_norm, self.eps, inv_freq, turn, ctx.positions,
                                  ctx.req_of_token, table, cache.page_size, cache.k, neighbours=neighbours, write=not self.borrows, latent=latent)
+        if self.expands(ctx):
+            ops.current_tag = "latent.expand"
+            places, blocks, _ = ctx.context_rows()
+            k, v = ops.latent_expanded(cache.k, places, table, self.w_ukv, H, self.dim, self.rd)
+            ops.current_tag = "latent.keys"
+            wide = ctx.query_tiles(ops.attention_flex_tc_tile_tokens(H, H), most_keys_first=(None, None))
+            a = ops.attention_flex(qn.view(H * T, self.dim), qr.view(H * T, self.rd) if self.rd else None, True, k, v, blocks, ctx.req_of_token, ctx.positions, H, self.scale,
+                                   max_context=ctx.max_context, sinks=self.sinks, wide_tiles=wide)
+            ops.current_tag = "latent.o"
+            return linear.matmul(a, self.w_o, rt, partials_ok=not ctx.hold_results)
         tiles = wide = None
         if not rt.is_fp32 and rt.tensor_cores:
             tokens = ops.attention_flex_wide(ctx.max_q_len, H, self.rank, self.rd, False, cache.k, cache.v, self.scale, ctx.q_lens, ctx.max_context, self.window)
