@@ -1,5 +1,5 @@
-// Matrix products on CUDA cores with FP32 fused multiply-adds: the fallback of the bfloat16 path for shapes the
-// tensor-core kernels refuse.  FP32 operands go to gemm_f32.cu.
+// Matrix products on CUDA cores with FP32 fused multiply-adds: the arithmetic of the true 32-bit
+// path, and the fallback of the bfloat16 path for shapes the tensor-core kernels refuse.
 //
 //   out[r, n] (+)= sum_k A[row(r), k] * W_g[n, k]        (W is [N, K], K contiguous, as the
 //   reference stores its projection weights: crates/engine/src/flint.rs:293-300)
@@ -11,9 +11,6 @@
 // Each output element is summed over k in an order that follows from K alone, so its value does not
 // depend on which tile or batch the row was in.
 #include "common.cuh"
-
-int q6k_gemm_f32(const float* A, int lda, const int* a_rows, const float* W, const float* W2, size_t w_group_stride, float* out, int ldo, int M, int N, int K, const int* tile_group,
-                 const int* tile_row0, const int* group_offsets, const int* num_tiles, int max_tiles, int epilogue, int act, float act_limit, cudaStream_t st);      // gemm_f32.cu
 
 namespace {
 
@@ -105,6 +102,155 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* A, int lda, con
     }
 }
 
+// FP32 operands.  The kernel above loads one value at a time into a transposed tile that everyone then waits for, and leaves the
+// multipliers idle two thirds of the time.  Here rows go to shared memory as they lie, 16 bytes a copy, two blocks of 32 k ahead of the one in
+// use, and the products go through the packed multiply-add, which takes two FP32 products an instruction: with operands read four k at a time,
+// the even and the odd k of an output are its two halves, so nothing has to be rearranged.  An output is then four sums over ascending k (even and
+// odd, of either half of each block of 32), added in the end: no larger an error than one sum, and the same for a row whatever its tile.
+// A block makes 32 x 64 outputs, half of its threads the first 16 k of every block and half the others: small enough that 512
+// rows fill the chip and that experts of some 60 rows waste little, with 4 x 4 outputs a thread all the same (8 loads of 16 bytes
+// for 64 products; rows 144 bytes apart, so that eight threads' reads fall into different banks).
+// The 20 products of a step of 509 tokens through four layers (1,024 wide, experts of 512): 1,835 -> 1,670 us against tiles of 64 x 64 with
+// an instruction per product (2,930 us with the kernel above).  What bounds it now: the FP32 pipe, half of its cycles, and reads of
+// shared memory, two thirds (3.3 wavefronts a read).  Warps of 8 x 128 outputs, whose reads of one address were to cost less, took 2,100 us.
+// WIDE: rows start on 16 bytes and K is a multiple of 4; else copies of 4 bytes.
+constexpr int FM = 32, FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 3;
+static_assert(BM == 2 * FM, "a tile of the tile lists is two of these");
+
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum_pair(unsigned long long v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+
+// grid (ceil(N / 64), tiles of 64 rows, 2), 256 threads.
+template <int EPI, bool WIDE>
+__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(const float* A, int lda, const int* a_rows, const float* W, const float* W2,
+                                                                                  size_t w_group_stride, float* out, int ldo, int M, int N, int K,
+                                                                                  const int* tile_group, const int* tile_row0, const int* group_offsets,
+                                                                                  const int* num_tiles, int act, float act_limit) {
+    pdl_enter();
+    constexpr bool DUAL = EPI == EPI_SWIGLU;
+    constexpr int MATS = DUAL ? 2 : 1, STAGE = (FM + MATS * FN) * FLD;
+    extern __shared__ __align__(16) float f_smem[];          // [FSTAGES][A 32 rows | W 64 | W2 64][FLD]
+    int g = 0, row0 = blockIdx.y * BM, row_end = M;
+    if (tile_group) {
+        if ((int)blockIdx.y >= *num_tiles) return;
+        g = tile_group[blockIdx.y];
+        row0 = tile_row0[blockIdx.y];
+        row_end = group_offsets[g + 1];
+    }
+    row0 += blockIdx.z * FM;
+    if (row0 >= row_end) return;
+    const int n0 = blockIdx.x * FN, tid = threadIdx.x;
+    // loader: WIDE pieces of 4 k of rows tid / 8 (+ 32), else single k of rows tid / 32 + 8 e
+    constexpr int STEP = WIDE ? 32 : 8, A_ROWS = FM / STEP, W_ROWS = FN / STEP;
+    const int lr = WIDE ? tid >> 3 : tid >> 5, lk = WIDE ? (tid & 7) * 4 : tid & 31;
+    const float *a_src[A_ROWS], *w_src[MATS][W_ROWS];
+#pragma unroll
+    for (int e = 0; e < A_ROWS; ++e) {
+        const int r = row0 + lr + e * STEP;
+        a_src[e] = r < row_end ? A + (size_t)(a_rows ? a_rows[r] : r) * lda : nullptr;
+    }
+#pragma unroll
+    for (int e = 0; e < W_ROWS; ++e) {
+        const int n = n0 + lr + e * STEP;
+        w_src[0][e] = n < N ? W + (size_t)g * w_group_stride + (size_t)n * K : nullptr;
+        if (DUAL) w_src[MATS - 1][e] = n < N ? W2 + (size_t)g * w_group_stride + (size_t)n * K : nullptr;
+    }
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(f_smem);
+    const int blocks = (K + FK - 1) / FK;
+    auto fetch = [&](int b) {
+        if (b < blocks) {
+            const int k = b * FK + lk;
+            const uint32_t at = base + 4 * ((b % FSTAGES) * STAGE + lr * FLD + lk);
+            auto copy = [&](const float* row, int to_row) {
+                const bool in = row != nullptr && k < K;
+                const float* from = in ? row + k : A;
+                if (WIDE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + 4 * to_row * FLD), "l"(from), "r"(in ? 16 : 0) : "memory");
+                else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + 4 * to_row * FLD), "l"(from), "r"(in ? 4 : 0) : "memory");
+            };
+#pragma unroll
+            for (int e = 0; e < A_ROWS; ++e) copy(a_src[e], e * STEP);
+#pragma unroll
+            for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                for (int e = 0; e < W_ROWS; ++e) copy(w_src[m][e], FM + m * FN + e * STEP);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // this thread's outputs: rows ty + 4 i, columns tx + 8 j; its k: 16 of each block's 32
+    const int half = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31, tx = (warp & 1) * 32 + (lane & 7), ty = (warp >> 1) * 16 + (lane >> 3);
+    unsigned long long acc[MATS][4][4] = {};
+    fetch(0);
+    fetch(1);
+    for (int b = 0; b < blocks; ++b) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                     // this block has landed for everyone; the one before it is done with
+        fetch(b + 2);
+        const float* As = f_smem + (b % FSTAGES) * STAGE + ty * FLD + half * (FK / 2);
+        const float* Ws = f_smem + (b % FSTAGES) * STAGE + (FM + tx) * FLD + half * (FK / 2);
+#pragma unroll
+        for (int k = 0; k < FK / 2; k += 4) {
+            ulonglong2 a[4], w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(As + i * 4 * FLD + k);
+#pragma unroll
+            for (int m = 0; m < MATS; ++m) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + (m * FN + j * 8) * FLD + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma_pair(acc[m][i][j], a[i].x, w[j].x);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma_pair(acc[m][i][j], a[i].y, w[j].y);
+            }
+        }
+    }
+    // the second half of the threads hands its sums over
+    __syncthreads();
+    float* sums = f_smem + (tid & 127);                      // [matrix, i, j][128 threads]
+    if (half == 1) {
+#pragma unroll
+        for (int e = 0; e < MATS * 16; ++e) sums[e * 128] = sum_pair(acc[e / 16][e / 4 % 4][e % 4]);
+    }
+    __syncthreads();
+    if (half == 1) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row0 + ty + 4 * i;
+        if (r >= row_end) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tx + 8 * j;
+            if (n >= N) continue;
+            float* o = out + (size_t)r * ldo + n;
+            const float v = sum_pair(acc[0][i][j]) + sums[(i * 4 + j) * 128];
+            if (EPI == EPI_STORE) *o = v;
+            else if (EPI == EPI_ADD) *o += v;
+            else if (EPI == EPI_ACT) *o = q6k_activation(v, act);
+            else {
+                const float up = sum_pair(acc[MATS - 1][i][j]) + sums[(MATS * 16 - 16 + i * 4 + j) * 128];
+                *o = act == 0 ? v / (1.0f + expf(-v)) * up : q6k_gated(v, up, act, act_limit);
+            }
+        }
+    }
+}
+
+template <int EPI>
+int launch_f32(dim3 grid, bool wide, cudaStream_t st, const float* A, int lda, const int* a_rows, const float* W, const float* W2, size_t w_group_stride,
+               float* out, int ldo, int M, int N, int K, const int* tile_group, const int* tile_row0, const int* group_offsets, const int* num_tiles, int act,
+               float act_limit) {
+    const size_t smem = (size_t)FSTAGES * (FM + (EPI == EPI_SWIGLU ? 2 : 1) * FN) * FLD * sizeof(float);
+    grid.z = BM / FM;
+    auto* kernel = wide ? gemm_f32_kernel<EPI, true> : gemm_f32_kernel<EPI, false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return q6k_check_launch("gemm_f32: shared memory attribute");
+    q6k_launch(kernel, grid, 256, smem, st, A, lda, a_rows, W, W2, w_group_stride, out, ldo, M, N, K, tile_group, tile_row0, group_offsets, num_tiles, act, act_limit);
+    return q6k_check_launch("gemm_f32");
+}
+
 // Row tiles of the groups: for offsets[0..G] the list of (group, first row) of every BM-row tile.
 // One block; groups are walked in order so the list is a function of the offsets only.
 __global__ void tile_list_kernel(const int* offsets, int G, int bm, int* tile_group, int* tile_row0, int* num_tiles,
@@ -174,8 +320,14 @@ Q6K_API int q6k_gemm_simt(const void* A, int lda, const int* a_rows, const void*
     Q6K_REQUIRE(ytiles <= 65535, "gemm: %d row tiles exceed the grid limit", ytiles);
     dim3 grid((N + BN - 1) / BN, ytiles);
     if (dtype == Q6K_F32) {
-        return q6k_gemm_f32((const float*)A, lda, a_rows, (const float*)W, (const float*)W2, (size_t)w_group_stride, (float*)out, ldo, M, N, K, tile_group, tile_row0, group_offsets,
-                            num_tiles, max_tiles, epilogue, act, act_param, st);
+        const bool wide = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W | (uintptr_t)W2) & 15) == 0 && w_group_stride % 4 == 0;
+#define LAUNCH_F32(EPI) launch_f32<EPI>(grid, wide, st, (const float*)A, lda, a_rows, (const float*)W, (const float*)W2, (size_t)w_group_stride, (float*)out, ldo, M, N, K, \
+                                        tile_group, tile_row0, group_offsets, num_tiles, act, act_param)
+        if (epilogue == EPI_STORE) return LAUNCH_F32(EPI_STORE);
+        if (epilogue == EPI_ADD) return LAUNCH_F32(EPI_ADD);
+        if (epilogue == EPI_ACT) return LAUNCH_F32(EPI_ACT);
+        return LAUNCH_F32(EPI_SWIGLU);
+#undef LAUNCH_F32
     }
     using T = __nv_bfloat16;
 #define LAUNCH(EPI)                                                                                                     \

@@ -239,7 +239,7 @@ def swiglu(gu: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     return act
 
 
-# --------------------------------------------------------------------------- matrix products (CUDA cores, FP32)
+# --------------------------------------------------------------------------- matrix products (CUDA cores)
 EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_ACT, EPI_BF16 = 0, 1, 2, 4, 5
 ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "relu2": 2}
 # A gate that takes a constant is named with it, ("clamped", limit): with g the gate's product and u the other one,
@@ -284,7 +284,7 @@ def _act_param(act) -> float:
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
               w2: Optional[torch.Tensor] = None, a_rows: Optional[torch.Tensor] = None, groups=None,
               rows: Optional[int] = None, act: Optional[str] = None) -> torch.Tensor:
-    """out[r] (+)= a[row(r)] @ w_g^T with FP32 fused multiply-adds, for FP32 operands as exact products of bfloat16 parts at FP32's precision.  act: the gate's activation when w2 is given (default
+    """out[r] (+)= a[row(r)] @ w_g^T with FP32 fused multiply-adds.  act: the gate's activation when w2 is given (default
     silu); without w2, out = act(a w^T) in a's dtype.
 
     a: [*, K]; w: [N, K] or, grouped, [G, N, K]; w2 (same shape) switches to the SwiGLU epilogue,
@@ -376,8 +376,7 @@ def tc_status() -> int:
     lib.q6k_attention_tc_status.restype = ctypes.c_int
     lib.q6k_router_status.restype = ctypes.c_int
     lib.q6k_attention_flex_tc_status.restype = ctypes.c_int
-    lib.q6k_gemm_f32_status.restype = ctypes.c_int
-    return (lib.q6k_gemm_f32_status() or lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_attention_flex_tc_status()
+    return (lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_attention_flex_tc_status()
             or lib.q6k_router_status())
 
 

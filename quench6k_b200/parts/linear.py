@@ -1,7 +1,7 @@
 """Chooses the matrix-product kernel for an operand dtype and shape.
 
-float32 operands always take the FP32 kernel (tensor cores on exact bfloat16 parts of the operands, sums at FP32's own
-precision; no reduced-precision matrix mode exists on that path).  bfloat16 operands take the tcgen05 tensor-core kernel where the shape allows (K a
+float32 operands always take the CUDA-core FP32 kernel (no reduced-precision matrix mode exists on
+that path).  bfloat16 operands take the tcgen05 tensor-core kernel where the shape allows (K a
 multiple of 8, rows starting on 16 bytes), the matrix-vector kernel or the mma.sync kernel for few tokens where the
 library prefers them (steps of at most 16 tokens), and the CUDA-core kernel otherwise.
 """
