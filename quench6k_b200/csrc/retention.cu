@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(128) time_mix_prep_kernel(const float* r, cons
 // chunk's results, [d^(i+1) Q | M] times [S | V] as one product of 64 x 128 outputs whose second factor comes by in slices of 32 rows.
 // FP32 throughout; powers of d are made in double precision.  C = 64: 32 would double the bytes of the states (one per chunk and head).
 // 2,550 tokens in three portions, 16 heads of 128 x 128: 202 us token by token, 41 + 14 + 95 us so.  What bounds the two products: reads of
-// shared memory beside the FP32 pipe, each about half of the time.
+// shared memory beside the FP32 pipe, each about half of the time.  Heads of 65 to 128 keys take chunks of 128 on the tensor cores instead (retention_tc.cuh).
 constexpr int RC = 64;
 
 __device__ __forceinline__ float ret_power(float d, int n) {
@@ -421,6 +421,10 @@ __device__ __forceinline__ float ret_power(float d, int n) {
         if (n & 1) p *= x;
     return (float)p;
 }
+
+}  // namespace
+#include "retention_tc.cuh"
+namespace {
 
 // grid (H, chunks, ceil(dk / 128) ceil(dv / 128)) (blocks of chunks that there are not come last), 256 threads, 64 KB of dynamic shared memory; KV: FP32 [chunks, H, dk, dv].
 __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const float* vp, int ld, const float* decay, const int* q_start, int R, int beyond, float* KV, int H, int dk,
@@ -476,17 +480,18 @@ __global__ void __launch_bounds__(256) ret_outer_kernel(const float* kp, const f
 }
 
 // The state every chunk starts from, in its sum's place, and the state a portion leaves.  grid (long requests * blocks), blocks = ceil(H dk dv / 1024).
+template <int CT>
 __global__ void __launch_bounds__(256) ret_fold_kernel(float* KV, const float* decay, float* state, const int* q_start, int R, int beyond, const int* slot_ids, int H, int cells) {
     pdl_enter();
     const size_t all = (size_t)H * cells;                   // cells = dk dv, a multiple of 4
     const unsigned blocks = (unsigned)((all + 1023) / 1024);
     int chunk0;
-    const int r = long_request<RC>(q_start, R, beyond, blockIdx.x / blocks, chunk0);
+    const int r = long_request<CT>(q_start, R, beyond, blockIdx.x / blocks, chunk0);
     if (r < 0) return;
-    const int n = q_start[r + 1] - q_start[r], count = (n + RC - 1) / RC;
+    const int n = q_start[r + 1] - q_start[r], count = (n + CT - 1) / CT;
     const size_t i = ((size_t)(blockIdx.x % blocks) * 256 + threadIdx.x) * 4;
     if (i >= all) return;
-    const float d = decay[i / cells], full = ret_power(d, RC), rest = ret_power(d, n - (count - 1) * RC);
+    const float d = decay[i / cells], full = ret_power(d, CT), rest = ret_power(d, n - (count - 1) * CT);
     float4* mine = reinterpret_cast<float4*>(state + (size_t)slot_ids[r] * all + i);
     float4 S = *mine;
     float* at = KV + (size_t)chunk0 * all + i;
@@ -675,7 +680,17 @@ Q6K_API int q6k_retention(const float* p, int ld, int q_col, int k_col, int v_co
 }
 
 // Floats of scratch for the same walk chunk by chunk.
-Q6K_API long long q6k_retention_chunk_floats(int T_, int R, int H, int dk, int dv, int beyond) { return (long long)most_chunks<RC>(T_, R, beyond) * H * dk * dv; }
+// Heads of more than 64 and up to 128 keys go on the tensor cores, in chunks of 128: narrower ones would fill half of their tiles (a head of 64 x 64,
+// 1,024 tokens of 16: 47 us in FP32, 37 us for the tiles of twice its size), wider ones do not fit.
+static bool retention_tc(int dk) { return dk > 64 && dk <= 128; }
+Q6K_API long long q6k_retention_chunk_floats(int T_, int R, int H, int dk, int dv, int beyond) {
+    return (long long)(retention_tc(dk) ? most_chunks<RT>(T_, R, beyond) : most_chunks<RC>(T_, R, beyond)) * H * dk * dv;
+}
+Q6K_API int q6k_retention_tc_status() {
+    int v = -1;
+    if (cudaMemcpyFromSymbol(&v, g_retention_tc_status, sizeof v) != cudaSuccess) return -1;
+    return v;
+}
 
 // Requests of more than `beyond` tokens in chunks of 64 (T_: rows of the step): rows and heads of q, k and v that start on 16 bytes,
 // dk and dv multiples of 4.
@@ -687,13 +702,28 @@ Q6K_API int q6k_retention_chunked(const float* p, int ld, int q_col, int k_col, 
                 "retention: chunks take rows and heads that start on 16 bytes");
     const int n_long = most_long(T_, R, beyond), n_chunks = most_chunks<RC>(T_, R, beyond), cols = (dv + 127) / 128, dkp = (dk + 31) / 32 * 32;
     if (n_long == 0) return 0;
+    const unsigned folds = (unsigned)(n_long * (((size_t)H * dk * dv + 1023) / 1024));
+    if (retention_tc(dk)) {
+        const long long tasks = (long long)most_chunks<RT>(T_, R, beyond) * H * cols;
+        Q6K_REQUIRE(tasks < 0x7fffffff - 1024, "retention: %lld tasks", tasks);
+        const unsigned grid = (unsigned)(tasks < 148 ? tasks : 148);
+        if (cudaFuncSetAttribute(ret_outer_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(ret_out_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_SMEM) != cudaSuccess)
+            return q6k_check_launch("retention: shared memory attribute");
+        q6k_launch(ret_outer_tc_kernel, grid, RT_THREADS, RT_SMEM, st, p + k_col, p + v_col, ld, decay, q_start, R, beyond, chunks, H, dk, dv, (int)tasks);
+        if (int rc = q6k_check_launch("ret_outer_tc")) return rc;
+        q6k_launch(ret_fold_kernel<RT>, dim3(folds), 256, 0, st, chunks, decay, state, q_start, R, beyond, slot_ids, H, dk * dv);
+        if (int rc = q6k_check_launch("ret_fold")) return rc;
+        q6k_launch(ret_out_tc_kernel, grid, RT_THREADS, RT_SMEM, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, beyond, o, H, dk, dv, (int)tasks);
+        return q6k_check_launch("ret_out_tc");
+    }
     const size_t smem1 = (size_t)2 * RC * 128 * sizeof(float), smem2 = (size_t)ret_out_floats(dkp) * sizeof(float);
     if (cudaFuncSetAttribute(ret_outer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
         cudaFuncSetAttribute(ret_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess)
         return q6k_check_launch("retention: shared memory attribute");
     q6k_launch(ret_outer_kernel, dim3(H, n_chunks, (dk + 127) / 128 * cols), 256, smem1, st, p + k_col, p + v_col, ld, decay, q_start, R, beyond, chunks, H, dk, dv);
     if (int rc = q6k_check_launch("ret_outer")) return rc;
-    q6k_launch(ret_fold_kernel, dim3((unsigned)(n_long * (((size_t)H * dk * dv + 1023) / 1024))), 256, 0, st, chunks, decay, state, q_start, R, beyond, slot_ids, H, dk * dv);
+    q6k_launch(ret_fold_kernel<RC>, dim3(folds), 256, 0, st, chunks, decay, state, q_start, R, beyond, slot_ids, H, dk * dv);
     if (int rc = q6k_check_launch("ret_fold")) return rc;
     q6k_launch(ret_out_kernel, dim3(H, n_chunks, cols), 256, smem2, st, p + q_col, p + k_col, p + v_col, ld, decay, chunks, q_start, R, beyond, o, H, dk, dv, dkp);
     return q6k_check_launch("ret_out");

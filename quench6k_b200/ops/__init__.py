@@ -376,7 +376,8 @@ def tc_status() -> int:
     lib.q6k_attention_tc_status.restype = ctypes.c_int
     lib.q6k_router_status.restype = ctypes.c_int
     lib.q6k_attention_flex_tc_status.restype = ctypes.c_int
-    return (lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_attention_flex_tc_status()
+    lib.q6k_retention_tc_status.restype = ctypes.c_int
+    return (lib.q6k_retention_tc_status() or lib.q6k_tc_status() or lib.q6k_attention_status() or lib.q6k_attention_tc_status() or lib.q6k_attention_flex_tc_status()
             or lib.q6k_router_status())
 
 
@@ -1779,7 +1780,8 @@ def retention_chunks(q_lens, H: int, dk: int, dv: int) -> bool:
     the longest portion decides (its blocks slow one another down once several share an SM); by chunks the rounds of 64-token chunks
     over the SMs do, and short portions wait for a launch of their own.  16 heads of 128 x 128, walk and chunks: 65 tokens 10 and
     35, 320 tokens 36 and 37, 512 tokens 56 and 38, eight portions of 200 91 and 118, two of 1,024 146 and 120, 65 beside 32 of one 30 and 54,
-    512 beside 8 of one 105 and 45."""
+    512 beside 8 of one 105 and 45, with FP32 multiply-adds by chunks.  Where the tensor cores take the keys the chunks are the faster form a little
+    earlier than this says (320 tokens 34, eight portions of 200 69, two of 1,024 63, 512 beside 8 of one 44); the line stays where it was."""
     longest = max(q_lens, default=0)
     if longest <= CHUNKS_BEYOND:
         return False
@@ -1800,7 +1802,7 @@ def retention(p: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.
               slot_ids: torch.Tensor, R: int, H: int, dk: int, dv: int, longest: int = 0, shortest: int = 0) -> torch.Tensor:
     """Per request and head, in token order: S <- decay[h] S + k v^T, o = S^T q.  p FP32 [T, N] with q, k (prepared) and v
     at their columns; state FP32 [slots, H, dk, dv], updated in place; returns o FP32 [T, H dv].  longest: tokens of the step's
-    longest portion; beyond 64 (the walk token by token takes 200 ns each), rows that start on 16 bytes go 64 tokens at a time, equal up to
+    longest portion; beyond 64 (the walk token by token takes 200 ns each), rows that start on 16 bytes go 64 or 128 tokens at a time, equal up to
     rounding, if the states of all the chunks take no more than 256 MB.  shortest: tokens of its shortest portion; where it says that
     there are portions of up to CHUNKS_BEYOND tokens beside the long ones, those are walked token by token all the same (the same bits as
     in a step of their own)."""
