@@ -208,160 +208,195 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
     if (sub == 0 && taps > 1) scan_move_tail(tail + (size_t)slot * (taps - 1) * C + c, xz + (size_t)first_req * ldx + c, ldx, C, n_req, taps);
 }
 
-// ---------------------------------------------------------------------------------------- a lane per state, one pass
+// ---------------------------------------------------------------------------------------- a lane per two states, one pass
 //
-// With up to 16 states a channel and enough channels, a portion needs no segments: a lane per state gives 16 C chains (2,048 warps for
-// 4,096 channels), which walk all the tokens once where the segments' two launches compute every decay twice.  A block takes 16
-// channels.  Per tile of 64 tokens its threads make dt, dt u, the gate and the skip of each (token, channel) once, from loads asked for
-// before the tile before was walked; then a lane steps through the tile, reading four tokens' dt, dt u, B and C at a time and leaving
-// S C in shared memory, and every 16 tokens the lanes sum the 16 values of each (token, channel).  The decays of two
-// tokens go through packed instructions.  2,048 tokens, 4,096 channels of 16 states: 171 us against 371 in segments (186 with tiles of 32
-// tokens).  What bounds it: issue slots, two thirds of them taken where four warps share a scheduler, and the chain through a tile's
-// preparation and its two barriers.
-// decay_minus_one of two tokens' dt (FP32, the first in the low half) times a, with packed arithmetic where FAST.
-template <bool FAST>
-__device__ __forceinline__ void decay_minus_one_pair(unsigned long long dt, float a, float* out) {
-    const float d0 = __uint_as_float((uint32_t)dt), d1 = __uint_as_float((uint32_t)(dt >> 32));
-    if (!FAST) {
-        out[0] = decay_minus_one<false>(d0 * a), out[1] = decay_minus_one<false>(d1 * a);
-        return;
-    }
-    auto both = [](float v) {
-        unsigned long long r;
-        asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-        return r;
-    };
-    auto mul = [](unsigned long long x, unsigned long long y) {
-        unsigned long long r;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
-        return r;
-    };
-    auto fma = [](unsigned long long x, unsigned long long y, unsigned long long z) {
-        unsigned long long r;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
-        return r;
-    };
-    const unsigned long long x = mul(dt, both(a)), y = mul(dt, both(a * 1.44269504088896341f));
-    unsigned long long p = fma(x, both(1.0f / 120.0f), both(1.0f / 24.0f));
-    p = fma(x, p, both(1.0f / 6.0f));
-    p = fma(x, p, both(0.5f));
-    p = mul(x, fma(x, p, both(1.0f)));
-    float e0, e1;                            // beyond e^-87 a decay is zero beside the 1 that is taken from it
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(__uint_as_float((uint32_t)y)));
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(__uint_as_float((uint32_t)(y >> 32))));
-    out[0] = __uint_as_float((uint32_t)x) > -0.25f ? __uint_as_float((uint32_t)p) : e0 - 1.0f;
-    out[1] = __uint_as_float((uint32_t)(x >> 32)) > -0.25f ? __uint_as_float((uint32_t)(p >> 32)) : e1 - 1.0f;
+// With up to 16 states a channel and enough channels, a portion needs no segments: a lane per two states gives 8 C chains, which walk all the tokens
+// once where the segments' two launches compute every decay twice.  A block takes 16 channels.  Half of its warps make dt, dt u, the gate and the skip
+// of each (token, channel) of the next 32 tokens once, from loads asked for a tile earlier, and store the results of the tile before; the other half
+// steps through a tile meanwhile, with packed instructions over its lanes' two states (the same operations as a state each, so the same states bit for
+// bit).  dt and dt u lie twice in shared memory, B and C as pairs of states of two tokens, so that every operand comes as the packed instruction
+// takes it; S C is left in shared memory, and every 16 tokens a lane sums the values of one channel's two tokens.
+// 2,048 tokens, 4,096 channels of 16 states: 150 us; a lane per state, every warp in both roles, 170; in segments 345.  What bounds it: issue slots, of
+// which a lane per state took twice as many for the same operands read from shared memory.  Not faster: every warp in both roles (225), tiles of 64
+// tokens (144 and 151 where tiles of 32 took 143 and 137 for one portion of 2,048 and three of 682: two blocks on an SM instead of three), registers
+// for four blocks (148 and 138), the operands of the next four tokens asked for ahead (152 against 145).
+// decay_minus_one of two states at one dt, which comes twice, with packed arithmetic where FAST.
+__device__ __forceinline__ unsigned long long ls_pair(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
+__device__ __forceinline__ unsigned long long ls_mul(unsigned long long x, unsigned long long y) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+__device__ __forceinline__ unsigned long long ls_add(unsigned long long x, unsigned long long y) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+__device__ __forceinline__ unsigned long long ls_fma(unsigned long long x, unsigned long long y, unsigned long long z) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+__device__ __forceinline__ float ls_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float ls_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+template <bool FAST>
+__device__ __forceinline__ unsigned long long decay_minus_one_pair(unsigned long long dt, unsigned long long a) {
+    const unsigned long long x = ls_mul(dt, a);
+    if (!FAST) return ls_pair(decay_minus_one<false>(ls_lo(x)), decay_minus_one<false>(ls_hi(x)));
+    constexpr float LOG2E = 1.44269504088896341f;
+    unsigned long long p = ls_fma(x, ls_pair(1.0f / 120.0f, 1.0f / 120.0f), ls_pair(1.0f / 24.0f, 1.0f / 24.0f));
+    p = ls_fma(x, p, ls_pair(1.0f / 6.0f, 1.0f / 6.0f));
+    p = ls_fma(x, p, ls_pair(0.5f, 0.5f));
+    p = ls_mul(x, ls_fma(x, p, ls_pair(1.0f, 1.0f)));
+    const unsigned long long y = ls_mul(x, ls_pair(LOG2E, LOG2E));
+    float e0, e1;                            // beyond e^-87 a decay is zero beside the 1 that is taken from it
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(ls_lo(y)));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(ls_hi(y)));
+    const unsigned long long far = ls_add(ls_pair(e0, e1), ls_pair(-1.0f, -1.0f));
+    return ls_pair(ls_lo(x) > -0.25f ? ls_lo(p) : ls_lo(far), ls_hi(x) > -0.25f ? ls_hi(p) : ls_hi(far));
+}
+constexpr int LS_N = 16, LS_CH = 16, LS_WALK = LS_N / 2 * LS_CH, LS_THREADS = 2 * LS_WALK, LS_TILE = 32, LS_LD = LS_TILE + 1;
+struct LsTile {
+    float4 dd[LS_CH][LS_LD];                     // [channel][token]: dt, dt, dt u, dt u
+    float2 gs[LS_CH][LS_LD];                     // [channel][token]: gate, skip
+    float bc[2][LS_TILE / 2][2 * LS_N];          // B, then C: [two tokens][two states][token of the two][state of the two]
+};
 
-constexpr int LS_N = 16, LS_CH = 16, LS_THREADS = LS_N * LS_CH, LS_TILE = 64, LS_LD = LS_TILE + 4;
-
+// grid (R, ceil(C / 16)), 256 threads: warps 0-3 walk, warps 4-7 make the next tile's values meanwhile and store the last tile's results.
 template <typename T>
-__global__ void __launch_bounds__(LS_THREADS) scan_lanes_kernel(const T* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col,
-                                                                int c_col, const float* A, const float* Dskip, const float* xz, int ldx, int z_col,
-                                                                float* state, float* tail, const int* q_start, const int* slot_ids, T* out, int C, int N,
-                                                                int taps) {
+__global__ void __launch_bounds__(LS_THREADS, 3) scan_lanes_kernel(const T* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col,
+                                                                   int c_col, const float* A, const float* Dskip, const float* xz, int ldx, int z_col,
+                                                                   float* state, float* tail, const int* q_start, const int* slot_ids, T* out, int C, int N,
+                                                                   int taps) {
     pdl_enter();
-    __shared__ __align__(16) float s_dt[LS_CH][LS_LD], s_du[LS_CH][LS_LD], s_gate[LS_CH][LS_LD], s_skip[LS_CH][LS_LD];       // [channel][token]
-    __shared__ __align__(16) float s_bc[2 * LS_N][LS_LD];                    // [state of B, then of C][token]
-    __shared__ __align__(16) float s_y[LS_THREADS / 32][8][68];              // a warp's S C: [pair of tokens][lane][token of it]
-    __shared__ T s_out[LS_TILE][LS_CH];
-    const int r = blockIdx.x, c0 = blockIdx.y * LS_CH, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    extern __shared__ __align__(16) uint8_t ls_smem[];
+    LsTile* tiles = reinterpret_cast<LsTile*>(ls_smem);
+    __shared__ __align__(16) float s_y[LS_WALK / 32][8][80];                 // a warp's S C: [two tokens][channel, 20 apart][lane][token of the two]
+    __shared__ T s_out[2][LS_TILE][LS_CH];
+    const int r = blockIdx.x, c0 = blockIdx.y * LS_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = q_start[r], n_tok = q_start[r + 1] - first;
     if (n_tok <= 0) return;
-    const int slot = slot_ids[r], cc = tid >> 4, n = tid & 15, c = c0 + cc;
-    const bool has = c < C && n < N;                                         // a state beyond N has A = B = C = 0 and stays zero
-    const float a = has ? A[(size_t)c * N + n] : 0.0f;
-    float S = has ? state[((size_t)slot * C + c) * N + n] : 0.0f;
-    // a thread's share of a tile: four (token, channel) and eight entries of B and C
-    const int pc = tid & 15, pt = tid >> 4, bn = tid & 31, bt = tid >> 5;
-    const bool p_in = c0 + pc < C, b_in = (bn & 15) < N;
-    const float bias = p_in ? dt_bias[c0 + pc] : 0.0f, skip = p_in ? Dskip[c0 + pc] : 0.0f;
-    const int col = bn < LS_N ? b_col + bn : c_col + bn - LS_N;
-    float f_dt[LS_TILE / 16], f_u[LS_TILE / 16], f_z[LS_TILE / 16], f_bc[LS_TILE / 8];
-    auto fetch = [&](int t0) {
+    const int n_tiles = (n_tok + LS_TILE - 1) / LS_TILE, slot = slot_ids[r];
+    if (warp >= LS_WALK / 32) {
+        constexpr int SHARE = LS_TILE * LS_CH / LS_WALK, SHARE_BC = LS_TILE * 2 * LS_N / LS_WALK;
+        const int tid = threadIdx.x - LS_WALK, pc = tid & 15, pt = tid >> 4, bn = tid & 31, bt = tid >> 5;
+        const bool p_in = c0 + pc < C, b_in = (bn & 15) < N;
+        const float bias = p_in ? dt_bias[c0 + pc] : 0.0f, skip = p_in ? Dskip[c0 + pc] : 0.0f;
+        const int col = bn < LS_N ? b_col + bn : c_col + bn - LS_N;
+        float f_dt[SHARE], f_u[SHARE], f_z[SHARE], f_bc[SHARE_BC];
+        auto fetch = [&](int t0) {
 #pragma unroll
-        for (int j = 0; j < LS_TILE / 16; ++j) {
-            const int t = t0 + pt + 16 * j;
-            const size_t row = (size_t)(first + t);
-            const bool in = p_in && t < n_tok;
-            f_dt[j] = in ? dt_raw[row * C + c0 + pc] : 0.0f;
-            f_u[j] = in ? to_f32(u[row * C + c0 + pc]) : 0.0f;
-            f_z[j] = in ? xz[row * ldx + z_col + c0 + pc] : 0.0f;
-        }
+            for (int j = 0; j < SHARE; ++j) {
+                const int t = t0 + pt + LS_WALK / LS_CH * j;
+                const size_t row = (size_t)(first + t);
+                const bool in = p_in && t < n_tok;
+                f_dt[j] = in ? dt_raw[row * C + c0 + pc] : 0.0f;
+                f_u[j] = in ? to_f32(u[row * C + c0 + pc]) : 0.0f;
+                f_z[j] = in ? xz[row * ldx + z_col + c0 + pc] : 0.0f;
+            }
 #pragma unroll
-        for (int j = 0; j < LS_TILE / 8; ++j) {
-            const int t = t0 + bt + 8 * j;
-            f_bc[j] = b_in && t < n_tok ? proj[(size_t)(first + t) * ldp + col] : 0.0f;
-        }
-    };
-    fetch(0);
-    for (int t0 = 0; t0 < n_tok; t0 += LS_TILE) {
-        const int nt = min(LS_TILE, n_tok - t0);
+            for (int j = 0; j < SHARE_BC; ++j) {
+                const int t = t0 + bt + LS_WALK / 32 * j;
+                f_bc[j] = b_in && t < n_tok ? proj[(size_t)(first + t) * ldp + col] : 0.0f;
+            }
+        };
+        auto make = [&](LsTile& x) {
 #pragma unroll
-        for (int j = 0; j < LS_TILE / 16; ++j) {
-            const int t = pt + 16 * j;
-            const float dt = softplus_f(f_dt[j] + bias);
-            s_dt[pc][t] = dt;
-            s_du[pc][t] = dt * f_u[j];
-            s_gate[pc][t] = silu_f(f_z[j]);
-            s_skip[pc][t] = skip * f_u[j];
-        }
+            for (int j = 0; j < SHARE; ++j) {
+                const int t = pt + LS_WALK / LS_CH * j;
+                const float dt = softplus_f(f_dt[j] + bias), du = dt * f_u[j];
+                x.dd[pc][t] = make_float4(dt, dt, du, du);
+                x.gs[pc][t] = make_float2(silu_f(f_z[j]), skip * f_u[j]);
+            }
 #pragma unroll
-        for (int j = 0; j < LS_TILE / 8; ++j) s_bc[bn][bt + 8 * j] = f_bc[j];
+            for (int j = 0; j < SHARE_BC; ++j) {
+                const int t = bt + LS_WALK / 32 * j;
+                x.bc[bn >> 4][t >> 1][((bn & 15) >> 1) * 4 + (t & 1) * 2 + (bn & 1)] = f_bc[j];
+            }
+        };
+        auto store = [&](int i) {
+            const int t0 = i * LS_TILE;
+#pragma unroll
+            for (int j = 0; j < SHARE; ++j) {
+                const int t = pt + LS_WALK / LS_CH * j;
+                if (p_in && t0 + t < n_tok) out[(size_t)(first + t0 + t) * C + c0 + pc] = s_out[i & 1][t][pc];
+            }
+        };
+        fetch(0);
+        make(tiles[0]);
+        fetch(LS_TILE);
         __syncthreads();
-        if (t0 + LS_TILE < n_tok) fetch(t0 + LS_TILE);
+        for (int i = 0; i < n_tiles; ++i) {
+            if (i + 1 < n_tiles) make(tiles[(i + 1) & 1]);
+            fetch((i + 2) * LS_TILE);
+            if (i > 0) store(i - 1);
+            __syncthreads();
+        }
+        store(n_tiles - 1);
+        return;
+    }
+    const int tid = threadIdx.x, cc = tid >> 3, n = (tid & 7) * 2, c = c0 + cc;
+    const bool has0 = c < C && n < N, has1 = c < C && n + 1 < N;             // a state beyond N has A = B = C = 0 and stays zero
+    const float a0 = has0 ? A[(size_t)c * N + n] : 0.0f, a1 = has1 ? A[(size_t)c * N + n + 1] : 0.0f;
+    const unsigned long long a = ls_pair(a0, a1);
+    float* mine = state + ((size_t)slot * C + (c < C ? c : 0)) * N + n;
+    unsigned long long S = ls_pair(has0 ? mine[0] : 0.0f, has1 ? mine[1] : 0.0f);
+    __syncthreads();
+    for (int i = 0; i < n_tiles; ++i) {
+        const LsTile& x = tiles[i & 1];
+        const int nt = min(LS_TILE, n_tok - i * LS_TILE);
 #pragma unroll 1
         for (int g = 0; g < LS_TILE; g += 16) {
             if (g >= nt) break;
             auto walk = [&](auto whole) {                    // whole: 16 tokens; else the nt - g that there are
 #pragma unroll
                 for (int q = 0; q < 16; q += 4) {
-                    const ulonglong2 dt4 = *reinterpret_cast<const ulonglong2*>(&s_dt[cc][g + q]);
-                    const float4 du4 = *reinterpret_cast<const float4*>(&s_du[cc][g + q]), b4 = *reinterpret_cast<const float4*>(&s_bc[n][g + q]);
-                    const float4 c4 = *reinterpret_cast<const float4*>(&s_bc[LS_N + n][g + q]);
-                    const float du_[4] = {du4.x, du4.y, du4.z, du4.w}, b_[4] = {b4.x, b4.y, b4.z, b4.w};
-                    float SS[4];
+                    unsigned long long near_one[4], du[4];
 #pragma unroll
-                    for (int e = 0; e < 4; e += 2) {
-                        float near_one[2];
-                        decay_minus_one_pair<sizeof(T) == 2>(e ? dt4.y : dt4.x, a, near_one);
-#pragma unroll
-                        for (int f = 0; f < 2; ++f) {
-                            // exp(dt A) S as S + expm1(dt A) S, as above
-                            const float next = fmaf(du_[e + f], b_[e + f], fmaf(near_one[f], S, S));
-                            if (decltype(whole)::value || g + q + e + f < nt) S = next;
-                            SS[e + f] = S;
-                        }
+                    for (int e = 0; e < 4; ++e) {
+                        const ulonglong2 dd = *reinterpret_cast<const ulonglong2*>(&x.dd[cc][g + q + e]);
+                        near_one[e] = decay_minus_one_pair<sizeof(T) == 2>(dd.x, a), du[e] = dd.y;
                     }
-                    *reinterpret_cast<float2*>(&s_y[warp][q / 2][lane * 2]) = make_float2(SS[0] * c4.x, SS[1] * c4.y);
-                    *reinterpret_cast<float2*>(&s_y[warp][q / 2 + 1][lane * 2]) = make_float2(SS[2] * c4.z, SS[3] * c4.w);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2*>(&x.bc[0][(g + q) / 2 + h][n * 2]), c2 = *reinterpret_cast<const ulonglong2*>(&x.bc[1][(g + q) / 2 + h][n * 2]);
+                        float y[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            // exp(dt A) S as S + expm1(dt A) S, as above
+                            const unsigned long long next = ls_fma(du[2 * h + e], e ? b2.y : b2.x, ls_fma(near_one[2 * h + e], S, S));
+                            if (decltype(whole)::value || g + q + 2 * h + e < nt) S = next;
+                            const unsigned long long sc = ls_mul(S, e ? c2.y : c2.x);
+                            y[e] = ls_lo(sc) + ls_hi(sc);
+                        }
+                        *reinterpret_cast<float2*>(&s_y[warp][q / 2 + h][(lane >> 3) * 20 + (lane & 7) * 2]) = make_float2(y[0], y[1]);
+                    }
                 }
             };
             if (g + 16 <= nt) walk(std::true_type{});
             else walk(std::false_type{});
             __syncwarp();
-            // a lane adds eight states' values of two tokens, then takes the other eight's sum of one of them from the lane 16 away
-            const int pair = lane & 7, ch = (lane >> 3) & 1, part = lane >> 4;
-            const float4* p = reinterpret_cast<const float4*>(&s_y[warp][pair][ch * 32 + part * 16]);
-            float y0 = 0.0f, y1 = 0.0f;
+            // a lane sums the eight lanes' values of one channel's two tokens
+            const int pair = lane >> 2, ch = lane & 3, c_at = warp * 4 + ch;
+            const ulonglong2* p = reinterpret_cast<const ulonglong2*>(&s_y[warp][pair][ch * 20]);
+            const ulonglong2 v0 = p[0], v1 = p[1], v2 = p[2], v3 = p[3];
+            const unsigned long long y2 = ls_add(ls_add(ls_add(v0.x, v0.y), ls_add(v1.x, v1.y)), ls_add(ls_add(v2.x, v2.y), ls_add(v3.x, v3.y)));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 v = p[k];
-                y0 += v.x, y1 += v.y, y0 += v.z, y1 += v.w;
+            for (int e = 0; e < 2; ++e) {
+                const int tok = g + 2 * pair + e;
+                const float2 gs = x.gs[c_at][tok];
+                s_out[i & 1][tok][c_at] = from_f32<T>(((e ? ls_hi(y2) : ls_lo(y2)) + gs.y) * gs.x);
             }
-            const float other = __shfl_xor_sync(0xffffffffu, part ? y0 : y1, 16), y = (part ? y1 : y0) + other;
-            const int tok = g + 2 * pair + part, c_at = 2 * warp + ch;
-            s_out[tok][c_at] = from_f32<T>((y + s_skip[c_at][tok]) * s_gate[c_at][tok]);
             __syncwarp();
         }
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < LS_TILE / 16; ++j) {
-            const int t = pt + 16 * j;
-            if (p_in && t < nt) out[(size_t)(first + t0 + t) * C + c0 + pc] = s_out[t][pc];
-        }
     }
-    if (has) state[((size_t)slot * C + c) * N + n] = S;
+    if (has0) mine[0] = ls_lo(S);
+    if (has1) mine[1] = ls_hi(S);
     if (c < C && n == 0 && taps > 1) scan_move_tail(tail + (size_t)slot * (taps - 1) * C + c, xz + (size_t)first * ldx + c, ldx, C, n_tok, taps);
 }
 
@@ -407,18 +442,18 @@ Q6K_API int q6k_selective_scan_lanes(int N) {
 // Tokens per segment when a portion is walked by several blocks.
 Q6K_API int q6k_selective_scan_segment() { return 64; }
 
-// Whether a step of T_ rows whose longest portion has up to `segments` segments goes a lane per state in one pass.  More than 16 states
-// take more lanes; fewer than 9 leave half of them idle.  A chain takes about 35 clocks a token however few there are; the segments'
-// launches take their 30 instructions per token and state, spread over the chip: with 592 schedulers the lines meet where the tokens of all
-// requests bring 24,000 chains for each token of the longest (65,536 chains: 171 against 371 us).  Without segments (up to 64 tokens) a walk of eight states a lane
-// takes 0.58 us a token of the longest portion, a lane per state 6.6 us for every round of blocks (four are resident on an SM), whatever their
-// tokens (4,096 channels: 64 tokens 40 and 9 us, 64 beside 8 of one 40 and 31, 32 portions of 8 28 and 88); from 25 tokens a request on the
-// latter has the fewer instructions too.  A step of single tokens keeps the former (nothing to fetch ahead).
+// Whether a step of T_ rows whose longest portion has up to `segments` segments goes a lane per two states in one pass.  More than 16 states
+// take more lanes; fewer than 9 leave half of them idle.  A chain takes about 45 ns a token however few there are; the segments' launches take 70 us
+// and their 30 instructions per token and state, spread over the chip: for one portion of 2,048 tokens the lines meet where its tokens bring 10,000
+// chains (768 channels: 90 against 95 us; 512: 90 against 86; 4,096: 150 against 345).  Without segments (up to 64 tokens) a walk of eight states a lane
+// takes 0.58 us a token of the longest portion, a lane per two states 4.4 us for every round of blocks (three are resident on an SM), whatever their
+// tokens (4,096 channels: 64 tokens 35 and 9 us, 64 beside 8 of one 41 and 32, 32 portions of 8 28 and 86); from 25 tokens a request on the
+// latter has the fewer instructions too (8 portions of 64: 53 and 41).  A step of single tokens keeps the former (nothing to fetch ahead).
 static bool lanes_taken(int T_, int R, int C, int N, int segments, int longest) {
     const long long blocks = (C + LS_CH - 1) / LS_CH;
     if (N <= 8 || N > LS_N || T_ < 8 * R || blocks > 65535) return false;
-    if (segments > 1) return (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 24000;
-    return T_ >= 25 * R || 5.0f + 6.6f * (float)(R * blocks) / (4 * 148) < 3.0f + 0.58f * (float)longest;
+    if (segments > 1) return (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 10000;
+    return T_ >= 25 * R || 5.0f + 4.4f * (float)(R * blocks) / (3 * 148) < 3.0f + 0.58f * (float)longest;
 }
 Q6K_API int q6k_selective_scan_lanes_taken(int T_, int R, int C, int N, int segments) { return lanes_taken(T_, R, C, N, segments, R > 0 ? T_ / R : 0); }
 
@@ -441,8 +476,12 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
     dim3 grid(R, (C + per_block - 1) / per_block);
     Q6K_REQUIRE(grid.y <= 65535, "selective_scan: %d channels exceed the grid limit", C);
     if (lanes_taken(T_, R, C, N, segments, longest > 0 ? longest : T_ / R)) {
-        Q6K_DISPATCH(dtype, q6k_launch(scan_lanes_kernel<T>, dim3(R, (C + LS_CH - 1) / LS_CH), LS_THREADS, 0, st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
-                                       A, Dskip, xz, ldx, z_col, state, tail, q_start, slot_ids, (T*)out, C, N, taps););
+        Q6K_DISPATCH(dtype, {
+            if (cudaFuncSetAttribute(scan_lanes_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(LsTile)) != cudaSuccess)
+                return q6k_check_launch("selective_scan: shared memory attribute");
+            q6k_launch(scan_lanes_kernel<T>, dim3(R, (C + LS_CH - 1) / LS_CH), LS_THREADS, 2 * sizeof(LsTile), st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
+                       A, Dskip, xz, ldx, z_col, state, tail, q_start, slot_ids, (T*)out, C, N, taps);
+        });
         return q6k_check_launch("selective_scan (lanes)");
     }
     const size_t smem = (size_t)SCAN_TILE * (2 * L * MAX_PER_LANE + 4 * per_block) * sizeof(float);

@@ -1148,8 +1148,8 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
     holding the convolution's inputs (columns 0..) and z (columns z_col..), state FP32 [slots, C, N], tail FP32
     [slots, taps-1, C] (moved on to the portion's end).  Returns [T, C] in u's dtype.
     segments = (most segments of any request, seg_base int32 [R] on the device, segments in all) from
-    selective_scan_segments(q_lens): long portions are then walked by several blocks each (three launches), unless a lane per state
-    takes the step in one pass.  longest: tokens of the longest portion, if known."""
+    selective_scan_segments(q_lens): long portions are then walked by several blocks each (three launches), unless a lane per two
+    states takes the step in one pass.  longest: tokens of the longest portion, if known."""
     _need(u, "u")
     T, C = u.shape
     N = A.shape[1]

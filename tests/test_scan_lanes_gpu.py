@@ -75,3 +75,32 @@ def test_which_walk_short_portions_take():
     assert taken(64, 1, 4096, 16, 1) and taken(64, 2, 4096, 16, 1) and taken(2048, 32, 4096, 16, 1)
     assert not taken(256, 32, 4096, 16, 1) and not taken(32, 32, 4096, 16, 1) and not taken(64, 1, 1 << 20, 16, 1 << 30)
     assert not taken(1 << 12, 1, (1 << 20) + 16, 16, 1)        # more blocks of channels than a grid has rows
+
+
+@pytest.mark.parametrize("C, N, dtype, lens", [(17, 9, torch.bfloat16, [32, 31, 33, 1, 96]), (16, 15, torch.float32, [64, 95, 97]), (33, 16, torch.float32, [30, 47, 48, 49])])
+def test_lanes_of_two_states_at_extremes(C, N, dtype, lens):
+    """Tiles of 32 tokens and odd state counts, with steps so short and so long that decays lie on both sides of their series' end, and gates out to
+    where the sigmoid is 0 or 1 (infinity included): every result is that of the walk of single tokens, up to the order in which 16 products are added."""
+    from quench6k_b200 import ops
+    g = torch.Generator().manual_seed(C * N)
+    T, R, taps = sum(lens), len(lens), 4
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    starts = [sum(lens[:i]) for i in range(R + 1)]
+    u, dt_raw, dt_b, proj = rnd(T, C).to(dtype), rnd(T, C) * 8, rnd(C) * 0.5, rnd(T, 2 * N)
+    A, D, xz, state, tail = -torch.exp(rnd(C, N)), rnd(C), rnd(T, 2 * C) * 30, rnd(R, C, N), rnd(R, taps - 1, C)
+    xz[::7, C] = float("inf")
+    xz[1::7, C] = -1e30
+    assert ops.library().q6k_selective_scan_lanes_taken(T, R, C, N, 1) == 1
+    s1, t1, s2, t2, walked = state.clone(), tail.clone(), state.clone(), tail.clone(), []
+    got = ops.selective_scan(u, dt_raw, dt_b, proj, 0, N, A, D, xz, C, s1, t1, i32(starts), i32(list(range(R))), R)
+    for r, n in enumerate(lens):
+        for t in range(starts[r], starts[r] + n):
+            walked.append(ops.selective_scan(u[t:t + 1], dt_raw[t:t + 1], dt_b, proj[t:t + 1], 0, N, A, D, xz[t:t + 1], C, s2, t2, i32([0, 1]), i32([r]), 1))
+    walked = torch.cat(walked)
+    finite = torch.isfinite(walked)
+    assert torch.equal(finite, torch.isfinite(got)) and torch.equal(walked[~finite], got[~finite]) and torch.equal(t1, t2)
+    torch.testing.assert_close(s1, s2, rtol=1e-6, atol=1e-6 * float(s2.abs().max()))
+    # 16 FP32 products and a skip in another order (some 20 roundings of 6e-8 of the largest), times the gate; bfloat16: a neighbouring value
+    scale = float(walked[finite].abs().max())
+    torch.testing.assert_close(got[finite], walked[finite], rtol=2 ** -7 if dtype == torch.bfloat16 else 2e-6, atol=2e-6 * scale)
