@@ -555,14 +555,22 @@ __host__ __device__ constexpr uint32_t umma_idesc_pair(int n) {
 }
 
 // HEADS: the results leave in bfloat16, a matrix of p.head_cols columns per head (whole blocks of 16 rows).
-template <int BT2, bool HEADS>
-__global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
-                                                           const __grid_constant__ CUtensorMap tm_out, const Params p) {
+//
+// DUAL: a gated product of two weight matrices.  A CTA's 128 weight rows are 64 of the one (lanes 0-63 of its accumulator) and the same 64 of the other
+// (lanes 64-127), so that a pair's tile of 256 tokens feeds both products and the tensor memory still holds two buffers.  Per 32 tokens the two warps
+// that hold a column's two products exchange half of theirs through shared memory, and each gates and sends 16 tokens.
+// 1,522 rows, 2 x 8,192 columns, K 2,048: 73 us (1,400 TFLOP/s) where one CTA a tile of 128 tokens takes 89, its MMAs waiting for shared memory;
+// 512 rows, 2 x 4,864: 24 and 31; 8,192 rows: 359 and 438.
+constexpr int GATE_BYTES = 4 * 2 * EPI_BLOCK_BYTES;        // DUAL: each warp's 16 tokens for its partner, two buffers
+template <int BT2, bool HEADS, bool DUAL>
+__global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_w2,
+                                                           const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_out, const Params p) {
     // The tiles follow from the launch alone: the pair sets itself up and sends for the weights of its first ring of
     // k-blocks before it waits for the kernel that makes the activations (and whose reader may still use the output).
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-    const int n_x = (p.N + 2 * WM - 1) / (2 * WM), total = n_x * p.n_y;
+    constexpr int COLS = DUAL ? WM / 2 : WM;               // output columns of a CTA's tile
+    const int n_x = (p.N + 2 * COLS - 1) / (2 * COLS), total = n_x * p.n_y;
     const int kb_total = (p.K + BK - 1) / BK;
 
     extern __shared__ uint8_t smem_raw[];
@@ -588,6 +596,7 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_a) : "memory");
+        if (DUAL) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w2) : "memory");
     }
     if (warp == 1) {                                       // the same warp of both CTAs allocates for the pair
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
@@ -604,11 +613,12 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
         if (elect_one()) {
             int pre = 0;                                   // k-blocks whose weights went out before the wait
             for (int t = pair; t < total && pre < stages; t += n_pairs) {
-                const int n0 = (t % n_x) * 2 * WM + (int)rank * WM;
+                const int n0 = (t % n_x) * 2 * COLS + (int)rank * COLS;
                 for (int i = 0; i < kb_total && pre < stages; ++i, ++pre) {
                     const uint32_t st = smem_u32(smem + (size_t)pre * STAGE_BYTES), fb = full0 + 8 * pre;
                     if (rank == 0) mbar_expect_tx(fb, 2 * STAGE_BYTES);
                     tma_load_2d_pair(st, &tm_w, i * BK, n0, fb);
+                    if (DUAL) tma_load_2d_pair(st + W_BYTES / 2, &tm_w2, i * BK, n0, fb);
                 }
             }
             pdl_wait();
@@ -616,7 +626,7 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
             uint32_t st = smem_u32(smem), phase = 0;
             bool ok = true;
             for (int t = pair; t < total && ok; t += n_pairs) {
-                const int n0 = (t % n_x) * 2 * WM + (int)rank * WM, row0 = (t / n_x) * BT2 + (int)rank * (BT2 / 2);
+                const int n0 = (t % n_x) * 2 * COLS + (int)rank * COLS, row0 = (t / n_x) * BT2 + (int)rank * (BT2 / 2);
                 for (int i = 0; i < kb_total; ++i) {
                     const uint32_t fb = full0 + 8 * s;
                     if (pre > 0) {                         // the first ring's stages are fresh and their weights on the way
@@ -629,6 +639,7 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
                         }
                         if (rank == 0) mbar_expect_tx(fb, 2 * STAGE_BYTES);
                         tma_load_2d_pair(st, &tm_w, i * BK, n0, fb);
+                        if (DUAL) tma_load_2d_pair(st + W_BYTES / 2, &tm_w2, i * BK, n0, fb);
                     }
                     tma_load_2d_pair(st + W_BYTES, &tm_a, i * BK, row0, fb);
                     if (++s == stages) s = 0, st = smem_u32(smem), phase ^= 1;
@@ -671,18 +682,59 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_kernel(const __grid_constant
     } else {
         const int quarter = warp & 3;
         const uint32_t out_smem = smem_u32(smem + (size_t)stages * STAGE_BYTES) + quarter * 2 * EPI_BLOCK_BYTES;
-        int nt = 0, sent = 0;
+        int nt = 0, sent = 0, turn = 0;
         pdl_wait();                                        // the output may still be in use by the kernel before
         for (int t = pair; t < total; t += n_pairs, ++nt) {
             const int buf = nt & 1;
             if (!mbar_wait(acc_full0 + 8 * buf, (nt >> 1) & 1)) {
                 if (lane == 0) atomicExch(&g_tc_status, 13);
-                break;
+                if (!DUAL) break;                           // DUAL: on to the barriers that the partner may be waiting at
             }
             tc_fence_after();
-            const int n = (t % n_x) * 2 * WM + (int)rank * WM + quarter * 32 + lane, tok0 = (t / n_x) * BT2;
+            const int n = (t % n_x) * 2 * COLS + (int)rank * COLS + (DUAL ? quarter & 1 : quarter) * 32 + lane, tok0 = (t / n_x) * BT2;
             const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * ACC_COLS;
             const int valid = min(BT2, p.rows_total - tok0);
+            if constexpr (DUAL) {
+                const uint32_t swap = out_smem + EPI_BYTES;            // this warp's two buffers; the partner's are two warps on
+                const uint32_t theirs = smem_u32(smem + (size_t)stages * STAGE_BYTES) + EPI_BYTES + (quarter ^ 2) * 2 * EPI_BLOCK_BYTES;
+                const bool gates = quarter < 2;                        // tokens 0-15 of 32; the other products' warp finishes 16-31
+#pragma unroll 1
+                for (int c0 = 0; c0 < valid; c0 += 32, ++turn) {
+                    float v[16], u[16];
+                    tmem_ld16(lane_addr + c0 + (gates ? 16 : 0), u);   // the partner's tokens
+                    tmem_ld16(lane_addr + c0 + (gates ? 0 : 16), v);
+                    if (c0 + 32 >= valid) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
+                    }
+                    const uint32_t at = (turn & 1) * EPI_BLOCK_BYTES + lane * 4;
+#pragma unroll
+                    for (int j = 0; j < EPI_TOKENS; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(swap + at + j * 128), "f"(u[j]) : "memory");
+                    // both have written; and the buffers of the turn before have been read
+                    if (quarter & 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+                    else asm volatile("bar.sync 1, 64;" ::: "memory");
+                    __nv_bfloat16 y[16];
+#pragma unroll
+                    for (int j = 0; j < EPI_TOKENS; ++j) {
+                        float other;
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(other) : "r"(theirs + at + j * 128) : "memory");
+                        u[j] = gates ? other : v[j], v[j] = gates ? v[j] : other;
+                    }
+                    rounded_results<true>(p, v, u, y);
+                    const int c1 = c0 + (gates ? 0 : 16), row = tok0 + c1;
+                    if (c1 >= valid || n - lane >= p.N) continue;
+                    if (p.out_tma && c1 + 16 <= valid) {
+                        send_block(&tm_out, out_smem, sent++, y, n - lane, row, false);
+                    } else if (n < p.N) {
+                        __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n;
+#pragma unroll
+                        for (int j = 0; j < EPI_TOKENS; ++j)
+                            if (c1 + j < valid) o[(size_t)j * p.ldo] = y[j];
+                    }
+                }
+                continue;
+            }
 #pragma unroll 1
             for (int c0 = 0; c0 < valid; c0 += 16) {
                 float v[16];
@@ -731,17 +783,17 @@ int make_map(CUtensorMap* map, const void* base, long long rows, int K, long lon
     return make_bf16_map(map, base, rows, K, pitch, box_rows, weights, "gemm_tc");
 }
 
-// Weight maps do not change between calls: keep them by (address, rows, K).
+// Weight maps do not change between calls: keep them by (address, rows, K, rows of a box).
 std::mutex g_map_mutex;
-std::map<std::tuple<const void*, long long, int>, CUtensorMap> g_weight_maps;
+std::map<std::tuple<const void*, long long, int, int>, CUtensorMap> g_weight_maps;
 
-int weight_map(CUtensorMap* out, const void* base, long long rows, int K) {
+int weight_map(CUtensorMap* out, const void* base, long long rows, int K, int box_rows = WM) {
     std::lock_guard<std::mutex> lock(g_map_mutex);
-    auto key = std::make_tuple(base, rows, K);
+    auto key = std::make_tuple(base, rows, K, box_rows);
     auto it = g_weight_maps.find(key);
     if (it == g_weight_maps.end()) {
         CUtensorMap m;
-        if (int rc = make_map(&m, base, rows, K, K, WM, true)) return rc;
+        if (int rc = make_map(&m, base, rows, K, K, box_rows, true)) return rc;
         it = g_weight_maps.emplace(key, m).first;
     }
     *out = it->second;
@@ -810,24 +862,25 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta,
 }
 
 // The CTA-pair kernel: tiles of [256 weights x BT2 tokens], one cluster of two CTAs per SM pair.
-template <int BT2, bool HEADS>
-int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const CUtensorMap* heads, Params p, cudaStream_t st) {
+template <int BT2, bool HEADS, bool DUAL>
+int launch_pair(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& ta, const CUtensorMap* heads, Params p, cudaStream_t st) {
+    constexpr int cols = DUAL ? WM : 2 * WM, out_bytes = EPI_BYTES + (DUAL ? GATE_BYTES : 0);
     constexpr int stage = WM * BK * 2 + (BT2 / 2) * BK * 2;
     CUtensorMap tout = tw;
     if (HEADS) tout = *heads;
-    else if (int rc = out_map(&tout, &p.out_tma, p.out, p.rows_total, p.N, p.ldo, false)) return rc;
-    int stages = (225 * 1024 - EPI_BYTES) / stage;
+    else if (int rc = out_map(&tout, &p.out_tma, p.out, p.rows_total, p.N, p.ldo, DUAL)) return rc;
+    int stages = (225 * 1024 - out_bytes) / stage;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     p.stages = stages;
     p.n_y = (p.rows_total + BT2 - 1) / BT2;
-    const size_t smem = (size_t)stages * stage + EPI_BYTES + 1024;
+    const size_t smem = (size_t)stages * stage + out_bytes + 1024;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BT2, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BT2, HEADS, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
             return q6k_check_launch("gemm_tc pair: shared memory attribute");
         configured = true;
     }
-    const long long total = (long long)((p.N + 2 * WM - 1) / (2 * WM)) * p.n_y;
+    const long long total = (long long)((p.N + cols - 1) / cols) * p.n_y;
     const int pairs = sm_count() / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (unsigned)(total < pairs ? total : pairs)), cfg.blockDim = dim3(192), cfg.dynamicSmemBytes = smem, cfg.stream = st;
@@ -837,26 +890,27 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const CUtensorMap*
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // the weights of the first ring are fetched under the kernel before
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = q6k_pdl_mode() != 0 ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2, HEADS>, tw, ta, tout, p);
+    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BT2, HEADS, DUAL>, tw, tw2, ta, tout, p);
     return q6k_check_launch("gemm_tc pair");
 }
 
 // Token tile of the pair kernel for (rows, N), or 0 when the one-CTA kernel serves the product:
 // plain dense products with at least 512 rows and 256 weight rows.  Q6K_TC_PAIR=0 switches it off.
-static int pair_tile(int rows, int N) {                    // the tile that ends the last round earlier
-    const long long n_x = (N + 2 * WM - 1) / (2 * WM), pairs = sm_count() / 2;
+static int pair_tile(int rows, int N, int cols = 2 * WM) {  // the tile that ends the last round earlier
+    const long long n_x = (N + cols - 1) / cols, pairs = sm_count() / 2;
     const long long r256 = (n_x * ((rows + 255) / 256) + pairs - 1) / pairs, r192 = (n_x * ((rows + 191) / 192) + pairs - 1) / pairs;
     return r192 * 192 < r256 * 256 ? 192 : 256;
 }
-static int pair_plan(int rows, int N, int K) {
+static int pair_plan(int rows, int N, int K, bool dual) {
+    const int cols = dual ? WM : 2 * WM;
     static const bool off = [] {
         const char* v = getenv("Q6K_TC_PAIR");
         return v && v[0] == '0';
     }();
-    if (off || rows < 512 || N < 2 * WM || K % 8 != 0) return 0;
-    const long long n_x = (N + 2 * WM - 1) / (2 * WM), pairs = sm_count() / 2;
+    if (off || rows < 512 || N < cols || K % 8 != 0) return 0;
+    const long long n_x = (N + cols - 1) / cols, pairs = sm_count() / 2;
     if (n_x * ((rows + 255) / 256) * 2 < pairs) return 0;   // too few tiles for the pairs: the one-CTA kernel narrows its tile
-    return pair_tile(rows, N);
+    return pair_tile(rows, N, cols);
 }
 
 }  // namespace
@@ -960,12 +1014,18 @@ Q6K_API int q6k_gemm_tc(const void* A, long long lda, int rows_total, const void
     tw2 = tw;
     if (dual)
         if (int rc = weight_map(&tw2, W2, (long long)groups * N, K)) return rc;
-    if (!grouped && !dual && planned_splits == 1) {
-        if (const int bt2 = pair_plan(rows_total, N, K)) {
+    if (!grouped && planned_splits == 1) {
+        if (const int bt2 = pair_plan(rows_total, N, K, dual)) {
             if (int rc = make_map(&ta, A, rows_total, K, lda, bt2 / 2, false)) return rc;
             Params pp{};
             pp.out = out, pp.rows_total = rows_total, pp.N = N, pp.K = K, pp.ldo = ldo, pp.epilogue = epilogue;
-            return bt2 == 192 ? launch_pair<192, false>(tw, ta, nullptr, pp, st) : launch_pair<256, false>(tw, ta, nullptr, pp, st);
+            if (dual) {
+                if (int rc = weight_map(&tw, W, N, K, WM / 2)) return rc;
+                if (int rc = weight_map(&tw2, W2, N, K, WM / 2)) return rc;
+                pp.act = act, pp.act_limit = act_param;
+                return bt2 == 192 ? launch_pair<192, false, true>(tw, tw2, ta, nullptr, pp, st) : launch_pair<256, false, true>(tw, tw2, ta, nullptr, pp, st);
+            }
+            return bt2 == 192 ? launch_pair<192, false, false>(tw, tw, ta, nullptr, pp, st) : launch_pair<256, false, false>(tw, tw, ta, nullptr, pp, st);
         }
     }
     if (int rc = make_map(&ta, A, rows_total, K, lda, bt, false)) return rc;
@@ -1033,7 +1093,7 @@ Q6K_API int q6k_gemm_tc_heads(const void* A, long long lda, int rows, const void
     if (int rc = make_map(&ta, A, rows, K, lda, bt2 / 2, false)) return rc;
     Params p{};
     p.out = out, p.rows_total = rows, p.N = N, p.K = K, p.epilogue = EPI_BF16, p.head_cols = head_cols, p.head_split = split, p.head_gap = gap;
-    return bt2 == 192 ? launch_pair<192, true>(tw, ta, &tout, p, st) : launch_pair<256, true>(tw, ta, &tout, p, st);
+    return bt2 == 192 ? launch_pair<192, true, false>(tw, tw, ta, &tout, p, st) : launch_pair<256, true, false>(tw, tw, ta, &tout, p, st);
 }
 
 // Few tokens (decode): one tile per (token, slot) pair instead of a permutation.  pair_expert:
