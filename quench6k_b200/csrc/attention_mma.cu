@@ -48,7 +48,7 @@ struct AttnParams {
     int n_work;
     int max_blocks, page_size, window, chunk, Hq, Hkv, G;
     float scale_log2;
-    int early;                               // the plan, the block tables and every key before a tile's first position are older than the
+    int early;                               // 2: see the kernel.  1: the plan, the block tables and every key before a tile's first position are older than the
                                              // kernel launched before this one: key tiles may be fetched before the wait for it
     int pool_rows;                           // rows of the [Hkv * pages * page_size, HD] view of a pool (TMA path)
     int num_pages;                           // pages of a pool (per KV head)
@@ -216,7 +216,10 @@ __global__ void __launch_bounds__((WIDE ? 8 : 4) * 32 + 32, WIDE ? 1 : 2) attent
     // written by an earlier step: the producer fetches those key tiles while the kernel launched before this one (the
     // one that writes this step's keys and q) still runs, and only then waits for it (programmatic dependent launch;
     // the plan and the block tables are older than that kernel too).  Wide tiles wait first, like any other kernel.
-    const bool EARLY = !WIDE && p.early != 0;
+    // Beside the tcgen05 attention of a step's prompt portions (early == 2) nothing here is the work of the kernel before: that one has signalled after
+    // its own wait, so all that is older is complete; this one works in the SMs that it leaves idle and waits for it only at the end, for the
+    // sake of what comes next.  1,501 prompt tokens (96 CTAs, 106 us) beside 21 decoding requests: 17 us behind it in turn, 5 left side by side.
+    const bool EARLY = !WIDE && p.early != 0, BESIDE = !WIDE && p.early == 2;
     if (EARLY) pdl_launch();
     else pdl_enter();
     constexpr int CW = WIDE ? 8 : 4;         // consumer warps
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__((WIDE ? 8 : 4) * 32 + 32, WIDE ? 1 : 2) attent
     if (warp == CW) {
         const int ps = p.page_size;
         if (TMA && !elect_one()) return;      // one elected lane issues the TMA loads; the copies of the other path take all 32
-        bool waited = !EARLY;
+        bool waited = !EARLY || BESIDE;
         // a launch that makes the new keys itself finds only keys of earlier steps in the pages: nothing there is the
         // work of the kernel before this one (the rows of this step's positions are replaced in shared memory)
         const bool makes_kv = !WIDE && p.qkv != nullptr && p.write_kv;
@@ -331,6 +334,7 @@ __global__ void __launch_bounds__((WIDE ? 8 : 4) * 32 + 32, WIDE ? 1 : 2) attent
             }
         }
         if (!TMA) cp_async_wait_all();        // nothing of this warp's is in flight when it leaves
+        if (BESIDE) pdl_wait();
         return;
     }
 
@@ -353,7 +357,7 @@ __global__ void __launch_bounds__((WIDE ? 8 : 4) * 32 + 32, WIDE ? 1 : 2) attent
         }
         asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory");
     }
-    if (EARLY) pdl_wait();                    // q (or the q/k/v product) is the work of the kernel before this one
+    if (EARLY && !BESIDE) pdl_wait();         // q (or the q/k/v product) is the work of the kernel before this one
     // the rows this thread holds in the accumulator fragments: block nb, rows nb*8 + 2*pair + {0, 1}
     int see_to[NB][2], see_from[NB][2];
 #pragma unroll
@@ -963,7 +967,8 @@ Q6K_API int q6k_attention_plan(const int* positions, const int* req_of_token, co
 // part_ml: FP32 [n_work * Hkv * rows * 2] (unused when n_work == n_tiles).
 // early != 0 (tiles of 8 or 16 rows only): the caller's word that the plan and the block table were made before the kernel
 // launched before this one started, and that this kernel writes this step's keys; key tiles older than a tile's first
-// position are then fetched while it still runs.
+// position are then fetched while it still runs.  early == 2 (q given): the kernel launched before this one reads other rows of q and the same pages and
+// writes other rows of out, was itself launched without overlap and signals only after its own wait: the two then run side by side.
 // qkv != null (tiles of 8 or 16 rows only; q is then unused): FP32 [qkv_splits, T, qkv_ld] rows of q heads | k heads | v heads
 // (slices qkv_split_stride floats apart, summed in order: split-K partial products), which the
 // kernel itself normalises per head (q_norm, k_norm: FP32 [hd] or null; eps), rotates (inv_freq: FP32 [rotary_dim / 2] or
@@ -987,6 +992,7 @@ Q6K_API int q6k_attention_mma(const void* q, const void* k_pages, const void* v_
     Q6K_REQUIRE(q6k_attention_mma_supported(hd, G, rows == 128) && G <= rows, "attention_mma: head_dim %d / group size %d is not covered by tiles of %d rows", hd, G, rows);
     Q6K_REQUIRE(page_size > 0 && max_blocks > 0 && window >= 0 && chunk >= 0 && n_work >= n_tiles && work && tile_plan,
                 "attention_mma: bad page_size %d / max_blocks %d / window %d / %d work items for %d tiles", page_size, max_blocks, window, n_work, n_tiles);
+    Q6K_REQUIRE(early != 2 || !qkv, "attention_mma: beside another kernel q is given%s", "");
     Q6K_REQUIRE(n_work == n_tiles || (part_o && part_ml), "attention_mma: splitting the keys needs the partial buffers");
     Q6K_REQUIRE(Hkv <= 65535 && n_tiles <= 65535, "attention_mma: grid limit exceeded (Hkv=%d, tiles=%d)", Hkv, n_tiles);
     AttnParams p{};

@@ -767,7 +767,7 @@ def attention_mma(q: Optional[torch.Tensor], k_pages: torch.Tensor, v_pages: tor
                   req_of_token: torch.Tensor, positions: torch.Tensor, tile_tok0: torch.Tensor, tile_ntok: torch.Tensor,
                   rows: int, window: Optional[int], sinks: Optional[torch.Tensor], max_splits: int = 1, min_tiles: int = 2,
                   scale: Optional[float] = None, out: Optional[torch.Tensor] = None, plan=None, plan_is_old: bool = False,
-                  prepare=None, chunk: Optional[int] = None) -> torch.Tensor:
+                  prepare=None, chunk: Optional[int] = None, beside_tc: bool = False) -> torch.Tensor:
     """bfloat16 tensor-core attention over the pages.  Tiles: tile_tok0[i] is the first row and
     tile_ntok[i] the number of tokens (consecutive positions of one request, at most rows // G;
     rows: 8, 16 or 128, see attention_mma_tile_rows) of tile i.  plan: attention_plan(...) of these tiles, this
@@ -782,7 +782,10 @@ def attention_mma(q: Optional[torch.Tensor], k_pages: torch.Tensor, v_pages: tor
     write (bool); qkv may be [slices, T, width] split-K partial products.  The kernel then normalises, rotates and rounds q itself, and with write=True
     makes the tiles' keys and values and puts them into the pages (every token of the step must
     then lie in a tile).  With plan_is_old the plan must be older than the kernel that made qkv
-    AND the one before it."""
+    AND the one before it.
+
+    beside_tc (with plan_is_old, without prepare): the launch just before this call was attention_tc over other rows of
+    the same q, pages and out; narrow tiles then run side by side with it."""
     _need(k_pages, "k_pages", torch.bfloat16)
     _need(v_pages, "v_pages", torch.bfloat16, k_pages.shape)
     Hkv, num_pages, page_size, hd = k_pages.shape
@@ -837,7 +840,7 @@ def attention_mma(q: Optional[torch.Tensor], k_pages: torch.Tensor, v_pages: tor
     _call("q6k_attention_mma", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ll(num_pages), _ptr(block_table),
           _i(block_table.shape[1]), _i(page_size), _ptr(work), _ptr(tile_plan), _i(n_work), _i(n_tiles), _i(rows),
           _i(window or 0), _i(chunk or 0), _ptr(sinks), _f(scale if scale is not None else 1.0 / math.sqrt(hd)), _ptr(out), _ptr(part_o), _ptr(part_ml),
-          _i(Hq), _i(Hkv), _i(hd), _i(1 if plan_is_old else 0), _ptr(qkv), _i(ld), _i(splits), _ll(split_stride), _ptr(q_norm), _ptr(k_norm), _f(eps),
+          _i(Hq), _i(Hkv), _i(hd), _i((2 if beside_tc and prepare is None else 1) if plan_is_old else 0), _ptr(qkv), _i(ld), _i(splits), _ll(split_stride), _ptr(q_norm), _ptr(k_norm), _f(eps),
           _ptr(inv_freq), _i(rotary_dim), _i(1 if write else 0), _stream())
     return out
 

@@ -338,10 +338,10 @@ class Attention(Mixer):
             (tok0, ntok), short = how[1], how[2]
             out = ops.attention_tc(q, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, tok0, ntok, self.window,
                                    self.sinks, scale=self.scale, chunk=self.chunk)
-            return out if short is None else self._split_keys(q, cache, table, ctx, short, out)
+            return out if short is None else self._split_keys(q, cache, table, ctx, short, out, beside_tc=True)
         return self._split_keys(q, cache, table, ctx, how[1])
 
-    def _split_keys(self, q, cache, table, ctx, planned, out=None, prepare=None):
+    def _split_keys(self, q, cache, table, ctx, planned, out=None, prepare=None, beside_tc=False):
         rows, tok0, ntok, plan, fresh = planned
         # The plan was made before this layer's first launch.  With q from qk_prep, the kernel before this one is that
         # one (or, beside prompt portions, the tcgen05 attention), which itself waited for everything before it: the plan
@@ -350,7 +350,7 @@ class Attention(Mixer):
         # is surely complete.
         return ops.attention_mma(q, cache.k, cache.v, table, ctx.req_of_token, ctx.positions, tok0, ntok, rows, self.window,
                                  self.sinks, scale=self.scale, out=out, plan=plan, plan_is_old=prepare is None or not fresh,
-                                 prepare=prepare, chunk=self.chunk)
+                                 prepare=prepare, chunk=self.chunk, beside_tc=beside_tc)
 
     def _sm_count(self) -> int:
         if "_sms" not in self.__dict__:
