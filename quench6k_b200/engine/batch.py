@@ -44,8 +44,8 @@ class StepContext:
     made: set = field(default_factory=set)        # keys of plans whose device-side part has been launched in this pass over the
                                                   # layers: the runner empties it before it records the step, so that a kernel
                                                   # that fills a plan from the step's positions is part of the recording
-    replayed: bool = False                        # the pass is, or will be, a recording that later steps replay at other positions: what a part
-                                                  # launches must not depend on the host's positions
+    replayed: bool = False                        # steps of this shape are recorded and replayed at other positions, this pass or a later one: the form
+                                                  # a part takes must not depend on the host's positions, in this pass as in the replays
     fed: Optional[torch.Tensor] = None            # int32 ids the step before sampled: a token id -(i + 1) stands for fed[i]
     hold_results: bool = False                    # a block that keeps a sublayer's result while other kernels run sets it: results
                                                   # must then be tensors of their own, not views of the products' scratch buffer

@@ -228,7 +228,9 @@ class ModelRunner:
             if not decode and seen < 2:
                 if len(self._shapes_seen) > 4096:
                     self._shapes_seen.clear()
-                return self.model.forward(self._context(entries), self.caches, self.states)
+                ctx = self._context(entries)
+                ctx.replayed = True                     # the same forms now as in the recording that the shape's next step makes
+                return self.model.forward(ctx, self.caches, self.states)
             # run the step eagerly from a static block, then record the same launches into a graph
             # (recording executes nothing)
             R, T = len(entries) + pad, sum(len(e.tokens) for e in entries) + pad

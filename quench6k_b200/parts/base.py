@@ -85,6 +85,8 @@ class Part:
     # and their slots are not: a part whose launches depend on them must leave this False (the
     # attention part plans its key splits on the device for that reason; the order of its
     # prompt tiles, which only balances the load, is the one thing it takes from pos_starts).
+    # A part may choose between forms by pos_starts only where ctx.replayed is False: the runner
+    # sets it on every pass of a shape that it records, the eager one before the recording included.
     graph_safe = False
 
     def tensors(self) -> List[TensorSpec]:
