@@ -108,8 +108,9 @@ class LatentAttention(Mixer):
         a row's two products, and a further 15 go to the products around the attention.  Expanded they take 2.5, in tiles of 128 tokens; the rows to
         expand take their product at 1.1 PFLOP/s and 1 a thousand for the copies.  Absorbed and expanded, both measured: 16 heads, 2,048 tokens 310 and 145; 130 tokens
         at 4,096 111 and 105, at 16,000 217 and 246; 8 heads, 300 tokens at 4,096 85 and 74, at 16,000 137 and 163.  Steps of a shape that is recorded
-        are absorbed in every pass: where their replays will stand is not known, and the same step must give the same bits each time it comes."""
-        if self.w_ukv is None or ctx.replayed or ctx.max_q_len < 64:         # a portion fills half a tile of its heads
+        are absorbed in every pass: where their replays will stand is not known, and the same step must give the same bits each time it comes; so are
+        steps whose positions the host does not know."""
+        if self.w_ukv is None or ctx.replayed or ctx.max_q_len < 64 or len(ctx.pos_starts) != len(ctx.q_lens):        # 64: half a tile of a head
             return False
         key = ("latent.expands", self.H, self.dim, self.rd, self.vd, self.rank)
         if key not in ctx.plans:
