@@ -553,16 +553,36 @@ __global__ void __launch_bounds__(256) latent_rows_kernel(const float* x, int ld
     for (int d = threadIdx.x; d < rd; d += 256) dst[rank + d] = from_f32<T>(turned(xs, d));
 }
 
-// The latents that prompt portions see, for the product that expands them: row i of `places` (request, position, or a negative position for a row that
-// nobody sees) from its page into lat [rows, rank] (zeros where nobody sees it), its rotated part behind each of the H heads' expanded keys, whose rows
-// of dim entries lie `pitch` apart, [H, rows, pitch].  16 bytes at a time: everything a multiple of 8 entries.  grid (rows), 128 threads.
-__global__ void __launch_bounds__(128) latent_context_kernel(const uint4* pages, const int2* places, const int* block_table, int max_blocks, int page_size, uint4* lat, uint4* keys,
-                                                             int rank8, int rd8, int dim8, int pitch8, int H) {
+// The latents that prompt portions see, for the product that expands them: every position of every request, a request after the other, each from a
+// multiple of 64 rows on, from its page into lat [rows, rank] (zeros in the rows between), its rotated part behind each of the H heads' expanded keys,
+// whose rows of dim entries lie `pitch` apart, [H, rows, pitch].  16 bytes at a time: everything a multiple of 8 entries.  Which request and position a
+// row is follows from q_start and pos_start (32 requests a look: a warp sums their blocks of 64 rows); blocks [R, wide] receives every request's blocks,
+// the last one in the places beyond.  (As lists made on the host this took two uploads of a step, which waited for the GPU.)  grid (rows), 128 threads.
+__global__ void __launch_bounds__(128) latent_context_kernel(const uint4* pages, const int* q_start, const int* pos_start, int R, const int* block_table, int max_blocks, int page_size,
+                                                             uint4* lat, uint4* keys, int* blocks, int wide, int rank8, int rd8, int dim8, int pitch8, int H) {
     pdl_enter();
-    const int row = blockIdx.x;
-    const int2 at = places[row];
-    const int page = at.y >= 0 ? block_table[(size_t)at.x * max_blocks + at.y / page_size] : -1;
-    const uint4* src = pages + ((size_t)max(page, 0) * page_size + max(at.y, 0) % page_size) * (rank8 + rd8);
+    const int row = blockIdx.x, block = row >> 6, lane = threadIdx.x & 31;
+    int r = -1, first = 0, count = 0, reach = 0;                                  // of this row's request: its first block, its blocks, its positions
+    for (int r0 = 0, before = 0; r0 < R && r < 0; r0 += 32) {
+        const int q = r0 + lane, sees = q < R ? pos_start[q] + q_start[q + 1] - q_start[q] : 0, n = (sees + 63) >> 6;
+        int sum = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        const unsigned beyond = __ballot_sync(0xffffffffu, before + sum > block);
+        if (beyond) {
+            const int l = __ffs(beyond) - 1;
+            r = r0 + l, count = __shfl_sync(0xffffffffu, n, l), reach = __shfl_sync(0xffffffffu, sees, l);
+            first = before + __shfl_sync(0xffffffffu, sum, l) - count;
+        }
+        before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    const int pos = row - first * 64, page = r >= 0 && pos < reach ? block_table[(size_t)r * max_blocks + pos / page_size] : -1;
+    if (r >= 0 && (row & 63) == 0)
+        for (int i = block - first + threadIdx.x; i < (block - first + 1 < count ? min(block - first + 1, wide) : wide); i += 128) blocks[(size_t)r * wide + i] = block;
+    const uint4* src = pages + ((size_t)max(page, 0) * page_size + pos % page_size) * (rank8 + rd8);
     const uint4 zero = make_uint4(0, 0, 0, 0);
     for (int i = threadIdx.x; i < rank8; i += 128) lat[(size_t)row * rank8 + i] = page >= 0 ? src[i] : zero;
     for (int i = threadIdx.x; i < H * rd8; i += 128) {
@@ -847,16 +867,16 @@ Q6K_API int q6k_latent_prep(const float* x, int ld, const float* xc, int ldc, in
     return q6k_check_launch("latent_prep");
 }
 
-// pages: bfloat16 [pages, page_size, rank + rd]; places: int32 [rows, 2]; lat: bfloat16 [rows, rank]; keys: bfloat16 [H, rows, pitch] (columns dim .. dim + rd
-// are written).
-Q6K_API int q6k_latent_context(const void* pages, const int* places, int rows, const int* block_table, int max_blocks, int page_size, void* lat, void* keys, int rank, int rd, int dim,
-                               int pitch, int H, cudaStream_t st) {
+// pages: bfloat16 [pages, page_size, rank + rd]; rows: 64 for every 64 positions (or part of them) that one of the R requests sees; lat: bfloat16 [rows, rank];
+// keys: bfloat16 [H, rows, pitch] (columns dim .. dim + rd are written); blocks: int32 [R, wide], wide the most blocks of a request.
+Q6K_API int q6k_latent_context(const void* pages, const int* q_start, const int* pos_start, int R, int rows, const int* block_table, int max_blocks, int page_size, void* lat,
+                               void* keys, int* blocks, int wide, int rank, int rd, int dim, int pitch, int H, cudaStream_t st) {
     if (rows == 0) return 0;
-    Q6K_REQUIRE(rows > 0 && rank > 0 && rank % 8 == 0 && rd >= 0 && rd % 8 == 0 && dim % 8 == 0 && pitch % 8 == 0 && pitch >= dim + rd && H > 0 && page_size > 0 &&
-                    (((uintptr_t)pages | (uintptr_t)lat | (uintptr_t)keys) & 15) == 0 && ((uintptr_t)places & 7) == 0,
+    Q6K_REQUIRE(rows > 0 && R > 0 && wide > 0 && rank > 0 && rank % 8 == 0 && rd >= 0 && rd % 8 == 0 && dim % 8 == 0 && pitch % 8 == 0 && pitch >= dim + rd && H > 0 &&
+                    page_size > 0 && (((uintptr_t)pages | (uintptr_t)lat | (uintptr_t)keys) & 15) == 0,
                 "latent_context: bad sizes rows=%d rank=%d rd=%d dim=%d", rows, rank, rd, dim);
-    q6k_launch(latent_context_kernel, dim3(rows), 128, 0, st, (const uint4*)pages, (const int2*)places, block_table, max_blocks, page_size, (uint4*)lat, (uint4*)keys, rank / 8, rd / 8,
-               dim / 8, pitch / 8, H);
+    q6k_launch(latent_context_kernel, dim3(rows), 128, 0, st, (const uint4*)pages, q_start, pos_start, R, block_table, max_blocks, page_size, (uint4*)lat, (uint4*)keys, blocks, wide,
+               rank / 8, rd / 8, dim / 8, pitch / 8, H);
     return q6k_check_launch("latent_context");
 }
 

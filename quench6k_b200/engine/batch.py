@@ -86,24 +86,6 @@ class StepContext:
             self.plans[key] = (both[0], both[1], len(first))
         return self.plans[key]
 
-    def context_rows(self):
-        """Every position that the step's requests see, a request after the other, each beginning at a multiple of 64: as device arrays
-        (request and position of every row, a negative position for the rows between; [R, blocks] the blocks of 64 rows of each request) and the
-        number of rows."""
-        key = "context_rows"
-        if key not in self.plans:
-            reach = [s + n for s, n in zip(self.pos_starts, self.q_lens)]
-            blocks = [-(-c // 64) for c in reach]
-            first = [sum(blocks[:r]) for r in range(len(blocks))]
-            req = torch.repeat_interleave(torch.arange(len(reach), dtype=torch.int32), torch.tensor(blocks) * 64)
-            pos = torch.cat([torch.arange(b * 64, dtype=torch.int32) for b in blocks])
-            pos = torch.where(pos < torch.tensor(reach, dtype=torch.int32)[req.long()], pos, -1)
-            wide = max(blocks)
-            table = torch.tensor([[f + min(i, b - 1) for i in range(wide)] for f, b in zip(first, blocks)], dtype=torch.int32)
-            device = self.token_ids.device
-            self.plans[key] = (torch.stack([req, pos], 1).contiguous().to(device, non_blocking=True), table.to(device, non_blocking=True), 64 * sum(blocks))
-        return self.plans[key]
-
     def short_requests(self, at_most: int):
         """The requests that bring at most `at_most` tokens to the step: (how many, first row,
         end row, most tokens of one, largest position + 1); rows of other requests may lie between."""

@@ -1261,22 +1261,26 @@ def latent_prep(x: torch.Tensor, H: int, dim: int, rd: int, rank: int, c_weight:
     return qn, qr
 
 
-def latent_expanded(pages: torch.Tensor, places: torch.Tensor, block_table: torch.Tensor, w: torch.Tensor, H: int, dim: int, rd: int):
-    """Keys and values of every head for the cached latents at `places` (int32 [rows, 2]: request and position, rows a multiple of 64; a negative position:
-    a row of zeros), as pages of 64 rows that attention_flex reads: views [H, rows / 64, 64, dim + rd] and [H, rows / 64, 64, vd] of one bfloat16 tensor.
+def latent_expanded(pages: torch.Tensor, reach: list, q_start: torch.Tensor, pos_start: torch.Tensor, block_table: torch.Tensor, w: torch.Tensor, H: int, dim: int, rd: int):
+    """Keys and values of every head for the cached latents that the step's requests see (reach: how many positions each; on the device they follow from
+    q_start and pos_start), as pages of 64 rows that attention_flex reads: views [H, rows / 64, 64, dim + rd] and [H, rows / 64, 64, vd] of one bfloat16
+    tensor, a request after the other, and the requests' block table over them [R, most blocks of one].
     pages: bfloat16 [1, pages, page, rank + rd]; w: [H (dim + vd), rank], a head's rows of the keys' up-projection before those of the values'."""
     _need(pages, "pages", torch.bfloat16)
-    _need(places, "places", torch.int32)
-    rows, rank, cols = places.shape[0], w.shape[1], w.shape[0] // H
+    counts = [-(-c // 64) for c in reach]
+    R, rows, wide, rank, cols = len(reach), 64 * sum(counts), max(counts), w.shape[1], w.shape[0] // H
     _need(w, "w", torch.bfloat16, (H * cols, rank))
-    if rows % 64 or pages.shape[-1] != rank + rd or cols <= dim:
-        raise KernelError(f"latent_expanded: {rows} rows, pages of {pages.shape[-1]} for a latent of {rank} + {rd}")
+    _need(q_start, "q_start", torch.int32, (R + 1,))
+    _need(pos_start, "pos_start", torch.int32, (R,))
+    if pages.shape[-1] != rank + rd or cols <= dim:
+        raise KernelError(f"latent_expanded: pages of {pages.shape[-1]} for a latent of {rank} + {rd}")
     lat = torch.empty((rows, rank), dtype=torch.bfloat16, device=pages.device)
     kv = torch.empty((H, rows // 64, 64, cols + rd), dtype=torch.bfloat16, device=pages.device)
-    _call("q6k_latent_context", _ptr(pages), _ptr(places), _i(rows), _ptr(block_table), _i(block_table.shape[1]), _i(pages.shape[2]), _ptr(lat), _ptr(kv), _i(rank), _i(rd), _i(dim),
-          _i(cols + rd), _i(H), _stream())
+    blocks = torch.empty((R, wide), dtype=torch.int32, device=pages.device)
+    _call("q6k_latent_context", _ptr(pages), _ptr(q_start), _ptr(pos_start), _i(R), _i(rows), _ptr(block_table), _i(block_table.shape[1]), _i(pages.shape[2]), _ptr(lat), _ptr(kv),
+          _ptr(blocks), _i(wide), _i(rank), _i(rd), _i(dim), _i(cols + rd), _i(H), _stream())
     _call("q6k_gemm_tc_heads", _ptr(lat), _ll(rank), _i(rows), _ptr(w), _i(H * cols), _i(rank), _ptr(kv), _i(cols), _i(dim), _i(rd), _i(cols + rd), _ll(rows * (cols + rd)), _stream())
-    return kv[..., :dim + rd], kv[..., dim + rd:]
+    return kv[..., :dim + rd], kv[..., dim + rd:], blocks
 
 
 def heads_to_rows(src: torch.Tensor, H: int, out_dtype: torch.dtype) -> torch.Tensor:

@@ -149,8 +149,8 @@ class LatentAttention(Mixer):
                                  ctx.req_of_token, table, cache.page_size, cache.k, neighbours=neighbours, write=not self.borrows, latent=latent)
         if self.expands(ctx):
             ops.current_tag = "latent.expand"
-            places, blocks, _ = ctx.context_rows()
-            k, v = ops.latent_expanded(cache.k, places, table, self.w_ukv, H, self.dim, self.rd)
+            reach = [s + n for s, n in zip(ctx.pos_starts, ctx.q_lens)]
+            k, v, blocks = ops.latent_expanded(cache.k, reach, ctx.q_start, ctx.pos_start, table, self.w_ukv, H, self.dim, self.rd)
             ops.current_tag = "latent.keys"
             wide = ctx.query_tiles(ops.attention_flex_tc_tile_tokens(H, H), most_keys_first=(None, None))
             a = ops.attention_flex(qn.view(H * T, self.dim), qr.view(H * T, self.rd) if self.rd else None, True, k, v, blocks, ctx.req_of_token, ctx.positions, H, self.scale,

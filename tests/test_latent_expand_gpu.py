@@ -88,3 +88,84 @@ def test_the_rule_leaves_recorded_steps_and_decoded_tokens_alone():
     assert not takes([2048], [0], True) and not takes([1] * 8, [40] * 8) and not takes([63], [0]) and not takes([130], [16000])
     rows = EXPAND_BYTES // (2 * (512 + 16 * 320))
     assert takes([2048], [rows - 2048 - 64]) and not takes([2048], [rows - 2048 + 64])
+
+
+def _layer_and_context(lens, starts, page=16, H=4, rank=256):
+    from quench6k_b200.parts.base import MIXERS, LayerCache, Runtime, make_part
+    from quench6k_b200.spec import PartSpec
+    D, dim, rd, vd = 192, 128, 64, 128
+    g = torch.Generator().manual_seed(sum(lens))
+    rnd = lambda *s, std=0.05: (torch.randn(s, generator=g) * std).to(torch.bfloat16).to(DEV)
+    weights = {"q_proj.weight": rnd(H * (dim + rd), D, std=0.1), "kv_down_proj.weight": rnd(rank + rd, D), "kv_norm.weight": torch.ones(rank), "k_up_proj.weight": rnd(H * dim, rank),
+               "v_up_proj.weight": rnd(H * vd, rank), "o_proj.weight": rnd(D, H * vd)}
+    mixer = make_part(MIXERS, "mixer", PartSpec("latent_attention", dict(num_heads=H, head_dim=dim, rot_dim=rd, v_dim=vd, kv_rank=rank, scale=192 ** -0.5, eps=1e-6,
+                                                                         pos=PartSpec("rope", {"head_dim": rd, "theta": 10000.0, "rotary_dim": rd}))), hidden_size=D)
+    mixer.bind(lambda name: weights[name], Runtime(torch.device(DEV), torch.bfloat16))
+    blocks = [-(-(s + n) // page) for s, n in zip(starts, lens)]
+    table = torch.zeros((len(lens), max(blocks)), dtype=torch.int32)
+    for r in range(len(lens)):
+        table[r, :blocks[r]] = torch.arange(sum(blocks[:r]), sum(blocks[:r + 1]))
+    k = rnd(1, sum(blocks), page, rank + rd, std=1.0)
+    x, out = rnd(sum(lens), D, std=1.0), torch.empty((sum(lens), D), device=DEV)
+    ctx = _context(lens, starts, table.to(DEV))
+    run = lambda ctx: mixer.forward(x, ctx, LayerCache(0, k, k[..., :rank], page), None, out)
+    return mixer, ctx, run
+
+
+def test_a_new_context_uploads_nothing_for_the_rows_it_expands():
+    """What an expanding step needs of its requests is on the device already: the tiles of its queries are all that goes up."""
+    import copy
+
+    from torch.utils._python_dispatch import TorchDispatchMode
+    mixer, ctx, run = _layer_and_context([300, 1, 130], [1000, 64, 0])
+
+    class Uploads(TorchDispatchMode):
+        count = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            if func in (torch.ops.aten._to_copy.default, torch.ops.aten.copy_.default):
+                src = args[1] if func is torch.ops.aten.copy_.default else args[0]
+                Uploads.count += out.is_cuda and not src.is_cuda
+            return out
+
+    assert mixer.expands(ctx)
+    run(ctx)                                                            # tensors that the process keeps are made
+    fresh = copy.copy(ctx)
+    fresh.plans, fresh.made = {}, set()
+    with Uploads():
+        run(fresh)
+    assert Uploads.count <= 1
+
+
+@pytest.mark.parametrize("lens, starts", [([64], [0]), ([1, 63, 65, 200], [128, 1, 0, 500]), ([1] * 33 + [70] + [2] * 40, [9 * i for i in range(74)])])
+def test_rows_and_blocks_of_every_request(lens, starts):
+    """Requests side by side, more than a warp looks at together: every row is the latent of its request and position, the rows between are zeros."""
+    from quench6k_b200 import ops
+    H, dim, rd, vd, rank, page = 2, 32, 8, 64, 64, 4
+    reach = [s + n for s, n in zip(starts, lens)]
+    need = [-(-c // page) for c in reach]
+    g = torch.Generator().manual_seed(len(lens))
+    order = torch.randperm(sum(need), generator=g, dtype=torch.int32)
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    for r in range(len(lens)):
+        table[r, :need[r]] = order[sum(need[:r]):sum(need[:r + 1])]
+    pages = torch.randn(1, sum(need), page, rank + rd, generator=g).to(torch.bfloat16)
+    w = (torch.randn(H * (dim + vd), rank, generator=g) * 0.1).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    k, v, blocks = ops.latent_expanded(pages.to(DEV), reach, i32([sum(lens[:i]) for i in range(len(lens) + 1)]), i32(starts), table.to(DEV), w.to(DEV), H, dim, rd)
+    counts = [-(-c // 64) for c in reach]
+    assert k.shape == (H, sum(counts), 64, dim + rd) and v.shape == (H, sum(counts), 64, vd)
+    first = [sum(counts[:r]) for r in range(len(lens))]
+    assert blocks.tolist() == [[f + min(i, n - 1) for i in range(max(counts))] for f, n in zip(first, counts)]
+    want = torch.zeros(sum(counts) * 64, rank + rd)
+    for r, c in enumerate(reach):
+        for p in range(c):
+            want[first[r] * 64 + p] = pages[0, table[r, p // page], p % page].float()
+    for h in range(H):
+        up = (want[:, :rank].double() @ w[h * (dim + vd):(h + 1) * (dim + vd)].double().T)
+        assert torch.equal(k[h, :, :, dim:].reshape(-1, rd).float().cpu(), want[:, rank:])
+        got = torch.cat([k[h, :, :, :dim], v[h]], -1).reshape(-1, dim + vd).double().cpu()
+        # a sum of 64 products of FP32, rounded to bfloat16
+        assert bool(((got - up).abs() <= up.abs() * 2.0 ** -8 + 1e-5).all())
+    assert ops.tc_status() == 0
