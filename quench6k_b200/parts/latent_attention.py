@@ -112,7 +112,7 @@ class LatentAttention(Mixer):
         steps whose positions the host does not know."""
         if self.w_ukv is None or ctx.replayed or ctx.max_q_len < 64 or len(ctx.pos_starts) != len(ctx.q_lens):        # 64: half a tile of a head
             return False
-        key = ("latent.expands", self.H, self.dim, self.rd, self.vd, self.rank)
+        key = LatentAttention._plan_key(self)
         if key not in ctx.plans:
             reach = [s + n for s, n in zip(ctx.pos_starts, ctx.q_lens)]
             pairs = self.H * 1e-6 * sum(n * (c - n / 2) for n, c in zip(ctx.q_lens, reach))
@@ -122,6 +122,20 @@ class LatentAttention(Mixer):
             fits = rows * (self.rank + self.H * (self.dim + self.rd + self.vd)) * 2 <= EXPAND_BYTES
             ctx.plans[key] = fits and 2.5 * tiled + rows * (flops / 1.1e9 + 1e-3) < 4.1e-3 * (3 * self.rank + self.rd) * pairs + 15.0
         return ctx.plans[key]
+
+    def _expanded(self, ctx, cache, table):
+        """Keys, values and block table of the positions that the step's requests see, or None where there is no memory left for them (up to 256 MB beside what
+        the absorbed form takes): the step is then absorbed, in this layer and in those like it."""
+        ops.current_tag = "latent.expand"
+        reach = [s + n for s, n in zip(ctx.pos_starts, ctx.q_lens)]
+        try:
+            return ops.latent_expanded(cache.k, reach, ctx.q_start, ctx.pos_start, table, self.w_ukv, self.H, self.dim, self.rd)
+        except torch.OutOfMemoryError:
+            ctx.plans[self._plan_key()] = False
+            return None
+
+    def _plan_key(self):
+        return ("latent.expands", self.H, self.dim, self.rd, self.vd, self.rank)
 
     def cache_request(self):
         if self.borrows:
@@ -147,10 +161,9 @@ class LatentAttention(Mixer):
         inv_freq, turn, neighbours = (None, 0, False) if self.pos.is_identity else self.pos.rotary_table()
         qn, qr = ops.latent_prep(x, H, self.dim, self.rd, self.rank, self.c_norm, self.eps, inv_freq, turn, ctx.positions,
                                  ctx.req_of_token, table, cache.page_size, cache.k, neighbours=neighbours, write=not self.borrows, latent=latent)
-        if self.expands(ctx):
-            ops.current_tag = "latent.expand"
-            reach = [s + n for s, n in zip(ctx.pos_starts, ctx.q_lens)]
-            k, v, blocks = ops.latent_expanded(cache.k, reach, ctx.q_start, ctx.pos_start, table, self.w_ukv, H, self.dim, self.rd)
+        expanded = self._expanded(ctx, cache, table) if self.expands(ctx) else None
+        if expanded is not None:
+            k, v, blocks = expanded
             ops.current_tag = "latent.keys"
             wide = ctx.query_tiles(ops.attention_flex_tc_tile_tokens(H, H), most_keys_first=(None, None))
             a = ops.attention_flex(qn.view(H * T, self.dim), qr.view(H * T, self.rd) if self.rd else None, True, k, v, blocks, ctx.req_of_token, ctx.positions, H, self.scale,

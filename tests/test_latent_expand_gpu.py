@@ -169,3 +169,20 @@ def test_rows_and_blocks_of_every_request(lens, starts):
         # a sum of 64 products of FP32, rounded to bfloat16
         assert bool(((got - up).abs() <= up.abs() * 2.0 ** -8 + 1e-5).all())
     assert ops.tc_status() == 0
+
+
+def test_where_the_expanded_rows_find_no_memory_the_step_is_absorbed(monkeypatch):
+    """The step then gives the bits of the absorbed form, which needs no such rows.  The failure is the host's: the call that allocates them raises."""
+    from quench6k_b200 import ops
+    mixer, ctx, run = _layer_and_context([300], [100])
+    assert mixer.expands(ctx)
+
+    def no_room(*a, **k):
+        raise torch.OutOfMemoryError("out of memory, says the test")
+
+    with monkeypatch.context() as m:
+        m.setattr(ops, "latent_expanded", no_room)
+        got = run(ctx).clone()
+    absorbed = _layer_and_context([300], [100])
+    monkeypatch.setattr(type(absorbed[0]), "expands", lambda self, ctx: False)
+    assert torch.equal(got, absorbed[2](absorbed[1])) and ops.tc_status() == 0
