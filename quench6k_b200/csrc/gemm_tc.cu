@@ -165,21 +165,29 @@ __device__ __forceinline__ void sent_blocks_done() {
 // The value that leaves in bfloat16: of EPI_SWIGLU (DUAL: gate and up), EPI_ACT or EPI_BF16.
 template <bool DUAL>
 __device__ __forceinline__ float rounded_result(const Params& p, float v, float up) {
-    if (DUAL) return p.act == 0 ? v / (1.0f + expf(-v)) * up : q6k_gated(v, up, p.act, p.act_limit);
+    if (DUAL) return q6k_gated(v, up, p.act, p.act_limit);
     return p.epilogue == EPI_ACT ? q6k_activation(v, p.act) : v;
 }
 
-// silu(v) * up where |v| < 80: the quotient of v and d = 1 + e^-v, d between 1 and e^81, by a reciprocal with one Newton step and one correction by the
-// remainder (Markstein 1990), which rounds as a division does.  A division's branches kept a warp's sixteen from overlapping, and the epilogue of a gated
-// product took longer than its tile's MMAs: 1,522 rows, 2 x 8,192 columns, K 2,048: 105 us with the division, 89 with this (600 rows: 56 and 45;
-// 64 rows: 20 and 18; 16 rows, 2 x 2,816 columns, K 1,024: 8 and 7).
-__device__ __forceinline__ float silu_times_within(float v, float up) {
-    const float d = 1.0f + expf(-v);
+// silu(v) * up: the quotient of v and d = 1 + e^-v by a reciprocal with one Newton step and one correction by the remainder (Markstein 1990); the results,
+// rounded to bfloat16, have the bits that a division gives (but v = -0 counts as +0, whatever stands beside it: keeping its sign took 0.9 us of 64 rows'
+// 9.6).  A division's branches kept a warp's sixteen from overlapping, and the epilogue of a gated product took longer than its tile's MMAs: 1,522 rows,
+// 2 x 8,192 columns, K 2,048: 105 us with the division, 89 with this (600 rows: 56 and 45; 64 rows: 20 and 18; 16 rows, 2 x 2,816 columns, K 1,024: 8
+// and 7).  Where |v| < 80, d is at most e^81 and its reciprocal a normal number.
+// ANY: for every v.  Below -64 both are taken 2^-32 times, which keeps reciprocal, quotient and remainder normal; beyond e^88.7 d is infinite, so the result
+// is -0 (not a number for v = -infinity); far above 0 d is 1.  No division here either: where gates spread over +-100, nearly every warp has one beyond
+// (4,096 rows, 2 x 4,096 columns, K 2,048, gates of deviation 45: 90 us; 235 with divisions where one is beyond 80, 193 with divisions throughout).
+template <bool ANY>
+__device__ __forceinline__ float silu_times(float v, float up) {
+    const float e = expf(-v), s = ANY && v < -64.0f ? 0x1p-32f : 1.0f;
+    const float d = ANY ? (1.0f + e) * s : 1.0f + e, n = ANY ? v * s : v;
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     r = fmaf(fmaf(-d, r, 1.0f), r, r);
-    const float q = v * r;
-    return fmaf(fmaf(-q, d, v), r, q) * up;
+    float q = n * r;
+    q = fmaf(fmaf(-q, d, n), r, q);
+    if (ANY) q = e > 3.402823466e38f ? v * 0.0f : v > 64.0f ? v : q;
+    return q * up;
 }
 // 16 results that leave in bfloat16.
 template <bool DUAL>
@@ -191,9 +199,12 @@ __device__ __forceinline__ void rounded_results(const Params& p, const float* v,
         for (int j = 0; j < EPI_TOKENS; ++j) most = fmaxf(most, fabsf(v[j])), numbers = numbers && v[j] == v[j];
         if (most < 80.0f && numbers) {
 #pragma unroll
-            for (int j = 0; j < EPI_TOKENS; ++j) y[j] = __float2bfloat16_rn(silu_times_within(v[j], up[j]));
-            return;
+            for (int j = 0; j < EPI_TOKENS; ++j) y[j] = __float2bfloat16_rn(silu_times<false>(v[j], up[j]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < EPI_TOKENS; ++j) y[j] = __float2bfloat16_rn(silu_times<true>(v[j], up[j]));
         }
+        return;
     }
 #pragma unroll
     for (int j = 0; j < EPI_TOKENS; ++j) y[j] = __float2bfloat16_rn(rounded_result<DUAL>(p, v[j], up[DUAL ? j : 0]));

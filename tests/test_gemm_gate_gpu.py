@@ -46,3 +46,57 @@ def test_pairs_as_rows_a_few_at_a_time(M, N, K, act):
     got = ops.gemm_tc(a, w, w2=w2, act=act)
     few = torch.cat([ops.gemm_tc(a[i:i + 256], w, w2=w2, act=act) for i in range(0, M, 256)])
     assert torch.equal(got, few) and ops.tc_status() == 0
+
+
+@pytest.mark.parametrize("M", [48, 304, 1040])                        # tiles of 64 and of 128 tokens, CTA pairs
+def test_a_gate_does_not_depend_on_the_rows_beside_it(M):
+    """A dense sweep of gates, from subnormal numbers to beyond where e^-v overflows: the bits of the division, alone or with a neighbour (of the 16
+    rows that a thread gates together) that is large."""
+    from quench6k_b200 import ops
+    N = 264
+    g = torch.Generator().manual_seed(M)
+    e = torch.rand(M, N, generator=g)
+    v = torch.where(e < 0.3, 10 ** (torch.rand(M, N, generator=g) * 42 - 41), torch.rand(M, N, generator=g) * 100)
+    v = torch.where(torch.rand(M, N, generator=g) < 0.5, -v, v)
+    v[3, :5] = torch.tensor([-87.0, -87.4, -88.7, -88.73, 1e38])
+    # one product a row and column: a one-hot row of A picks the gate from W, so v (two bfloat16 parts, exact in FP32) comes out as it is
+    first = v.to(torch.bfloat16)
+    second = (v - first.float()).to(torch.bfloat16)
+    K = (2 * M + 7) // 8 * 8
+    a = torch.zeros(M, K, dtype=torch.bfloat16)
+    a[torch.arange(M), torch.arange(M)] = 1
+    a[torch.arange(M), M + torch.arange(M)] = 1
+    w, w2 = torch.zeros(N, K, dtype=torch.bfloat16), torch.zeros(N, K, dtype=torch.bfloat16)
+    w[:, :M], w[:, M:2 * M] = first.T, second.T
+    w2[:, :M] = torch.randn(N, M, generator=g).to(torch.bfloat16)
+    a, w, w2 = a.cuda(), w.cuda(), w2.cuda()
+    gate, up = ops.gemm_tc(a, w), ops.gemm_tc(a, w2)                   # the products themselves, FP32
+    want = (gate / (1.0 + torch.exp(-gate)) * up).to(torch.bfloat16)
+    alone = ops.gemm_tc(a, w, w2=w2)
+    assert torch.equal(alone.view(torch.int16), want.view(torch.int16))
+    w[:, 15:M:16] = torch.tensor([300.0, -300.0, 1e30, -1e30], dtype=torch.bfloat16, device="cuda").repeat(N // 4 + 1)[:N, None]
+    beside = ops.gemm_tc(a, w, w2=w2)
+    rows = torch.arange(M) % 16 != 15
+    assert torch.equal(beside[rows].view(torch.int16), alone[rows].view(torch.int16))
+    assert ops.tc_status() == 0
+
+
+def test_gates_beyond_80_cost_no_divisions():
+    """Gates that spread over +-100 (nearly every warp holds one beyond 80) take the time of small ones: 90 and 88 us here, 235 with divisions for those."""
+    from quench6k_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    a, w, w2 = r(4096, 2048).bfloat16(), r(4096, 2048) * 2048 ** -0.5, (r(4096, 2048) * 2048 ** -0.5).bfloat16()
+    took = {}
+    for spread in (1, 45, 1, 45):
+        ws = (w * spread).bfloat16()
+        ops.gemm_tc(a, ws, w2=w2)
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        for _ in range(3):
+            begin.record()
+            for _ in range(10):
+                ops.gemm_tc(a, ws, w2=w2)
+            end.record()
+            end.synchronize()
+            took[spread] = min(took.get(spread, 1e9), begin.elapsed_time(end))
+    assert took[45] <= 1.5 * took[1], took
