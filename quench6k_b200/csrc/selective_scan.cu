@@ -266,7 +266,10 @@ struct LsTile {
     float bc[2][LS_TILE / 2][2 * LS_N];          // B, then C: [two tokens][two states][token of the two][state of the two]
 };
 
-// grid (R, ceil(C / 16)), 256 threads: warps 0-3 walk, warps 4-7 make the next tile's values meanwhile and store the last tile's results.
+// grid (R ceil(C / 16)), a request's blocks of channels side by side, the requests from that end of the list on where the longer one stands (a step lists its
+// decoding requests before its prompt portions): a long portion's blocks so start together, on SMs of their own (1,500 tokens beside 8 requests of one,
+// 1,536 channels: 151 us with the requests' blocks in turn, 73 so).  256 threads: warps 0-3 walk, warps 4-7 make the next tile's values meanwhile and
+// store the last tile's results.
 template <typename T>
 __global__ void __launch_bounds__(LS_THREADS, 3) scan_lanes_kernel(const T* u, const float* dt_raw, const float* dt_bias, const float* proj, int ldp, int b_col,
                                                                    int c_col, const float* A, const float* Dskip, const float* xz, int ldx, int z_col,
@@ -277,8 +280,9 @@ __global__ void __launch_bounds__(LS_THREADS, 3) scan_lanes_kernel(const T* u, c
     LsTile* tiles = reinterpret_cast<LsTile*>(ls_smem);
     __shared__ __align__(16) float s_y[LS_WALK / 32][8][80];                 // a warp's S C: [two tokens][channel, 20 apart][lane][token of the two]
     __shared__ T s_out[2][LS_TILE][LS_CH];
-    const int r = blockIdx.x, c0 = blockIdx.y * LS_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = q_start[r], n_tok = q_start[r + 1] - first;
+    const int of_request = (C + LS_CH - 1) / LS_CH, last = gridDim.x / of_request - 1, place = blockIdx.x / of_request;
+    const int r = q_start[1] - q_start[0] > q_start[last + 1] - q_start[last] ? place : last - place;
+    const int c0 = blockIdx.x % of_request * LS_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = q_start[r], n_tok = q_start[r + 1] - first;
     if (n_tok <= 0) return;
     const int n_tiles = (n_tok + LS_TILE - 1) / LS_TILE, slot = slot_ids[r];
     if (warp >= LS_WALK / 32) {
@@ -452,7 +456,7 @@ Q6K_API int q6k_selective_scan_segment() { return 64; }
 // latter has the fewer instructions too (8 portions of 64: 53 and 41).  A step of single tokens keeps the former (nothing to fetch ahead).
 static bool lanes_taken(int T_, int R, int C, int N, int segments, int longest) {
     const long long blocks = (C + LS_CH - 1) / LS_CH;
-    if (N <= 8 || N > LS_N || T_ < 8 * R || blocks > 65535) return false;
+    if (N <= 8 || N > LS_N || T_ < 8 * R || blocks > 65535 || R * blocks > 0x7fffffffLL) return false;
     if (segments > 1) return (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 10000;
     return T_ >= 25 * R || 5.0f + 4.4f * (float)(R * blocks) / (3 * 148) < 3.0f + 0.58f * (float)longest;
 }
@@ -480,7 +484,7 @@ Q6K_API int q6k_selective_scan(const void* u, const float* dt_raw, const float* 
         Q6K_DISPATCH(dtype, {
             if (cudaFuncSetAttribute(scan_lanes_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(LsTile)) != cudaSuccess)
                 return q6k_check_launch("selective_scan: shared memory attribute");
-            q6k_launch(scan_lanes_kernel<T>, dim3(R, (C + LS_CH - 1) / LS_CH), LS_THREADS, 2 * sizeof(LsTile), st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
+            q6k_launch(scan_lanes_kernel<T>, dim3((unsigned)R * ((C + LS_CH - 1) / LS_CH)), LS_THREADS, 2 * sizeof(LsTile), st, (const T*)u, dt_raw, dt_bias, proj, ldp, b_col, c_col,
                        A, Dskip, xz, ldx, z_col, state, tail, q_start, slot_ids, (T*)out, C, N, taps);
         });
         return q6k_check_launch("selective_scan (lanes)");

@@ -104,3 +104,31 @@ def test_lanes_of_two_states_at_extremes(C, N, dtype, lens):
     # 16 FP32 products and a skip in another order (some 20 roundings of 6e-8 of the largest), times the gate; bfloat16: a neighbouring value
     scale = float(walked[finite].abs().max())
     torch.testing.assert_close(got[finite], walked[finite], rtol=2 ** -7 if dtype == torch.bfloat16 else 2e-6, atol=2e-6 * scale)
+
+
+@pytest.mark.parametrize("lens", [[1500] + [1] * 8, [1] * 8 + [1500]])
+def test_a_portion_beside_requests_of_a_token_takes_its_own_time(lens):
+    """The portion's blocks of channels start together, on SMs of their own: 74 us where the portion alone takes 71 (151 with the requests' blocks in turn)."""
+    from quench6k_b200 import ops
+    C, N = 1536, 16
+    g = torch.Generator().manual_seed(7)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+
+    def took(lens):
+        T, R = sum(lens), len(lens)
+        u, dt_raw, dt_b, proj = rnd(T, C).bfloat16(), rnd(T, C), rnd(C), rnd(T, 2 * N)
+        A, D, xz, state, tail = -torch.exp(rnd(C, N)), rnd(C), rnd(T, 2 * C), rnd(R, C, N), rnd(R, 3, C)
+        starts, slots, segments = i32([sum(lens[:i]) for i in range(R + 1)]), i32(list(range(R))), ops.selective_scan_segments(lens, u.device)
+        best = 1e9
+        for _ in range(4):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(8):
+                ops.selective_scan(u, dt_raw, dt_b, proj, 0, N, A, D, xz, C, state, tail, starts, slots, R, segments=segments, longest=max(lens))
+            end.record()
+            end.synchronize()
+            best = min(best, begin.elapsed_time(end) / 8)
+        return best
+
+    assert took(lens) <= 1.5 * took([1500])
