@@ -448,16 +448,22 @@ Q6K_API int q6k_selective_scan_lanes(int N) {
 Q6K_API int q6k_selective_scan_segment() { return 64; }
 
 // Whether a step of T_ rows whose longest portion has up to `segments` segments goes a lane per two states in one pass.  More than 16 states
-// take more lanes; fewer than 9 leave half of them idle.  A chain takes about 45 ns a token however few there are; the segments' launches take 70 us
-// and their 30 instructions per token and state, spread over the chip: for one portion of 2,048 tokens the lines meet where its tokens bring 10,000
-// chains (768 channels: 90 against 95 us; 512: 90 against 86; 4,096: 150 against 345).  Without segments (up to 64 tokens) a walk of eight states a lane
+// take more lanes; fewer than 9 leave half of them idle.  A chain takes 46 ns a token however few there are, and more from a block an SM on; the segments'
+// launches take 70 us and then what their 30 instructions per token and state take, spread over the chip (W million states of tokens: 1.3 us each beside
+// the 70, 2.45 once they fill it).  One pass and segments, both measured (us, bfloat16): one portion of 2,048 tokens, 640 channels 94 and 100, 4,096 channels
+// 146 and 349; of 4,096, 768 channels 184 and 150, 1,024 185 and 191, 1,536 185 and 255; of 8,192, 640 channels 362 and 230, 1,024 395 and 364, 1,536 401
+// and 527.  Below 10,000 chains for each token of the longest portion segments stay.  Without segments (up to 64 tokens) a walk of eight states a lane
 // takes 0.58 us a token of the longest portion, a lane per two states 4.4 us for every round of blocks (three are resident on an SM), whatever their
 // tokens (4,096 channels: 64 tokens 35 and 9 us, 64 beside 8 of one 41 and 32, 32 portions of 8 28 and 86); from 25 tokens a request on the
 // latter has the fewer instructions too (8 portions of 64: 53 and 41).  A step of single tokens keeps the former (nothing to fetch ahead).
 static bool lanes_taken(int T_, int R, int C, int N, int segments, int longest) {
     const long long blocks = (C + LS_CH - 1) / LS_CH;
     if (N <= 8 || N > LS_N || T_ < 8 * R || blocks > 65535 || R * blocks > 0x7fffffffLL) return false;
-    if (segments > 1) return (long long)T_ * C * N >= (long long)segments * q6k_selective_scan_segment() * 10000;
+    if (segments > 1) {
+        const float most = (float)segments * q6k_selective_scan_segment(), W = (float)T_ * C * LS_N * 1e-6f;       // tokens of the longest portion, rounded up
+        const float one_pass = 3.0f + most * fmaxf(0.046f, 0.043f * ((float)T_ / most) * (float)blocks / 148), in_segments = fmaxf(70.0f + 1.3f * W, 30.0f + 2.45f * W);
+        return (float)T_ * C * N >= most * 10000.0f && one_pass < in_segments;
+    }
     return T_ >= 25 * R || 5.0f + 4.4f * (float)(R * blocks) / (3 * 148) < 3.0f + 0.58f * (float)longest;
 }
 Q6K_API int q6k_selective_scan_lanes_taken(int T_, int R, int C, int N, int segments) { return lanes_taken(T_, R, C, N, segments, R > 0 ? T_ / R : 0); }
