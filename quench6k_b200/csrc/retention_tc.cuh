@@ -78,22 +78,72 @@ __device__ __forceinline__ bool rt_done(uint32_t bar, uint32_t parity) {
     return ok;
 }
 
-// One result with multiply-adds, no value of a later token among them.
-__device__ __noinline__ float ret_out_plain(const float* q, const float* k, const float* v, const float* S, int ld, int dk, int dv, int row, const float* pw) {
-    float s = 0.0f;
-    for (int i = 0; i < dk; ++i) s = fmaf(q[i] * pw[row + 1], S[(size_t)i * dv], s);
-    for (int t = 0; t <= row; ++t) {
-        float dot = 0.0f;
-        for (int i = 0; i < dk; ++i) dot = fmaf(q[i], k[(size_t)t * ld + i], dot);
-        s = fmaf(dot * pw[row - t], v[(size_t)t * ld], s);
+// Where results are not finite, the whole block sums its tile again with multiply-adds, from rows in shared memory; only those that are not finite are taken.
+// (A result at a time from global memory held a block up for 11 ms: 2,550 tokens with one key that is not a number 77 ms, so 0.24.)
+constexpr int RP_LD = RT + 1, RP_STAGE = 132;                                 // floats a row: of an operand, of the results
+// This thread's 4 x 8 sums: rows 4 (tid / 16) + r, columns tid % 16 + 16 c.  TRANS: A lies with the terms as rows; LOWER: terms up to a row's own only.
+template <bool A_TRANS, bool B_TRANS, bool LOWER>
+__device__ __forceinline__ void rp_product(float (&acc)[4][8], const float* A, const float* B, int terms) {
+    const int tx = threadIdx.x & 15, r0 = (threadIdx.x >> 4) * 4;
+    for (int i = 0; i < terms; ++i) {
+        float b[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) b[c] = B_TRANS ? B[(tx + 16 * c) * RP_LD + i] : B[i * RP_LD + tx + 16 * c];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            if (LOWER && i > r0 + r) continue;
+            const float a = A_TRANS ? A[i * RP_LD + r0 + r] : A[(r0 + r) * RP_LD + i];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(a, b[c], acc[r][c]);
+        }
     }
-    return s;
 }
-
-__device__ __noinline__ float ret_outer_plain(const float* k, const float* v, int ld, int n, const float* pw) {
-    float s = 0.0f;
-    for (int i = 0; i < n; ++i) s = fmaf(k[(size_t)i * ld] * pw[i], v[(size_t)i * ld], s);
-    return s;
+__device__ __forceinline__ void rp_fetch(float* to, const float* src, size_t ld, int rows, int cols) {
+    for (int i = threadIdx.x; i < RT * RT; i += RT_THREADS) to[(i >> 7) * RP_LD + (i & 127)] = (i >> 7) < rows && (i & 127) < cols ? src[(size_t)(i >> 7) * ld + (i & 127)] : 0.0f;
+}
+__device__ __forceinline__ void rp_store(float* to, const float (&acc)[4][8], int ld) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) to[((threadIdx.x >> 4) * 4 + r) * ld + (threadIdx.x & 15) + 16 * c] = acc[r][c];
+}
+// K'^T V to smem [128][RP_STAGE].
+__device__ __noinline__ void ret_outer_plain(float* smem, const float* k, const float* v, int ld, int n, int dk, int cols, const float* pw) {
+    float *A = smem, *B = smem + RT * RP_LD, acc[4][8] = {};
+    rp_fetch(A, k, ld, n, dk);
+    rp_fetch(B, v, ld, n, cols);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * RT; i += RT_THREADS) A[(i >> 7) * RP_LD + (i & 127)] *= pw[i >> 7];
+    __syncthreads();
+    rp_product<true, false, false>(acc, A, B, n);
+    __syncthreads();
+    rp_store(smem, acc, RP_STAGE);
+    __syncthreads();
+}
+// d^(i+1) (Q S)_i + (M V)_i to smem [128][RP_STAGE].
+__device__ __noinline__ void ret_out_plain(float* smem, const float* q, const float* k, const float* v, const float* S, int ld, int dk, int dv, int n, int cols, const float* pw) {
+    float *A = smem, *B = smem + RT * RP_LD, m[4][8] = {}, acc[4][8] = {};
+    rp_fetch(A, q, ld, n, dk);
+    rp_fetch(B, k, ld, n, dk);
+    __syncthreads();
+    rp_product<false, true, false>(m, A, B, dk);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) m[r][c] *= pw[max(0, (int)(threadIdx.x >> 4) * 4 + r - (int)(threadIdx.x & 15) - 16 * c)];       // above the diagonal nothing is read
+    __syncthreads();
+    for (int i = threadIdx.x; i < RT * RT; i += RT_THREADS) A[(i >> 7) * RP_LD + (i & 127)] *= pw[(i >> 7) + 1];
+    rp_fetch(B, S, dv, dk, cols);
+    __syncthreads();
+    rp_product<false, false, false>(acc, A, B, dk);
+    __syncthreads();
+    rp_store(A, m, RP_LD);
+    rp_fetch(B, v, ld, n, cols);
+    __syncthreads();
+    rp_product<false, false, true>(acc, A, B, n);
+    __syncthreads();
+    rp_store(smem, acc, RP_STAGE);
+    __syncthreads();
 }
 
 // Task t of a launch: one (head, 128 value columns) of one chunk, the heads fastest.
@@ -159,22 +209,27 @@ __global__ void __launch_bounds__(RT_THREADS, 1) ret_outer_tc_kernel(const float
         float acc[32];
         tmem_ld32_issue(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0, acc);
         tmem_ld_wait();
+        float* stage = reinterpret_cast<float*>(smem) + row * RP_STAGE + c0;         // through shared memory, which no product reads any more: whole rows leave
+        bool finite = true;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            if (row < dk && c0 + c < now.cols && !(fabsf(acc[c]) <= 3.402823466e38f)) {
-                acc[c] = ret_outer_plain(kp + (size_t)now.first * ld + (size_t)now.head * dk + row, vp + (size_t)now.first * ld + (size_t)now.head * dv + now.col0 + c0 + c, ld, n, pw);
-            }
-        }
-        float* stage = reinterpret_cast<float*>(smem) + row * 132 + c0;              // through shared memory, which no product reads any more: whole rows leave
+        for (int c = 0; c < 32; ++c) finite = finite && !(row < dk && c0 + c < now.cols && !(fabsf(acc[c]) <= 3.402823466e38f));
 #pragma unroll
         for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(stage + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
         tc_fence_before();
-        __syncthreads();
+        if (!__syncthreads_and(finite)) {
+            ret_outer_plain(reinterpret_cast<float*>(smem), kp + (size_t)now.first * ld + (size_t)now.head * dk, vp + (size_t)now.first * ld + (size_t)now.head * dv + now.col0, ld, n, dk,
+                            now.cols, pw);
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+                if (fabsf(acc[c]) <= 3.402823466e38f) stage[c] = acc[c];
+            fetch(task);                                                             // its registers need not outlast the sums above
+            __syncthreads();
+        }
         float* out = KV + ((size_t)now.chunk * H + now.head) * dk * dv + now.col0;
         if (ok)
             for (int i = threadIdx.x; i < dk * 32; i += RT_THREADS) {
                 const int r = i >> 5, c = (i & 31) * 4;
-                if (c < now.cols) *reinterpret_cast<float4*>(out + (size_t)r * dv + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * 132 + c);
+                if (c < now.cols) *reinterpret_cast<float4*>(out + (size_t)r * dv + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * RP_STAGE + c);
             }
         __syncthreads();
         if (!ok) break;
@@ -263,22 +318,27 @@ __global__ void __launch_bounds__(RT_THREADS, 1) ret_out_tc_kernel(const float* 
 #pragma unroll
             for (int c = 0; c < 16; ++c) x[h + c] = fmaf(p, x[h + c], y[c]);
         }
+        float* stage = reinterpret_cast<float*>(smem) + row * RP_STAGE + c0;
+        bool finite = true;
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (row < n && c0 + c < now.cols && !(fabsf(x[c]) <= 3.402823466e38f)) {
-                const size_t at = (size_t)now.first * ld + (size_t)now.head * dk;
-                x[c] = ret_out_plain(qp + at + (size_t)row * ld, kp + at, v + c0 + c, S + c0 + c, ld, dk, dv, row, pw);
-            }
-        float* stage = reinterpret_cast<float*>(smem) + row * 132 + c0;
+        for (int c = 0; c < 32; ++c) finite = finite && !(row < n && c0 + c < now.cols && !(fabsf(x[c]) <= 3.402823466e38f));
 #pragma unroll
         for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(stage + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
         tc_fence_before();
-        __syncthreads();
+        if (!__syncthreads_and(finite)) {
+            const size_t at = (size_t)now.first * ld + (size_t)now.head * dk;
+            ret_out_plain(reinterpret_cast<float*>(smem), qp + at, kp + at, v, S, ld, dk, dv, n, now.cols, pw);
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+                if (fabsf(x[c]) <= 3.402823466e38f) stage[c] = x[c];
+            fetch(task);
+            __syncthreads();
+        }
         if (ok)
             for (int i = threadIdx.x; i < n * 32; i += RT_THREADS) {
                 const int r = i >> 5, c = (i & 31) * 4;
                 if (c < now.cols)
-                    *reinterpret_cast<float4*>(o + ((size_t)(now.first + r) * H + now.head) * dv + now.col0 + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * 132 + c);
+                    *reinterpret_cast<float4*>(o + ((size_t)(now.first + r) * H + now.head) * dv + now.col0 + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * RP_STAGE + c);
             }
         __syncthreads();
         if (!ok) break;

@@ -51,3 +51,34 @@ def test_an_infinite_value_reaches_no_earlier_token():
     assert torch.allclose(got[:200], clean[:200], rtol=1e-5, atol=1e-4) and torch.isfinite(got[:200]).all()
     assert torch.equal(torch.isfinite(got), torch.isfinite(walk)) and torch.equal(torch.isfinite(s), torch.isfinite(s_walk))
     assert torch.equal(got[300:], clean[300:])
+
+
+def test_results_that_are_not_finite_do_not_hold_a_step_up():
+    """A key that is not a number makes a head's results of every later token so: they are summed again, those of other heads and requests keep their bits, and
+    the step takes a few times its time (single results one by one took 480 times)."""
+    H, dk, dv, lens = 8, 128, 128, [700, 600]
+    p, decay, state, starts, run = _case(lens, H, dk, dv)
+    decay.fill_(0.99)
+    clean, s_clean = run(longest=max(lens))
+
+    def took():
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = 1e9
+        for _ in range(3):
+            a.record()
+            run(longest=max(lens))
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    at_first = took()
+    p[200, H * dk + dk + 7] = float("nan")                              # head 1 of the first request
+    p[300, 2 * H * dk + 2 * dv + 9] = float("inf")                      # one value column of head 2
+    got, s = run(longest=max(lens))
+    walk, s_walk = run()
+    assert torch.equal(torch.isfinite(got), torch.isfinite(walk)) and torch.equal(torch.isfinite(s), torch.isfinite(s_walk))
+    same, heads = torch.isfinite(got), [0] + list(range(3, H))
+    assert not same.all() and torch.allclose(got[same], clean[same], rtol=1e-5, atol=1e-4) and torch.equal(s[torch.isfinite(s)], s_clean[torch.isfinite(s)])
+    assert torch.equal(got[700:], clean[700:]) and torch.equal(got.view(-1, H, dv)[:, heads], clean.view(-1, H, dv)[:, heads])
+    assert took() <= 30 * at_first
