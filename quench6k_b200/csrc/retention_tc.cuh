@@ -231,8 +231,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1) ret_outer_tc_kernel(const float
                 const int r = i >> 5, c = (i & 31) * 4;
                 if (c < now.cols) *reinterpret_cast<float4*>(out + (size_t)r * dv + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * RP_STAGE + c);
             }
-        __syncthreads();
-        if (!ok) break;
+        if (!__syncthreads_and(ok)) break;                                          // all threads or none: a wait may run out in one and not in the next
     }
     rt_end(tmem, 128);
 }
@@ -340,8 +339,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1) ret_out_tc_kernel(const float* 
                 if (c < now.cols)
                     *reinterpret_cast<float4*>(o + ((size_t)(now.first + r) * H + now.head) * dv + now.col0 + c) = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * RP_STAGE + c);
             }
-        __syncthreads();
-        if (!ok) break;
+        if (!__syncthreads_and(ok)) break;                                          // all threads or none: a wait may run out in one and not in the next
     }
     rt_end(tmem, 512);
 }
