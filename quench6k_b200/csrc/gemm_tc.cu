@@ -694,12 +694,14 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_pair_kernel(const __grid_const
         const int quarter = warp & 3;
         const uint32_t out_smem = smem_u32(smem + (size_t)stages * STAGE_BYTES) + quarter * 2 * EPI_BLOCK_BYTES;
         int nt = 0, sent = 0, turn = 0;
+        bool ok = true;
         pdl_wait();                                        // the output may still be in use by the kernel before
         for (int t = pair; t < total; t += n_pairs, ++nt) {
             const int buf = nt & 1;
-            if (!mbar_wait(acc_full0 + 8 * buf, (nt >> 1) & 1)) {
+            if (ok && !mbar_wait(acc_full0 + 8 * buf, (nt >> 1) & 1)) {
                 if (lane == 0) atomicExch(&g_tc_status, 13);
-                if (!DUAL) break;                           // DUAL: on to the barriers that the partner may be waiting at
+                if (!DUAL) break;
+                ok = false;                                 // DUAL: on to the barriers that the partner may be waiting at, with no further wait
             }
             tc_fence_after();
             const int n = (t % n_x) * 2 * COLS + (int)rank * COLS + (DUAL ? quarter & 1 : quarter) * 32 + lane, tok0 = (t / n_x) * BT2;
