@@ -57,3 +57,20 @@ def test_groups_end_inside_a_block():
     gate = ops.gemm_tc(a, w, w2=w2, groups=tiles, bt=128, rows=rows)
     assert float((gate.double() - want).abs().max()) <= 1e-2 * float(want.abs().max())
     assert ops.tc_status() == 0
+
+
+@pytest.mark.parametrize("M", [300, 1041])                           # one CTA a tile, CTA pairs; a last block that leaves from registers
+def test_additions_of_subnormal_numbers(M):
+    """What blocks add in L2 and what a thread adds itself are the same bits, also where an operand or the sum is subnormal (PTX lets the former flush them)."""
+    from quench6k_b200 import ops
+    N, K, tiny = 2048, 64, 2.0 ** -126                                  # the smallest normal number
+    a, w = torch.zeros(M, K, device=DEV, dtype=torch.bfloat16), torch.zeros(N, K, device=DEV, dtype=torch.bfloat16)
+    a[:, 0], w[:, 0], w[::2, 0] = 1, tiny, -tiny
+    for shift in (0, 1):
+        out = torch.zeros(M * N + 8, device=DEV)[4 + shift:4 + shift + M * N].view(M, N)
+        out.fill_(1.5 * tiny)                                           # less tiny: subnormal
+        out[:, 1::4] = tiny / 16                                        # subnormal before
+        want = out.double() + a.double() @ w.double().T
+        ops.gemm_tc(a, w, out=out, accumulate=True)
+        assert torch.equal(out.double(), want) and float(out.abs().min()) < tiny
+    assert ops.tc_status() == 0
