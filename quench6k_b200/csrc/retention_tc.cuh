@@ -9,7 +9,8 @@
 // A result that is not finite is summed again as the FP32 kernels do it: a value of a later token, were it infinite, must not reach an earlier one, and the
 // zeros of M do not keep it away.
 // Blocks walk the (head, chunk)s, the next one's rows on their way in registers under the last product of this one.  2,550 tokens in three portions, 16 heads
-// of 128 x 128: 97 + 42 us with FP32 multiply-adds in chunks of 64, 52 + 34 us so, and the fold between them 15 -> 9.5 us (half as many states).
+// of 128 x 128: 97 + 42 us with FP32 multiply-adds in chunks of 64, 52 + 34 us so, and the fold between them 15 -> 9.5 us (half as many states); the three
+// launches together 100 us, 88 since sums of results that are not finite leave the products' registers alone.
 // What bounds it: the phases of a block follow one another (rows from L2, the split, 1.6 us a product), and shared memory lets one block to an SM; the
 // last round of blocks (336 on 148 SMs).  Distance to float64 of the state left behind and of the results: as before (the products' own is smaller).
 #pragma once

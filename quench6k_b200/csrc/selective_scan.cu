@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(const T* u, const f
 // steps through a tile meanwhile, with packed instructions over its lanes' two states (the same operations as a state each, so the same states bit for
 // bit).  dt and dt u lie twice in shared memory, B and C as pairs of states of two tokens, so that every operand comes as the packed instruction
 // takes it; S C is left in shared memory, and every 16 tokens a lane sums the values of one channel's two tokens.
-// 2,048 tokens, 4,096 channels of 16 states: 150 us; a lane per state, every warp in both roles, 170; in segments 345.  What bounds it: issue slots, of
+// 2,048 tokens, 4,096 channels of 16 states: 146 us; a lane per state, every warp in both roles, 170; in segments 345.  What bounds it: issue slots, of
 // which a lane per state took twice as many for the same operands read from shared memory.  Not faster: every warp in both roles (225), tiles of 64
 // tokens (144 and 151 where tiles of 32 took 143 and 137 for one portion of 2,048 and three of 682: two blocks on an SM instead of three), registers
 // for four blocks (148 and 138), the operands of the next four tokens asked for ahead (152 against 145).
