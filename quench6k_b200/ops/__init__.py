@@ -1783,12 +1783,13 @@ def retention_prep(p: torch.Tensor, H: int, dk: int, q_col: int, k_col: int, rot
 
 def retention_chunks(q_lens, H: int, dk: int, dv: int) -> bool:
     """Whether a step of these portions should go chunk by chunk: the recurrence's time (us) by either form, from measurements of 65 to
-    1,024 tokens in 1 to 8 portions, alone and beside 1 to 32 requests of a token, with 8 and 16 heads of 64, 128 and 256 keys.  Token by token
-    the longest portion decides (its blocks slow one another down once several share an SM); by chunks the rounds of 64-token chunks
-    over the SMs do, and short portions wait for a launch of their own.  16 heads of 128 x 128, walk and chunks: 65 tokens 10 and
-    35, 320 tokens 36 and 37, 512 tokens 56 and 38, eight portions of 200 91 and 118, two of 1,024 146 and 120, 65 beside 32 of one 30 and 54,
-    512 beside 8 of one 105 and 45, with FP32 multiply-adds by chunks.  Where the tensor cores take the keys the chunks are the faster form a little
-    earlier than this says (320 tokens 34, eight portions of 200 69, two of 1,024 63, 512 beside 8 of one 44); the line stays where it was."""
+    2,048 tokens in 1 to 16 portions, alone and beside 1 to 32 requests of a token, with 8 and 16 heads of 64, 128 and 256 keys.  Token by token
+    the longest portion decides (its blocks slow one another down once several share an SM); by chunks the rounds of the chunks
+    over the SMs do (of 64 tokens in FP32; of 128 on tensor cores for heads of 65 to 128 keys, 28 us a round), and short portions wait for a launch of
+    their own.  16 heads of 128 x 128, walk and chunks: 65 tokens 11 and 31, 320 tokens 37 and 35, 512 tokens 57 and 35, three portions of 300 64 and 40, three
+    of 1,021 204 and 90, two of 1,024 148 and 60, 65 beside 32 of one 31 and 51, 512 beside 8 of one 107 and 46; 8 heads, three of 400 60 and 37.  16 heads of 64 x 64,
+    two of 1,024 74 and 93.  On tensor cores a step leaves the walk for a gain of a quarter (eight portions of 200, 93 and 67, are predicted
+    closer than that and stay), or where FP32 chunks would have gained."""
     longest = max(q_lens, default=0)
     if longest <= CHUNKS_BEYOND:
         return False
@@ -1799,10 +1800,12 @@ def retention_chunks(q_lens, H: int, dk: int, dv: int) -> bool:
     shared = 0.72 * load if load < 4 else 2.9 + 0.45 * (load - 4)
     walk = 3 + per_token * longest * max(shared, 1.3 if len(q_lens) * H * -(-dv // 16) > sms else 1.0)
     rounds = -(-sum(-(-n // 64) for n in q_lens if n > CHUNKS_BEYOND) * H * -(-dv // 128) // sms)
-    chunks = 5 + rounds * (10 + 0.17 * dk)
-    if short:
-        chunks += 5 + per_token * max(short) + 0.55 * len(short) * (H * dk * dv / 262144)
-    return 1.04 * chunks < walk
+    beside = 5 + per_token * max(short) + 0.55 * len(short) * (H * dk * dv / 262144) if short else 0
+    if 64 < dk <= 128:
+        rounds_tc = -(-sum(-(-n // 128) for n in q_lens if n > CHUNKS_BEYOND) * H * -(-dv // 128) // sms)
+        if 1.3 * (8 + 28 * rounds_tc + 1.1 * (long_ones - 1) + beside) < walk:
+            return True
+    return 1.04 * (5 + rounds * (10 + 0.17 * dk) + beside) < walk
 
 
 def retention(p: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
